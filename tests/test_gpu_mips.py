@@ -49,3 +49,23 @@ def test_gpu_mips_match_oracle_device_buffers(cg, filt, srgb, wrap):
     got = cg.generate_mipmaps(torch.from_numpy(img).cuda(), filt, 0.9, srgb, wrap, alpha=True, levels=4)
     for l, (a, b) in enumerate(zip(got, want)):
         assert np.array_equal(a.cpu().numpy(), b), (filt, l)
+
+
+# sides below the eight rows / columns and the pairs a warp takes, windows over one staged chunk
+# (320 positions in rows, 128 in columns) by size and by filter scale, levels of at most 16 and of
+# more samples, power-of-two and other scales, wrap far outside the image
+@pytest.mark.parametrize("w,h,filt,scale,wrap,alpha", [
+    (1, 1, "kaiser", 0.9, False, True), (1, 37, "kaiser", 0.9, True, True), (41, 2, "tent", 1.2, False, False),
+    (9, 7, "box", 0.9, True, True), (66, 34, "mitchell", 0.9, False, True), (700, 9, "lanczos4", 1.0, True, True),
+    (11, 530, "kaiser", 0.9, False, False), (128, 64, "kaiser", 9.0, True, True), (530, 133, "lanczos4", 3.0, False, True),
+])
+def test_gpu_mips_edges_match_oracle(cg, w, h, filt, scale, wrap, alpha):
+    from oracle import mip_oracle
+    from crunch2_gb300 import texgen
+    img = texgen.colour_texture(w, h, w * 7 + h, with_alpha_noise=True)
+    levels = max(w, h).bit_length()
+    want = mip_oracle.generate_mipmaps(img, filt, scale, True, wrap, alpha=alpha, levels=levels)
+    got = cg.generate_mipmaps(torch.from_numpy(img).cuda(), filt, scale, True, wrap, alpha=alpha)
+    assert len(got) == levels
+    for l in range(1, levels):
+        assert np.array_equal(got[l].cpu().numpy(), want[l] if len(want) == levels else want[l - 1]), l
