@@ -10,12 +10,9 @@
 //
 // Inference (crngpu_mlp_forward, the learned encode) runs as one fused persistent kernel,
 // k_mlp_infer: weights resident in shared memory, activations kept on the SM.
-// Training GEMMs go through k_gemm_tc: C[M x N] = sum_k A(m, k) B(n, k), a 128 x BN tile per CTA,
-// K staged 64 at a time into shared memory in the no-swizzle K-major core-matrix layout
-// (8 x 8 BF16 core matrices, 128 bytes each), four K=16 MMAs per stage issued by one thread,
-// completion through tcgen05.commit on an mbarrier (bounded wait), epilogue from TMEM with
-// tcgen05.ld. Operands are fp32, bf16 or raw RGBA8 blocks with arbitrary strides, so the
-// transposed products of the backward pass need no separate transpose kernels.
+// Training runs in three kernels: k_train_tile (per 128 samples: forward, loss gradient and the
+// backward products that stay within the samples), k_train_weight_grads (the products over the
+// batch, split over it) and k_train_reduce (the slices' sum and, in a training step, AdamW).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -34,38 +31,8 @@ namespace crngpu {
 namespace mlp {
 
 constexpr int kIn = 48, kHid = 256, kOut = 8, kOutPad = 16;
-constexpr int BM = 128, BK = 64;
-constexpr int kTmemCols = 128;
+constexpr int BM = 128;
 constexpr uint32_t kWaitLimit = 1u << 24;  // bounded mbarrier polls (~ tens of ms), then error
-
-enum OpKind : int { OP_F32 = 0, OP_BF16 = 1, OP_PIXELS = 2 };
-// epilogues
-enum Epi : int {
-  EPI_STORE = 0,       // C = acc (+ bias)
-  EPI_BIAS_GELU = 1,   // Cpre = acc + bias (fp32), Cb = bf16(gelu(Cpre))
-  EPI_GELU_GRAD = 2,   // Cb = bf16(acc * gelu'(pre)), C (fp32) = same value
-};
-
-struct Operand {
-  const void* p;
-  int kind;
-  long long s_row, s_k;  // element (row, k) at p[row * s_row + k * s_k]; OP_PIXELS: see load_op
-  int pix_sample_is_row; // OP_PIXELS: 1 -> row = sample, k = feature; 0 -> row = feature, k = sample
-};
-
-struct GemmArgs {
-  Operand a, b;
-  int M, N, K;
-  int epi;
-  float* C;              // fp32 out (row-major, ldc)
-  __nv_bfloat16* Cb;     // bf16 out (row-major, ldc)
-  const float* pre;      // EPI_GELU_GRAD: pre-activation (row-major, ldc)
-  const float* bias;     // per column
-  int ldc;
-  uint32_t* err;         // set to 1 if an mbarrier wait timed out
-  int kslice;            // split K: CTA z covers K columns [z * kslice, (z + 1) * kslice) (0: all of K)
-  float* part;           // split K: CTA z writes its raw partial tile to part + z * M * N (row-major, N)
-};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -85,25 +52,12 @@ __device__ __forceinline__ float gelu(float x) {
   const float c = 0.7978845608f;  // sqrt(2/pi), tanh form
   return 0.5f * x * (1.f + tanhf(c * (x + 0.044715f * x * x * x)));
 }
-__device__ __forceinline__ float gelu_grad(float x) {
+// gelu(x) and its derivative from one tanh
+__device__ __forceinline__ float gelu_both(float x, float& grad) {
   const float c = 0.7978845608f;
   const float t = tanhf(c * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * x * x);
-}
-
-__device__ __forceinline__ float load_op(const Operand& o, int row, int k, int rows, int ks) {
-  if (row >= rows || k >= ks) return 0.f;
-  switch (o.kind) {
-    // read-only inputs of the product: non-coherent loads, which the compiler may also move ahead of
-    // the shared-memory stores of the staging loop
-    case OP_F32: return __ldg(reinterpret_cast<const float*>(o.p) + row * o.s_row + k * o.s_k);
-    case OP_BF16: return __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(o.p) + row * o.s_row + k * o.s_k));
-    default: {
-      const int s = o.pix_sample_is_row ? row : k, f = o.pix_sample_is_row ? k : row;
-      const uint8_t* px = reinterpret_cast<const uint8_t*>(o.p);
-      return (float)__ldg(px + (long long)s * 64 + (f / 3) * 4 + f % 3) * (1.0f / 255.0f);
-    }
-  }
+  grad = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * x * x);
+  return 0.5f * x * (1.f + t);
 }
 
 // Polls of a first wait on a tcgen05.commit (a test hook can lower it to force the timeout path);
@@ -121,167 +75,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
                  : "r"(bar), "r"(parity));
   }
   return done != 0;
-}
-
-// C tile (blockIdx.x: 128 rows of M, blockIdx.y: BN columns of N) = A x B^T over all of K, or --
-// split K, for products whose M x N has few tiles but whose K is the batch -- over the slice of K
-// of blockIdx.z, written raw to g.part for k_splitk_sum.
-template <int BN>
-__global__ void __launch_bounds__(128) k_gemm_tc(GemmArgs g) {
-  __shared__ __align__(1024) unsigned char sa[BM * BK * 2];
-  __shared__ __align__(1024) unsigned char sb[BN * BK * 2];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "n"(kTmemCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base;
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-  uint32_t phase = 0;
-  bool ok = true;
-  const int kbeg = g.kslice ? (int)blockIdx.z * g.kslice : 0;
-  const int kend = g.kslice ? min(g.K, kbeg + g.kslice) : g.K;
-  const int nk = (kend - kbeg + BK - 1) / BK;
-  for (int kc = 0; kc < nk; kc++) {
-    const int k0 = kbeg + kc * BK;
-    // stage A (BM x BK) and B (BN x BK); the faster-varying index follows the operand's
-    // contiguous dimension so global reads coalesce. Eight elements per thread at a time: their
-    // loads are all in flight before the first conversion and store.
-    auto stage = [&](const Operand& o, int rows_tile, int row0, int rows, unsigned char* dst) {
-      if (o.kind == OP_BF16 && o.s_k == 1 && (o.s_row & 7) == 0 && ((uintptr_t)o.p & 15) == 0) {
-        // BF16 rows with K contiguous: 8 consecutive K of a row are one 16-byte segment of the
-        // K-major core-matrix layout, copied with one load and one store
-        const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(o.p);
-#pragma unroll 4
-        for (int e = tid; e < rows_tile * (BK / 8); e += 128) {
-          const int r = e / (BK / 8), kg = e - r * (BK / 8);
-          const int row = row0 + r, k = k0 + kg * 8;
-          uint4 v = make_uint4(0u, 0u, 0u, 0u);
-          if (row < rows && k + 8 <= g.K) {
-            v = __ldg(reinterpret_cast<const uint4*>(src + (long long)row * o.s_row + k));
-          } else if (row < rows) {
-            __nv_bfloat16 h[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) h[u] = k + u < g.K ? src[(long long)row * o.s_row + k + u] : __float2bfloat16(0.f);
-            v = *reinterpret_cast<const uint4*>(h);
-          }
-          *reinterpret_cast<uint4*>(dst + kmaj_off(r, kg * 8, BK)) = v;
-        }
-        return;
-      }
-      const bool rmaj = o.kind != OP_PIXELS && o.s_row == 1;
-      for (int e0 = tid; e0 < rows_tile * BK; e0 += 128 * 8) {
-        float v[8];
-        int rr[8], kk[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int e = e0 + u * 128;
-          if (rmaj) { rr[u] = e % rows_tile; kk[u] = e / rows_tile; } else { kk[u] = e % BK; rr[u] = e / BK; }
-          v[u] = e < rows_tile * BK ? load_op(o, row0 + rr[u], k0 + kk[u], rows, g.K) : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-          if (e0 + u * 128 < rows_tile * BK)
-            *reinterpret_cast<__nv_bfloat16*>(dst + kmaj_off(rr[u], kk[u], BK)) = __float2bfloat16(v[u]);
-      }
-    };
-    stage(g.a, BM, m0, g.M, sa);
-    stage(g.b, BN, n0, g.N, sb);
-    asm volatile("fence.proxy.async.shared::cta;");  // generic-proxy smem writes -> tensor core reads
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll
-      for (int ks = 0; ks < BK / 16; ks++) {
-        const uint64_t ad = make_desc(smem_u32(sa) + ks * 256, 128, (BK / 8) * 128);
-        const uint64_t bd = make_desc(smem_u32(sb) + ks * 256, 128, (BK / 8) * 128);
-        const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
-        asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(&mbar)));
-    }
-    // the MMAs read shared memory asynchronously: wait before restaging it
-    const bool done = mbar_wait(smem_u32(&mbar), phase, g_mma_wait_polls);
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    ok = __syncthreads_and(done) != 0;  // uniform across the CTA
-    if (!ok) {
-      // drain the in-flight MMAs (long bound) before TMEM is released
-      if (tid == 0) atomicAdd(&g_mma_wait_timeouts, 1u);
-      mbar_wait(smem_u32(&mbar), phase, kDrainPolls);
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      break;
-    }
-    phase ^= 1;
-  }
-  if (!ok) {
-    if (tid == 0) atomicExch(g.err, 1u);
-  } else {
-    // epilogue: warp w owns rows 32w..32w+31 of the tile, 16 columns per tcgen05.ld
-    const int row = m0 + warp * 32 + lane;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-      uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;");
-      if (row < g.M) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int col = n0 + c0 + j;
-          if (col >= g.N) continue;
-          float v = __uint_as_float(r[j]);
-          if (g.part) {
-            g.part[((long long)blockIdx.z * g.M + row) * g.N + col] = v;
-            continue;
-          }
-          const long long o = (long long)row * g.ldc + col;
-          if (g.epi == EPI_STORE) {
-            if (g.bias) v += g.bias[col];
-            if (g.C) g.C[o] = v;
-            if (g.Cb) g.Cb[o] = __float2bfloat16(v);
-          } else if (g.epi == EPI_BIAS_GELU) {
-            v += g.bias[col];
-            g.C[o] = v;
-            g.Cb[o] = __float2bfloat16(gelu(v));
-          } else {
-            v *= gelu_grad(g.pre[o]);
-            if (g.C) g.C[o] = v;
-            g.Cb[o] = __float2bfloat16(v);
-          }
-        }
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols));
-}
-
-// Split K: C[row, col] (+ bias) = the sum of the slices' partial tiles, in slice order.
-__global__ void k_splitk_sum(const float* __restrict__ part, int slices, int M, int N, float* __restrict__ C, int ldc,
-                             const float* __restrict__ bias) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * N) return;
-  const int row = i / N, col = i - row * N;
-  float v = 0.f;
-  for (int z = 0; z < slices; z++) v += part[(long long)z * M * N + i];
-  if (bias) v += bias[col];
-  C[(long long)row * ldc + col] = v;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -492,59 +285,441 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 }
 
 // ------------------------------------------------------------------------------------------
-// elementwise / reduction kernels
+// Training. Everything a sample's forward and backward pass needs of other samples is the weight
+// gradients, so a tile of 128 samples runs through all layers, forward and back, in one CTA
+// (k_train_tile), its activations in shared and tensor memory; what the weight gradients need of
+// it (both hidden layers, their gradients, the features and output gradients, BF16) is written
+// transposed, [feature][sample], in the K-major core-matrix layout those products stage as is. The
+// weight gradients' K is the batch: k_train_weight_grads gives a run of tiles to each of about 128
+// CTAs, k_train_reduce adds the runs' partial sums in a fixed order and applies AdamW. Bias
+// gradients and the loss are summed in FP32 per 32 samples with warp shuffles, then in a fixed
+// order. A step is bound by the latency of its serial parts (six dependent MMAs and four epilogues
+// of 32,768 tanh or products each per tile), not by its 4 GFLOP. A step of batch 8192 with separate
+// GEMMs, one thread per column for the bias sums and an AdamW launch per parameter took 1.39 ms.
+constexpr int kTrainThreads = 512;
+constexpr int kGradCols = kHid + kIn + kOutPad;             // dW2 | dW1 | dW3^T columns of a partial sum
+constexpr int kBiasSums = 2 * kHid + kOutPad + 1;           // db1, db2, db3, loss
+constexpr uint32_t kTileT = kHid * BM * 2, kTileX = kIn * BM * 2, kTileDy = kOutPad * BM * 2;
 
-// Loss gradient dY and loss partial sums. Outputs 0..5 (endpoints): squared error, dY = 2 (y - t) / B.
-// Output 6 (the error bound): squared error when tau <= 0; otherwise the quantile (pinball) loss
-// bw * max(tau (t - y), (1 - tau) (y - t)), whose minimiser is the tau-quantile of the plain
-// optimizer's error given the block, i.e. an upper bound that holds for a fraction tau of blocks.
-__global__ void k_loss_grad(const float* __restrict__ y, const float* __restrict__ t, int B, float* __restrict__ dy,
-                            float* __restrict__ loss, float tau, float bw) {
-  float acc = 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B * kOutPad; i += gridDim.x * blockDim.x) {
-    const int s = i / kOutPad, c = i % kOutPad;
-    float g = 0.f;
-    if (c < 7) {
-      const float d = y[(long long)s * kOutPad + c] - t[(long long)s * kOut + c];
-      if (c == 6 && tau > 0.f) {
-        acc += bw * (d > 0.f ? (1.f - tau) * d : -tau * d);
-        g = bw * (d > 0.f ? (1.f - tau) : -tau) / (float)B;
+// k_train_tile's shared memory. W2's place takes W2^T for the backward product; W1's, once layer 1
+// is done, the warps' transposing buffers and W3^T; H is features, h1, h2, dY and dpre2 in turn.
+constexpr uint32_t kTrW2 = 0, kTrH = kTrW2 + kHid * kHid * 2, kTrW1 = kTrH + BM * kHid * 2, kTrBuf = kTrW1,
+                   kTrW3T = kTrBuf + (kTrainThreads / 32) * 1024, kTrW3 = kTrW1 + kHid * kIn * 2,
+                   kTrB1 = kTrW3 + kOutPad * kHid * 2, kTrB2 = kTrB1 + kHid * 4, kTrB3 = kTrB2 + kHid * 4,
+                   kTrBar = kTrB3 + kOutPad * 4, kTrTmem = kTrBar + 8, kTrainSmem = kTrTmem + 8;
+static_assert(kTrW3T + kHid * kOutPad * 2 <= kTrW3, "transposing buffers and W3^T fit in W1's place");
+static_assert(kTrainSmem <= 232448, "k_train_tile exceeds the 227 KB shared-memory limit");
+
+struct TrainArgs {
+  const uint8_t* blocks;
+  const float* targets;
+  int n, tiles;
+  float tau, bw;
+  const __nv_bfloat16 *W1, *W2, *W2T, *W3, *W3T;
+  const float *b1, *b2, *b3;
+  unsigned char *h1T, *h2T, *d1T, *d2T, *xT, *dyT;  // per tile: [feature][128 samples] core-matrix tiles
+  float *g1, *g2;                                   // per tile: gelu' of both layers, [feature][128 samples]
+  float* bias;                                      // [kBiasSums][4 * tiles]: sums of 32 samples
+  float* part;                                      // [slices][kGradCols][kHid] partial weight gradients
+  int slices, slice_tiles;
+  uint32_t* err;
+};
+
+__device__ __forceinline__ void async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+}
+
+// row-major BF16 [rows x kt] -> K-major core matrices at dst
+__device__ __forceinline__ void async_weights(uint32_t dst, const __nv_bfloat16* w, int rows, int kt) {
+  const int segs = kt >> 3;
+  for (int e = threadIdx.x; e < rows * segs; e += kTrainThreads) {
+    const int r = e / segs, kg = e - r * segs;
+    async16(dst + kseg(r, kg, kt), w + (size_t)r * kt + kg * 8);
+  }
+}
+
+// 16 features (first c0) of this warp's 32 samples (`quarter` of the tile), BF16, into the
+// [feature][sample] tile: through the warp's 1 KB buffer, then 16 bytes (8 samples) a lane
+__device__ __forceinline__ void store_transposed(unsigned char* buf, unsigned char* tile, int quarter, int c0,
+                                                 const uint32_t* packed) {
+  const int lane = threadIdx.x & 31;
+  uint16_t* b16 = reinterpret_cast<uint16_t*>(buf);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    b16[(2 * j) * 32 + lane] = (uint16_t)packed[j];
+    b16[(2 * j + 1) * 32 + lane] = (uint16_t)(packed[j] >> 16);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = lane; u < 64; u += 32) {
+    const int c = c0 + (u >> 2), sg = quarter * 4 + (u & 3);
+    *reinterpret_cast<uint4*>(tile + (c >> 3) * (BM / 8 * 128) + sg * 128 + (c & 7) * 16) =
+        *reinterpret_cast<const uint4*>(buf + u * 16);
+  }
+  __syncwarp();
+}
+
+// sums of v[0..15] over the warp's lanes: lane 2c (and 2c + 1) returns column c's
+__device__ __forceinline__ float column_sums(float (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int half = 8; half > 0; half >>= 1) {
+    const bool up = (lane & (2 * half)) != 0;
+#pragma unroll
+    for (int j = 0; j < half; j++) {
+      const float give = up ? v[j] : v[j + half], keep = up ? v[j + half] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, 2 * half);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 1);
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_train_tile(TrainArgs a) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  unsigned char* sH = sm + kTrH;
+  float* sB1 = reinterpret_cast<float*>(sm + kTrB1);
+  float* sB2 = reinterpret_cast<float*>(sm + kTrB2);
+  float* sB3 = reinterpret_cast<float*>(sm + kTrB3);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kTrTmem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, cg = warp >> 2, row = quarter * 32 + lane;  // TMEM lane = tile row; 64 columns
+  const int tile = blockIdx.x;
+  const long long row0 = (long long)tile * BM;
+  unsigned char* buf = sm + kTrBuf + warp * 1024;
+  const uint32_t base = smem_u32(sm), bar = base + kTrBar;
+  async_weights(base + kTrW1, a.W1, kHid, kIn);
+  asm volatile("cp.async.commit_group;");
+  async_weights(base + kTrW2, a.W2, kHid, kHid);
+  async_weights(base + kTrW3, a.W3, kOutPad, kHid);
+  asm volatile("cp.async.commit_group;");
+  if (tid < kHid) { sB1[tid] = a.b1[tid]; sB2[tid] = a.b2[tid]; }
+  if (tid < kOutPad) sB3[tid] = a.b3[tid];
+  if (tid < 2 * BM) {  // features: texels 8 * hf .. + 7 of a sample, and their transposed copy
+    const int r = tid & (BM - 1), hf = tid >> 7;
+    uint32_t px[8] = {};
+    if (row0 + r < a.n) {
+      const uint8_t* src = a.blocks + (row0 + r) * 64 + hf * 32;
+      if (((uintptr_t)a.blocks & 15) == 0) {
+        const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(src)), v1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        px[0] = v0.x; px[1] = v0.y; px[2] = v0.z; px[3] = v0.w;
+        px[4] = v1.x; px[5] = v1.y; px[6] = v1.z; px[7] = v1.w;
       } else {
-        acc += d * d;
-        g = 2.f * d / (float)B;
+#pragma unroll
+        for (int t = 0; t < 8; t++) px[t] = (uint32_t)__ldg(src + 4 * t) | (uint32_t)__ldg(src + 4 * t + 1) << 8 | (uint32_t)__ldg(src + 4 * t + 2) << 16;
       }
     }
-    dy[i] = g;
+    uint32_t f[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      const int i = 2 * k, j = 2 * k + 1;
+      f[k] = pack_bf16((float)((px[i / 3] >> (8 * (i % 3))) & 255u) * (1.0f / 255.0f),
+                       (float)((px[j / 3] >> (8 * (j % 3))) & 255u) * (1.0f / 255.0f));
+    }
+    unsigned char* xt = a.xT + (size_t)tile * kTileX;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      *reinterpret_cast<uint16_t*>(xt + kmaj_off(hf * 24 + 2 * k, r, BM)) = (uint16_t)f[k];
+      *reinterpret_cast<uint16_t*>(xt + kmaj_off(hf * 24 + 2 * k + 1, r, BM)) = (uint16_t)(f[k] >> 16);
+    }
+#pragma unroll
+    for (int g = 0; g < 3; g++)
+      *reinterpret_cast<uint4*>(sH + kseg(r, hf * 3 + g, kIn)) = make_uint4(f[4 * g], f[4 * g + 1], f[4 * g + 2], f[4 * g + 3]);
   }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc / (float)B);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+  asm volatile("cp.async.wait_group 1;");
+  const uint32_t id256 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kHid >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  const uint32_t id16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kOutPad >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  auto to_mma = [&]() {  // shared-memory writes and TMEM reads of all threads before the next product
+    asm volatile("fence.proxy.async.shared::cta;");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+  };
+  to_mma();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+  uint32_t phase = 0;
+  // TMEM columns 0.. = A [128 x kt] x B [N x kt]^T, both K-major in shared memory; false on a timeout
+  auto product = [&](uint32_t at, uint32_t bt, int kt, uint32_t idesc) {
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t sbo = (uint32_t)(kt >> 3) * 128;
+      for (int ks = 0; ks < kt / 16; ks++)
+        mma_bf16(tmem, make_desc(base + at + ks * 256, 128, sbo), make_desc(base + bt + ks * 256, 128, sbo), idesc, ks > 0);
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
+    }
+    const bool ok = tile_wait(bar, phase);
+    phase ^= 1;
+    return ok;
+  };
+  const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+  auto hidden = [&](const float* bias, float* grad, unsigned char* hT) {
+#pragma unroll 1
+    for (int c0 = cg * 64; c0 < cg * 64 + 64; c0 += 16) {
+      uint32_t r[16], w[8];
+      tmem_ld16(taddr + (uint32_t)c0, r);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        float ga, gb;
+        const float x = gelu_both(__uint_as_float(r[j]) + bias[c0 + j], ga);
+        const float y = gelu_both(__uint_as_float(r[j + 1]) + bias[c0 + j + 1], gb);
+        w[j / 2] = pack_bf16(x, y);
+        grad[(c0 + j) * BM + row] = ga;  // read back by this thread alone
+        grad[(c0 + j + 1) * BM + row] = gb;
+      }
+      *reinterpret_cast<uint4*>(sH + kseg(row, c0 >> 3, kHid)) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(sH + kseg(row, (c0 >> 3) + 1, kHid)) = make_uint4(w[4], w[5], w[6], w[7]);
+      store_transposed(buf, hT, quarter, c0, w);
+    }
+  };
+  auto back = [&](const float* grad, unsigned char* dT, float* bias, bool keep) {
+#pragma unroll 1
+    for (int c0 = cg * 64; c0 < cg * 64 + 64; c0 += 16) {
+      uint32_t r[16], w[8];
+      float v[16];
+      tmem_ld16(taddr + (uint32_t)c0, r);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]) * grad[(c0 + j) * BM + row];
+#pragma unroll
+      for (int j = 0; j < 8; j++) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+      if (keep) {
+        *reinterpret_cast<uint4*>(sH + kseg(row, c0 >> 3, kHid)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(sH + kseg(row, (c0 >> 3) + 1, kHid)) = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+      store_transposed(buf, dT, quarter, c0, w);
+      const float s = column_sums(v);
+      if (!(lane & 1)) bias[(size_t)(c0 + (lane >> 1)) * 4 * a.tiles] = s;
+    }
+  };
+  float* g1 = a.g1 + (size_t)tile * kHid * BM;
+  float* g2 = a.g2 + (size_t)tile * kHid * BM;
+  float* bias = a.bias + (size_t)tile * 4 + quarter;
+  const size_t bias_row = (size_t)4 * a.tiles;
+  bool ok;
+  do {
+    if (!(ok = product(kTrH, kTrW1, kIn, id256))) break;
+    async_weights(base + kTrW3T, a.W3T, kHid, kOutPad);  // into W1's place
+    asm volatile("cp.async.commit_group;");
+    hidden(sB1, g1, a.h1T + (size_t)tile * kTileT);
+    asm volatile("cp.async.wait_group 0;");
+    to_mma();
+    if (!(ok = product(kTrH, kTrW2, kHid, id256))) break;
+    async_weights(base + kTrW2, a.W2T, kHid, kHid);  // into W2's place
+    asm volatile("cp.async.commit_group;");
+    hidden(sB2, g2, a.h2T + (size_t)tile * kTileT);
+    to_mma();
+    if (!(ok = product(kTrH, kTrW3, kHid, id16))) break;
+    if (cg == 0) {
+      // Loss gradient. Outputs 0..5 (endpoints): squared error, dY = 2 (y - t) / B. Output 6 (the
+      // error bound): squared error when tau <= 0; otherwise the quantile (pinball) loss
+      // bw * max(tau (t - y), (1 - tau) (y - t)), whose minimiser is the tau-quantile of the plain
+      // optimizer's error given the block, i.e. an upper bound that holds for a fraction tau of blocks.
+      uint32_t r[16], w[8];
+      float v[16], loss = 0.f;
+      tmem_ld16(taddr, r);
+#pragma unroll
+      for (int c = 0; c < 16; c++) v[c] = 0.f;
+      if (row0 + row < a.n) {
+        const float* t = a.targets + (row0 + row) * kOut;
+#pragma unroll
+        for (int c = 0; c < 7; c++) {
+          const float d = __uint_as_float(r[c]) + sB3[c] - __ldg(t + c);
+          if (c == 6 && a.tau > 0.f) {
+            loss += a.bw * (d > 0.f ? (1.f - a.tau) * d : -a.tau * d);
+            v[c] = a.bw * (d > 0.f ? (1.f - a.tau) : -a.tau) / (float)a.n;
+          } else {
+            loss += d * d;
+            v[c] = 2.f * d / (float)a.n;
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+      *reinterpret_cast<uint4*>(sH + kseg(row, 0, kOutPad)) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(sH + kseg(row, 1, kOutPad)) = make_uint4(w[4], w[5], w[6], w[7]);
+      store_transposed(buf, a.dyT + (size_t)tile * kTileDy, quarter, 0, w);
+      const float s = column_sums(v);
+      if (!(lane & 1)) bias[(2 * kHid + (lane >> 1)) * bias_row] = s;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
+      if (lane == 0) bias[(2 * kHid + kOutPad) * bias_row] = loss / (float)a.n;
+    }
+    to_mma();
+    if (!(ok = product(kTrH, kTrW3T, kOutPad, id256))) break;  // dY W3
+    back(g2, a.d2T + (size_t)tile * kTileT, bias + kHid * bias_row, true);
+    asm volatile("cp.async.wait_group 0;");
+    to_mma();
+    if (!(ok = product(kTrH, kTrW2, kHid, id256))) break;  // dpre2 W2
+    back(g1, a.d1T + (size_t)tile * kTileT, bias, false);
+  } while (false);
+  if (!ok && tid == 0) atomicExch(a.err, 1u);
+  asm volatile("cp.async.wait_group 0;");
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
 }
 
-// column sums of a row-major [rows x cols] fp32 matrix -> out[cols]
-__global__ void k_colsum(const float* __restrict__ x, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; r++) s += x[(long long)r * cols + c];
-  out[c] = s;
+// blockIdx.x: half of the 256 rows, blockIdx.y: slice of the tiles. Rows [128 half, + 128) of
+// dW2 = dpre2^T h1, dW1 = dpre1^T X and dW3^T = h2^T dY over the slice, accumulated in TMEM (columns
+// 0.., 256.., 304..), written column by column ([kGradCols][kHid]: 32 rows a warp store).
+constexpr uint32_t kWgD2 = 0, kWgH1 = kWgD2 + kTileT / 2, kWgD1 = kWgH1 + kTileT, kWgX = kWgD1 + kTileT / 2,
+                   kWgH2 = kWgX + kTileX, kWgDy = kWgH2 + kTileT / 2, kWgBar = kWgDy + kTileDy, kWgTmem = kWgBar + 8,
+                   kWgSmem = kWgTmem + 8;
+static_assert(kWgSmem <= 232448, "k_train_weight_grads exceeds the 227 KB shared-memory limit");
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_train_weight_grads(TrainArgs a) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kWgTmem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t base = smem_u32(sm), bar = base + kWgBar, half = blockIdx.x;
+  const int t0 = blockIdx.y * a.slice_tiles, t1 = min(a.tiles, t0 + a.slice_tiles);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+  uint32_t phase = 0;
+  bool ok = true;
+  auto copy = [&](uint32_t dst, const unsigned char* src, uint32_t bytes) {
+    for (uint32_t e = tid * 16; e < bytes; e += kTrainThreads * 16) async16(base + dst + e, src + e);
+  };
+  for (int t = t0; t < t1; t++) {
+    const size_t at = (size_t)t * kTileT + half * (kTileT / 2);
+    copy(kWgD2, a.d2T + at, kTileT / 2);
+    copy(kWgH1, a.h1T + (size_t)t * kTileT, kTileT);
+    copy(kWgD1, a.d1T + at, kTileT / 2);
+    copy(kWgX, a.xT + (size_t)t * kTileX, kTileX);
+    copy(kWgH2, a.h2T + at, kTileT / 2);
+    copy(kWgDy, a.dyT + (size_t)t * kTileDy, kTileDy);
+    asm volatile("cp.async.commit_group;");
+    asm volatile("cp.async.wait_group 0;");
+    asm volatile("fence.proxy.async.shared::cta;");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      auto idesc = [](int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); };
+      constexpr uint32_t sbo = BM / 8 * 128;
+#pragma unroll
+      for (int ks = 0; ks < BM / 16; ks++) {
+        const uint32_t acc = t > t0 || ks > 0;
+        auto desc = [&](uint32_t o) { return make_desc(base + o + ks * 256, 128, sbo); };
+        mma_bf16(tmem, desc(kWgD2), desc(kWgH1), idesc(kHid), acc);
+        mma_bf16(tmem + kHid, desc(kWgD1), desc(kWgX), idesc(kIn), acc);
+        mma_bf16(tmem + kHid + kIn, desc(kWgH2), desc(kWgDy), idesc(kOutPad), acc);
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
+    }
+    if (!(ok = tile_wait(bar, phase))) break;
+    phase ^= 1;
+  }
+  if (!ok) {
+    if (tid == 0) atomicExch(a.err, 1u);
+  } else {
+    const int quarter = warp & 3, cg = warp >> 2;
+    float* dst = a.part + (size_t)blockIdx.y * kGradCols * kHid + half * BM + quarter * 32 + lane;
+#pragma unroll 1
+    for (int c0 = cg * (kGradCols / 4); c0 < (cg + 1) * (kGradCols / 4); c0 += 16) {
+      uint32_t r[16];
+      tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
+#pragma unroll
+      for (int j = 0; j < 16; j++) dst[(size_t)(c0 + j) * kHid] = __uint_as_float(r[j]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
-// AdamW on fp32 master weights; refreshes the bf16 copy. mask: parameters that stay zero.
-__global__ void k_adamw(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                        __nv_bfloat16* __restrict__ wb, int n, float lr, float b1, float b2, float eps, float wd,
-                        float bc1, float bc2, int rows_live, int row_len) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (i / row_len >= rows_live) { w[i] = 0.f; if (wb) wb[i] = __float2bfloat16(0.f); continue; }
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float wi = w[i] * (1.f - lr * wd);
-    wi -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
+// A parameter's buffers: FP32 gradient, weights and Adam moments, BF16 copy and transposed copy.
+struct ParamPtrs {
+  float *g, *w, *m, *v;
+  __nv_bfloat16 *wb, *wbT;
+};
+struct ReduceArgs {
+  const float *part, *bias;
+  int slices, bias_sums;
+  ParamPtrs W1, b1, W2, b2, W3, b3;
+  float* loss;
+  const uint32_t* err;
+  int update;  // AdamW after the gradients
+  float lr, beta1, beta2, eps, wd, bc1, bc2;
+};
+
+// AdamW on the FP32 master weight; returns it
+__device__ __forceinline__ float adamw(const ReduceArgs& a, const ParamPtrs& p, size_t i, float gi, float wd) {
+  const float mi = a.beta1 * p.m[i] + (1.f - a.beta1) * gi;
+  const float vi = a.beta2 * p.v[i] + (1.f - a.beta2) * gi * gi;
+  p.m[i] = mi;
+  p.v[i] = vi;
+  float wi = p.w[i] * (1.f - a.lr * wd);
+  wi -= a.lr * (mi / a.bc1) / (sqrtf(vi / a.bc2) + a.eps);
+  p.w[i] = wi;
+  return wi;
+}
+
+// Blocks 0..79: a 32 x 32 tile of the weight gradients ([kGradCols][kHid] partial sums, added slice
+// after slice); the others: one bias gradient (or the loss) per warp. After a timed-out wait (err)
+// nothing is written.
+constexpr int kReduceTiles = (kHid / 32) * (kGradCols / 32), kReduceBlocks = kReduceTiles + (kBiasSums + 31) / 32;
+static_assert(kGradCols % 32 == 0 && (kHid + kIn) % 32 == 16, "the last column tile is half W1, half W3");
+
+__global__ void __launch_bounds__(1024) k_train_reduce(ReduceArgs a) {
+  if (*a.err) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.x >= kReduceTiles) {
+    const int o = (blockIdx.x - kReduceTiles) * 32 + warp;
+    if (o >= kBiasSums) return;
+    const float* src = a.bias + (size_t)o * a.bias_sums;
+    float s = 0.f;
+    for (int k = lane; k < a.bias_sums; k += 32) s += src[k];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, k);
+    if (lane) return;
+    if (o == 2 * kHid + kOutPad) { *a.loss = s; return; }
+    const ParamPtrs& p = o < kHid ? a.b1 : o < 2 * kHid ? a.b2 : a.b3;
+    const int i = o < kHid ? o : o < 2 * kHid ? o - kHid : o - 2 * kHid;
+    p.g[i] = s;
+    if (a.update) adamw(a, p, i, s, 0.f);
+    return;
   }
+  __shared__ float t[32][33];
+  const int r0 = (blockIdx.x % (kHid / 32)) * 32, c0 = (blockIdx.x / (kHid / 32)) * 32;
+  {
+    const float* src = a.part + (size_t)(c0 + warp) * kHid + r0 + lane;
+    float s = 0.f;
+#pragma unroll 8
+    for (int z = 0; z < a.slices; z++) s += src[(size_t)z * kGradCols * kHid];
+    const int o = c0 + warp - kHid - kIn;
+    if (o >= 0) {  // W3 [16 x 256]: rows 7.. stay zero
+      const size_t i = (size_t)o * kHid + r0 + lane;
+      a.W3.g[i] = s;
+      if (a.update) {
+        float w = 0.f;
+        if (o < 7) w = adamw(a, a.W3, i, s, a.wd); else a.W3.w[i] = 0.f;
+        a.W3.wb[i] = __float2bfloat16(w);
+        a.W3.wbT[(size_t)(r0 + lane) * kOutPad + o] = __float2bfloat16(w);
+      }
+    }
+    t[warp][lane] = s;
+  }
+  __syncthreads();
+  const int row = r0 + warp, col = c0 + lane;
+  if (col >= kHid + kIn) return;
+  const ParamPtrs& p = col < kHid ? a.W2 : a.W1;
+  const size_t i = col < kHid ? (size_t)row * kHid + col : (size_t)row * kIn + col - kHid;
+  const float s = t[lane][warp];
+  p.g[i] = s;
+  if (!a.update) return;
+  const __nv_bfloat16 w = __float2bfloat16(adamw(a, p, i, s, a.wd));
+  p.wb[i] = w;
+  if (col < kHid) p.wbT[(size_t)col * kHid + row] = w;
 }
 
 // Training targets from the plain optimizer's blocks: endpoints of the 4-colour solution in
@@ -723,6 +898,7 @@ __global__ void k_scatter_idx(const uint8_t* __restrict__ enc, const uint32_t* _
 struct Param {
   int rows, cols, rows_live;
   DevBuf w, g, m, v, wb;  // fp32 master, grad, Adam moments, bf16 copy (weights only)
+  DevBuf wbT;             // bf16 transposed copy (W2, W3: the backward products)
   size_t n() const { return (size_t)rows * cols; }
 };
 
@@ -732,16 +908,16 @@ struct Net {
   Param W1, b1, W2, b2, W3, b3;
   int step = 0;
   float bound_tau = 0.f, bound_weight = 1.f;  // loss of the error-bound output (see k_loss_grad)
-  // activations / scratch sized for the largest batch seen
+  // training scratch sized for the largest batch seen (tiles of 128 samples, see TrainArgs)
   int cap = 0;
-  DevBuf pre1, h1, pre2, h2, y, dy, dpre2, dpre1, dh_b, dh_b1, targets, loss, errflag;
-  DevBuf splitk;  // partial tiles of the split-K weight-gradient products
+  DevBuf h1T, h2T, d1T, d2T, xT, dyT, g1, g2, bias, part;
+  DevBuf errflag;  // [0] a wait timed out, [1] the loss
   // learned encode scratch
   DevBuf fb_idx, fb_count, fb_in, fb_out, chunk_y;
   std::vector<Param*> params() { return {&W1, &b1, &W2, &b2, &W3, &b3}; }
 };
 
-int alloc_param(Param& p, int rows, int cols, int rows_live, bool bf16) {
+int alloc_param(Param& p, int rows, int cols, int rows_live, bool bf16, bool transposed) {
   p.rows = rows; p.cols = cols; p.rows_live = rows_live;
   cudaError_t e;
   if ((e = p.w.ensure(p.n() * 4)) != cudaSuccess) return cuda_check(e, "alloc weights");
@@ -752,6 +928,7 @@ int alloc_param(Param& p, int rows, int cols, int rows_live, bool bf16) {
   cudaMemset(p.v.ptr, 0, p.n() * 4);
   cudaMemset(p.g.ptr, 0, p.n() * 4);
   if (bf16 && (e = p.wb.ensure(p.n() * 2)) != cudaSuccess) return cuda_check(e, "alloc bf16 weights");
+  if (transposed && (e = p.wbT.ensure(p.n() * 2)) != cudaSuccess) return cuda_check(e, "alloc bf16 weights");
   return CRNGPU_OK;
 }
 
@@ -764,110 +941,32 @@ int upload(Param& p, const std::vector<float>& host) {
     if ((e = cudaMemcpy(p.wb.ptr, hb.data(), p.n() * 2, cudaMemcpyHostToDevice)) != cudaSuccess)
       return cuda_check(e, "upload bf16 weights");
   }
+  if (p.wbT.ptr) {
+    std::vector<__nv_bfloat16> hb(p.n());
+    for (int r = 0; r < p.rows; r++)
+      for (int c = 0; c < p.cols; c++) hb[(size_t)c * p.rows + r] = __float2bfloat16(host[(size_t)r * p.cols + c]);
+    if ((e = cudaMemcpy(p.wbT.ptr, hb.data(), p.n() * 2, cudaMemcpyHostToDevice)) != cudaSuccess)
+      return cuda_check(e, "upload bf16 weights");
+  }
   return CRNGPU_OK;
 }
 
-int ensure_batch(Net& net, int B) {
-  if (B <= net.cap) return CRNGPU_OK;
+// Slices of the weight gradients' sum: with two halves of the rows each, about as many CTAs as SMs.
+constexpr int kMaxSlices = 64;
+
+int ensure_batch(Net& net, int tiles) {
   cudaError_t e;
-  const size_t hid = (size_t)B * kHid;
-  DevBuf* f32[] = {&net.pre1, &net.pre2, &net.dpre2, &net.dpre1};
-  for (DevBuf* b : f32)
-    if ((e = b->ensure(hid * 4)) != cudaSuccess) return cuda_check(e, "alloc activations");
-  DevBuf* b16[] = {&net.h1, &net.h2, &net.dh_b, &net.dh_b1};
-  for (DevBuf* b : b16)
-    if ((e = b->ensure(hid * 2)) != cudaSuccess) return cuda_check(e, "alloc activations");
-  if ((e = net.y.ensure((size_t)B * kOutPad * 4)) != cudaSuccess) return cuda_check(e, "alloc outputs");
-  if ((e = net.dy.ensure((size_t)B * kOutPad * 4)) != cudaSuccess) return cuda_check(e, "alloc output grads");
-  if ((e = net.targets.ensure((size_t)B * kOut * 4)) != cudaSuccess) return cuda_check(e, "alloc targets");
-  if ((e = net.loss.ensure(16)) != cudaSuccess) return cuda_check(e, "alloc loss");
   if ((e = net.errflag.ensure(16)) != cudaSuccess) return cuda_check(e, "alloc flag");
-  net.cap = B;
+  if (tiles <= net.cap) return CRNGPU_OK;
+  struct { DevBuf* b; size_t bytes; } need[] = {
+      {&net.h1T, kTileT}, {&net.h2T, kTileT}, {&net.d1T, kTileT}, {&net.d2T, kTileT}, {&net.xT, kTileX},
+      {&net.dyT, kTileDy}, {&net.g1, kHid * BM * 4}, {&net.g2, kHid * BM * 4}, {&net.bias, kBiasSums * 4 * 4}};
+  for (auto& n : need)
+    if ((e = n.b->ensure(n.bytes * (size_t)tiles)) != cudaSuccess) return cuda_check(e, "alloc training scratch");
+  if ((e = net.part.ensure((size_t)std::min(tiles, kMaxSlices) * kGradCols * kHid * 4)) != cudaSuccess)
+    return cuda_check(e, "alloc partial gradients");
+  net.cap = tiles;
   return CRNGPU_OK;
-}
-
-Operand op_f32(const float* p, long long s_row, long long s_k) { return Operand{p, OP_F32, s_row, s_k, 0}; }
-Operand op_bf16(const __nv_bfloat16* p, long long s_row, long long s_k) { return Operand{p, OP_BF16, s_row, s_k, 0}; }
-Operand op_pixels(const uint8_t* p, bool sample_is_row) { return Operand{p, OP_PIXELS, 0, 0, sample_is_row ? 1 : 0}; }
-
-// Each CTA allocates kTmemCols of the SM's 512 tensor-memory columns; an unused dynamic
-// shared-memory reservation brings every CTA to about 57 KB so at most 4 CTAs share an SM and
-// the allocations never wait on each other.
-int gemm(GemmArgs g, cudaStream_t s, DevBuf* split_scratch = nullptr) {
-  static bool attr_done[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> lock(device_setup_mutex());
-    if (dev >= 0 && dev < 64 && !attr_done[dev]) {  // > 48 KB per CTA in total needs the opt-in
-      cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 << 10);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tc<48>, cudaFuncAttributeMaxDynamicSharedMemorySize, 36 << 10);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 24 << 10);
-      if (e != cudaSuccess) return cuda_check(e, "set k_gemm_tc shared memory");
-      attr_done[dev] = true;
-    }
-  }
-  const unsigned gx = (g.M + BM - 1) / BM;
-  const unsigned bn = g.N <= 16 ? 16u : g.N <= 48 ? 48u : 128u;
-  const unsigned gy = (g.N + bn - 1) / bn;
-  // Products with few output tiles and a long K (the weight gradients: K is the batch) split K so
-  // that about 128 CTAs share the work; the slices are summed by k_splitk_sum in a fixed order.
-  unsigned gz = 1;
-  g.kslice = 0;
-  g.part = nullptr;
-  if (split_scratch && g.epi == EPI_STORE && g.C && !g.Cb && gx * gy < 32 && g.K >= 4 * BK) {
-    gz = std::min<unsigned>(128 / (gx * gy), (unsigned)((g.K + BK - 1) / BK));
-    const int slice = ((g.K + (int)gz - 1) / (int)gz + BK - 1) / BK * BK;
-    gz = (unsigned)((g.K + slice - 1) / slice);
-    cudaError_t e = split_scratch->ensure((size_t)gz * g.M * g.N * sizeof(float));
-    if (e != cudaSuccess) return cuda_check(e, "alloc split-K scratch");
-    g.kslice = slice;
-    g.part = static_cast<float*>(split_scratch->ptr);
-  }
-  const dim3 grid(gx, gy, gz);
-  if (bn == 16) k_gemm_tc<16><<<grid, 128, 40 << 10, s>>>(g);
-  else if (bn == 48) k_gemm_tc<48><<<grid, 128, 36 << 10, s>>>(g);
-  else k_gemm_tc<128><<<grid, 128, 24 << 10, s>>>(g);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_check(e, "launch k_gemm_tc");
-  if (g.part) {
-    k_splitk_sum<<<(g.M * g.N + 255) / 256, 256, 0, s>>>(g.part, (int)gz, g.M, g.N, g.C, g.ldc, g.bias);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_check(e, "launch k_splitk_sum");
-  }
-  return CRNGPU_OK;
-}
-
-GemmArgs args(Operand a, Operand b, int M, int N, int K, int epi, float* C, __nv_bfloat16* Cb, const float* pre,
-              const float* bias, int ldc, Net& net) {
-  GemmArgs g;
-  g.a = a; g.b = b; g.M = M; g.N = N; g.K = K; g.epi = epi; g.C = C; g.Cb = Cb; g.pre = pre; g.bias = bias; g.ldc = ldc;
-  g.err = static_cast<uint32_t*>(net.errflag.ptr);
-  g.kslice = 0;
-  g.part = nullptr;
-  return g;
-}
-
-// forward over B samples whose pixels are `blocks` (device); y -> net.y [B x 16]
-int forward(Net& net, const uint8_t* blocks, int B, cudaStream_t s) {
-  int rc;
-  float* pre1 = static_cast<float*>(net.pre1.ptr);
-  float* pre2 = static_cast<float*>(net.pre2.ptr);
-  __nv_bfloat16* h1 = static_cast<__nv_bfloat16*>(net.h1.ptr);
-  __nv_bfloat16* h2 = static_cast<__nv_bfloat16*>(net.h2.ptr);
-  // L1: pre1 = X W1^T + b1, h1 = gelu(pre1)
-  if ((rc = gemm(args(op_pixels(blocks, true), op_bf16(static_cast<__nv_bfloat16*>(net.W1.wb.ptr), kIn, 1), B, kHid,
-                      kIn, EPI_BIAS_GELU, pre1, h1, nullptr, static_cast<float*>(net.b1.w.ptr), kHid, net),
-                 s)) != CRNGPU_OK)
-    return rc;
-  if ((rc = gemm(args(op_bf16(h1, kHid, 1), op_bf16(static_cast<__nv_bfloat16*>(net.W2.wb.ptr), kHid, 1), B, kHid,
-                      kHid, EPI_BIAS_GELU, pre2, h2, nullptr, static_cast<float*>(net.b2.w.ptr), kHid, net),
-                 s)) != CRNGPU_OK)
-    return rc;
-  return gemm(args(op_bf16(h2, kHid, 1), op_bf16(static_cast<__nv_bfloat16*>(net.W3.wb.ptr), kHid, 1), B, kOutPad, kHid,
-                   EPI_STORE, static_cast<float*>(net.y.ptr), nullptr, nullptr, static_cast<float*>(net.b3.w.ptr),
-                   kOutPad, net),
-              s);
 }
 
 // inference over n blocks (device) -> y [n x 16] with the fused kernel, one persistent CTA per SM
@@ -898,54 +997,83 @@ int infer(Net& net, const uint8_t* blocks, uint32_t n, float* y, cudaStream_t s)
   return cuda_check(cudaGetLastError(), "launch k_mlp_infer");
 }
 
-// gradients of the mean squared error for targets in net.targets; loss -> net.loss
-int backward(Net& net, const uint8_t* blocks, int B, cudaStream_t s) {
-  int rc;
-  float* dy = static_cast<float*>(net.dy.ptr);
-  float* dpre2 = static_cast<float*>(net.dpre2.ptr);
-  float* dpre1 = static_cast<float*>(net.dpre1.ptr);
-  __nv_bfloat16* dhb = static_cast<__nv_bfloat16*>(net.dh_b.ptr);    // bf16 dpre2
-  __nv_bfloat16* dhb1 = static_cast<__nv_bfloat16*>(net.dh_b1.ptr);  // bf16 dpre1 (own buffer: dhb is read meanwhile)
-  cudaMemsetAsync(net.loss.ptr, 0, 4, s);
-  k_loss_grad<<<256, 256, 0, s>>>(static_cast<float*>(net.y.ptr), static_cast<float*>(net.targets.ptr), B, dy,
-                                  static_cast<float*>(net.loss.ptr), net.bound_tau, net.bound_weight);
-  // dW3 [16 x 256] = dY^T H2 ; db3 = colsum(dY)
-  if ((rc = gemm(args(op_f32(dy, 1, kOutPad), op_bf16(static_cast<__nv_bfloat16*>(net.h2.ptr), 1, kHid), kOutPad, kHid,
-                      B, EPI_STORE, static_cast<float*>(net.W3.g.ptr), nullptr, nullptr, nullptr, kHid, net),
-                 s, &net.splitk)) != CRNGPU_OK)
-    return rc;
-  k_colsum<<<1, kOutPad, 0, s>>>(dy, B, kOutPad, static_cast<float*>(net.b3.g.ptr));
-  // dpre2 = (dY W3) * gelu'(pre2)
-  if ((rc = gemm(args(op_f32(dy, kOutPad, 1), op_f32(static_cast<float*>(net.W3.w.ptr), 1, kHid), B, kHid, kOutPad,
-                      EPI_GELU_GRAD, dpre2, dhb, static_cast<float*>(net.pre2.ptr), nullptr, kHid, net),
-                 s)) != CRNGPU_OK)
-    return rc;
-  // dW2 [256 x 256] = dpre2^T H1 ; db2
-  if ((rc = gemm(args(op_bf16(dhb, 1, kHid), op_bf16(static_cast<__nv_bfloat16*>(net.h1.ptr), 1, kHid), kHid, kHid, B,
-                      EPI_STORE, static_cast<float*>(net.W2.g.ptr), nullptr, nullptr, nullptr, kHid, net),
-                 s, &net.splitk)) != CRNGPU_OK)
-    return rc;
-  k_colsum<<<(kHid + 127) / 128, 128, 0, s>>>(dpre2, B, kHid, static_cast<float*>(net.b2.g.ptr));
-  // dpre1 = (dpre2 W2) * gelu'(pre1)
-  if ((rc = gemm(args(op_bf16(dhb, kHid, 1), op_f32(static_cast<float*>(net.W2.w.ptr), 1, kHid), B, kHid, kHid,
-                      EPI_GELU_GRAD, dpre1, dhb1, static_cast<float*>(net.pre1.ptr), nullptr, kHid, net),
-                 s)) != CRNGPU_OK)
-    return rc;
-  // dW1 [256 x 48] = dpre1^T X ; db1
-  if ((rc = gemm(args(op_bf16(dhb1, 1, kHid), op_pixels(blocks, false), kHid, kIn, B, EPI_STORE,
-                      static_cast<float*>(net.W1.g.ptr), nullptr, nullptr, nullptr, kIn, net),
-                 s, &net.splitk)) != CRNGPU_OK)
-    return rc;
-  k_colsum<<<(kHid + 127) / 128, 128, 0, s>>>(dpre1, B, kHid, static_cast<float*>(net.b1.g.ptr));
-  return cuda_check(cudaGetLastError(), "backward kernels");
+struct Adam {
+  float lr, wd;
+};
+
+// Loss and gradients of B samples, and with `adam` one AdamW step (betas 0.9/0.999, eps 1e-8); the
+// loss goes to errflag[1].
+int train_pass(Net& net, const uint8_t* blocks, const float* targets, int B, const Adam* adam, cudaStream_t s) {
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_check(e, "cudaGetDevice");
+  if (dev < 0 || dev >= 64) { set_error("device index out of range"); return CRNGPU_E_DEVICE; }
+  {
+    std::lock_guard<std::mutex> lock(device_setup_mutex());
+    if (!attr_done[dev]) {
+      e = cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_train_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
+      if (e != cudaSuccess) return cuda_check(e, "set up the training kernels");
+      attr_done[dev] = true;
+    }
+  }
+  const int tiles = (int)(((long long)B + BM - 1) / BM);
+  int rc = ensure_batch(net, tiles);
+  if (rc != CRNGPU_OK) return rc;
+  auto f32 = [](DevBuf& b) { return static_cast<float*>(b.ptr); };
+  auto bf = [](DevBuf& b) { return static_cast<__nv_bfloat16*>(b.ptr); };
+  auto u8 = [](DevBuf& b) { return static_cast<unsigned char*>(b.ptr); };
+  uint32_t* err = static_cast<uint32_t*>(net.errflag.ptr);
+  TrainArgs t;
+  t.blocks = blocks;
+  t.targets = targets;
+  t.n = B;
+  t.tiles = tiles;
+  t.tau = net.bound_tau;
+  t.bw = net.bound_weight;
+  t.W1 = bf(net.W1.wb); t.W2 = bf(net.W2.wb); t.W2T = bf(net.W2.wbT); t.W3 = bf(net.W3.wb); t.W3T = bf(net.W3.wbT);
+  t.b1 = f32(net.b1.w); t.b2 = f32(net.b2.w); t.b3 = f32(net.b3.w);
+  t.h1T = u8(net.h1T); t.h2T = u8(net.h2T); t.d1T = u8(net.d1T); t.d2T = u8(net.d2T); t.xT = u8(net.xT); t.dyT = u8(net.dyT);
+  t.g1 = f32(net.g1); t.g2 = f32(net.g2);
+  t.bias = f32(net.bias);
+  t.part = f32(net.part);
+  t.slice_tiles = (tiles + kMaxSlices - 1) / kMaxSlices;
+  t.slices = (tiles + t.slice_tiles - 1) / t.slice_tiles;
+  t.err = err;
+  ReduceArgs r;
+  auto ptrs = [&](Param& p) { return ParamPtrs{f32(p.g), f32(p.w), f32(p.m), f32(p.v), bf(p.wb), bf(p.wbT)}; };
+  r.W1 = ptrs(net.W1); r.b1 = ptrs(net.b1); r.W2 = ptrs(net.W2); r.b2 = ptrs(net.b2); r.W3 = ptrs(net.W3); r.b3 = ptrs(net.b3);
+  r.part = t.part;
+  r.bias = t.bias;
+  r.slices = t.slices;
+  r.bias_sums = 4 * tiles;
+  r.loss = reinterpret_cast<float*>(err + 1);
+  r.err = err;
+  r.update = adam != nullptr;
+  r.beta1 = 0.9f;
+  r.beta2 = 0.999f;
+  r.eps = 1e-8f;
+  r.lr = adam ? adam->lr : 0.f;
+  r.wd = adam ? adam->wd : 0.f;
+  r.bc1 = 1.f - std::pow(r.beta1, (float)(net.step + 1));
+  r.bc2 = 1.f - std::pow(r.beta2, (float)(net.step + 1));
+  if ((e = cudaMemsetAsync(err, 0, 8, s)) != cudaSuccess) return cuda_check(e, "clear flag");
+  k_train_tile<<<tiles, kTrainThreads, kTrainSmem, s>>>(t);
+  k_train_weight_grads<<<dim3(2, t.slices), kTrainThreads, kWgSmem, s>>>(t);
+  k_train_reduce<<<kReduceBlocks, 1024, 0, s>>>(r);
+  return cuda_check(cudaGetLastError(), "launch the training kernels");
 }
 
-int check_flag(Net& net, cudaStream_t s) {
-  uint32_t f = 0;
-  cudaError_t e = cudaMemcpyAsync(&f, net.errflag.ptr, 4, cudaMemcpyDeviceToHost, s);
+// Waits for the stream; the flag (and with `loss` the loss) of what ran on it.
+int check_flag(Net& net, cudaStream_t s, float* loss = nullptr) {
+  uint32_t f[2] = {};
+  cudaError_t e = cudaMemcpyAsync(f, net.errflag.ptr, loss ? 8 : 4, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_check(e, "read mma status");
-  if (f) { set_error("tensor-core wait timed out"); return CRNGPU_E_DEVICE; }
+  if (f[0]) { set_error("tensor-core wait timed out"); return CRNGPU_E_DEVICE; }
+  if (loss) std::memcpy(loss, &f[1], 4);
   return CRNGPU_OK;
 }
 
@@ -976,7 +1104,7 @@ extern "C" void* crngpu_mlp_create(uint64_t seed) try {
   cudaGetDevice(&net->device);
   std::mt19937_64 rng(seed);
   auto init = [&](Param& p, int rows, int cols, int rows_live, bool is_bias, int fan_in) {
-    if (alloc_param(p, rows, cols, rows_live, !is_bias) != CRNGPU_OK) return false;
+    if (alloc_param(p, rows, cols, rows_live, !is_bias, &p == &net->W2 || &p == &net->W3) != CRNGPU_OK) return false;
     std::vector<float> h(p.n(), 0.f);
     if (!is_bias) {
       const float bound = std::sqrt(6.0f / (float)fan_in) * 0.5f;
@@ -1064,14 +1192,8 @@ extern "C" int crngpu_mlp_gradients(void* h, const uint8_t* d_blocks, const floa
   Net* net = static_cast<Net*>(h);
   if (!net || net->magic != 0x4D4C5030u || !d_blocks || !d_targets || !n) return CRNGPU_E_PARAM;
   cudaStream_t s = as_stream(stream);
-  int rc = ensure_batch(*net, (int)n);
-  if (rc != CRNGPU_OK) return rc;
-  cudaMemsetAsync(net->errflag.ptr, 0, 4, s);
-  cudaMemcpyAsync(net->targets.ptr, d_targets, (size_t)n * kOut * 4, cudaMemcpyDeviceToDevice, s);
-  if ((rc = forward(*net, d_blocks, (int)n, s)) != CRNGPU_OK) return rc;
-  if ((rc = backward(*net, d_blocks, (int)n, s)) != CRNGPU_OK) return rc;
-  if (loss) cudaMemcpyAsync(loss, net->loss.ptr, 4, cudaMemcpyDeviceToHost, s);
-  return check_flag(*net, s);
+  int rc = train_pass(*net, d_blocks, d_targets, (int)n, nullptr, s);
+  return rc != CRNGPU_OK ? rc : check_flag(*net, s, loss);
 } catch (...) {
   return crngpu::exception_status();
 }
@@ -1079,21 +1201,15 @@ extern "C" int crngpu_mlp_gradients(void* h, const uint8_t* d_blocks, const floa
 // One AdamW step (betas 0.9/0.999, eps 1e-8) on a batch: forward, backward, update.
 extern "C" int crngpu_mlp_train_step(void* h, const uint8_t* d_blocks, const float* d_targets, uint32_t n, float lr,
                                      float weight_decay, float* loss, void* stream) try {
-  int rc = crngpu_mlp_gradients(h, d_blocks, d_targets, n, loss, stream);
-  if (rc != CRNGPU_OK) return rc;
+  clear_error();
   Net* net = static_cast<Net*>(h);
+  if (!net || net->magic != 0x4D4C5030u || !d_blocks || !d_targets || !n) return CRNGPU_E_PARAM;
   cudaStream_t s = as_stream(stream);
+  const Adam adam = {lr, weight_decay};
+  int rc = train_pass(*net, d_blocks, d_targets, (int)n, &adam, s);
+  if (rc != CRNGPU_OK || (rc = check_flag(*net, s, loss)) != CRNGPU_OK) return rc;
   net->step++;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float bc1 = 1.f - std::pow(b1, (float)net->step), bc2 = 1.f - std::pow(b2, (float)net->step);
-  for (Param* p : net->params()) {
-    const bool is_bias = p->rows == 1;
-    k_adamw<<<64, 256, 0, s>>>(static_cast<float*>(p->w.ptr), static_cast<float*>(p->g.ptr),
-                               static_cast<float*>(p->m.ptr), static_cast<float*>(p->v.ptr),
-                               static_cast<__nv_bfloat16*>(p->wb.ptr), (int)p->n(), lr, b1, b2, 1e-8f,
-                               is_bias ? 0.f : weight_decay, bc1, bc2, is_bias ? 1 : p->rows_live, p->cols);
-  }
-  return cuda_check(cudaGetLastError(), "launch k_adamw");
+  return CRNGPU_OK;
 } catch (...) {
   return crngpu::exception_status();
 }

@@ -159,3 +159,34 @@ def test_shipped_network_on_held_out_textures(L):
     assert got["rmse_learned"] - r["rmse_plain"] <= 0.1
     assert got["speedup"] > 2.0
     assert 0.0 < got["fallback_frac"] < 0.25
+
+
+# one sample, a tile's last sample, one past it, more tiles than slices of the weight gradients, and
+# blocks that are not 16-byte aligned; the bounds are test_gradients_match_oracle's (BF16 operands)
+@pytest.mark.parametrize("n,shift", [(1, 0), (128, 0), (129, 4), (8197, 0), (64 * 128 + 128 + 3, 1)])
+def test_gradients_at_tile_and_slice_edges(L, n, shift):
+    from oracle import mlp_oracle
+    rng = np.random.default_rng(n)
+    blocks = rng.integers(0, 256, (n, 64), np.uint8)
+    targets = rng.random((n, 8)).astype(np.float32)
+    net = L.EndpointNet(seed=12)
+    raw = torch.zeros(n * 64 + shift, dtype=torch.uint8, device="cuda")
+    raw[shift:] = torch.from_numpy(blocks.reshape(-1)).cuda()
+    loss = net.gradients(raw[shift:].view(n, 64), torch.from_numpy(targets).cuda())
+    ref_loss, ref = mlp_oracle.gradients(net.state(), blocks, targets)
+    assert abs(loss - ref_loss) / ref_loss < 1e-2
+    for i, name in enumerate(L.PARAM_NAMES):
+        assert rel_err(net.get(i, grad=True).astype(np.float64), ref[name]) < 3e-2, name
+
+
+def test_training_steps_are_repeatable(L):
+    """No sum depends on the order CTAs finish in: two networks trained alike end alike."""
+    blocks = L.training_blocks(1, 256, seed0=1000)
+    targets, _ = L.make_targets(blocks)
+    states = []
+    for _ in range(2):
+        net = L.EndpointNet(seed=3)
+        L.train(net, blocks, targets, steps=5, batch=1000)
+        states.append(net.state())
+    for name in L.PARAM_NAMES:
+        assert np.array_equal(states[0][name], states[1][name]), name
