@@ -32,7 +32,7 @@
 namespace crngpu {
 
 // Device status word values (written by k_crn_decode_textures, read back by the host).
-enum : uint32_t { kStOk = 0, kStBadCode = 1, kStBadIndex = 2 };
+enum : uint32_t { kStOk = 0, kStBadCode = 1, kStBadIndex = 2, kStWait = 3 };
 
 // Model slots in a context's device model array.
 enum { kMRef = 0, kMEp0 = 1, kMSel0 = 2, kMEp1 = 3, kMSel1 = 4, kNumModels = 5 };
@@ -1073,6 +1073,733 @@ __global__ void __launch_bounds__(kWThreads, 1) k_crn_decode_wide(const StreamJo
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// The largest levels of a plan: k_crn_decode_walk, many CTAs per level stream.
+//
+// The wide decoder keeps one CTA busy with everything a level needs, and its walk, one dependent
+// shared-memory load (about 47 cycles) per chunk or block, bounds it: 1.74 ms for the 1024 x 1024
+// level of a DXT1 file while the other SMs idle (0.50 ms here). Here the other SMs build richer step tables, so
+// that the walk takes a step per four chunks (even rows) or four blocks (odd rows), and the symbol
+// decode and the endpoint indices leave the walking CTA:
+//
+//  * Tables, per bit position p: C4[p] = four times the bits of four chunks starting at p (low half; the
+//    distance to the next entry in bytes) and, for the row below, which of their eight blocks carry endpoint deltas; O4[p][k] = bits - 1 of four
+//    blocks, for each of the 16 combinations k of which carry deltas (a block is at most 64 bits,
+//    so four fit a byte less one). Where a row's blocks are not a multiple of eight, O2 and C1 (two
+//    blocks, one chunk) for the row's end. A lookup never depends on where the walk is, so every
+//    position's entry is computed by all SMs at once.
+//  * Segments. A level's stream is cut into segments; launch s builds the tables of segment s,
+//    walks segment s - 1, decodes the symbols of the groups the walk passed in segment s - 2 and
+//    resolves the endpoint indices of the rows decoded from segment s - 3, each in CTAs of its own.
+//    The launches follow each other on one stream: no CTA waits for another. Two table buffers of a
+//    segment each stay in L2. Small segments overlap the stages better, large ones launch less
+//    often: a segment is kWalkSegment positions of the plan's largest level, and the plan's other
+//    levels are cut in as many.
+//  * A segment's tables go on for one window (kWalkHalo positions) after its end, so that the walk,
+//    which tests the position of the group before, may step over the end.
+// Past the end of the stream every bit is zero: the walk stays at the first such position.
+constexpr uint32_t kWalkThreads = 512;
+constexpr uint32_t kWalkTile = 4096;       // positions per builder CTA
+constexpr uint32_t kWalkReach = 640;       // positions past a tile that its entries depend on: 3 chunks of 144 bits,
+                                           // a chunk's three codes and their 16-bit windows
+constexpr uint32_t kWalkExt = kWalkTile + kWalkReach;
+constexpr uint32_t kWalkHalo = 2048;       // > two groups of 576 bits
+constexpr uint32_t kWalkSegment = 98304;
+constexpr uint32_t kWalkMaxSegments = 64;
+constexpr uint32_t kWalkPosBits = 28;      // anchors: position | combination << 28
+
+// A level's progress between launches (zero at the start).
+struct WalkState {
+  uint32_t p, r, e, groups;                // the walk: position, row, chunk or block in the row, groups passed
+  uint32_t rows, carry, bad, pad;          // the resolver: rows resolved, running indices; 1: bad code, 2: bad index
+  uint32_t passed[kWalkMaxSegments + 1];   // groups passed after each segment
+  uint32_t bits[kWMaxW / 32];              // the current even row's combinations, a byte per four chunks
+};
+
+struct WalkJob {
+  StreamJob j;
+  uint4* o4;          // two buffers of `cap` entries
+  uint32_t* c4;
+  uint2* rem;         // (O2, C1), or null when rows are multiples of eight blocks
+  uint32_t* anchors;  // position of every group
+  uint32_t* blocks;   // decoded blocks, padded rows: ref | delta A << 2 | selector A << 16 | ref of the block
+                      // below << 30, and for two-endpoint formats a plane of delta B | selector B << 16
+  uint16_t* above;    // endpoint indices A, then B, of the last resolved row
+  WalkState* st;
+  uint32_t bits;      // bits of the stream
+  uint32_t seg, segs; // positions per segment, segments
+  uint32_t cap;       // entries of a table buffer: seg + kWalkHalo
+  uint32_t tile0, tiles;  // this level's builder CTAs in a launch
+};
+
+struct WalkShape {
+  uint32_t W, H, W2, rows, ge, go;  // ge, go: groups of an even and an odd row
+};
+__host__ __device__ inline WalkShape walk_shape(uint32_t bx, uint32_t by, uint32_t faces) {
+  WalkShape s;
+  s.W = (bx + 1) & ~1u;
+  s.H = (by + 1) & ~1u;
+  s.W2 = s.W >> 1;
+  s.rows = s.H * faces;
+  s.ge = s.W2 / 4 + s.W2 % 4;  // whole groups, then a group per chunk
+  s.go = (s.W + 3) / 4;
+  return s;
+}
+
+// Shared memory: the walk's ring of table windows (four windows; smaller ones when it holds the row
+// ends' tables too; the first window is copied again behind the last, so that a group of steps that
+// begins in the last window runs on without wrapping), the builders' arrays, the decoder's tables.
+template <bool REM>
+struct WalkRing {
+  static constexpr uint32_t kWindow = REM ? 1024u : 2048u, kSlots = 4u, kMask = kWindow * kSlots - 1u;
+  static constexpr uint32_t kO4 = 0, kC4 = kO4 + kWindow * (kSlots + 1) * 16u, kRem = kC4 + kWindow * (kSlots + 1) * 4u,
+                            kEnd = kRem + (REM ? kWindow * (kSlots + 1) * 8u : 0u);
+};
+constexpr uint32_t kWalkLuts = 5u * (4u << kLutBits);
+constexpr uint32_t kWalkBuildSmem = kWalkLuts + wide_align16((kWalkExt / 32 + 4) * 4u) + 10u * kWalkExt + 3u * 4u * kWalkExt;
+constexpr uint32_t kWalkSmem = WalkRing<false>::kEnd > kWalkBuildSmem ? WalkRing<false>::kEnd : kWalkBuildSmem;
+static_assert(WalkRing<true>::kEnd <= kWalkSmem && kWalkSmem + 2048u <= 227u << 10, "walk decoder shared memory");
+
+struct WalkShared {
+  uint32_t aux[5][kAuxWords];
+  uint32_t scan[2][4][2];
+  uint32_t carry[2];
+  uint32_t bits[kWMaxW / 32];
+  uint32_t walking;  // 0: the walk is over
+  uint64_t full[4], empty[4];
+};
+
+// The models a level's format reads, staged: first-level tables at `luts`, long-code bounds.
+__device__ __forceinline__ uint32_t walk_stage_models(const StreamJob& J, uint32_t* luts, WalkShared& S) {
+  const bool colour = J.kind == kKDxt1 || J.kind == kKDxt5;
+  const uint32_t nm = models_used(J.kind);
+  const int srcm[5] = {kMRef, colour ? kMEp0 : kMEp1, colour ? kMSel0 : kMSel1, kMEp1, kMSel1};
+  for (uint32_t t = 0; t < nm; t++) {
+    const uint4* src = reinterpret_cast<const uint4*>(J.models[srcm[t]].lut);
+    uint4* dst = reinterpret_cast<uint4*>(luts + (t << kLutBits));
+    for (uint32_t k = threadIdx.x; k < (1u << kLutBits) / 4; k += kWalkThreads) dst[k] = __ldg(src + k);
+  }
+  if (threadIdx.x < nm * kAuxWords) {
+    const uint32_t t = threadIdx.x / kAuxWords, k = threadIdx.x - t * kAuxWords;
+    const DevModel* md = J.models + srcm[t];
+    S.aux[t][k] = k < 5 ? __ldg(&md->limit[kLutBits + 1 + k])
+                : k < 10 ? (uint32_t)__ldg(&md->base[kLutBits + 1 + k - 5])
+                : k == 10 ? __ldg(&md->num_syms) : 0u;
+  }
+  return nm;
+}
+
+// ---- tables of positions [tile * kWalkTile, + kWalkTile) of segment k
+__device__ __forceinline__ void walk_build(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t tile) {
+  const StreamJob& J = job.j;
+  const uint32_t P0 = k * job.seg + tile * kWalkTile, tid = threadIdx.x;
+  if (P0 > job.bits + kWalkHalo) return;
+  const bool two = J.kind == kKDxt5 || J.kind == kKDxn, five = J.kind == kKDxt5;
+  uint32_t* luts = reinterpret_cast<uint32_t*>(wide_smem);
+  uint32_t* words = luts + kWalkLuts / 4;
+  uint32_t* C1 = words + wide_align16((kWalkExt / 32 + 4) * 4u) / 4;
+  uint32_t* C2 = C1 + kWalkExt;
+  uint32_t* O2 = C2 + kWalkExt;
+  uint8_t* lenR = reinterpret_cast<uint8_t*>(O2 + kWalkExt);
+  uint8_t *grp = lenR + kWalkExt, *lenDA = grp + kWalkExt, *lenSA = lenDA + kWalkExt, *L0 = lenSA + kWalkExt,
+          *L1 = L0 + kWalkExt, *lenDB = L1 + kWalkExt, *lenSB = lenDB + kWalkExt, *selB = lenSB + kWalkExt,
+          *endB = selB + kWalkExt;
+  walk_stage_models(J, luts, S);
+  for (uint32_t m = tid; m < kWalkExt / 32 + 4; m += kWalkThreads) words[m] = stream_word(J.src, J.src_size, P0 / 32 + m);
+  __syncthreads();
+  const uint32_t* lR = luts;
+  const uint32_t* lDA = luts + (1u << kLutBits);
+  const uint32_t* lSA = luts + (2u << kLutBits);
+  const uint32_t* lDB = luts + (3u << kLutBits);
+  const uint32_t* lSB = luts + (4u << kLutBits);
+  auto in = [](uint32_t j) { return min(j, kWalkExt - 1u); };  // entries near the end are beyond every tile entry's reach
+  for (uint32_t j = tid; j < kWalkExt; j += kWalkThreads) {
+    const uint32_t v = window_bits(words, j) >> 16;
+    uint32_t len, junk = 0;
+    grp[j] = (uint8_t)code_sym(v, lR, S.aux[0], J.models + kMRef, nullptr, 0u, len, junk);
+    lenR[j] = (uint8_t)len;
+    lenDA[j] = (uint8_t)code_len(v, lDA, S.aux[1]);
+    lenSA[j] = (uint8_t)code_len(v, lSA, S.aux[2]);
+    if (five) {
+      lenDB[j] = (uint8_t)code_len(v, lDB, S.aux[3]);
+      lenSB[j] = (uint8_t)code_len(v, lSB, S.aux[4]);
+    }
+  }
+  __syncthreads();
+  const uint8_t *sel = lenSA, *end = lenDA;
+  if (two) {
+    const uint8_t *d2 = five ? lenDB : lenDA, *s2 = five ? lenSB : lenSA;
+    for (uint32_t j = tid; j < kWalkExt; j += kWalkThreads) {
+      selB[j] = (uint8_t)(lenSA[j] + s2[in(j + lenSA[j])]);
+      endB[j] = (uint8_t)(lenDA[j] + d2[in(j + lenDA[j])]);
+    }
+    __syncthreads();
+    sel = selB;
+    end = endB;
+  }
+  for (uint32_t j = tid; j < kWalkExt; j += kWalkThreads) {
+    L0[j] = sel[j];
+    L1[j] = (uint8_t)(end[j] + sel[in(j + end[j])]);
+  }
+  __syncthreads();
+  for (uint32_t j = tid; j < kWalkExt; j += kWalkThreads) {
+    const uint32_t g = grp[j];
+    uint32_t q = in(j + lenR[j]);
+    q = in(q + ((g & 3u) ? L0 : L1)[q]);
+    const uint32_t end2 = q + (((g >> 4) & 3u) ? L0 : L1)[q];
+    C1[j] = (end2 - j) | ((((g >> 2) & 3u) ? 0u : 1u) | (((g >> 6) & 3u) ? 0u : 2u)) << 16;
+    const uint32_t d0 = L0[j], d1 = L1[j], q0 = in(j + d0), q1 = in(j + d1);
+    O2[j] = (d0 + L0[q0]) | (d1 + L0[q1]) << 8 | (d0 + L1[q0]) << 16 | (d1 + L1[q1]) << 24;
+  }
+  __syncthreads();
+  for (uint32_t j = tid; j < kWalkExt; j += kWalkThreads) {
+    const uint32_t a = C1[j], b = C1[in(j + (a & 0xFFFFu))];
+    C2[j] = ((a & 0xFFFFu) + (b & 0xFFFFu)) | ((a >> 16) << 2 | b >> 16) << 16;
+  }
+  __syncthreads();
+  const size_t at = (size_t)(k & 1u) * job.cap + tile * kWalkTile;
+  for (uint32_t j = tid; j < kWalkTile; j += kWalkThreads) {
+    const uint32_t a = C2[j], b = C2[j + (a & 0xFFFFu)];
+    job.c4[at + j] = 4u * ((a & 0xFFFFu) + (b & 0xFFFFu)) | (a >> 16 | (b >> 16) << 4) << 16;
+    const uint32_t o = O2[j];
+    uint32_t w[4];
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const uint32_t d = (o >> (8 * f)) & 255u;
+      w[f] = O2[j + d] + (d - 1u) * 0x01010101u;  // bytes of at most 128 + 127
+    }
+    job.o4[at + j] = make_uint4(w[0], w[1], w[2], w[3]);
+    if (job.rem) job.rem[at + j] = make_uint2(o, C1[j]);
+  }
+}
+
+// ---- the walk over segment k: thread 0 of the CTA, with thread 32 bringing the windows of the
+// tables by bulk copies up to three windows ahead (every wait is bounded; one that runs out ends
+// the walk with an error). A step's chain is a shared-memory load and the addition that gives the
+// next load's address; the loop's own instructions (test, stores) cost as much as the chain unless
+// groups go in fours. Measured on the 1024 x 1024 DXT1 level, cycles per step: 124 with cp.async by
+// the other warps, a barrier per window and a test per group; 103 with bulk copies issued by the
+// walking thread and groups in fours; 72 so.
+constexpr uint32_t kWalkWaitLimit = 1u << 22;
+__device__ __forceinline__ bool walk_wait(uint32_t bar, uint32_t parity, const volatile uint32_t* walking = nullptr) {
+  uint32_t done = 0;
+  for (uint32_t i = 0; i < kWalkWaitLimit && !done && !(walking && !*walking); i++)
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
+  uint32_t v;
+  asm volatile("{\n.reg .u16 t;\nld.shared.u8 t, [%1];\ncvt.u32.u16 %0, t;\n}" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+  uint32_t v;
+  asm volatile("{\n.reg .u16 t;\nld.shared.u16 t, [%1];\ncvt.u32.u16 %0, t;\n}" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+template <bool REM>
+__device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t* status) {
+  using R = WalkRing<REM>;
+  const StreamJob& J = job.j;
+  const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
+  WalkState& st = *job.st;
+  const uint32_t tid = threadIdx.x, base = k * job.seg;
+  if (tid < kWMaxW / 32) S.bits[tid] = st.bits[tid];
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(wide_smem);
+  const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
+  const uint32_t windows = (job.seg + R::kWindow - 1) / R::kWindow, staged = job.cap / R::kWindow;
+  if (tid == 0) {
+    for (uint32_t i = 0; i < R::kSlots; i++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8 * i));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    S.walking = st.r < sh.rows ? 1u : 0u;
+  }
+  __syncthreads();
+  const size_t buf = (size_t)(k & 1u) * job.cap;
+  if (tid == 32) {
+    // the producer: window w into slot w & 3 once the walk has left window w - 4; it ends when the
+    // walk does (S.walking), after its copies have landed
+    volatile uint32_t* walking = &S.walking;
+    uint32_t w = 0;
+    for (; w < staged && *walking; w++) {
+      const uint32_t slot = w & (R::kSlots - 1), bar = full + 8 * slot;
+      if (w >= R::kSlots && !walk_wait(empty + 8 * slot, (w / R::kSlots - 1) & 1u, walking)) {
+        if (*walking) atomicMax(status, (uint32_t)kStWait);
+        break;
+      }
+      const bool mirror = slot == 0 && w > 0;
+      constexpr uint32_t kBytes = R::kWindow * (REM ? 28u : 20u);
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(mirror ? 2 * kBytes : kBytes)
+                   : "memory");
+      const size_t at = buf + (size_t)w * R::kWindow;
+      auto copy = [&](uint32_t dst, const void* src, uint32_t bytes) {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm0 + dst),
+                     "l"(src), "r"(bytes), "r"(bar)
+                     : "memory");
+      };
+      for (uint32_t to = slot; to <= R::kSlots; to += R::kSlots) {
+        copy(R::kO4 + to * R::kWindow * 16u, job.o4 + at, R::kWindow * 16u);
+        copy(R::kC4 + to * R::kWindow * 4u, job.c4 + at, R::kWindow * 4u);
+        if (REM) copy(R::kRem + to * R::kWindow * 8u, job.rem + at, R::kWindow * 8u);
+        if (!mirror) break;
+      }
+    }
+    // the last copies of each slot
+    for (uint32_t v = w > R::kSlots ? w - R::kSlots : 0u; v < w; v++)
+      if (!walk_wait(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u)) atomicMax(status, (uint32_t)kStWait);
+  }
+  if (tid) return;
+  uint32_t r = st.r, e = st.e, q = st.p - base, groups = st.groups;
+  if (r < sh.rows) {
+    const uint8_t* bits = reinterpret_cast<const uint8_t*>(S.bits);
+    uint8_t* bits_w = reinterpret_cast<uint8_t*>(S.bits);
+    const uint32_t o4 = sm0 + R::kO4, c4 = sm0 + R::kC4;
+    const uint2* RM = reinterpret_cast<const uint2*>(wide_smem + R::kRem);
+    const uint32_t left = job.bits > base ? job.bits - base : 0u;  // positions before the end of the stream
+    uint32_t* out = job.anchors + groups;
+    bool ok = walk_wait(full, 0u);
+    for (uint32_t w = 0; w < windows && ok && r < sh.rows; w++) {
+      if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u);
+      if (!ok) break;
+      const uint32_t lim = min(min((w + 1) * R::kWindow, job.seg), left);
+      // four groups of chunks may start while the last of them starts inside window w + 1
+      constexpr uint32_t kOver = 3u * 576u + 1u > R::kWindow ? 3u * 576u + 1u - R::kWindow : 0u;
+      const uint32_t lim_c = min(lim, (w + 1) * R::kWindow - kOver);
+      while (r < sh.rows && q < lim) {
+        if (!(r & 1u)) {
+          if (!(e & 15u) && e + 16 <= sh.W2 && q < lim_c) {
+            // a: shared address of the entry; z: what turns it into a position
+            uint32_t a = c4 + 4u * (q & R::kMask);
+            const uint32_t z = base + q - (a >> 2);
+            do {
+              const uint32_t a1 = a + lds_u16(a), a2 = a1 + lds_u16(a1), a3 = a2 + lds_u16(a2), a4 = a3 + lds_u16(a3);
+              const uint32_t b0 = lds_u8(a + 2), b1 = lds_u8(a1 + 2), b2 = lds_u8(a2 + 2), b3 = lds_u8(a3 + 2);
+              out[0] = z + (a >> 2);
+              out[1] = z + (a1 >> 2);
+              out[2] = z + (a2 >> 2);
+              out[3] = z + (a3 >> 2);
+              S.bits[e >> 4] = b0 | b1 << 8 | b2 << 16 | b3 << 24;
+              a = a4;
+              out += 4;
+              e += 16;
+              q = z + (a >> 2) - base;
+            } while (e + 16 <= sh.W2 && q < lim_c && a < c4 + 4u * R::kWindow * R::kSlots);
+          }
+          while (e + 4 <= sh.W2 && q < lim) {
+            if (!(e & 15u) && e + 16 <= sh.W2 && q < lim_c) break;
+            const uint32_t a = c4 + 4u * (q & R::kMask), t = lds_u16(a);
+            *out++ = base + q;
+            bits_w[e >> 2] = (uint8_t)lds_u8(a + 2);
+            q += t >> 2;
+            e += 4;
+          }
+          if (REM) {
+            while (e < sh.W2 && e + 4 > sh.W2 && q < lim) {
+              const uint32_t t = RM[q & R::kMask].y, s = ((e & 3u) * 2u) ^ 2u;
+              *out++ = base + q;
+              const uint32_t old = (e & 3u) ? bits[e >> 2] : 0u;
+              bits_w[e >> 2] = (uint8_t)(old | (t >> 16) << s);
+              q += t & 0xFFFFu;
+              e++;
+            }
+          }
+          if (e == sh.W2) { e = 0; r++; }
+        } else {
+          // (four groups of blocks are at most 1024 bits: the last of them starts inside window w + 1)
+          if (!(e & 15u) && e + 16 <= sh.W) {
+            uint32_t a = o4 + 16u * (q & R::kMask);
+            const uint32_t z = base + q - (a >> 4);  // the ring starts on 16 bytes: z + (address >> 4) is the position
+            uint32_t n = S.bits[e >> 5] >> (e & 16u);
+            do {
+              const uint32_t n0 = n & 15u, n1 = (n >> 4) & 15u, n2 = (n >> 8) & 15u, n3 = (n >> 12) & 15u;
+              const uint32_t a0 = a + n0;
+              const uint32_t a1 = lds_u8(a0) * 16u + (a + 16u + n1);
+              const uint32_t a2 = lds_u8(a1) * 16u + (a1 + 16u - n1 + n2);
+              const uint32_t a3 = lds_u8(a2) * 16u + (a2 + 16u - n2 + n3);
+              a = lds_u8(a3) * 16u + (a3 + 16u - n3);
+              e += 16;
+              n = S.bits[min(e, sh.W - 1u) >> 5] >> (e & 16u);
+              out[0] = (z + (a0 >> 4)) | n0 << kWalkPosBits;
+              out[1] = (z + (a1 >> 4)) | n1 << kWalkPosBits;
+              out[2] = (z + (a2 >> 4)) | n2 << kWalkPosBits;
+              out[3] = (z + (a3 >> 4)) | n3 << kWalkPosBits;
+              out += 4;
+              q = z + (a >> 4) - base;
+            } while (e + 16 <= sh.W && q < lim && a < o4 + 16u * R::kWindow * R::kSlots);
+          }
+          while (e + 4 <= sh.W && q < lim) {
+            if (!(e & 15u) && e + 16 <= sh.W) break;
+            const uint32_t nib = (bits[e >> 3] >> (e & 4u)) & 15u;
+            *out++ = (base + q) | nib << kWalkPosBits;
+            q += lds_u8(o4 + 16u * (q & R::kMask) + nib) + 1u;
+            e += 4;
+          }
+          if (REM && e < sh.W && e + 4 > sh.W && q < lim) {  // the row's last two blocks
+            const uint32_t nib = (bits[e >> 3] >> (e & 4u)) & 15u;
+            *out++ = (base + q) | nib << kWalkPosBits;
+            q += (RM[q & R::kMask].x >> (8u * (nib >> 2))) & 255u;
+            e += 2;
+          }
+          if (e == sh.W) { e = 0; r++; }
+        }
+      }
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * (w & (R::kSlots - 1))) : "memory");
+    }
+    *(volatile uint32_t*)&S.walking = 0u;
+    if (!ok) atomicMax(status, (uint32_t)kStWait);
+    if (k + 1 == job.segs && ok && r < sh.rows) {
+      // the stream has ended (a corrupt or truncated one): every further group starts in its zeros
+      const uint32_t zero = (uint32_t)(job.c4[buf + left] >> 16) & 255u;
+      while (r < sh.rows) {
+        if (!(r & 1u)) {
+          if (e + 4 <= sh.W2) {
+            bits_w[e >> 2] = (uint8_t)zero;
+            e += 4;
+          } else {
+            const uint32_t s = ((e & 3u) * 2u) ^ 2u, old = (e & 3u) ? bits[e >> 2] : 0u;
+            bits_w[e >> 2] = (uint8_t)(old | (zero & 3u) << s);
+            e++;
+          }
+          *out++ = job.bits;
+          if (e == sh.W2) { e = 0; r++; }
+        } else {
+          const uint32_t nib = (bits[e >> 3] >> (e & 4u)) & 15u;
+          *out++ = job.bits | nib << kWalkPosBits;
+          e = min(e + 4, sh.W);
+          if (e == sh.W) { e = 0; r++; }
+        }
+      }
+    }
+    groups = (uint32_t)(out - job.anchors);
+    for (uint32_t i = 0; i < kWMaxW / 32; i++) st.bits[i] = S.bits[i];
+  }
+  st.p = base + q;
+  st.r = r;
+  st.e = e;
+  st.groups = groups;
+  st.passed[k] = groups;
+}
+
+// ---- symbols of the groups passed in segment k, this CTA's share of them
+template <int KIND>
+__device__ __forceinline__ void walk_decode(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t part, uint32_t parts) {
+  constexpr bool colour = KIND == kKDxt1 || KIND == kKDxt5;
+  constexpr bool two = KIND == kKDxt5 || KIND == kKDxn, five = KIND == kKDxt5;
+  constexpr uint32_t sDB = five ? 3u : 1u, sSB = five ? 4u : 2u;
+  const StreamJob& J = job.j;
+  const uint32_t g0 = k ? job.st->passed[k - 1] : 0u, g1 = job.st->passed[k];
+  if (g0 + part * kWalkThreads >= g1) return;
+  const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
+  uint32_t* luts = reinterpret_cast<uint32_t*>(wide_smem);
+  walk_stage_models(J, luts, S);
+  __syncthreads();
+  const DevModel* mDA = J.models + (colour ? kMEp0 : kMEp1);
+  const DevModel* mSA = J.models + (colour ? kMSel0 : kMSel1);
+  uint32_t* plane_b = job.blocks + (size_t)sh.rows * sh.W;
+  uint32_t bad = 0;
+  for (uint32_t g = g0 + part * kWalkThreads + threadIdx.x; g < g1; g += parts * kWalkThreads) {
+    const uint32_t anchor = job.anchors[g], p = anchor & ((1u << kWalkPosBits) - 1u), nib = anchor >> kWalkPosBits;
+    const uint32_t pair = g / (sh.ge + sh.go), rem = g - pair * (sh.ge + sh.go);
+    // a bit reader in registers: `have` stream bits MSB first in acc, one word refills
+    uint32_t wi = p >> 5;
+    const uint32_t s = p & 31u;
+    uint32_t w0 = stream_word(J.src, J.src_size, wi), w1 = stream_word(J.src, J.src_size, wi + 1),
+             w2 = stream_word(J.src, J.src_size, wi + 2), w3 = stream_word(J.src, J.src_size, wi + 3);
+    uint64_t acc = (uint64_t)__funnelshift_l(w1, w0, s) << 32 | __funnelshift_l(w2, w1, s);
+    int have = 64;
+    wi += 4;  // w2, w3: the words after acc's; the next load is word wi
+    auto dec = [&](uint32_t slot, const DevModel* m) {
+      if (have <= 32) {
+        acc |= (uint64_t)__funnelshift_l(w3, w2, s) << (32 - have);
+        have += 32;
+        w2 = w3;
+        w3 = stream_word(J.src, J.src_size, wi++);
+      }
+      uint32_t len;
+      const uint32_t sym = code_sym((uint32_t)(acc >> 48), luts + (slot << kLutBits), S.aux[slot], m, nullptr, 0u, len, bad);
+      acc <<= len;
+      have -= (int)len;
+      return sym;
+    };
+    auto block = [&](uint32_t ref, uint32_t below, size_t at) {
+      uint32_t dA = 0, dB = 0;
+      if (!ref) {
+        dA = dec(1, mDA);
+        if (two) dB = dec(sDB, J.models + kMEp1);
+      }
+      const uint32_t sA = dec(2, mSA), sB = two ? dec(sSB, J.models + kMSel1) : 0u;
+      job.blocks[at] = ref | dA << 2 | sA << 16 | below << 30;
+      if (two) plane_b[at] = dB | sB << 16;
+    };
+    if (rem < sh.ge) {
+      const uint32_t full = sh.W2 / 4, x = rem < full ? 4 * rem : 4 * full + (rem - full), n = rem < full ? 4u : 1u;
+      size_t at = (size_t)pair * 2 * sh.W + 2 * x;
+      for (uint32_t c = 0; c < n; c++, at += 2) {
+        const uint32_t grp = dec(0, J.models + kMRef) & 0xFFu;
+        block(grp & 3u, (grp >> 2) & 3u, at);
+        block((grp >> 4) & 3u, grp >> 6, at + 1);
+      }
+    } else {
+      const uint32_t x = 4 * (rem - sh.ge), n = min(4u, sh.W - x);
+      const size_t at = (size_t)(pair * 2 + 1) * sh.W + x;
+      // nib: first two blocks in bits 2 and 3, the others in bits 0 and 1; set: deltas (reference 0)
+      for (uint32_t c = 0; c < n; c++) block(((nib >> (c ^ 2u)) & 1u) ^ 1u, 0u, at + c);
+    }
+  }
+  if (bad) atomicOr(&job.st->bad, 1u);
+}
+
+// ---- endpoint indices of the rows whose groups had all been decoded by the launch before: a row
+// at a time on four warps, a thread taking kPer neighbouring blocks of every row (so a block's
+// index in the row above is the thread's own), the rows' words staged in shared memory. A row is a
+// scan's latency (two shuffles' worth of warps and one barrier); with a block per thread on sixteen
+// warps and three words per operator it was their issue slots, 1,900 cycles a row of 256 blocks
+// against 1,000 now.
+constexpr uint32_t kResolveThreads = 128;
+__device__ __forceinline__ void resolve_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kResolveThreads) : "memory"); }
+__device__ __forceinline__ bool resolve_sync_or(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "n"(kResolveThreads)
+      : "memory");
+  return r != 0u;
+}
+
+template <bool TWO, uint32_t kPer>
+__device__ __forceinline__ void walk_resolve(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t* status) {
+  const StreamJob& J = job.j;
+  const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
+  WalkState& st = *job.st;
+  const uint32_t passed = st.passed[k], pairs = passed / (sh.ge + sh.go);
+  const uint32_t ready = 2 * pairs + (passed - pairs * (sh.ge + sh.go) >= sh.ge ? 1u : 0u);
+  uint32_t r = st.rows;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, W = sh.W;
+  const uint32_t nA = J.n_a, nB = J.n_b, nSA = J.n_sa, nSB = J.n_sb;
+  const uint32_t x0 = tid * kPer;  // rows are even: a pair of blocks is inside or outside
+  const uint32_t* plane_b = job.blocks + (size_t)sh.rows * W;
+  // the decoded blocks of as many rows as fit, staged
+  uint32_t* rows0 = reinterpret_cast<uint32_t*>(wide_smem) + 3 * kWMaxW;
+  const uint32_t most = (kWalkSmem / 4u - 3u * kWMaxW) / (W * (TWO ? 2u : 1u)) & ~1u;
+  // Indices are handled in pairs, A in the low half and B in the high half of a word. In the exact
+  // case (sizes of at most 2^14, deltas and indices below them) a sum of two is below 2^15, and its
+  // remainder is the smaller of it and, modulo 2^16, it less the size.
+  const uint32_t less = ((0u - nA) & 0xFFFFu) | (TWO ? (0u - nB) << 16 : 0u);
+  const bool never_exact = nA == 0 || nA > 16384u || (TWO && (nB == 0 || nB > 16384u));
+  auto add = [&](uint32_t u, uint32_t v) { return __viaddmin_u16x2(u + v, less, u + v); };
+  auto outside = [&](uint32_t u) { return (u & 0xFFFFu) >= nA || (TWO && (u >> 16) >= nB); };
+  const uint32_t below = (1u << lane) - 1u;
+  uint32_t ab[kPer], low[kPer];  // indices of the row above; its blocks' references for this row
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; i++) {
+    const uint32_t x = x0 + i;
+    ab[i] = x < W ? job.above[x] | (TWO ? (uint32_t)job.above[kWMaxW + x] << 16 : 0u) : 0u;
+    low[i] = (r & 1u) && x < W ? job.blocks[(size_t)(r - 1) * W + x] >> 30 : 0u;
+  }
+  if (tid == 0) S.carry[r & 1u] = st.carry;
+  resolve_sync();
+  bool badi = false;
+  uint32_t first = r, staged = 0, f = r / sh.H, y = r - f * sh.H;
+  for (; r < ready; r++) {
+    if (r == first + staged) {
+      first = r;
+      staged = min(most, ready - r);
+      resolve_sync();
+      auto stage = [&](const uint32_t* from, uint32_t* to) {
+        for (uint32_t i = tid; i < staged * (W / 2); i += kResolveThreads)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 2 * i)),
+                       "l"(from + 2 * i)
+                       : "memory");
+      };
+      stage(job.blocks + (size_t)r * W, rows0);
+      if (TWO) stage(plane_b + (size_t)r * W, rows0 + most * W);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      resolve_sync();
+    }
+    const uint32_t* row_a = rows0 + (r - first) * W;
+    const uint32_t* row_b = row_a + most * W;
+    const uint32_t cur = r & 1u;
+    uint32_t w0[kPer], w1[kPer], val[kPer], ref[kPer];
+    bool inexact = never_exact;
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i += 2) {
+      uint2 v = make_uint2(1u, 1u), u = make_uint2(0u, 0u);  // past the row: keep the running index
+      if (x0 + i < W) {
+        v = *reinterpret_cast<const uint2*>(row_a + x0 + i);
+        if (TWO) u = *reinterpret_cast<const uint2*>(row_b + x0 + i);
+      }
+      w0[i] = v.x;
+      w0[i + 1] = v.y;
+      w1[i] = u.x;
+      w1[i + 1] = u.y;
+    }
+    // A block adds its deltas to the running indices (reference 0), keeps them (1), or takes those of
+    // the row above. `mine`: what the thread's blocks add, or with `set` what they leave.
+    uint32_t mine = 0;
+    bool set = false;
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i++) {
+      ref[i] = x0 + i >= W ? 1u : cur ? low[i] : w0[i] & 3u;
+      low[i] = w0[i] >> 30;
+      val[i] = ref[i] == 0 ? ((w0[i] >> 2) & 0x3FFFu) | (TWO ? w1[i] << 16 : 0u) : ref[i] == 1 ? 0u : ab[i];
+      inexact |= ref[i] != 1 && outside(val[i]);
+      mine = ref[i] > 1 ? val[i] : add(mine, val[i]);
+      set |= ref[i] > 1;
+    }
+    // inclusive scan over the lanes, which starts anew at every lane that sets
+    const unsigned sets = __ballot_sync(0xFFFFFFFFu, set);
+    const int from = 31 - __clz((int)(sets & (below | 1u << lane)));  // the last such lane up to this one, or -1
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, mine, d);
+      if ((int)lane - d >= max(from, 0)) mine = add(mine, o);
+    }
+    if (lane == 31) {
+      S.scan[cur][warp][0] = mine;
+      S.scan[cur][warp][1] = sets;
+    }
+    uint32_t pre = __shfl_up_sync(0xFFFFFFFFu, mine, 1);  // of the lanes before
+    if (lane == 0) pre = 0;
+    const bool any_inexact = resolve_sync_or(inexact);
+    const uint32_t carry = S.carry[cur];
+    if (any_inexact || outside(carry)) {
+      // an index or a delta at or above its palette size: the reference's sequential rule, on one
+      // thread, over indices in shared memory
+      uint32_t* sAB = reinterpret_cast<uint32_t*>(wide_smem);
+      uint32_t* sR = sAB + kWMaxW;
+#pragma unroll
+      for (uint32_t i = 0; i < kPer; i++)
+        if (x0 + i < W) { sAB[x0 + i] = ab[i]; sR[x0 + i] = ref[i]; }
+      resolve_sync();
+      if (tid == 0) {
+        uint32_t iA = carry & 0xFFFFu, iB = carry >> 16;
+        for (uint32_t x = 0; x < W; x++) {
+          if (sR[x] == 0) {
+            iA += (row_a[x] >> 2) & 0x3FFFu;
+            if (iA >= nA) iA -= nA;
+            if (TWO) {
+              iB += row_b[x] & 0xFFFFu;
+              if (iB >= nB) iB -= nB;
+            }
+          } else if (sR[x] >= 2) {
+            iA = sAB[x] & 0xFFFFu;
+            iB = sAB[x] >> 16;
+          }
+          // the row above holds 16-bit indices: larger ones are corrupt in any case
+          if (iA > 0xFFFFu || iB > 0xFFFFu) badi = true;
+          iA &= 0xFFFFu;
+          iB &= 0xFFFFu;
+          sAB[x] = iA | iB << 16;
+        }
+        S.carry[cur ^ 1u] = iA | iB << 16;
+      }
+      resolve_sync();
+#pragma unroll
+      for (uint32_t i = 0; i < kPer; i++)
+        if (x0 + i < W) ab[i] = sAB[x0 + i];
+      resolve_sync();
+    } else {
+      uint32_t run = carry;
+#pragma unroll
+      for (uint32_t w = 0; w + 1 < kResolveThreads / 32; w++)
+        if (w < warp) run = S.scan[cur][w][1] ? S.scan[cur][w][0] : add(run, S.scan[cur][w][0]);
+      run = (sets & below) ? pre : add(run, pre);
+#pragma unroll
+      for (uint32_t i = 0; i < kPer; i++) ab[i] = run = ref[i] > 1 ? val[i] : add(run, val[i]);
+      if (x0 < W && x0 + kPer >= W) S.carry[cur ^ 1u] = run;  // positions past the row keep the last block's index
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i++) {
+      const uint32_t x = x0 + i;
+      const uint32_t sA = (w0[i] >> 16) & 0x3FFFu, sB = TWO ? w1[i] >> 16 : 0u;
+      if (x < W && (outside(ab[i]) || sA >= nSA || (TWO && sB >= nSB))) badi = true;
+      if (y < J.by && x < J.bx) {
+        const size_t at = ((size_t)f * J.by + y) * J.bx + x;
+        if (TWO) reinterpret_cast<uint64_t*>(J.rec)[at] = (uint64_t)((ab[i] & 0xFFFFu) | sA << 16) | (uint64_t)(ab[i] >> 16 | sB << 16) << 32;
+        else reinterpret_cast<uint32_t*>(J.rec)[at] = (ab[i] & 0xFFFFu) | sA << 16;
+      }
+    }
+    if (++y == sh.H) { y = 0; f++; }
+  }
+  if (badi) atomicOr(&st.bad, 2u);
+  resolve_sync();
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; i++)
+    if (x0 + i < W) {
+      job.above[x0 + i] = (uint16_t)ab[i];
+      if (TWO) job.above[kWMaxW + x0 + i] = (uint16_t)(ab[i] >> 16);
+    }
+  if (tid == 0) {
+    st.rows = ready;
+    st.carry = S.carry[ready & 1u];
+    const uint32_t bad = k + 1 == job.segs ? atomicOr(&st.bad, 0u) : 0u;
+    if (bad) atomicMax(status, (bad & 1u) ? (uint32_t)kStBadCode : (uint32_t)kStBadIndex);
+  }
+}
+template <bool TWO>
+__device__ __forceinline__ void walk_resolve_rows(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t* status) {
+  if (threadIdx.x >= kResolveThreads) return;
+  const uint32_t W = (job.j.bx + 1) & ~1u;
+  static_assert(8 * kResolveThreads == kWMaxW, "blocks of a thread");
+  if (W <= 2 * kResolveThreads) walk_resolve<TWO, 2>(job, S, k, status);
+  else if (W <= 4 * kResolveThreads) walk_resolve<TWO, 4>(job, S, k, status);
+  else walk_resolve<TWO, 8>(job, S, k, status);
+}
+
+// Launch `step` of a plan, over the first n jobs (the ones with work left; jobs are ordered by their
+// number of segments): CTAs [0, n) walk segment step - 1 of their level, [n, 2n) resolve rows from
+// segment step - 3, [2n, 2n + n * parts) decode the groups of segment step - 2, the others build
+// tables of segment `step` of the first nb jobs.
+__global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJob* __restrict__ jobs, uint32_t n,
+                                                                     uint32_t nb, uint32_t parts, uint32_t step,
+                                                                     uint32_t* status) {
+  __shared__ WalkShared S;
+  uint32_t b = blockIdx.x;
+  if (b < n) {
+    const WalkJob job = jobs[b];
+    const uint32_t k = step - 1;
+    if (step < 1 || k >= job.segs) return;
+    if (job.rem) walk_segment<true>(job, S, k, status); else walk_segment<false>(job, S, k, status);
+    return;
+  }
+  b -= n;
+  if (b < n) {
+    const WalkJob job = jobs[b];
+    const uint32_t k = step - 3;
+    if (step < 3 || k >= job.segs) return;
+    if (record_bytes(job.j.kind) == 8u) walk_resolve_rows<true>(job, S, k, status); else walk_resolve_rows<false>(job, S, k, status);
+    return;
+  }
+  b -= n;
+  if (b < n * parts) {
+    const WalkJob job = jobs[b / parts];
+    const uint32_t k = step - 2, part = b % parts;
+    if (step < 2 || k >= job.segs) return;
+    switch (job.j.kind) {
+      case kKDxt1: walk_decode<kKDxt1>(job, S, k, part, parts); break;
+      case kKDxt5: walk_decode<kKDxt5>(job, S, k, part, parts); break;
+      case kKDxn: walk_decode<kKDxn>(job, S, k, part, parts); break;
+      default: walk_decode<kKDxt5a>(job, S, k, part, parts); break;
+    }
+    return;
+  }
+  b -= n * parts;
+  uint32_t lo = 0, hi = nb;  // the last level whose first tile is at or before this one
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(&jobs[mid].tile0) <= b) lo = mid; else hi = mid;
+  }
+  const WalkJob job = jobs[lo];
+  if (step < job.segs) walk_build(job, S, step, b - job.tile0);
+}
+
 // Palette entry index, clamped so that records left unwritten by a stream the decoder rejected
 // as corrupt can never read outside the palette (valid records are already in range).
 __device__ __forceinline__ uint32_t clamp_idx(uint32_t i, uint32_t n) { return i < n ? i : 0u; }
@@ -1517,6 +2244,13 @@ struct Plan {
   uint32_t n_wide = 0;      // level streams for k_crn_decode_wide (one CTA each, largest first)
   uint32_t wide_smem = 0;   // its dynamic shared memory (the largest format's layout)
   size_t wide_ofs = 0;
+  uint32_t n_walk = 0;      // level streams for k_crn_decode_walk
+  uint32_t walk_steps = 0;  // its launches
+  struct WalkStep { uint32_t jobs, builds, tiles; };  // jobs with work left, jobs building, their builder CTAs
+  HVec<WalkStep> walk_step;
+  size_t walk_ofs = 0;
+  uint64_t walk_bytes = 0, walk_zero = 0;  // its scratch, and how much of that is cleared before the first launch
+  uint8_t* walk_scratch = nullptr;         // set by place_walk
   uint32_t rb_words = 2;    // largest row-buffer need of one texture job (words)
   uint32_t lut_words = 0;   // first-level tables staged per texture job (words)
   size_t stream_ofs = 0, expand_ofs = 0;
@@ -1538,6 +2272,12 @@ std::atomic<uint32_t> g_wide_min_blocks{0};
 // DXN), measured on GB300: the lane decoder's serial chain and one wide CTA's phase loop.
 constexpr double kLaneUsPerBlock = 0.20, kWideUsPerBlock = 0.03;
 constexpr uint32_t kWideMinBlocks = 256;  // smaller levels always go to the lane decoder
+// The walk decoder: its walk per block (as above), the tables of a bit of stream on all SMs, a launch.
+// Measured on GB300: the top level of a 1024 x 1024 DXT1 file 0.50 ms (13 launches, 46 us each while
+// it walks) against 1.74 ms wide; the largest level of a 24-texture batch, 2048 x 1024 DXT5, 1.2 ms
+// against 5.5 ms.
+constexpr double kWalkUsPerBlock = 0.0055, kWalkUsPerBit = 2e-5, kWalkLaunchUs = 3.0;
+constexpr double kWalkWaveUs = 2.0, kLaneLaunchUs = 8.0;  // a wave of CTAs of one launch; the lane decoder's launch
 
 uint64_t task_blocks(const LevelTask& t) {
   const LevelInfo& li = t.file->level[t.level];
@@ -1550,50 +2290,151 @@ bool wide_eligible(const LevelTask& t) {
   return ((li.blocks_x + 1) & ~1u) <= kWMaxW && t.src_size < (1u << 27);
 }
 
-// Per task: true if it goes to the wide decoder. The lane decoder runs every stream side by side
-// and finishes with its longest stream; the wide decoder runs `wide_slots` CTAs at once and
-// finishes when its queue drains, but never before its largest level. The two run one after the
-// other on the caller's stream. With the levels sorted by cost, the first k go wide for the k that
-// minimises wide time + lane time of level k + 1.
-HVec<bool> decide_wide(const HVec<LevelTask>& tasks, uint32_t wide_slots) {
-  HVec<bool> wide(tasks.size(), false);
+bool walk_eligible(const LevelTask& t) {
+  // anchors hold a bit position below 2^kWalkPosBits, past the stream's end by at most a segment's halo
+  return wide_eligible(t) && t.src_size < (1u << (kWalkPosBits - 3)) - 4096u;
+}
+
+// Where each task's level stream is decoded.
+enum Decoder : uint8_t { kLane = 0, kWide = 1, kWalk = 2 };
+
+// The lane decoder runs every stream side by side and finishes with its longest stream; the wide
+// decoder runs `wide_slots` CTAs at once and finishes when its queue drains, but never before its
+// largest level; the walk decoder (if `walk`) finishes with its largest level's walk or when the
+// SMs have built every level's tables, whichever is later, plus its launches. The three run one
+// after the other on the caller's stream. With the levels sorted by cost, the first k go to the
+// walk decoder and the next m wide, for the k and m that minimise the sum.
+HVec<uint8_t> decide_decoders(const HVec<LevelTask>& tasks, uint32_t wide_slots, bool walk) {
+  HVec<uint8_t> to(tasks.size(), (uint8_t)kLane);
   const uint32_t fixed = g_wide_min_blocks.load(std::memory_order_relaxed);
   if (fixed) {
-    for (size_t i = 0; i < tasks.size(); i++) wide[i] = wide_eligible(tasks[i]) && task_blocks(tasks[i]) >= fixed;
-    return wide;
+    for (size_t i = 0; i < tasks.size(); i++)
+      if (wide_eligible(tasks[i]) && task_blocks(tasks[i]) >= fixed) to[i] = kWide;
+    return to;
   }
-  HVec<std::pair<double, size_t>> cost;  // lane cost, task
-  double lane_rest = 0;                         // longest lane stream among the ineligible ones
+  HVec<std::pair<double, size_t>> cost;  // blocks (twice for two-endpoint formats), task
+  double lane_rest = 0;                  // longest lane stream among the ineligible ones
   for (size_t i = 0; i < tasks.size(); i++) {
     const double w = (tasks[i].file->kind == Kind::DXT5 || tasks[i].file->kind == Kind::DXN) ? 2.0 : 1.0;
     const double c = (double)task_blocks(tasks[i]) * w;
-    if (wide_eligible(tasks[i]) && task_blocks(tasks[i]) >= kWideMinBlocks) cost.push_back({c, i});
+    if (wide_eligible(tasks[i])) cost.push_back({c, i});
     else lane_rest = std::max(lane_rest, c * kLaneUsPerBlock);
   }
   std::stable_sort(cost.begin(), cost.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-  double best = std::max(lane_rest, cost.empty() ? 0.0 : cost[0].first * kLaneUsPerBlock), sum = 0;
+  const size_t n = cost.size();
+  const uint32_t sms = std::max<uint32_t>(1, wide_slots);  // a wide or a walk CTA has an SM to itself
   constexpr double kWideLaunchUs = 10.0;  // a second kernel launch and its fixed set-up
-  size_t best_k = 0;
-  for (size_t k = 1; k <= cost.size(); k++) {
-    sum += cost[k - 1].first * kWideUsPerBlock;
-    const double wide_t = std::max(cost[0].first * kWideUsPerBlock, sum / std::max<uint32_t>(1, wide_slots));
-    const double lane_t = std::max(lane_rest, k < cost.size() ? cost[k].first * kLaneUsPerBlock : 0.0);
-    if (wide_t + lane_t + kWideLaunchUs < best) {
-      best = wide_t + lane_t + kWideLaunchUs;
-      best_k = k;
+  double best = 1e300;
+  size_t best_k = 0, best_m = 0;
+  double walk_bits = 0, max_bits = 0;
+  for (size_t k = 0; k <= n; k++) {
+    double walk_t = 0;
+    if (k) {
+      const LevelTask& t = tasks[cost[k - 1].second];
+      if (!walk || !walk_eligible(t)) break;
+      walk_bits += 8.0 * t.src_size;
+      max_bits = std::max(max_bits, 8.0 * t.src_size);
+      walk_t = std::max(cost[0].first * kWalkUsPerBlock, walk_bits * kWalkUsPerBit) +
+               (std::min<double>(kWalkMaxSegments, max_bits / kWalkSegment) + 4) *
+                   (kWalkLaunchUs + kWalkWaveUs * (double)(3 * k / sms));
+    }
+    if (walk_t >= best) break;  // grows with k
+    double sum = 0;
+    for (size_t m = 0; k + m <= n; m++) {
+      if (m && task_blocks(tasks[cost[k + m - 1].second]) < kWideMinBlocks) break;
+      if (m) sum += cost[k + m - 1].first * kWideUsPerBlock;
+      const double wide_t = m ? std::max(cost[k].first * kWideUsPerBlock, sum / sms) + kWideLaunchUs : 0.0;
+      double lane_t = std::max(lane_rest, k + m < n ? cost[k + m].first * kLaneUsPerBlock : 0.0);
+      if (lane_t > 0) lane_t += kLaneLaunchUs;
+      if (walk_t + wide_t + lane_t < best) {
+        best = walk_t + wide_t + lane_t;
+        best_k = k;
+        best_m = m;
+      }
+      if (walk_t + wide_t >= best) break;
     }
   }
-  for (size_t k = 0; k < best_k; k++) wide[cost[k].second] = true;
-  return wide;
+  for (size_t i = 0; i < best_k; i++) to[cost[i].second] = kWalk;
+  for (size_t i = best_k; i < best_k + best_m; i++) to[cost[i].second] = kWide;
+  return to;
+}
+
+// The walk decoder's jobs: how each level is cut, and where its scratch lies (offsets in the
+// pointers until place_walk).
+void plan_walk(HVec<WalkJob>& jobs, Plan& p) {
+  uint64_t longest = 1;
+  for (const WalkJob& w : jobs) longest = std::max<uint64_t>(longest, w.bits);
+  const uint32_t cuts = (uint32_t)std::min<uint64_t>(kWalkMaxSegments, std::max<uint64_t>(1, (longest + kWalkSegment / 2) / kWalkSegment));
+  uint64_t o = 0;
+  auto take = [&](uint64_t bytes) {
+    const uint64_t at = o;
+    o += (bytes + 255) & ~(uint64_t)255;
+    return reinterpret_cast<uint8_t*>(at);
+  };
+  for (WalkJob& w : jobs) {
+    w.st = reinterpret_cast<WalkState*>(take(sizeof(WalkState)));
+    w.above = reinterpret_cast<uint16_t*>(take(2 * kWMaxW * sizeof(uint16_t)));
+  }
+  p.walk_zero = o;
+  for (WalkJob& w : jobs) {
+    const WalkShape sh = walk_shape(w.j.bx, w.j.by, w.j.faces);
+    w.tiles = (uint32_t)(((uint64_t)w.bits / cuts + 1 + kWalkHalo + kWalkTile - 1) / kWalkTile);
+    w.cap = w.tiles * kWalkTile;
+    w.seg = w.cap - kWalkHalo;
+    w.segs = w.bits / w.seg + 1;
+    p.walk_steps = std::max(p.walk_steps, w.segs + 3);
+    const bool two = record_bytes(w.j.kind) == 8u;
+    w.anchors = reinterpret_cast<uint32_t*>(take((uint64_t)sh.rows / 2 * (sh.ge + sh.go) * 4));
+    w.blocks = reinterpret_cast<uint32_t*>(take((uint64_t)sh.rows * sh.W * (two ? 8 : 4)));
+    w.o4 = reinterpret_cast<uint4*>(take(2ull * w.cap * 16));
+    w.c4 = reinterpret_cast<uint32_t*>(take(2ull * w.cap * 4));
+    w.rem = sh.W % 8 ? reinterpret_cast<uint2*>(take(2ull * w.cap * 8)) : nullptr;
+  }
+  std::stable_sort(jobs.begin(), jobs.end(), [](const WalkJob& a, const WalkJob& b) { return a.segs > b.segs; });
+  uint32_t tiles = 0;
+  for (WalkJob& w : jobs) {
+    w.tile0 = tiles;
+    tiles += w.tiles;
+  }
+  for (uint32_t step = 0; step < p.walk_steps; step++) {
+    Plan::WalkStep at{0, 0, 0};
+    for (const WalkJob& w : jobs) {
+      if (step && step < w.segs + 3) at.jobs++;
+      if (step < w.segs) { at.builds++; at.tiles += w.tiles; }
+    }
+    p.walk_step.push_back(at);
+  }
+  p.n_walk = (uint32_t)jobs.size();
+  p.walk_bytes = o;
+}
+
+// Rebases the walk jobs of a plan's image to their scratch (p.walk_bytes bytes, 256-byte aligned).
+void place_walk(Plan& p, uint8_t* scratch) {
+  p.walk_scratch = scratch;
+  WalkJob* jobs = reinterpret_cast<WalkJob*>(p.image.data() + p.walk_ofs);
+  auto move = [&](auto*& q) { q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(scratch + reinterpret_cast<uintptr_t>(q)); };
+  for (uint32_t i = 0; i < p.n_walk; i++) {
+    WalkJob& w = jobs[i];
+    const bool rem = w.rem != nullptr;
+    move(w.st);
+    move(w.above);
+    move(w.anchors);
+    move(w.blocks);
+    move(w.o4);
+    move(w.c4);
+    if (rem) move(w.rem);
+  }
 }
 
 // false if a texture job would not fit the decoder (more than 32 levels or rows too wide).
 // `wide_slots`: CTAs of k_crn_decode_wide resident at once on the device (wide_slots()).
-bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots) {
+// `walk`: the plan may use the walk decoder (its scratch is the caller's to place, place_walk).
+bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots, bool walk) {
   HVec<TexJob> items;
   HVec<HVec<StreamJob>> item_streams;
   HVec<StreamJob> wide;
-  const HVec<bool> to_wide = decide_wide(tasks, wide_slots);
+  HVec<WalkJob> walks;
+  const HVec<uint8_t> to = decide_decoders(tasks, wide_slots, walk);
   for (size_t i = 0; i < tasks.size();) {
     size_t k = i;
     while (k < tasks.size() && tasks[k].item == tasks[i].item) k++;
@@ -1620,8 +2461,15 @@ bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots) {
       j.n_b = tasks[t].pal.n_aep;
       j.n_sa = colour ? tasks[t].pal.n_csel : tasks[t].pal.n_asel;
       j.n_sb = tasks[t].pal.n_asel;
-      if (to_wide[t]) {
+      if (to[t] == kWide) {
         wide.push_back(j);
+        continue;
+      }
+      if (to[t] == kWalk) {
+        WalkJob w{};
+        w.j = j;
+        w.bits = 8u * j.src_size;
+        walks.push_back(w);
         continue;
       }
       j.rb_ofs = rb;
@@ -1646,6 +2494,8 @@ bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots) {
   std::stable_sort(wide.begin(), wide.end(), [](const StreamJob& a, const StreamJob& b) {
     return (uint64_t)a.bx * a.by * a.faces * record_bytes(a.kind) > (uint64_t)b.bx * b.by * b.faces * record_bytes(b.kind);
   });
+  std::stable_sort(walks.begin(), walks.end(), [](const WalkJob& a, const WalkJob& b) { return a.bits > b.bits; });
+  plan_walk(walks, p);
   for (const StreamJob& j : wide) p.wide_smem = std::max(p.wide_smem, wide_layout(models_used(j.kind)).total);
   // largest textures first: the persistent warps then finish at about the same time
   HVec<size_t> order(items.size());
@@ -1693,7 +2543,8 @@ bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots) {
   p.stream_ofs = al(sizeof(TexJob) * it_sorted.size());
   p.expand_ofs = p.stream_ofs + al(sizeof(StreamJob) * sj.size());
   p.wide_ofs = p.expand_ofs + al(sizeof(ExpandJob) * ej.size());
-  size_t end = p.wide_ofs + al(sizeof(StreamJob) * wide.size());
+  p.walk_ofs = p.wide_ofs + al(sizeof(StreamJob) * wide.size());
+  size_t end = p.walk_ofs + al(sizeof(WalkJob) * walks.size());
   for (int ts = 0; ts < kTileSizes; ts++) {
     p.tile_ofs[ts] = end;
     p.tile_ctas[ts] = (uint32_t)tiles[ts].size();
@@ -1704,6 +2555,7 @@ bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots) {
   std::memcpy(p.image.data() + p.stream_ofs, sj.data(), sizeof(StreamJob) * sj.size());
   std::memcpy(p.image.data() + p.expand_ofs, ej.data(), sizeof(ExpandJob) * ej.size());
   if (!wide.empty()) std::memcpy(p.image.data() + p.wide_ofs, wide.data(), sizeof(StreamJob) * wide.size());
+  if (!walks.empty()) std::memcpy(p.image.data() + p.walk_ofs, walks.data(), sizeof(WalkJob) * walks.size());
   for (int ts = 0; ts < kTileSizes; ts++)
     std::memcpy(p.image.data() + p.tile_ofs[ts], tiles[ts].data(), sizeof(uint2) * tiles[ts].size());
   return true;
@@ -1736,6 +2588,9 @@ int decode_device(const DecodeDevice** out) {
     if ((e = cudaFuncSetAttribute(k_crn_decode_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)wide_layout(5).total)) != cudaSuccess)
       return cuda_check(e, "wide decoder shared memory attribute");
+    if ((e = cudaFuncSetAttribute(k_crn_decode_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem)) !=
+        cudaSuccess)
+      return cuda_check(e, "walk decoder shared memory attribute");
     for (int v = 0; v < kExpandVariants; v++)
       if ((kVariantStage[v] || kVariantTmaBytes[v]) &&
           (e = cudaFuncSetAttribute(kExpandKernels[v], cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1789,8 +2644,19 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
   const TexJob* tj = reinterpret_cast<const TexJob*>(d_jobs);
   const StreamJob* sj = reinterpret_cast<const StreamJob*>(d_jobs + p.stream_ofs);
   const ExpandJob* ej = reinterpret_cast<const ExpandJob*>(d_jobs + p.expand_ofs);
-  if (decode && (p.n_item || p.n_wide)) {
+  if (decode && (p.n_item || p.n_wide || p.n_walk)) {
     if ((e = cudaMemsetAsync(words, 0, 8, s)) != cudaSuccess) return cuda_check(e, "clear work counter");
+  }
+  if (decode && p.n_walk) {
+    const WalkJob* kj = reinterpret_cast<const WalkJob*>(d_jobs + p.walk_ofs);
+    if ((e = cudaMemsetAsync(p.walk_scratch, 0, p.walk_zero, s)) != cudaSuccess) return cuda_check(e, "clear walk state");
+    for (uint32_t step = 0; step < p.walk_steps; step++) {
+      const Plan::WalkStep& at = p.walk_step[step];
+      const uint32_t parts = at.jobs ? std::max(1u, 16u / at.jobs) : 0;  // decoder CTAs of a level
+      k_crn_decode_walk<<<at.jobs * (2 + parts) + at.tiles, kWalkThreads, kWalkSmem, s>>>(kj, at.jobs, at.builds, parts,
+                                                                                           step, words + 1);
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_crn_decode_walk");
   }
   if (decode && p.n_wide) {
     const StreamJob* wj = reinterpret_cast<const StreamJob*>(d_jobs + p.wide_ofs);
@@ -1817,10 +2683,53 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
 
 int status_to_rc(uint32_t st) {
   if (!st) return CRNGPU_OK;
+  if (st == kStWait) { set_error("a wait of the transcoder timed out"); return CRNGPU_E_DEVICE; }
   set_error(st == kStBadCode ? "corrupt block stream (no such prefix code)"
                              : "corrupt block stream (palette index out of range)");
   return CRNGPU_E_CORRUPT;
 }
+
+// The walk decoder's scratch of one call: stream-ordered memory from a per-device pool, given back
+// in stream order. The pool keeps at most kWalkPoolBytes between calls.
+constexpr uint64_t kWalkPoolBytes = 128ull << 20;
+struct WalkScratch {
+  cudaStream_t s;
+  void* ptr = nullptr;
+  explicit WalkScratch(cudaStream_t stream) : s(stream) {}
+  WalkScratch(const WalkScratch&) = delete;
+  ~WalkScratch() {
+    if (ptr) cudaFreeAsync(ptr, s);
+  }
+  int get(uint64_t bytes) {
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_check(e, "cudaGetDevice");
+    if (dev < 0 || dev >= 64) { set_error("device index out of range"); return CRNGPU_E_PARAM; }
+    cudaMemPool_t pool;
+    {
+      std::lock_guard<std::mutex> lock(device_setup_mutex());
+      if (!pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t made;
+        if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess) return cuda_check(e, "create decode pool");
+        uint64_t keep = kWalkPoolBytes;
+        if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
+          return cuda_check(e, "decode pool attribute");
+        pools[dev] = made;
+      }
+      pool = pools[dev];
+    }
+    if ((e = cudaMallocFromPoolAsync(&ptr, bytes, pool, s)) != cudaSuccess) {
+      ptr = nullptr;
+      return cuda_check(e, "alloc decode scratch");
+    }
+    return CRNGPU_OK;
+  }
+};
 
 // Decodes and expands a list of levels of one context (destinations device memory), then
 // reads the status word back (synchronises `s`).
@@ -1839,7 +2748,12 @@ int run_levels(UnpackContext* c, HVec<LevelTask>& tasks, cudaStream_t s) {
   uint32_t slots = 0;
   int rc0 = wide_slots(&slots);
   if (rc0 != CRNGPU_OK) return rc0;
-  if (!make_plan(tasks, p, slots)) { set_error("too many levels in one texture job"); return CRNGPU_E_PARAM; }
+  if (!make_plan(tasks, p, slots, true)) { set_error("too many levels in one texture job"); return CRNGPU_E_PARAM; }
+  WalkScratch scratch(s);
+  if (p.n_walk) {
+    if ((rc0 = scratch.get(p.walk_bytes)) != CRNGPU_OK) return rc0;
+    place_walk(p, static_cast<uint8_t*>(scratch.ptr));
+  }
   if ((e = c->d_jobs.ensure(p.image.size() + 16)) != cudaSuccess) return cuda_check(e, "alloc jobs");
   if ((e = cudaMemcpyAsync(c->d_jobs.ptr, p.image.data(), p.image.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
     return cuda_check(e, "copy jobs");
@@ -2025,7 +2939,7 @@ struct UnpackBatch : HostObject {
   uint32_t magic = 0x42415443u;
   int device = -1;
   Plan plan;
-  DevBuf d_jobs, d_records, d_words;
+  DevBuf d_jobs, d_records, d_words, d_walk;
   uint32_t words_host[2] = {0, 0};
   cudaGraphExec_t graph = nullptr;
   bool decoded = false;
@@ -2161,7 +3075,11 @@ extern "C" crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
   for (LevelTask& t : tasks) t.rec = static_cast<uint8_t*>(b->d_records.ptr) + reinterpret_cast<uintptr_t>(t.rec);
   uint32_t slots = 0;
   if (wide_slots(&slots) != CRNGPU_OK) return nullptr;
-  if (!make_plan(tasks, b->plan, slots)) { set_error("too many levels in one batch item"); return nullptr; }
+  if (!make_plan(tasks, b->plan, slots, true)) { set_error("too many levels in one batch item"); return nullptr; }
+  if (b->plan.n_walk) {
+    if ((e = b->d_walk.ensure(b->plan.walk_bytes)) != cudaSuccess) { cuda_check(e, "alloc decode scratch"); return nullptr; }
+    place_walk(b->plan, static_cast<uint8_t*>(b->d_walk.ptr));
+  }
   if ((e = b->d_jobs.ensure(b->plan.image.size() + 16)) != cudaSuccess) { cuda_check(e, "alloc jobs"); return nullptr; }
   if ((e = cudaMemcpy(b->d_jobs.ptr, b->plan.image.data(), b->plan.image.size(), cudaMemcpyHostToDevice)) !=
       cudaSuccess) {
@@ -2452,7 +3370,7 @@ extern "C" int crngpu_unpack_level_noalloc(const void* crn_data, uint32_t crn_si
   Plan p;
   uint32_t slots = 0;
   if ((rc = wide_slots(&slots)) != CRNGPU_OK) return rc;
-  if (!make_plan({t}, p, slots)) { set_error("bad level"); return CRNGPU_E_PARAM; }
+  if (!make_plan({t}, p, slots, false)) { set_error("bad level"); return CRNGPU_E_PARAM; }
   const size_t need = o_jobs + al(p.image.size());
   if (need > kNoAllocScratchBytes) {
     set_error("level needs " + std::to_string(need) + " bytes of scratch; the allocation-free entry point has " +

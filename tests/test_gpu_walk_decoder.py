@@ -1,0 +1,123 @@
+"""The transcoder's walk decoder (the largest levels of a plan) against the lane decoder, which has
+one serial chain per level: rows that are and are not multiples of eight blocks (row ends of one,
+two and three chunks, of two blocks), several table segments, every format, cube maps, batches, and
+streams cut short or overwritten (the status and every byte that the two write)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def cg():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import crunch2_gb300
+    crunch2_gb300.lib()
+    return crunch2_gb300
+
+
+def texture(fmt, w, h, seed):
+    from crunch2_gb300 import texgen
+    if fmt == "dxn":
+        return texgen.normal_map(w, h, seed)
+    return texgen.colour_texture(w, h, seed, with_alpha_noise=fmt != "dxt1")
+
+
+def make(cg, fmt, w, h, seed, levels=3, faces=1, quality=128):
+    from crunch2_gb300 import texgen
+    f = {"dxt1": cg.FMT_DXT1, "dxt5": cg.FMT_DXT5, "dxn": cg.FMT_DXN_XY, "dxt5a": cg.FMT_DXT5A}[fmt]
+    return cg.compress_crn([texgen.mip_chain(texture(fmt, w, h, seed + i), levels) for i in range(faces)], f, quality)
+
+
+def decode(cg, crn, split, levels=None):
+    cg.set_decode_split(split)
+    try:
+        with cg.unpack_begin(crn) as ctx:
+            n = levels or ctx.levels
+            out = torch.full((sum(ctx.level_bytes(l) for l in range(n)),), 0xCD, dtype=torch.uint8, device="cuda")
+            try:
+                ctx.unpack_levels(0, n, out=out)
+                code = 0
+            except cg.CrnGpuError as e:
+                code = e.code
+            torch.cuda.synchronize()
+            return code, out.cpu().numpy()
+    finally:
+        cg.set_decode_split(cg.DECODE_SPLIT_DEFAULT)
+
+
+@pytest.mark.parametrize("fmt,w,h,faces", [
+    ("dxt1", 512, 512, 1), ("dxt5", 256, 320, 1), ("dxn", 264, 200, 1), ("dxt5a", 260, 260, 1),
+    ("dxt1", 1020, 90, 1), ("dxt5", 332, 180, 1), ("dxt1", 333, 444, 1), ("dxn", 148, 257, 1),
+    ("dxt1", 128, 128, 6), ("dxt5", 4096, 32, 1),
+])
+def test_walk_matches_lane(cg, fmt, w, h, faces):
+    crn = make(cg, fmt, w, h, w + h, faces=faces)
+    lane = decode(cg, crn, cg.DECODE_LANE_ONLY)
+    assert lane[0] == 0
+    walk = decode(cg, crn, cg.DECODE_SPLIT_DEFAULT)
+    assert walk[0] == 0 and np.array_equal(walk[1], lane[1])
+
+
+@pytest.mark.parametrize("fmt,quality", [("dxt1", 255), ("dxt5", 192)])
+def test_many_segments(cg, fmt, quality):
+    crn = make(cg, fmt, 1024, 768, 5, levels=1, quality=quality)
+    lane = decode(cg, crn, cg.DECODE_LANE_ONLY)
+    walk = decode(cg, crn, cg.DECODE_SPLIT_DEFAULT)
+    assert lane[0] == walk[0] == 0 and np.array_equal(walk[1], lane[1])
+
+
+@pytest.mark.parametrize("fmt,w", [("dxt1", 512), ("dxt5", 300)])
+@pytest.mark.parametrize("damage", ["cut", "zeros", "ones", "noise"])
+def test_damaged_streams(cg, fmt, w, damage):
+    """A level stream overwritten from a point on: the file's own level 0 lies before the others."""
+    crn = bytearray(make(cg, fmt, w, 512, 9, levels=1))
+    tail = len(crn) // 3
+    rng = np.random.default_rng(1)
+    fill = {"cut": b"\0" * tail, "zeros": b"\0" * tail, "ones": b"\xff" * tail,
+            "noise": rng.integers(0, 256, tail, np.uint8).tobytes()}[damage]
+    crn[len(crn) - tail:] = fill
+    if damage == "cut":  # the stream ends early: segmented entry with a shorter buffer
+        crn = bytes(make(cg, fmt, w, 512, 9, levels=1))
+        with cg.unpack_begin(crn) as ctx:
+            size = ctx.level_bytes(0)
+        outs = []
+        for split in (cg.DECODE_LANE_ONLY, cg.DECODE_SPLIT_DEFAULT):
+            cg.set_decode_split(split)
+            with cg.unpack_begin(crn) as ctx:
+                out = torch.full((size,), 0xCD, dtype=torch.uint8, device="cuda")
+                import ctypes
+                faces = (ctypes.c_void_p * 1)(out.data_ptr())
+                half = torch.from_numpy(np.frombuffer(crn[-len(crn) // 2:], np.uint8)[:len(crn) // 3].copy()).cuda()
+                pad = torch.cat([half, torch.zeros(64, dtype=torch.uint8, device="cuda")])
+                rc = cg.lib().crngpu_unpack_level_segmented(ctx.handle, pad.data_ptr(), half.numel(), faces, size, 0, 0,
+                                                            cg.MEM_DEVICE, None)
+                torch.cuda.synchronize()
+                outs.append((rc, out.cpu().numpy()))
+            cg.set_decode_split(cg.DECODE_SPLIT_DEFAULT)
+        lane, walk = outs
+    else:
+        lane, walk = (decode(cg, bytes(crn), s) for s in (cg.DECODE_LANE_ONLY, cg.DECODE_SPLIT_DEFAULT))
+    assert walk[0] == lane[0]
+    assert np.array_equal(walk[1], lane[1])
+
+
+def test_batch_of_walks(cg):
+    specs = [("dxt1", 512, 256), ("dxt5", 300, 300), ("dxn", 256, 512), ("dxt1", 130, 260), ("dxt1", 64, 64)]
+    crns = [make(cg, f, w, h, 20 + i) for i, (f, w, h) in enumerate(specs)]
+    want = [decode(cg, c, cg.DECODE_LANE_ONLY)[1] for c in crns]
+    ctxs = [cg.unpack_begin(c) for c in crns]
+    outs = [torch.zeros(len(w), dtype=torch.uint8, device="cuda") for w in want]
+    with cg.UnpackBatch([(c, 0, c.levels, o) for c, o in zip(ctxs, outs)]) as b:
+        for graph in (False, True, True):
+            for o in outs:
+                o.zero_()
+            b.launch(use_graph=graph)
+            b.status()
+            for o, w in zip(outs, want):
+                assert np.array_equal(o.cpu().numpy(), w)
+    for c in ctxs:
+        c.close()
