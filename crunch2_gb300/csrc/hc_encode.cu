@@ -1,7 +1,7 @@
 // Clustered ("hierarchical") DXT1 compression on the GPU: crnlib's dxt_hc
 // (crnlib/crn_dxt_hc.cpp:97-316) restated as batched kernels.
 //
-//   k_hc_tiles        per 2x2-block chunk: the nine candidate tiles (four blocks, two 8x4, two 4x8,
+//   k_hc_tile_*       per 2x2-block chunk: the nine candidate tiles (four blocks, two 8x4, two 4x8,
 //                     the 8x8 chunk) are compressed with the dxt_fast colour compressor and scored;
 //                     of the eight tile layouts the best PSNR minus a per-layout derating wins
 //                     (determine_tiles_task, :386-561); each chosen tile gets its two-colour
@@ -469,41 +469,50 @@ __host__ __device__ uint32_t fast_alpha_error(int n, const uint32_t* px, int com
   return err;
 }
 
+#ifdef __CUDACC__
 // dxt5_endpoint_optimizer::compute at quality Normal with 8-value blocks only, for the tile
 // decision (crn_dxt_hc.cpp:475-490): the smallest error over all pairs of the tile's unique
-// values (crnlib/crn_dxt5a.cpp:40-100, 198-262).
-__host__ __device__ uint32_t alpha_tile_error(int n, const uint32_t* px, int comp) {
-  uint8_t uv[64];
-  uint32_t uw[64];
+// values (crnlib/crn_dxt5a.cpp:40-100, 198-262), a warp per tile. A pair's eight values are the
+// same set either way round, so the pairs are taken over the sorted values, a lane per pair; a lane
+// leaves a pair once its error is above the least that it has seen. hist: 256 words of the warp's
+// own, zero before and after; val: its 64 (value | pixels << 8).
+__device__ __forceinline__ uint32_t alpha_tile_error(int n, const uint32_t* px, uint32_t* hist, uint32_t* val) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (int i = (int)lane; i < n; i += 32) atomicAdd(&hist[px[i]], 1u);
+  __syncwarp();
   int U = 0;
-  for (int i = 0; i < n; i++) {
-    const uint8_t a = (uint8_t)((px[i] >> (8 * comp)) & 255u);
-    int k = 0;
-    while (k < U && uv[k] != a) k++;
-    if (k == U) { uv[U] = a; uw[U] = 0; U++; }
-    uw[k]++;
-  }
-  if (U == 1) return 0;
-  unsigned long long best = ~0ull;
-  for (int i = 0; i < U - 1; i++) {
-    for (int j = i + 1; j < U; j++) {
-      const int l = uv[i], h = uv[j];
-      const int v[8] = {l, h, (l * 6 + h) / 7, (l * 5 + h * 2) / 7, (l * 4 + h * 3) / 7, (l * 3 + h * 4) / 7,
-                        (l * 2 + h * 5) / 7, (l + h * 6) / 7};
-      unsigned long long e = 0;
-      for (int u = 0; u < U && e <= best; u++) {
-        int bd = 0x7FFFFFFF;
-        for (int k = 0; k < 8; k++) {
-          const int d = (int)uv[u] - v[k];
-          bd = min(bd, d * d);
-        }
-        e += (unsigned long long)bd * uw[u];
-      }
-      if (e < best) best = e;
+  for (uint32_t base = 0; base < 256; base += 32) {
+    const uint32_t c = hist[base + lane];
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, c != 0);
+    if (c) {
+      val[U + __popc(m & ((1u << lane) - 1u))] = (base + lane) | c << 8;
+      hist[base + lane] = 0;
     }
+    U += __popc(m);
   }
-  return (uint32_t)best;
+  __syncwarp();
+  if (U == 1) return 0;
+  uint32_t best = 0xFFFFFFFFu;
+  const int pairs = U * (U - 1) / 2;
+  int i = 0, row = 0;  // pair p is (i, i + 1 + p - row)
+  for (int p = (int)lane; p < pairs; p += 32) {
+    while (p >= row + U - 1 - i) row += U - 1 - i++;
+    const int l = (int)(val[i] & 255u), h = (int)(val[i + 1 + p - row] & 255u);
+    const int v[8] = {l, h, (l * 6 + h) / 7, (l * 5 + h * 2) / 7, (l * 4 + h * 3) / 7, (l * 3 + h * 4) / 7,
+                      (l * 2 + h * 5) / 7, (l + h * 6) / 7};
+    uint32_t e = 0;
+    for (int u = 0; u < U && e <= best; u++) {
+      const uint32_t x = val[u];
+      int bd = 255;
+#pragma unroll
+      for (int k = 0; k < 8; k++) bd = min(bd, abs((int)(x & 255u) - v[k]));
+      e += (uint32_t)(bd * bd) * (x >> 8);
+    }
+    best = min(best, e);
+  }
+  return __reduce_min_sync(0xFFFFFFFFu, best);
 }
+#endif
 
 // split_vectors<vec1F> (crn_tree_clusterizer.h:573-753) for up to 64 weighted values: the two
 // centroids of a 1-D 2-means split seeded by the furthest/opposite values.
@@ -586,16 +595,22 @@ __host__ __device__ __forceinline__ uint32_t ld_px(const uint32_t* p) {
 #endif
 }
 
-__host__ __device__ __forceinline__ void chunk_pixels(const uint32_t* __restrict__ blocks, uint32_t b, uint32_t width,
-                                                      uint32_t* px /* 128 */) {
-  const uint32_t bl[4] = {b, b + width, b + 1, b + width + 1};  // [0..63]: TL, BL, TR, BR blocks
-  for (int q = 0; q < 4; q++)
-    for (int i = 0; i < 16; i++) px[q * 16 + i] = ld_px(blocks + (size_t)bl[q] * 16 + i);
-  // [64..127]: top 8x4 then bottom 8x4, row-major (t & 32: lower blocks, t & 4: right block)
-  for (int t = 0; t < 64; t += 4) {
-    const uint32_t blk = b + ((t & 32) ? width : 0) + ((t & 4) ? 1 : 0);
-    const int row = (t >> 1) & 12;
-    for (int i = 0; i < 4; i++) px[64 + t + i] = ld_px(blocks + (size_t)blk * 16 + row + i);
+// Pixels [ofs, ofs + n) of a chunk's 128-pixel image (both multiples of four): its blocks TL, BL, TR,
+// BR, then the whole chunk row by row (t & 32: lower blocks, t & 4: right block).
+__host__ __device__ __forceinline__ void chunk_pixels(const uint32_t* __restrict__ blocks, const Chunk& ch, int ofs, int n,
+                                                      uint32_t* px) {
+  for (int i = 0; i < n; i += 4) {
+    const int at = ofs + i;
+    uint32_t blk = ch.b;
+    int src = at & 15;
+    if (at < 64) {
+      blk += ((at & 16) ? ch.width : 0u) + ((at & 32) ? 1u : 0u);
+    } else {
+      const int t = at - 64;
+      blk += ((t & 32) ? ch.width : 0u) + ((t & 4) ? 1u : 0u);
+      src = (t >> 1) & 12;
+    }
+    for (int k = 0; k < 4; k++) px[i + k] = ld_px(blocks + (size_t)blk * 16 + src + k);
   }
 }
 
@@ -635,27 +650,64 @@ __host__ __device__ void palettize(const uint32_t* px, int n, bool perc, float* 
   for (int k = 0; k < 6; k++) out6[k] = res[k];
 }
 
-// One chunk of determine_tiles_task (crn_dxt_hc.cpp:386-561): tile errors, layout choice, the
-// chosen tiles' colour vec6 / alpha vec2, and each block's tile slot and layout. Returns the layout.
-__host__ __device__ int hc_tile_chunk(const uint32_t* __restrict__ blocks, uint32_t c, const Chunk& ch,
-                                      const float* __restrict__ derating, const float* __restrict__ level_weight,
-                                      bool perceptual, const SolidTables* __restrict__ st, const TileCfg& cfg,
-                                      Tile* __restrict__ tiles, uint32_t* __restrict__ block_tile,
-                                      uint8_t* __restrict__ block_enc) {
+// determine_tiles_task (crn_dxt_hc.cpp:386-561) in three steps: the errors of every chunk's nine
+// tiles (k_hc_tile_errors, and k_hc_alpha_errors for the alpha channels' pair search), the chunk's
+// layout from them (k_hc_tile_layout), and the chosen tiles' vectors (k_hc_tile_vectors). A thread
+// has one tile (errors: all of a warp's tiles the same size), not one chunk: with a thread per chunk
+// a 333 x 180 DXT5 chain was 21 CTAs of two warps, 4.8 ms; now TBD. The tile errors are
+// [channel][tile][chunk].
+__global__ void __launch_bounds__(64) k_hc_tile_errors(const uint32_t* __restrict__ blocks, const Chunk* __restrict__ chunks,
+                                                       uint32_t nchunks, const SolidTables* __restrict__ st, TileCfg cfg,
+                                                       uint32_t* __restrict__ terr) {
   const uint8_t tile_ofs[9] = HC_TILE_OFS;
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nchunks) return;
+  const int t = blockIdx.y, n = 16 << (t >> 2);
+  uint32_t px[64];
+  chunk_pixels(blocks, chunks[c], tile_ofs[t], n, px);
+  if (cfg.has_color) terr[(size_t)t * nchunks + c] = fast_tile_error(n, px, st);
+  if (cfg.qdxt)
+    for (int a = 0; a < cfg.num_alpha; a++) terr[((size_t)(1 + a) * 9 + t) * nchunks + c] = fast_alpha_error(n, px, cfg.comp[a]);
+}
+
+// a warp per chunk, blockIdx.y: tile, blockIdx.z: alpha channel
+constexpr int kAlphaErrWarps = 8;
+__global__ void __launch_bounds__(kAlphaErrWarps * 32) k_hc_alpha_errors(const uint32_t* __restrict__ blocks,
+                                                                         const Chunk* __restrict__ chunks,
+                                                                         uint32_t nchunks, TileCfg cfg,
+                                                                         uint32_t* __restrict__ terr) {
+  __shared__ uint32_t s_hist[kAlphaErrWarps][256], s_px[kAlphaErrWarps][64], s_val[kAlphaErrWarps][64];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, c = blockIdx.x * kAlphaErrWarps + warp;
+  if (c >= nchunks) return;  // whole warps
+  const int t = blockIdx.y, n = 16 << (t >> 2), comp = cfg.comp[blockIdx.z];
+  for (uint32_t i = lane; i < 256; i += 32) s_hist[warp][i] = 0;
+  const Chunk ch = chunks[c];
+  for (int i = 4 * (int)lane; i < n; i += 128) {
+    uint32_t px[4];
+    chunk_pixels(blocks, ch, c_tile_ofs[t] + i, 4, px);
+    for (int k = 0; k < 4; k++) s_px[warp][i + k] = (px[k] >> (8 * comp)) & 255u;
+  }
+  __syncwarp();
+  const uint32_t err = alpha_tile_error(n, s_px[warp], s_hist[warp], s_val[warp]);
+  if (lane == 0) terr[((size_t)(1 + blockIdx.z) * 9 + t) * nchunks + c] = err;
+}
+
+__global__ void __launch_bounds__(128) k_hc_tile_layout(const Chunk* __restrict__ chunks, uint32_t nchunks,
+                                                        const uint32_t* __restrict__ tile_err,
+                                                        const float* __restrict__ derating /* [level][8] */,
+                                                        const float* __restrict__ level_weight, TileCfg cfg,
+                                                        Tile* __restrict__ tiles, uint32_t* __restrict__ block_tile,
+                                                        uint8_t* __restrict__ block_enc) {
   const uint8_t layout_tiles[8][4] = HC_LAYOUT_TILES;
   const uint8_t layout_ntiles[8] = HC_LAYOUT_NTILES;
   const uint8_t tile_map[8][2][2] = HC_TILE_MAP;
-  uint32_t px[128];
-  chunk_pixels(blocks, ch.b, ch.width, px);
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nchunks) return;
+  const Chunk ch = chunks[c];
   uint32_t terr[3][9];
-  for (int t = 0; t < 9; t++) {
-    const int n = 16 << (t >> 2);
-    if (cfg.has_color) terr[0][t] = fast_tile_error(n, px + tile_ofs[t], st);
-    for (int a = 0; a < cfg.num_alpha; a++)
-      terr[1 + a][t] = cfg.qdxt ? fast_alpha_error(n, px + tile_ofs[t], cfg.comp[a])
-                                : alpha_tile_error(n, px + tile_ofs[t], cfg.comp[a]);
-  }
+  for (int k = 0; k < 3; k++)
+    for (int t = 0; t < 9; t++)
+      terr[k][t] = (k ? k <= cfg.num_alpha : cfg.has_color != 0) ? tile_err[((size_t)k * 9 + t) * nchunks + c] : 0u;
   float best_q = 0.0f;
   int best_e = 0;
   if (cfg.qdxt && !cfg.has_color) {
@@ -701,43 +753,13 @@ __host__ __device__ int hc_tile_chunk(const uint32_t* __restrict__ blocks, uint3
     }
     if (q > best_q) { best_q = q; best_e = e; }
   }
-  const float lw = level_weight[ch.level];
   for (int k = 0; k < 4; k++) {
     Tile& T = tiles[4 * c + k];
-    if (k >= layout_ntiles[best_e]) { T.kind = 0xFFu; T.chunk = c; T.weight = 0; continue; }
-    const int t = layout_tiles[best_e][k];
-    const int n = 16 << (t >> 2);
     T.chunk = c;
+    if (k >= layout_ntiles[best_e]) { T.kind = 0xFFu; T.weight = 0; continue; }
+    const int t = layout_tiles[best_e][k];
     T.kind = (uint32_t)t;
-    T.weight = (float)n * lw;
-    if (cfg.qdxt && !cfg.has_color) {
-      // qdxt5: the representative pair of the channel's values (as grey pixels), weighted by the
-      // squared distance / 8, 1..8
-      uint32_t grey[64];
-      for (int i = 0; i < n; i++) grey[i] = ((px[tile_ofs[t] + i] >> (8 * cfg.comp[0])) & 255u) * 0x010101u;
-      int lo[3], hi[3];
-      find_rep_colors(n, grey, lo, hi);
-      const uint32_t dist = (uint32_t)((lo[0] - hi[0]) * (lo[0] - hi[0]));
-      const uint32_t w = dist / 8u < 1u ? 1u : dist / 8u > 8u ? 8u : dist / 8u;
-      T.va[0][0] = (float)lo[0];
-      T.va[0][1] = (float)hi[0];
-      T.weight = (float)(w * (uint32_t)(n / 16));
-      continue;
-    }
-    if (cfg.qdxt) {
-      // representative colours as the training vector of each of the tile's blocks, weighted by
-      // their distance (squared RGB / 5000, 1..8)
-      int lo[3], hi[3];
-      find_rep_colors(n, px + tile_ofs[t], lo, hi);
-      const int d0 = lo[0] - hi[0], d1 = lo[1] - hi[1], d2 = lo[2] - hi[2];
-      const uint32_t dist = (uint32_t)(d0 * d0 + d1 * d1 + d2 * d2);
-      const uint32_t w = dist / 5000u < 1u ? 1u : dist / 5000u > 8u ? 8u : dist / 5000u;
-      for (int k2 = 0; k2 < 3; k2++) { T.v[k2] = (float)lo[k2]; T.v[3 + k2] = (float)hi[k2]; }
-      T.weight = (float)(w * (uint32_t)(n / 16));
-      continue;
-    }
-    if (cfg.has_color) palettize(px + tile_ofs[t], n, perceptual, T.v);
-    for (int a = 0; a < cfg.num_alpha; a++) palettize_alpha(px + tile_ofs[t], n, cfg.comp[a], T.va[a]);
+    T.weight = (float)(16 << (t >> 2)) * level_weight[ch.level];
   }
   for (int by = 0; by < 2; by++)
     for (int bx = 0; bx < 2; bx++) {
@@ -745,7 +767,46 @@ __host__ __device__ int hc_tile_chunk(const uint32_t* __restrict__ blocks, uint3
       block_tile[blk] = 4 * c + tile_map[best_e][by][bx];
       block_enc[blk] = (uint8_t)best_e;
     }
-  return best_e;
+}
+
+// blockIdx.y: tile slot of the chunk; the chosen tiles' colour vec6 / alpha vec2
+__global__ void __launch_bounds__(64) k_hc_tile_vectors(const uint32_t* __restrict__ blocks, const Chunk* __restrict__ chunks,
+                                                        uint32_t nchunks, int perceptual, TileCfg cfg,
+                                                        Tile* __restrict__ tiles) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nchunks) return;
+  Tile& T = tiles[4 * c + blockIdx.y];
+  if (T.kind == 0xFFu) return;
+  const int t = (int)T.kind, n = 16 << (t >> 2);
+  uint32_t px[64];
+  chunk_pixels(blocks, chunks[c], c_tile_ofs[t], n, px);
+  if (cfg.qdxt && !cfg.has_color) {
+    // qdxt5: the representative pair of the channel's values (as grey pixels), weighted by the
+    // squared distance / 8, 1..8
+    for (int i = 0; i < n; i++) px[i] = ((px[i] >> (8 * cfg.comp[0])) & 255u) * 0x010101u;
+    int lo[3], hi[3];
+    find_rep_colors(n, px, lo, hi);
+    const uint32_t dist = (uint32_t)((lo[0] - hi[0]) * (lo[0] - hi[0]));
+    const uint32_t w = dist / 8u < 1u ? 1u : dist / 8u > 8u ? 8u : dist / 8u;
+    T.va[0][0] = (float)lo[0];
+    T.va[0][1] = (float)hi[0];
+    T.weight = (float)(w * (uint32_t)(n / 16));
+    return;
+  }
+  if (cfg.qdxt) {
+    // representative colours as the training vector of each of the tile's blocks, weighted by
+    // their distance (squared RGB / 5000, 1..8)
+    int lo[3], hi[3];
+    find_rep_colors(n, px, lo, hi);
+    const int d0 = lo[0] - hi[0], d1 = lo[1] - hi[1], d2 = lo[2] - hi[2];
+    const uint32_t dist = (uint32_t)(d0 * d0 + d1 * d1 + d2 * d2);
+    const uint32_t w = dist / 5000u < 1u ? 1u : dist / 5000u > 8u ? 8u : dist / 5000u;
+    for (int k = 0; k < 3; k++) { T.v[k] = (float)lo[k]; T.v[3 + k] = (float)hi[k]; }
+    T.weight = (float)(w * (uint32_t)(n / 16));
+    return;
+  }
+  if (cfg.has_color) palettize(px, n, perceptual != 0, T.v);
+  for (int a = 0; a < cfg.num_alpha; a++) palettize_alpha(px, n, cfg.comp[a], T.va[a]);
 }
 
 // the dxt_fast alpha selectors of every block's channel comp (qdxt5::init's distinct-selector
@@ -774,16 +835,6 @@ __global__ void k_fast_selector_words(const uint32_t* __restrict__ blocks, uint3
   uint32_t w = 0;
   for (int i = 0; i < 16; i++) w |= (uint32_t)sel[i] << (2 * i);
   words[b] = w;
-}
-
-__global__ void __launch_bounds__(64) k_hc_tiles(const uint32_t* __restrict__ blocks, const Chunk* __restrict__ chunks,
-                                                 uint32_t nchunks, const float* __restrict__ derating /* [level][8] */,
-                                                 const float* __restrict__ level_weight, int perceptual,
-                                                 const SolidTables* __restrict__ st, TileCfg cfg, Tile* __restrict__ tiles,
-                                                 uint32_t* __restrict__ block_tile, uint8_t* __restrict__ block_enc) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchunks) return;
-  hc_tile_chunk(blocks, c, chunks[c], derating, level_weight, perceptual != 0, st, cfg, tiles, block_tile, block_enc);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -846,50 +897,83 @@ __device__ __forceinline__ void block_argmax(float& v, uint32_t& pos, float* rv,
     if (rv[w] > v || (rv[w] == v && rp[w] < pos)) { v = rv[w]; pos = rp[w]; }
 }
 
-// Cluster-wide exchange slots: each reduction writes its CTA's partial into slot[phase] and flips
-// the phase, so a slot is rewritten only after a later cluster barrier, by which time every CTA has
-// read it.
+// The warp's totals of N per-lane values: put(k, total) is called by a lane for each k. The sum of a
+// value is the butterfly's (lanes 16 apart, then 8, 4, 2, 1; the same bits in every lane, since an
+// addition's operands may change places), but a lane passes on the half of its values that it does
+// not keep, so 32 values take 31 shuffles instead of 160.
+template <int P>
+__device__ __forceinline__ float fold_columns(float* v) {
+  const unsigned lane = threadIdx.x & 31u;
+  int width = P;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (width > 1) {
+      const bool up = (lane & (unsigned)o) != 0;
+      width >>= 1;
+#pragma unroll
+      for (int j = 0; j < P / 2; j++) {
+        if (j >= width) break;
+        const float give = up ? v[j] : v[j + width], keep = up ? v[j + width] : v[j];
+        v[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, o);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], o);
+    }
+  }
+  return v[0];
+}
+template <int N, int BASE = 0, class Put>
+__device__ __forceinline__ void warp_totals(const float* vals, Put put) {
+  constexpr int kLeft = N - BASE;
+  constexpr int P = kLeft >= 17 ? 32 : kLeft >= 9 ? 16 : kLeft >= 5 ? 8 : kLeft >= 3 ? 4 : kLeft;
+  const int lane = threadIdx.x & 31;
+  float v[P];
+#pragma unroll
+  for (int k = 0; k < P; k++) v[k] = BASE + k < N ? vals[BASE + k] : 0.f;
+  const float t = fold_columns<P>(v);
+  constexpr int kLanes = 32 / P;  // lanes that end with the same column
+  if (lane % kLanes == 0 && BASE + lane / kLanes < N) put(BASE + lane / kLanes, t);
+  if constexpr (BASE + P < N) warp_totals<N, BASE + P>(vals, put);
+}
+
+// Cluster-wide exchange: each reduction's partials go straight into every CTA's slots of the phase,
+// which then flips, so a slot is rewritten only after a later cluster barrier, by which time every
+// CTA has read it.
 constexpr int kVqSlot = 40;
 struct VqShared {
-  float red[kVqSlot * 16];
+  float red[kVqSlot * 17];
   float rv[16];
   uint32_t rp[16];
-  float part[2][kVqSlot];
-  uint32_t upart[2][2];
+  float part[2][16][kVqSlot];
+  uint32_t pos[2][16];
   float tot[kVqSlot];
-  float stage[16][kVqSlot];
   uint32_t ustage[16][2];
   uint32_t scan[2][kVqThreads / 32 + 1];
 };
 
 // cluster-wide sum of N floats per thread; every CTA adds the partials in rank order, so all of
-// them hold bit-identical totals and take the same branches. Warps reduce by shuffles; N threads
-// add the warps' partials; the CTAs' partials are fetched through distributed shared memory in one
-// parallel round trip and added by N threads.
+// them hold bit-identical totals and take the same branches. Warps reduce by shuffles; the CTA's
+// total of a value is added by one thread per CTA of the cluster, which writes it there (a remote
+// write is not waited for; the barrier that it ends with makes it seen). With N threads adding,
+// partials read from the other CTAs after the barrier, and five shuffles a value, a split round of a
+// 1024 x 1024 DXT1 chain's selector tree took 128 us; now TBD.
 template <int N>
 __device__ __forceinline__ void cluster_sum(float* vals, VqShared& sh, int& phase, cg::cluster_group& cl) {
   static_assert(N <= kVqSlot, "cluster_sum slot");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < N; k++)
-    for (int o = 16; o > 0; o >>= 1) vals[k] += __shfl_xor_sync(0xFFFFFFFFu, vals[k], o);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < N; k++) sh.red[k * 16 + warp] = vals[k];
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  warp_totals<N>(vals, [&](int k, float t) { sh.red[k * 17 + warp] = t; });
   __syncthreads();
-  if (threadIdx.x < N) {
+  const unsigned C = cl.num_blocks(), r = cl.block_rank();
+  for (unsigned i = threadIdx.x; i < N * C; i += blockDim.x) {
+    const unsigned q = i / N, k = i % N;
     float t = 0.f;
-    for (int wi = 0; wi < nw; wi++) t += sh.red[threadIdx.x * 16 + wi];
-    sh.part[phase][threadIdx.x] = t;
+    for (int wi = 0; wi < nw; wi++) t += sh.red[k * 17 + wi];
+    *cl.map_shared_rank(&sh.part[phase][r][k], q) = t;
   }
   cl.sync();
-  const unsigned C = cl.num_blocks();
-  for (unsigned t = threadIdx.x; t < N * C; t += blockDim.x)
-    sh.stage[t / N][t % N] = cl.map_shared_rank(&sh.part[phase][0], t / N)[t % N];
-  __syncthreads();
   if (threadIdx.x < N) {
     float t = 0.f;
-    for (unsigned q = 0; q < C; q++) t += sh.stage[q][threadIdx.x];
+    for (unsigned q = 0; q < C; q++) t += sh.part[phase][q][threadIdx.x];
     sh.tot[threadIdx.x] = t;
   }
   __syncthreads();
@@ -900,20 +984,17 @@ __device__ __forceinline__ void cluster_sum(float* vals, VqShared& sh, int& phas
 
 __device__ __forceinline__ void cluster_argmax(float& v, uint32_t& pos, VqShared& sh, int& phase, cg::cluster_group& cl) {
   block_argmax(v, pos, sh.rv, sh.rp);
-  if (threadIdx.x == 0) { sh.part[phase][0] = v; sh.upart[phase][0] = pos; }
-  cl.sync();
-  const unsigned C = cl.num_blocks();
+  const unsigned C = cl.num_blocks(), r = cl.block_rank();
   if (threadIdx.x < C) {
-    sh.stage[threadIdx.x][0] = cl.map_shared_rank(&sh.part[phase][0], threadIdx.x)[0];
-    sh.ustage[threadIdx.x][0] = cl.map_shared_rank(&sh.upart[phase][0], threadIdx.x)[0];
+    *cl.map_shared_rank(&sh.part[phase][r][0], threadIdx.x) = v;
+    *cl.map_shared_rank(&sh.pos[phase][r], threadIdx.x) = pos;
   }
-  __syncthreads();
+  cl.sync();
   for (unsigned q = 0; q < C; q++) {
-    const float qv = sh.stage[q][0];
-    const uint32_t qp = sh.ustage[q][0];
+    const float qv = sh.part[phase][q][0];
+    const uint32_t qp = sh.pos[phase][q];
     if (qv > v || (qv == v && qp < pos)) { v = qv; pos = qp; }
   }
-  __syncthreads();
   phase ^= 1;
 }
 
@@ -951,10 +1032,10 @@ __device__ __forceinline__ float dist2(const float* a, const float* b) {
 // until the variance stops falling. vec[2] / w[2]: the two buffers (N x D floats, N weights).
 // One cluster of CTAs per job; CTA r of C works on the r-th contiguous slice of the node's range.
 template <int D>
-__global__ void __launch_bounds__(kVqThreads) k_vq_split(float* __restrict__ vec0, float* __restrict__ vec1,
-                                                         float* __restrict__ w0, float* __restrict__ w1,
-                                                         VqNode<D>* __restrict__ nodes, const SplitJob* __restrict__ jobs) {
-  __shared__ VqShared sh;
+__device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float* __restrict__ vec1,
+                                                 float* __restrict__ w0, float* __restrict__ w1,
+                                                 VqNode<D>* __restrict__ nodes, const SplitJob* __restrict__ jobs,
+                                                 VqShared& sh) {
   __shared__ float s_c[D];
   cg::cluster_group cl = cg::this_cluster();
   const unsigned C = cl.num_blocks(), r = cl.block_rank();
@@ -969,7 +1050,7 @@ __global__ void __launch_bounds__(kVqThreads) k_vq_split(float* __restrict__ vec
   const uint32_t per = (b1 - b0 + C - 1) / C;
   const uint32_t s0 = min(b1, b0 + r * per), s1 = min(b1, s0 + per);  // this CTA's slice
   if (threadIdx.x < D) s_c[threadIdx.x] = P.c[threadIdx.x];
-  __syncthreads();
+  cl.sync();  // every CTA has started: its shared memory may be written
   float c[D];
 #pragma unroll
   for (int k = 0; k < D; k++) c[k] = s_c[k];
@@ -1135,17 +1216,17 @@ __global__ void __launch_bounds__(kVqThreads) k_vq_split(float* __restrict__ vec
     }
     my_left += (uint32_t)__syncthreads_count(left);
   }
-  if (threadIdx.x == 0) { sh.upart[phase][0] = my_left; sh.upart[phase][1] = s1 - s0; }
+  if (threadIdx.x < C) {
+    *cl.map_shared_rank(&sh.ustage[r][0], threadIdx.x) = my_left;
+    *cl.map_shared_rank(&sh.ustage[r][1], threadIdx.x) = s1 - s0;
+  }
   cl.sync();
-  if (threadIdx.x < 2 * C) sh.ustage[threadIdx.x >> 1][threadIdx.x & 1] = cl.map_shared_rank(&sh.upart[phase][0], threadIdx.x >> 1)[threadIdx.x & 1];
-  __syncthreads();
   uint32_t left_before = 0, right_before = 0, left_total = 0;
   for (unsigned q = 0; q < C; q++) {
     const uint32_t ql = sh.ustage[q][0], qn = sh.ustage[q][1];
     left_total += ql;
     if (q < r) { left_before += ql; right_before += qn - ql; }
   }
-  phase ^= 1;
   uint32_t lrun = b0 + left_before, rrun = b0 + left_total + right_before;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   int sb = 0;
@@ -1195,15 +1276,17 @@ __global__ void __launch_bounds__(kVqThreads) k_vq_split(float* __restrict__ vec
   cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// The same split for small nodes, one warp per job (8 jobs per CTA): the reductions are warp
-// butterflies, which leave bit-identical totals in every lane, and no CTA-wide barrier is needed.
+// The same split for small nodes, one warp per job: no CTA-wide barrier is needed.
 constexpr uint32_t kVqWarpMax = 256;  // nodes up to this many vectors take the warp kernel
 
+// the totals go to all lanes through the warp's own `tot`
 template <int N>
-__device__ __forceinline__ void warp_sum(float* vals) {
+__device__ __forceinline__ void warp_sum(float* vals, float* tot) {
+  __syncwarp();  // the totals before have been read
+  warp_totals<N>(vals, [&](int k, float t) { tot[k] = t; });
+  __syncwarp();
 #pragma unroll
-  for (int k = 0; k < N; k++)
-    for (int o = 16; o > 0; o >>= 1) vals[k] += __shfl_xor_sync(0xFFFFFFFFu, vals[k], o);
+  for (int k = 0; k < N; k++) vals[k] = tot[k];
 }
 
 __device__ __forceinline__ void warp_argmax(float& v, uint32_t& pos) {
@@ -1215,14 +1298,10 @@ __device__ __forceinline__ void warp_argmax(float& v, uint32_t& pos) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(256, 2) k_vq_split_warp(float* __restrict__ vec0, float* __restrict__ vec1,
-                                                       float* __restrict__ w0, float* __restrict__ w1,
-                                                       VqNode<D>* __restrict__ nodes, const SplitJob* __restrict__ jobs,
-                                                       uint32_t njobs) {
-  const uint32_t jid = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (jid >= njobs) return;  // whole warps only
+__device__ __forceinline__ void vq_split_warp(float* __restrict__ vec0, float* __restrict__ vec1,
+                                              float* __restrict__ w0, float* __restrict__ w1,
+                                              VqNode<D>* __restrict__ nodes, const SplitJob job, float* tot) {
   const uint32_t lane = threadIdx.x & 31;
-  const SplitJob job = jobs[jid];
   VqNode<D>& P = nodes[job.parent];
   const uint32_t b0 = P.begin, b1 = P.end, src = P.buf;
   const float* __restrict__ vec = src ? vec1 : vec0;
@@ -1281,7 +1360,7 @@ __global__ void __launch_bounds__(256, 2) k_vq_split_warp(float* __restrict__ ve
 #pragma unroll
         for (int k = 0; k < D; k++) acc[k] += d[k] * ww;
       }
-      warp_sum<D>(acc);
+      warp_sum<D>(acc, tot);
       float mx = acc[0];
 #pragma unroll
       for (int k = 1; k < D; k++) mx = fmaxf(mx, acc[k]);
@@ -1317,7 +1396,7 @@ __global__ void __launch_bounds__(256, 2) k_vq_split_warp(float* __restrict__ ve
       acc[2 * D] += wl;
       acc[2 * D + 1] += wr;
     }
-    warp_sum<2 * D + 2>(acc);
+    warp_sum<2 * D + 2>(acc, tot);
     if (acc[2 * D] > 0.f && acc[2 * D + 1] > 0.f) {
 #pragma unroll
       for (int k = 0; k < D; k++) { L[k] = acc[k] / acc[2 * D]; R[k] = acc[D + k] / acc[2 * D + 1]; }
@@ -1345,7 +1424,7 @@ __global__ void __launch_bounds__(256, 2) k_vq_split_warp(float* __restrict__ ve
       acc[2 * D + 2] += sq * wl;
       acc[2 * D + 3] += sq * wr;
     }
-    warp_sum<2 * D + 4>(acc);
+    warp_sum<2 * D + 4>(acc, tot);
     lw = acc[2 * D]; rw = acc[2 * D + 1];
     if (!(lw > 0.f) || !(rw > 0.f)) break;
     float ll = 0.f, rr = 0.f;
@@ -1415,6 +1494,23 @@ __global__ void __launch_bounds__(256, 2) k_vq_split_warp(float* __restrict__ ve
   }
 }
 
+// A round's splits: the first nbig jobs on a cluster of CTAs each, then a warp per job. Both kinds
+// in one launch, so that the small nodes' chains run beside the large ones'.
+template <int D>
+__global__ void __launch_bounds__(kVqThreads) k_vq_split(float* __restrict__ vec0, float* __restrict__ vec1,
+                                                         float* __restrict__ w0, float* __restrict__ w1,
+                                                         VqNode<D>* __restrict__ nodes, const SplitJob* __restrict__ jobs,
+                                                         uint32_t nbig, uint32_t njobs) {
+  __shared__ VqShared sh;
+  const uint32_t ctas = nbig * (uint32_t)cg::this_cluster().num_blocks();
+  if (blockIdx.x < ctas) {  // whole clusters
+    vq_split_cluster<D>(vec0, vec1, w0, w1, nodes, jobs, sh);
+    return;
+  }
+  const uint32_t warp = threadIdx.x >> 5, jid = nbig + (blockIdx.x - ctas) * (kVqThreads / 32) + warp;
+  if (jid < njobs) vq_split_warp<D>(vec0, vec1, w0, w1, nodes, jobs[jid], &sh.part[0][0][0] + warp * kVqSlot);
+}
+
 // Root node statistics (centroid, weight, variance of all vectors) and the first buffer: the
 // caller's vectors and integer weights copied as floats. One cluster over all vectors.
 template <int D>
@@ -1441,6 +1537,7 @@ __global__ void __launch_bounds__(kVqThreads) k_vq_root(const float* __restrict_
     acc[D] += ww;
     acc[D + 1] += sq * ww;
   }
+  cl.sync();  // every CTA has started: its shared memory may be written
   cluster_sum<D + 2>(acc, sh, phase, cl);
   if (r == 0 && threadIdx.x == 0) {
     VqNode<D>& rt = nodes[0];
@@ -1587,15 +1684,13 @@ int tree_vq(const float* d_vec, const uint32_t* d_w, uint32_t n, uint32_t max_en
     if ((e = cudaMemcpyAsync(d_jobs.ptr, jobs.data(), sizeof(SplitJob) * take, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cuda_check(e, "copy vq jobs");
     const SplitJob* dj = static_cast<const SplitJob*>(d_jobs.ptr);
-    if (nbig) {
-      const unsigned C = vq_cluster_size(largest, max_split_cluster);
-      if ((e = launch_clustered(k_vq_split<D>, (unsigned)nbig * C, C, s, v0, v1, w0, w1, nodes, dj)) != cudaSuccess)
+    {
+      const unsigned C = nbig ? vq_cluster_size(largest, max_split_cluster) : 1u;
+      const unsigned small = ((unsigned)(take - nbig) + kVqThreads / 32 - 1) / (kVqThreads / 32);
+      const unsigned grid = ((unsigned)nbig * C + small + C - 1) / C * C;
+      if ((e = launch_clustered(k_vq_split<D>, grid, C, s, v0, v1, w0, w1, nodes, dj, (uint32_t)nbig, (uint32_t)take)) !=
+          cudaSuccess)
         return cuda_check(e, "launch k_vq_split");
-    }
-    if (nbig < take) {
-      const uint32_t nsmall = (uint32_t)(take - nbig);
-      k_vq_split_warp<D><<<(nsmall + 7) / 8, 256, 0, s>>>(v0, v1, w0, w1, nodes, dj + nbig, nsmall);
-      if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_vq_split_warp");
     }
     // only the new children are read back; a failed split is flagged on its left child
     if ((e = cudaMemcpyAsync(h.data() + first_new, nodes + first_new, sizeof(Node) * (used - first_new),
@@ -2757,6 +2852,7 @@ struct HcBuffers {
       cstart, clist, clusters, bweight, block_cluster, selvec, selw, cb16, cbsel, block_sel, entry_err, entry_used,
       levels, flags, iota, used, keys, keys2, cub_tmp, sse, avec, aw, aitems, tile_ac, cb2, acount, alist, astart,
       aclusters, aitem_cluster, aselvec, aselw, acb16, acbsel, aitem_sel, aentry_err;
+  DevBuf tile_err;  // errors of every chunk's nine tiles, per channel
   hc::VqScratch vq;
   bool clean = true;  // the last call ended with its stream synchronised
 };
@@ -2916,16 +3012,28 @@ int hc_compress_impl(const uint8_t* d_blocks, const crngpu_hc_params& P, uint32_
       (e = up(B.st, st_host, sizeof(SolidTables))) != cudaSuccess ||
       (e = up(B.levels, lv.data(), sizeof(Level) * lv.size())) != cudaSuccess)
     return cuda_check(e, "upload hc tables");
-  if ((e = B.tiles.ensure(sizeof(Tile) * ntiles)) != cudaSuccess || (e = B.block_tile.ensure(4 * N)) != cudaSuccess ||
+  if ((e = B.tile_err.ensure(sizeof(uint32_t) * 27 * (size_t)nchunks)) != cudaSuccess ||
+      (e = B.tiles.ensure(sizeof(Tile) * ntiles)) != cudaSuccess || (e = B.block_tile.ensure(4 * N)) != cudaSuccess ||
       (e = B.block_enc.ensure(N)) != cudaSuccess)
     return cuda_check(e, "alloc tiles");
   const uint32_t* blocks = reinterpret_cast<const uint32_t*>(d_blocks);
   Tile* tiles = static_cast<Tile*>(B.tiles.ptr);
-  k_hc_tiles<<<(nchunks + 63) / 64, 64, 0, s>>>(blocks, static_cast<Chunk*>(B.chunks.ptr), nchunks,
-                                                 static_cast<float*>(B.derating.ptr), static_cast<float*>(B.lweight.ptr),
-                                                 P.perceptual, static_cast<SolidTables*>(B.st.ptr), cfg, tiles,
-                                                 static_cast<uint32_t*>(B.block_tile.ptr), static_cast<uint8_t*>(B.block_enc.ptr));
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_hc_tiles");
+  {
+    const Chunk* ch = static_cast<Chunk*>(B.chunks.ptr);
+    uint32_t* terr = static_cast<uint32_t*>(B.tile_err.ptr);
+    const unsigned g64 = (nchunks + 63) / 64;
+    if (cfg.has_color || cfg.qdxt)
+      k_hc_tile_errors<<<dim3(g64, 9), 64, 0, s>>>(blocks, ch, nchunks, static_cast<SolidTables*>(B.st.ptr), cfg, terr);
+    if (cfg.num_alpha && !cfg.qdxt)
+      k_hc_alpha_errors<<<dim3((nchunks + kAlphaErrWarps - 1) / kAlphaErrWarps, 9, (unsigned)cfg.num_alpha),
+                          kAlphaErrWarps * 32, 0, s>>>(blocks, ch, nchunks, cfg, terr);
+    k_hc_tile_layout<<<(nchunks + 127) / 128, 128, 0, s>>>(ch, nchunks, terr, static_cast<float*>(B.derating.ptr),
+                                                           static_cast<float*>(B.lweight.ptr), cfg, tiles,
+                                                           static_cast<uint32_t*>(B.block_tile.ptr),
+                                                           static_cast<uint8_t*>(B.block_enc.ptr));
+    k_hc_tile_vectors<<<dim3(g64, 4), 64, 0, s>>>(blocks, ch, nchunks, P.perceptual, cfg, tiles);
+  }
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch the tile kernels");
   // the used tiles, compacted in tile order (so the result is reproducible)
   if ((e = B.count.ensure(16)) != cudaSuccess || (e = B.flags.ensure(ntiles)) != cudaSuccess ||
       (e = B.iota.ensure(4 * ntiles)) != cudaSuccess || (e = B.used.ensure(4 * ntiles)) != cudaSuccess ||
