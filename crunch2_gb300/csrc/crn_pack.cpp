@@ -240,6 +240,15 @@ unsigned pack_threads(uint64_t nblocks) {
   return std::max(1u, std::min(hw ? hw : 4u, 16u));
 }
 
+// The palettes' order is quadratic in their sizes, whatever the image's: with 2,570 colour and 2,094
+// alpha endpoints a 333 x 180 DXT5 chain's writer spent 15 of its 20 ms there on one thread (16 Grace
+// cores). Below 2^19 pairs (about 0.3 ms) a thread's start is not worth it.
+unsigned order_threads(uint64_t pairs) {
+  if (pairs < (1u << 19)) return 1;
+  const unsigned hw = std::thread::hardware_concurrency();
+  return std::max(1u, std::min(hw ? hw : 4u, 16u));
+}
+
 // symbol_codec's static model transmission, the inverse of
 // decode_receive_static_data_model (inc/crn_decomp.h:3044-3123): 14-bit symbol count, the 21
 // code-length-code lengths in transmission order (3 bits each), then the code lengths coded with
@@ -839,6 +848,9 @@ extern "C" int64_t crngpu_crn_pack(const uint8_t* blocks, uint32_t width, uint32
   Palette* ep_pal[2] = {&cep, &aep};
   Palette* sel_pal[2] = {&csel, &asel};
   std::vector<uint32_t> ep_rank[2], sel_rank[2];
+  uint64_t pairs = 0;
+  for (const Palette* q : {&cep, &csel, &aep, &asel}) pairs += (uint64_t)q->values.size() * q->values.size();
+  const unsigned order_workers = std::max(threads, order_threads(pairs));
   {
     std::vector<std::function<void()>> workers;  // per model: the selector order, the endpoint order
     // the endpoint trials of model m: coded size of the palette plus the index deltas
@@ -946,7 +958,7 @@ extern "C" int64_t crngpu_crn_pack(const uint8_t* blocks, uint32_t width, uint32
         std::vector<uint32_t> trial[4];
         uint64_t bits[4];
         static_assert(4000u * 3 / 2 <= 65535u && 4000u <= 10922u, "grow_chain's 16-bit similarity");
-        parallel_jobs(4, threads, [&](size_t t, unsigned) {
+        parallel_jobs(4, order_workers, [&](size_t t, unsigned) {
           if (t == 0) {
             // least distance between distinct endpoints: one 6-bit green step (4^2) or one alpha step
             trial[0] = nearest_chain_comps(u, m ? 1u : 16u);
@@ -961,7 +973,7 @@ extern "C" int64_t crngpu_crn_pack(const uint8_t* blocks, uint32_t width, uint32
         ep_rank[m] = std::move(trial[best]);
       });
     }
-    parallel_jobs(workers.size(), threads, [&](size_t j, unsigned) { workers[j](); });
+    parallel_jobs(workers.size(), order_workers, [&](size_t j, unsigned) { workers[j](); });
   }
   for (int m = 0; m < 2; m++) {
     if (comp_lo[m] == comp_hi[m]) continue;
