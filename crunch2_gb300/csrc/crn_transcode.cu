@@ -2276,8 +2276,10 @@ constexpr uint32_t kWideMinBlocks = 256;  // smaller levels always go to the lan
 // Measured on GB300: the top level of a 1024 x 1024 DXT1 file 0.50 ms (13 launches, 46 us each while
 // it walks) against 1.74 ms wide; the largest level of a 24-texture batch, 2048 x 1024 DXT5, 1.2 ms
 // against 5.5 ms.
-constexpr double kWalkUsPerBlock = 0.0055, kWalkUsPerBit = 2e-5, kWalkLaunchUs = 3.0;
-constexpr double kWalkWaveUs = 2.0, kLaneLaunchUs = 8.0;  // a wave of CTAs of one launch; the lane decoder's launch
+constexpr double kWalkUsPerBlock = 0.007, kWalkUsPerBit = 2e-5, kWalkLaunchUs = 5.0;
+// A wave of CTAs of one launch; the state's clearing, the scratch and the tables' pipeline filling; the
+// lane decoder's launch. (32 x 32: 35 us of walk against 15 of lane decoder; 64 x 64: 38 against 44.)
+constexpr double kWalkWaveUs = 2.0, kWalkFixedUs = 14.0, kLaneLaunchUs = 3.0;
 
 uint64_t task_blocks(const LevelTask& t) {
   const LevelInfo& li = t.file->level[t.level];
@@ -2335,8 +2337,9 @@ HVec<uint8_t> decide_decoders(const HVec<LevelTask>& tasks, uint32_t wide_slots,
       walk_bits += 8.0 * t.src_size;
       max_bits = std::max(max_bits, 8.0 * t.src_size);
       walk_t = std::max(cost[0].first * kWalkUsPerBlock, walk_bits * kWalkUsPerBit) +
-               (std::min<double>(kWalkMaxSegments, max_bits / kWalkSegment) + 4) *
-                   (kWalkLaunchUs + kWalkWaveUs * (double)(3 * k / sms));
+               (std::min<double>(kWalkMaxSegments, std::max(1.0, max_bits / kWalkSegment)) + 3) *
+                   (kWalkLaunchUs + kWalkWaveUs * (double)(3 * k / sms)) +
+               kWalkFixedUs;
     }
     if (walk_t >= best) break;  // grows with k
     double sum = 0;
