@@ -69,9 +69,6 @@ __device__ __forceinline__ uint32_t canon_lo(uint32_t lo, uint32_t hi) { return 
 __device__ __forceinline__ uint32_t canon_hi(uint32_t lo, uint32_t hi) { return lo < hi ? lo : hi; }
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
-// exact float (integer value in [0, 2^23)) -> uint via the 2^23 magic constant
-__device__ __forceinline__ uint32_t f2u_exact(float v) { return __float_as_uint(__fadd_rn(v, 8388608.0f)) - 0x4B000000u; }
-
 
 // A DXT1 solution (dxt1_endpoint_optimizer::potential_solution, crn_dxt1.h:272-311) minus its
 // selectors, which are recomputed from it when needed.
@@ -93,13 +90,17 @@ struct State {
 };
 
 // Candidate list kinds consumed by run_list (the reference's candidate loops).
-enum : int { LK_TABLE = 0, LK_PAIRS, LK_NEIGH, LK_MOVE2, LK_REFINE, LK_COMB, LK_COMPS };
+enum : int { LK_TABLE = 0, LK_PAIRS, LK_LATTICE, LK_REFINE, LK_COMB, LK_COMPS };
+// LK_LATTICE: the 26 adjacent cells, then (Uber) +-2 along each axis, together a warp's 32 candidates:
+// the two lists one after the other took 3.62 ms for a 1024 x 1024 chain, one batch for both 3.38.
+constexpr int kNeighbours = 26;
 
 struct ListDesc {
   int kind, count, dependent, alt, stop_on_accept;
   int side, nh, row;
-  int base[3];  // NEIGH/MOVE2: centre; COMPS: unpacked high endpoint
+  int base[3];  // LATTICE: centre (packed, base[0]); COMPS: unpacked high endpoint
   int e[6];     // REFINE: fitted endpoints (At1 triple, At2 triple)
+  uint32_t pk[2];  // and packed
   // COMPS: per-component error tables and running bounds
   int comp, p0;
   uint32_t packed_lo, e0, best_err;
@@ -128,18 +129,29 @@ struct SeedShared {
   uint64_t bar;
 };
 
+// A unique colour as the evaluation loop reads it, in two 16-byte loads: each component times -2 and
+// twice, for the packed multiply-adds that take two palette entries at a time; the weighted |x|^2
+// plus 2^23, so that adding the rest of a squared distance gives its integer in the low mantissa
+// bits; the weight. (With these, and the colours two to an iteration, a 1024 x 1024 chain's encode
+// went from 4.11 to 3.85 ms.)
+struct __align__(16) EvalColour {
+  float nx[2], ny[2];
+  float nz[2], xb;
+  uint32_t w;
+};
+
 // Per-warp shared state of the search kernel: the block's seed and the phase-2 working set.
 struct WarpShared {
   float4 ucf[16];     // r, g, b as floats, X2 = weighted |x|^2
   int ucw[16];        // weights
   // the same colours in evaluation order (farthest from the block's mean first, by weighted
   // distance): an error sum is exact in any order, and this order makes the early-out fire sooner
-  float4 ecf[16];
-  uint32_t ecw[16], eci[16];
+  EvalColour ecv[17];  // and one of weight 0 after the last: they are taken two at a time
+  uint32_t eci[16];
   uint32_t uci[16];   // r | g << 8 | b << 16
   uint2 lbr[32], lbg[64], lbb[32];  // plane lower bounds: .x = low, .y = high
-  uint16_t list[64];  // low-endpoint probes / combinatorial endpoints
-  uint16_t list2[32]; // high-endpoint probes
+  uint16_t list[64];  // combinatorial endpoints
+  uint16_t list2[32];
   uint32_t cand[64];  // table candidates (lo | hi << 16) / combinatorial scratch colours
   uint2 pq[64];       // run_list's queue of unpruned candidates of a fixed list: (lo | hi << 16, bound)
   State st;
@@ -522,6 +534,13 @@ __device__ __forceinline__ float4 entry(float wr, float wg, int r, int g, int b)
   return make_float4(2.f * wr * fr, 2.f * wg * fg, 2.f * fb, wr * fr * fr + wg * fg * fg + fb * fb);
 }
 
+// The same for the evaluation loop, whose colours carry the factor 2: (w p, w.p^2). Every product
+// and sum is an integer below 2^24, so the fused ones are exact.
+__device__ __forceinline__ float4 half_entry(float wr, float wg, float fr, float fg, float fb) {
+  const float hr = wr * fr, hg = wg * fg;
+  return make_float4(hr, hg, fb, fmaf(hr, fr, fmaf(hg, fg, fb * fb)));
+}
+
 // color::RGB_to_Y (crnlib/crn_color.h:792-796): fixed-point luma
 __device__ __forceinline__ int luma(int r, int g, int b) { return (r * 19595 + g * 38470 + b * 7471 + 32768) >> 16; }
 
@@ -532,11 +551,38 @@ __device__ __forceinline__ float4 entry_m(bool gray, float wr, float wg, int r, 
   const float y = (float)luma(r, g, b);
   return make_float4(2.f * y, 0.f, 0.f, y * y);
 }
+__device__ __forceinline__ float4 half_entry_m(bool gray, float wr, float wg, float r, float g, float b) {
+  if (!gray) return half_entry(wr, wg, r, g, b);
+  const float y = (float)luma((int)r, (int)g, (int)b);
+  return make_float4(y, 0.f, 0.f, y * y);
+}
 __device__ __forceinline__ float dist_part(const float4& x, const float4& q) {
   float t = fmaf(-x.x, q.x, q.w);
   t = fmaf(-x.y, q.y, t);
   return fmaf(-x.z, q.z, t);
 }
+
+// Two palette entries' distance parts at once: each half rounds as its own fmaf.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// exact float in [2^23, 2^24) -> its integer above 2^23
+__device__ __forceinline__ uint32_t b2u_exact(float v) { return __float_as_uint(v) - 0x4B000000u; }
 
 // Selector of unique colour i for solution s; ties go to the lowest index, which is how both
 // the uber trial loop and compute_selectors_hc (crn_dxt1.cpp:1845-1869) resolve them.
@@ -623,7 +669,8 @@ __device__ __forceinline__ void accept(WarpShared& S, uint32_t lo, uint32_t hi, 
 }
 
 // Candidate i of the current list (descriptor in S.d); false when the reference skips it.
-__device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDesc& d, int i, uint32_t& lo, uint32_t& hi) {
+__device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDesc& d, int i, int pa, int pb, uint32_t far,
+                                              uint32_t& lo, uint32_t& hi) {
   switch (d.kind) {
     case LK_TABLE: {
       const uint32_t v = S.cand[i];
@@ -631,40 +678,38 @@ __device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDes
       return true;
     }
     case LK_PAIRS: {
-      // i / nh through a float reciprocal: exact for i < 2^10, nh <= 31 (the fraction of
-      // (i + 0.5) / nh is at least 1 / 62 away from an integer)
-      const int a = __float2int_rz(__fmul_rn(__fadd_rn((float)i, 0.5f), __frcp_rn((float)d.nh))), b = i - a * d.nh;
-      const uint32_t p0 = S.list[a], p1 = S.list2[b];
-      lo = canon_lo(p0, p1); hi = canon_hi(p0, p1);
+      const uint32_t p0 = S.list[pa], p1 = S.list2[pb];
+      lo = max(p0, p1); hi = min(p0, p1);
       return true;
     }
-    case LK_NEIGH:
-    case LK_MOVE2: {
-      int c[3] = {d.base[0], d.base[1], d.base[2]};
-      if (d.kind == LK_NEIGH) {
+    case LK_LATTICE: {
+      const bool near = i < kNeighbours;
+      const uint32_t base = near ? (uint32_t)d.base[0] : far;
+      int r = (int)(base >> 11), g = (int)((base >> 5) & 63), b = (int)(base & 31);
+      if (near) {
         // g_adjacency order (crn_dxt1.cpp:489-522): x fastest, then y, then z, centre skipped
-        const int idx = i < 13 ? i : i + 1;
-        c[0] += idx % 3 - 1; c[1] += (idx / 3) % 3 - 1; c[2] += idx / 9 - 1;
-        if (c[0] < 0 || c[0] > 31 || c[1] < 0 || c[1] > 63 || c[2] < 0 || c[2] > 31) return false;
+        const int idx = i < 13 ? i : i + 1, row = idx / 3, z = row / 3;
+        r += idx - 3 * row - 1;
+        g += row - 3 * z - 1;
+        b += z - 1;
       } else {
-        const int a = i >> 1;
-        c[a] += (i & 1) ? 2 : -2;
-        if (c[a] < 0 || c[a] > (a == 1 ? 63 : 31)) return false;
+        const int a = (i - kNeighbours) >> 1, by = (i & 1) ? 2 : -2;
+        r += a == 0 ? by : 0;
+        g += a == 1 ? by : 0;
+        b += a == 2 ? by : 0;
       }
-      const uint32_t moved = pack565(c[0], c[1], c[2]);
-      const uint32_t p0 = d.side ? S.st.best.lo : moved, p1 = d.side ? moved : S.st.best.hi;
-      lo = canon_lo(p0, p1); hi = canon_hi(p0, p1);
+      if ((unsigned)r > 31u || (unsigned)g > 63u || (unsigned)b > 31u) return false;
+      const uint32_t moved = pack565(r, g, b), other = d.side ? S.st.best.lo : S.st.best.hi;
+      lo = max(moved, other); hi = min(moved, other);
       return true;
     }
     case LK_REFINE: {
-      const int which = i / 27, rr = (i / 9) % 3 - 1, gr = (i / 3) % 3 - 1, br = i % 3 - 1;
-      int c[6] = {d.e[0], d.e[1], d.e[2], d.e[3], d.e[4], d.e[5]};
-      const int o = which * 3;
-      c[o] = clampi(c[o] + rr, 0, 31);
-      c[o + 1] = clampi(c[o + 1] + gr, 0, 63);
-      c[o + 2] = clampi(c[o + 2] + br, 0, 31);
-      const uint32_t p0 = pack565(c[0], c[1], c[2]), p1 = pack565(c[3], c[4], c[5]);
-      lo = canon_lo(p0, p1); hi = canon_hi(p0, p1);
+      const int which = i >= 27 ? 1 : 0, j = which ? i - 27 : i, row = j / 3, z = row / 3;
+      const int* e = d.e + 3 * which;
+      const uint32_t moved = pack565(clampi(e[0] + z - 1, 0, 31), clampi(e[1] + row - 3 * z - 1, 0, 63),
+                                     clampi(e[2] + j - 3 * row - 1, 0, 31));
+      const uint32_t other = d.pk[which ^ 1];
+      lo = max(moved, other); hi = min(moved, other);
       return true;
     }
     case LK_COMB:
@@ -706,65 +751,72 @@ __device__ __noinline__ int run_list(WarpShared& S, int start, uint32_t& work) {
   int i0 = start;
   // Lists whose candidates do not depend on the running best are compacted: the candidates that
   // survive the plane-table prune (against the best when they are generated) queue up in list order
-  // in S.pq, and each batch evaluates 32 of them, so the colour loop runs on full warps. The prune
-  // is repeated against the best at the start of the batch; acceptances follow list order, as in
-  // the sparse form. Lists regenerated after each acceptance run sparse, 32 positions at a time.
+  // in S.pq (a ring of 64), and each batch evaluates 32 of them, so the colour loop runs on full
+  // warps. The prune is repeated against the best at the start of the batch; acceptances follow list
+  // order, as in the sparse form. Lists regenerated after each acceptance run sparse, 32 positions
+  // at a time. Both forms go through the one copy of the generation and of the evaluation: waiting
+  // for instructions is the kernel's largest stall, and with a copy each, a queue shifted down after
+  // every batch and candidates through indexed local arrays this routine was 17.5 KB of code, 11 now
+  // (1024 x 1024 chain 3.85 -> 3.79 ms).
   const bool compact = !d.dependent;
-  int qn = 0;  // queued candidates (compact lists)
-  // No tried-solution set (m_solutions_tried, crn_dxt1.cpp:1323-1330): a candidate evaluated
-  // before had an error at or above the best of that time, and the best only falls, so evaluating
-  // it again cannot accept it. The current best itself (once there is one; same palette rounding,
-  // endpoints not bumped apart by the equal-endpoint rule) is skipped, as its error would only
-  // reach the best at its last colour.
-  auto not_best = [&](uint32_t lo, uint32_t hi) {
-    const Sol& b = S.st.best;
-    return d.alt || b.err == kInf || b.alt || b.enforce || (lo | (hi << 16)) != (b.lo | (b.hi << 16));
-  };
+  int qh = 0, qn = 0;  // the queue's head and length
+  // position i of a list of probe pairs is pair (i / nh, i % nh), followed from batch to batch
+  const int nh = d.kind == LK_PAIRS ? d.nh : 32;
+  int pa = (int)lane / nh, pb = (int)lane - pa * nh;
+  const int da = 32 / nh, db = 32 - da * nh;
+  // A lattice list's +-2 moves are around the endpoint that the adjacent cells leave: the running
+  // best's when the last of those has been tried (an acceptance restarts the batch after it)
+  uint32_t far = 0;
   for (;;) {
-    uint32_t lo = 0, hi = 0, lb = kInf;
-    bool live;
-    int take = 32;
     const uint32_t B0 = S.st.best.err;
-    if (compact) {
-      while (qn < 32 && i0 < d.count) {
+    uint32_t word = 0, lb = kInf;  // this lane's candidate (lo | hi << 16) and its bound; kInf: none
+    if (!compact || qn < 32) {
+      if (i0 < d.count) {
         const int i = i0 + (int)lane;
-        uint32_t clo = 0, chi = 0;
-        const bool valid = i < d.count && gen_candidate(S, d, i, clo, chi);
-        const uint32_t clb = valid ? lower_bound(S, clo, chi) : kInf;
-        const bool keep = valid && clb < S.st.best.err && not_best(clo, chi);
-        const unsigned m = __ballot_sync(FULL_MASK, keep);
-        if (keep) S.pq[qn + __popc(m & ((1u << lane) - 1u))] = make_uint2(clo | (chi << 16), clb);
-        qn += __popc(m);
-        i0 += 32;
+        if (i0 <= kNeighbours) far = d.side ? S.st.best.hi : S.st.best.lo;
+        uint32_t lo = 0, hi = 0;
+        // No tried-solution set (m_solutions_tried, crn_dxt1.cpp:1323-1330): a candidate evaluated
+        // before had an error at or above the best of that time, and the best only falls, so
+        // evaluating it again cannot accept it. The current best itself (once there is one; same
+        // palette rounding, endpoints not bumped apart by the equal-endpoint rule) is skipped, as its
+        // error would only reach the best at its last colour.
+        if (i < d.count && gen_candidate(S, d, i, pa, pb, far, lo, hi)) {
+          lb = lower_bound(S, lo, hi);
+          word = lo | (hi << 16);
+          const Sol& b = S.st.best;
+          if (lb >= B0 || (word == (b.lo | (b.hi << 16)) && !d.alt && B0 != kInf && !b.alt && !b.enforce)) lb = kInf;
+        }
+        if (compact) {
+          const unsigned m = __ballot_sync(FULL_MASK, lb != kInf);
+          if (lb != kInf) S.pq[(qh + qn + __popc(m & ((1u << lane) - 1u))) & 63] = make_uint2(word, lb);
+          qn += __popc(m);
+          i0 += 32;
+          pa += da;
+          pb += db;
+          if (pb >= nh) { pb -= nh; pa++; }
+          if (qn < 32 && i0 < d.count) continue;
+        }
+      } else if (!compact) {
+        break;
       }
-      __syncwarp();
-      if (!qn) break;
-      take = min(qn, 32);
-      if ((int)lane < take) {
-        const uint2 v = S.pq[lane];
-        lo = v.x & 0xFFFFu; hi = v.x >> 16; lb = v.y;
-      }
-      live = (int)lane < take && lb < B0;
-    } else {
-      if (i0 >= d.count) break;
-      const int i = i0 + (int)lane;
-      const bool valid = i < d.count && gen_candidate(S, d, i, lo, hi);
-      lb = valid ? lower_bound(S, lo, hi) : kInf;
-      live = valid && lb < B0 && not_best(lo, hi);
     }
+    if (compact) {
+      if (!qn) break;
+      __syncwarp();
+      const int take = min(qn, 32);
+      const uint2 v = S.pq[(qh + (int)lane) & 63];
+      word = v.x;
+      lb = (int)lane < take ? v.y : kInf;
+      qh += take;
+      qn -= take;
+      __syncwarp();
+    }
+    const bool live = lb < B0;
     if (!__any_sync(FULL_MASK, live)) {  // the whole batch is pruned: nothing to evaluate
-      if (compact) {
-        const int rest = qn - take;
-        const uint2 v = (int)lane < rest ? S.pq[take + lane] : make_uint2(0u, 0u);
-        __syncwarp();
-        if ((int)lane < rest) S.pq[lane] = v;
-        __syncwarp();
-        qn = rest;
-      } else {
-        i0 += 32;
-      }
+      if (!compact) i0 += 32;
       continue;
     }
+    const uint32_t lo = word & 0xFFFFu, hi = word >> 16;
     // evaluate every lane's candidate (uber: 4- and 3-colour; hc: 4-colour; fast: the selector
     // by projection, then its distance), stopping early once no live lane can still beat the
     // running best. Blocks with transparent texels evaluate 3-colour blocks only.
@@ -773,40 +825,64 @@ __device__ __noinline__ int run_list(WarpShared& S, int start, uint32_t& work) {
       const int a = d.alt;
       const int r0 = exp5(lo >> 11), g0 = exp6((lo >> 5) & 63), b0 = exp5(lo & 31);
       const int r1 = exp5(hi >> 11), g1 = exp6((hi >> 5) & 63), b1 = exp5(hi & 31);
-      const float4 q0 = entry_m(gray, wr, wg, r0, g0, b0), q1 = entry_m(gray, wr, wg, r1, g1, b1);
-      const float4 q2 = entry_m(gray, wr, wg, (r0 * 2 + r1 + a) / 3, (g0 * 2 + g1 + a) / 3, (b0 * 2 + b1 + a) / 3);
-      const float4 q3 = entry_m(gray, wr, wg, (r1 * 2 + r0 + a) / 3, (g1 * 2 + g0 + a) / 3, (b1 * 2 + b0 + a) / 3);
-      const float4 q4 = entry_m(gray, wr, wg, (r0 + r1 + a) >> 1, (g0 + g1 + a) >> 1, (b0 + b1 + a) >> 1);
-      if (__any_sync(FULL_MASK, live)) {
+      // the palette in floats (converted integer palettes: 3.69 ms for the chain, now 3.62): a third's or a
+      // half's floor through 2^23's unit in the last place
+      // (2 x + y + a is at most 766, and 1/3 rounds up, so a multiple of three stays at or above its third)
+      const float fa = (float)a;
+      const float fr0 = (float)r0, fg0 = (float)g0, fb0 = (float)b0, fr1 = (float)r1, fg1 = (float)g1, fb1 = (float)b1;
+      auto third = [&](float x, float y) { return __fmaf_rz(fmaf(2.f, x, y + fa), 0.33333334f, 8388608.f) - 8388608.f; };
+      auto half = [&](float x, float y) { return __fmaf_rz(x + (y + fa), 0.5f, 8388608.f) - 8388608.f; };
+      const float4 q0 = half_entry_m(gray, wr, wg, fr0, fg0, fb0), q1 = half_entry_m(gray, wr, wg, fr1, fg1, fb1);
+      const float4 q2 = half_entry_m(gray, wr, wg, third(fr0, fr1), third(fg0, fg1), third(fb0, fb1));
+      const float4 q3 = half_entry_m(gray, wr, wg, third(fr1, fr0), third(fg1, fg0), third(fb1, fb0));
+      const float4 q4 = half_entry_m(gray, wr, wg, half(fr0, fr1), half(fg0, fg1), half(fb0, fb1));
+      {
         int k = 0;
         if (!fast) {
-          for (; k < n; k++) {
-            const float4 x = S.ecf[k];
-            const uint32_t w = S.ecw[k];
-            const float m01 = fminf(dist_part(x, q0), dist_part(x, q1));
-            e0 += w * f2u_exact(__fadd_rn(x.w, fminf(m01, fminf(dist_part(x, q2), dist_part(x, q3)))));
-            if (three) e1 += w * f2u_exact(__fadd_rn(x.w, fminf(m01, dist_part(x, q4))));
-            if ((k & 1) == 1 &&
-                __all_sync(FULL_MASK, !live || (only3 ? e1 : (three ? min(e0, e1) : e0)) >= B0)) { k++; break; }
+          const uint64_t ax = pack2(q0.x, q1.x), ay = pack2(q0.y, q1.y), az = pack2(q0.z, q1.z), aw = pack2(q0.w, q1.w);
+          const uint64_t cx = pack2(q2.x, q3.x), cy = pack2(q2.y, q3.y), cz = pack2(q2.z, q3.z), cw = pack2(q2.w, q3.w);
+          auto colour = [&](const EvalColour& v) {
+            const ulonglong2 xy = reinterpret_cast<const ulonglong2*>(&v)[0];
+            const ulonglong2 zw = reinterpret_cast<const ulonglong2*>(&v)[1];
+            float d0, d1, d2, d3, xb, wf;
+            unpack2(fma2(zw.x, az, fma2(xy.y, ay, fma2(xy.x, ax, aw))), d0, d1);
+            unpack2(fma2(zw.x, cz, fma2(xy.y, cy, fma2(xy.x, cx, cw))), d2, d3);
+            unpack2(zw.y, xb, wf);
+            const uint32_t w = __float_as_uint(wf);
+            const float m01 = fminf(d0, d1);
+            e0 += w * b2u_exact(__fadd_rn(xb, min3(m01, d2, d3)));
+            float nx, ny, nz, u;
+            unpack2(xy.x, nx, u);
+            unpack2(xy.y, ny, u);
+            unpack2(zw.x, nz, u);
+            e1 += w * b2u_exact(__fadd_rn(xb, fminf(m01, fmaf(nz, q4.z, fmaf(ny, q4.y, fmaf(nx, q4.x, q4.w))))));
+          };
+          #pragma unroll 1
+          for (; k < n; k += 2) {
+            colour(S.ecv[k]);
+            colour(S.ecv[k + 1]);
+            if (__all_sync(FULL_MASK, !live || (only3 ? e1 : (three ? min(e0, e1) : e0)) >= B0)) { k += 2; break; }
           }
+          k = min(k, n);
         } else {
           FastSel f4, f3;
           const bool perc = S.st.perceptual != 0;
           f4.init(perc, false, a, r0, g0, b0, r1, g1, b1);
           f3.init(perc, true, a, r0, g0, b0, r1, g1, b1);
           for (; k < n; k++) {
-            const float4 x = S.ecf[k];
+            const EvalColour& v = S.ecv[k];
+            const float4 x = make_float4(-v.nx[0], -v.ny[0], -v.nz[0], v.xb);  // twice the colour
             const uint32_t c = S.eci[k];
-            const uint32_t w = S.ecw[k];
+            const uint32_t w = v.w;
             if (!only3) {
               const int s4 = f4.pick(c);
               const float4 q = s4 == 0 ? q0 : s4 == 1 ? q1 : s4 == 2 ? q2 : q3;
-              e0 += w * f2u_exact(__fadd_rn(x.w, dist_part(x, q)));
+              e0 += w * b2u_exact(__fadd_rn(x.w, dist_part(x, q)));
             }
             if (three) {
               const int s3 = f3.pick(c);
               const float4 q = s3 == 0 ? q0 : s3 == 1 ? q1 : q4;
-              e1 += w * f2u_exact(__fadd_rn(x.w, dist_part(x, q)));
+              e1 += w * b2u_exact(__fadd_rn(x.w, dist_part(x, q)));
             }
             if ((k & 3) == 3 &&
                 __all_sync(FULL_MASK, !live || (only3 ? e1 : (three ? min(e0, e1) : e0)) >= B0)) { k++; break; }
@@ -833,17 +909,10 @@ __device__ __noinline__ int run_list(WarpShared& S, int start, uint32_t& work) {
       ok = __ballot_sync(FULL_MASK, live && lb < B && err < B) & after;
     }
     __syncwarp();
-    if (compact) {
-      const int rest = qn - take;
-      const uint2 v = (int)lane < rest ? S.pq[take + lane] : make_uint2(0u, 0u);
-      __syncwarp();
-      if ((int)lane < rest) S.pq[lane] = v;
-      __syncwarp();
-      qn = rest;
-    } else if (last >= 0) {
+    if (!compact && last >= 0) {
       if (d.stop_on_accept) return i0 + last;
       i0 += last + 1;
-    } else {
+    } else if (!compact) {
       i0 += 32;
     }
   }
@@ -892,16 +961,12 @@ __device__ __noinline__ bool refine(WarpShared& S, uint32_t& work, int level = 1
     comp = clampi(__double2int_rz(v), 0, k == 1 ? 63 : 31);
   }
   const int mine = comp;
-  for (int k = 0; k < 6; k++) {
-    const int v = __shfl_sync(FULL_MASK, mine, k);
-    if (lane == 0) S.d.e[k] = v;
-  }
+  if (lane < 6) S.d.e[lane] = mine;
+  __syncwarp();
+  if (lane < 2) S.d.pk[lane] = pack565(S.d.e[3 * lane], S.d.e[3 * lane + 1], S.d.e[3 * lane + 2]);
   __syncwarp();
   if (level == 0) {
-    if (lane == 0) {
-      const uint32_t p0 = pack565(S.d.e[0], S.d.e[1], S.d.e[2]), p1 = pack565(S.d.e[3], S.d.e[4], S.d.e[5]);
-      S.cand[0] = canon_lo(p0, p1) | (canon_hi(p0, p1) << 16);
-    }
+    if (lane == 0) S.cand[0] = canon_lo(S.d.pk[0], S.d.pk[1]) | (canon_hi(S.d.pk[0], S.d.pk[1]) << 16);
     set_list(S, LK_TABLE, 1, 0, 0);
   } else {
     set_list(S, LK_REFINE, 54, 0, 0);
@@ -992,7 +1057,11 @@ __device__ __noinline__ void comp_errors(WarpShared& S, int comp) {
         m = min(m, W[k] * pv * pv - WP2[k] * pv + WPP[k]);
       }
     } else {
-      for (uint32_t v = lane; v < 256; v += 32) m = min(m, W[k] * v * v - WP2[k] * v + WPP[k]);
+      // over all 256 values: the quadratic is least next to the weighted mean WP2 / 2W, which the 32
+      // values around its rounded quotient hold (a weight of 0 makes it 0 everywhere)
+      const float mean = __fdividef((float)WP2[k], (float)(2u * W[k]));
+      const uint32_t v = (uint32_t)clampi((W[k] ? (int)mean : 0) - 15 + (int)lane, 0, 255);
+      m = W[k] * v * v - WP2[k] * v + WPP[k];
     }
     rem[k] = __reduce_min_sync(FULL_MASK, m);
   }
@@ -1032,11 +1101,17 @@ __device__ __noinline__ void optimize_comps(WarpShared& S, uint32_t& work) {
     uint32_t best_err = E(0, ex(lo_u[comp])) + E(1, ex(hi_u[comp])) + E(2, (uint32_t)((p0s * 2 + p1s) / 3)) +
                         E(3, (uint32_t)((p0s + p1s * 2) / 3));
     if (rem[0] >= best_err) continue;
+    // the low components whose table error leaves room below the best's, from `from` on, 32 at a time
+    // (each visit looks again: an acceptance changes the tables and the best)
     #pragma unroll 1
-    for (int c0 = 0; c0 < limit; c0++) {
+    for (int from = 0; from < limit;) {
+      const int cl = (from & ~31) + (int)lane;
+      const unsigned room = __ballot_sync(FULL_MASK, cl >= from && E(0, ex(cl)) + rem[1] < best_err);
+      if (!room) { from = (from & ~31) + 32; continue; }
+      const int c0 = (from & ~31) + __ffs(room) - 1;
+      from = c0 + 1;
       const uint32_t p0 = ex(c0);
       uint32_t e0 = E(0, p0);
-      if (e0 + rem[1] >= best_err) continue;
       {
         // does any c1 pass the component-table prune for this c0 (:456-466)? lane c1 and c1 + 32;
         // a pair passes exactly when its component error is below the best's
@@ -1230,16 +1305,13 @@ __device__ void optimize(WarpShared& S, uint32_t& work) {
     // lattice neighbours: low endpoint (26 adjacent cells, then +-2 per axis), then high
     #pragma unroll 1
     for (int side = 0; side < (quality >= kQNormal ? 2 : 0); side++) {
-      for (int kind = LK_NEIGH; kind <= (quality == kQUber ? LK_MOVE2 : LK_NEIGH); kind++) {
-        if (lane == 0) {
-          const uint32_t base = side ? S.st.best.hi : S.st.best.lo;
-          S.d.base[0] = (int)(base >> 11); S.d.base[1] = (int)((base >> 5) & 63); S.d.base[2] = (int)(base & 31);
-          S.d.kind = kind; S.d.count = kind == LK_NEIGH ? 26 : 6; S.d.dependent = 1; S.d.alt = 0;
-          S.d.stop_on_accept = 0; S.d.side = side;
-        }
-        __syncwarp();
-        run_list<G>(S, 0, work);
+      if (lane == 0) {
+        S.d.base[0] = (int)(side ? S.st.best.hi : S.st.best.lo);
+        S.d.kind = LK_LATTICE; S.d.count = quality == kQUber ? kNeighbours + 6 : kNeighbours; S.d.dependent = 1; S.d.alt = 0;
+        S.d.stop_on_accept = 0; S.d.side = side;
       }
+      __syncwarp();
+      run_list<G>(S, 0, work);
     }
     if (!S.st.best.err || (pass && S.st.best.err == prev)) break;
     if (quality == kQUber) refine<G>(S, work);
@@ -1404,7 +1476,16 @@ __device__ uint32_t phase2_block(WarpShared& S, const uint8_t* __restrict__ px, 
       const float kj = __shfl_sync(FULL_MASK, key, j);
       rank += (kj > key || (kj == key && j < (int)lane)) ? 1 : 0;
     }
-    if ((int)lane < n) { S.ecf[rank] = x; S.ecw[rank] = w; S.eci[rank] = c; }
+    if ((int)lane < n) {
+      EvalColour& v = S.ecv[rank];
+      v.nx[0] = v.nx[1] = -2.f * x.x;
+      v.ny[0] = v.ny[1] = -2.f * x.y;
+      v.nz[0] = v.nz[1] = -2.f * x.z;
+      v.xb = __fadd_rn(x.w, 8388608.0f);
+      v.w = w;
+      S.eci[rank] = c;
+    }
+    if (lane == 16) S.ecv[n] = EvalColour{{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, 8388608.0f, 0u};
   }
   // m_evaluate_hc (:2085): Uber, no 3-colour blocks, no transparency, no grayscale sampling
   const bool hc = quality == kQUber && !use_alpha && !has_t && !gray;
