@@ -1716,138 +1716,163 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
 // ------------------------------------------------------------------------------------------
 // DXT5A: warp per block, lane per (low, high) candidate.
 
-struct Alpha5 {
-  int n;
-  uint32_t val[16], wt[16];
-  bool both;
-  // error of both block types for one (l, h); 8-value preferred on ties
-  __device__ __forceinline__ void eval(int l, int h, uint32_t& err, int& type) const {
-    int p8[8], p6[8];
-    p8[0] = l; p8[1] = h;
-    p8[2] = (l * 6 + h) / 7; p8[3] = (l * 5 + h * 2) / 7; p8[4] = (l * 4 + h * 3) / 7;
-    p8[5] = (l * 3 + h * 4) / 7; p8[6] = (l * 2 + h * 5) / 7; p8[7] = (l + h * 6) / 7;
-    p6[0] = l; p6[1] = h;
-    p6[2] = (l * 4 + h) / 5; p6[3] = (l * 3 + h * 2) / 5; p6[4] = (l * 2 + h * 3) / 5; p6[5] = (l + h * 4) / 5;
-    p6[6] = 0; p6[7] = 255;
-    uint32_t e8 = 0, e6 = 0;
-    for (int i = 0; i < n; i++) {
-      const int v = (int)val[i];
-      int m8 = 1 << 30, m6 = 1 << 30;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int d8 = v - p8[j], d6 = v - p6[j];
-        m8 = min(m8, d8 * d8);
-        m6 = min(m6, d6 * d6);
-      }
-      e8 += (uint32_t)m8 * wt[i];
-      e6 += (uint32_t)m6 * wt[i];
-    }
-    if (both && e6 < e8) { err = e6; type = 1; }
-    else { err = e8; type = 0; }
+// A warp's block: its unique values in evaluation order, farthest from the middle of their range first
+// so that the sums pass the best's early, two at a time (one of weight 0 pads them).
+struct AlphaShared {
+  float4 val[17];     // v, v + 2^23, weight, distance to 0 or 255
+  uint32_t uniq[16];  // first-occurrence order, the order of the pairs
+};
+
+// A lane's candidate (l, h), for the distance of a value to the nearest of lo + floor(k (hi - lo) / n),
+// k = 0 .. n. The value's own position in units of (hi - lo) / n, rounded down, gives the two entries
+// around it (an integer between two reals is between their floors too; at a rounding error across a
+// whole position the value is the entry itself and in both brackets), so a value costs 11 operations
+// for a block type and not the 24 of all eight entries. Floors are multiply-adds onto 2^23, rounded
+// down. hi == lo gives a NaN, which saturates to position 0. Sums of weighted squares are integers
+// below 2^24. With the integer loop over both palettes a channel of a 2048 x 2048 image took 237 us.
+struct AlphaRange {
+  float r, o, d7, d5, base;
+  __device__ __forceinline__ AlphaRange(int l, int h) {
+    const float lo = (float)min(l, h), d = (float)max(l, h) - lo;
+    r = __fdividef(1.f, d);
+    o = -lo * r;
+    d7 = __fmul_ru(d, 0.14285715f);
+    d5 = __fmul_ru(d, 0.2f);
+    base = lo + 8388608.f;
+  }
+  __device__ __forceinline__ float position(float v) const { return __saturatef(fmaf(v, r, o)); }
+  __device__ __forceinline__ float nearest(float v23, float u, float below_n, float dn) const {
+    const float k = __fmaf_rd(u, below_n, 8388608.f) - 8388608.f;
+    return fminf(fabsf(v23 - __fmaf_rd(k, dn, base)), fabsf(__fmaf_rd(k + 1.f, dn, base) - v23));
   }
 };
+
+// The errors of the warp's candidates, 8-value preferred on ties; where no lane's can be below `best`
+// any more the rest of the values is left out, and what is returned is at or above `best`.
+__device__ __forceinline__ float alpha_errors(const AlphaShared& S, int n, bool both, bool valid, int l, int h,
+                                              float best, int& type) {
+  const AlphaRange c(l, h);
+  float e8 = valid ? 0.f : 1e30f, e6 = valid && both ? 0.f : 1e30f;
+#pragma unroll 1
+  for (int i = 0; i < n; i += 2) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float4 x = S.val[i + k];
+      const float u = c.position(x.x);
+      const float m8 = c.nearest(x.y, u, 6.9999995f, c.d7);
+      e8 = fmaf(m8 * m8, x.z, e8);
+      if (both) {
+        const float m6 = fminf(c.nearest(x.y, u, 4.9999995f, c.d5), x.w);
+        e6 = fmaf(m6 * m6, x.z, e6);
+      }
+    }
+    if (__all_sync(FULL_MASK, fminf(e8, e6) >= best)) break;
+  }
+  type = e6 < e8;
+  return fminf(e8, e6);
+}
 
 // One DXT5A element (dxt5_endpoint_optimizer::compute, crnlib/crn_dxt5a.cpp:40-196) of the 4x4
 // RGBA8 block px on channel comp, written as 8 bytes to o; a whole warp, lane per candidate.
 // quality: crn_dxt_quality; the probe grid is +-16 at Uber, +-8 at Better and absent below (:105-110).
-__device__ __forceinline__ void alpha_block(const uint8_t* __restrict__ px, int comp, int both, uint32_t quality,
-                                            uint8_t* __restrict__ o) {
+__device__ __forceinline__ void alpha_block(AlphaShared& S, const uint8_t* __restrict__ px, int comp, bool both,
+                                            uint32_t quality, uint8_t* __restrict__ o) {
   const uint32_t lane = lane_id();
   const uint32_t v = lane < 16 ? __ldg(px + lane * 4 + comp) : 0x100u + lane;
   const unsigned match = __match_any_sync(FULL_MASK, v);
   const int leader = __ffs(match) - 1;
   const bool is_leader = lane < 16 && leader == (int)lane;
   const unsigned lmask = __ballot_sync(FULL_MASK, is_leader);
-  Alpha5 A;
-  A.n = __popc(lmask);
-  A.both = both != 0;
-  const int uidx = __popc(lmask & ((1u << leader) - 1u));
-  // every lane gets the unique values (first-occurrence order) and weights
-  {
-    unsigned m = lmask;
-    for (int i = 0; i < A.n; i++) {
-      const int src = __ffs(m) - 1;
-      m &= m - 1;
-      A.val[i] = __shfl_sync(FULL_MASK, v, src);
-      A.wt[i] = (uint32_t)__popc(__shfl_sync(FULL_MASK, match, src));
-    }
-  }
-  uint32_t first = 0, second = 0, berr = kInf;
-  int btype = 0;
-  if (A.n == 1) {
-    if (lane == 0) {
-      uint2 w = make_uint2(A.val[0] | (A.val[0] << 8), 0u);
-      *reinterpret_cast<uint2*>(o) = w;
-    }
+  const int n = __popc(lmask);
+  if (n == 1) {
+    if (lane == 0) *reinterpret_cast<uint2*>(o) = make_uint2(v | (v << 8), 0u);
     return;
   }
-  auto accept_chain = [&](bool valid, int l, int h, uint32_t err, int type, bool dependent) -> int {
-    unsigned ok = __ballot_sync(FULL_MASK, valid && err < berr);
+  {
+    // order of evaluation: by distance from the middle of the range, in half units
+    const int vmin = (int)__reduce_min_sync(FULL_MASK, lane < 16 ? v : 255u);
+    const int vmax = (int)__reduce_max_sync(FULL_MASK, lane < 16 ? v : 0u);
+    const int far = abs(2 * (int)v - vmin - vmax);
+    int rank = 0;
+    for (unsigned m = lmask; m; m &= m - 1) {
+      const int j = __ffs(m) - 1, other = __shfl_sync(FULL_MASK, far, j);
+      rank += other > far || (other == far && j < (int)lane);
+    }
+    __syncwarp();  // the previous block's reads are done
+    if (is_leader) {
+      const float fv = (float)v;
+      S.val[rank] = make_float4(fv, fv + 8388608.f, (float)__popc(match), fminf(fv, 255.f - fv));
+      S.uniq[__popc(lmask & ((1u << lane) - 1u))] = v;
+    }
+    if (lane == 0) S.val[n] = make_float4(0.f, 8388608.f, 0.f, 0.f);
+    __syncwarp();
+  }
+  int first = 0, second = 0, btype = 0;
+  float berr = 1e30f;
+  auto accept_chain = [&](int l, int h, float err, int type, bool dependent) -> int {
+    unsigned ok = __ballot_sync(FULL_MASK, err < berr);
     int last = -1;
     while (ok) {
       const int j = __ffs(ok) - 1;
       berr = __shfl_sync(FULL_MASK, err, j);
-      first = (uint32_t)__shfl_sync(FULL_MASK, l, j);
-      second = (uint32_t)__shfl_sync(FULL_MASK, h, j);
-      btype = __shfl_sync(FULL_MASK, type, j);
       last = j;
       if (dependent) break;
       const unsigned after = j == 31 ? 0u : (FULL_MASK << (j + 1));
-      ok = __ballot_sync(FULL_MASK, valid && err < berr) & after;
+      ok = __ballot_sync(FULL_MASK, err < berr) & after;
+    }
+    if (last >= 0) {
+      first = __shfl_sync(FULL_MASK, l, last);
+      second = __shfl_sync(FULL_MASK, h, last);
+      btype = __shfl_sync(FULL_MASK, type, last);
     }
     return last;
   };
   // all unique value pairs i < j (compute :83-96)
-  const int npairs = A.n * (A.n - 1) / 2;
+  const int npairs = n * (n - 1) / 2;
+  const float half = (float)n - 0.5f;
+#pragma unroll 1
   for (int p0 = 0; p0 < npairs; p0 += 32) {
     const int p = p0 + (int)lane;
-    int l = 0, h = 0;
-    const bool valid = p < npairs;
-    if (valid) {
-      int i = 0, rem = p;
-      while (rem >= A.n - 1 - i) { rem -= A.n - 1 - i; i++; }
-      l = (int)A.val[i];
-      h = (int)A.val[i + 1 + rem];
+    int l = 0, h = 0, type;
+    if (p < npairs) {
+      // i (2 n - 1 - i) / 2 pairs are before row i; 1e-4 is far below the root's distance to the next row's
+      const int i = (int)(half - sqrtf(half * half - (float)(2 * p)) + 1e-4f);
+      l = (int)S.uniq[i];
+      h = (int)S.uniq[p - i * (2 * n - 1 - i) / 2 + i + 1];
     }
-    uint32_t err = kInf;
-    int type = 0;
-    if (valid) A.eval(l, h, err, type);
-    accept_chain(valid, l, h, err, type, false);
+    const float err = alpha_errors(S, n, both, p < npairs, l, h, berr, type);
+    accept_chain(l, h, err, type, false);
   }
   // +-R probe around the running best (:98-141); the centre moves with each improvement
   const int R = quality == kQUber ? 16 : 8, D = 2 * R + 1;
-  if (berr && quality >= kQBetter) {
-    int pos = 0, row_l = (int)first - R;
+  const int over_d = R == 16 ? 1986 : 3856;  // p / D is p * over_d >> 16 for the p below
+  if (berr != 0.f && quality >= kQBetter) {
+    int pos = 0, row_l = first - R;
     const int total = D * D;
+#pragma unroll 1
     while (pos < total) {
       const int p = pos + (int)lane;
-      const int row0 = pos / D;
-      int l = 0, h = 0;
-      bool valid = p < total;
-      if (valid) {
-        const int r = p / D, c = p % D;
-        l = r == row0 ? row_l : (int)first + (r - R);
-        h = (int)second + (c - R);
-        valid = l >= 0 && l <= 255 && h >= 0 && h <= 255;
-      }
-      uint32_t err = kInf;
-      int type = 0;
-      if (valid) A.eval(l, h, err, type);
-      const int last = accept_chain(valid, l, h, err, type, true);
+      const int row0 = pos * over_d >> 16, r = p * over_d >> 16;
+      int type;
+      const int l = r == row0 ? row_l : first + (r - R);
+      const int h = second + (p - r * D - R);
+      const bool valid = p < total && (unsigned)l <= 255u && (unsigned)h <= 255u;
+      const float err = alpha_errors(S, n, both, valid, l, h, berr, type);
+      const int last = accept_chain(l, h, err, type, true);
       const int next = last >= 0 ? pos + last + 1 : pos + 32;
-      const int nrow = next / D;
+      const int nrow = next * over_d >> 16;
       // the reference fixes l when a row starts: a row begun inside this batch used the
       // centre from before the batch, unless it is the accepted candidate's own row
-      const int last_row = last >= 0 ? (pos + last) / D : -1;
+      const int last_row = last >= 0 ? (pos + last) * over_d >> 16 : -1;
       if (last >= 0 && nrow == last_row) row_l = __shfl_sync(FULL_MASK, l, last);
-      else if (nrow != row0) row_l = (int)first + (nrow - R);
+      else if (nrow != row0) row_l = first + (nrow - R);
       pos = next;
     }
   }
   // selectors of the winner, reorder rules (:143-185), pack (dxt5_block, crn_dxt.h:318-361)
   int sel = 0;
   if (lane < 16) {
-    const int l = (int)first, h = (int)second;
+    const int l = first, h = second;
     int pv[8];
     pv[0] = l; pv[1] = h;
     if (btype == 0) {
@@ -1857,26 +1882,25 @@ __device__ __forceinline__ void alpha_block(const uint8_t* __restrict__ px, int 
       pv[2] = (l * 4 + h) / 5; pv[3] = (l * 3 + h * 2) / 5; pv[4] = (l * 2 + h * 3) / 5; pv[5] = (l + h * 4) / 5;
       pv[6] = 0; pv[7] = 255;
     }
-    const int x = (int)A.val[uidx];
+    const int x = (int)v;
     int bd = 1 << 30;
+#pragma unroll
     for (int j = 0; j < 8; j++) {
       const int d = (x - pv[j]) * (x - pv[j]);
       if (d < bd) { bd = d; sel = j; }
     }
   }
-  uint32_t f = first, s = second;
+  uint32_t f = (uint32_t)first, s = (uint32_t)second;
   if (f == s) {
     sel = 0;
   } else if (btype) {
     if (f > s) {
       const uint32_t t = f; f = s; s = t;
-      const int inv6[8] = {1, 0, 5, 4, 3, 2, 6, 7};
-      sel = inv6[sel];
+      sel = 0x76234501 >> (4 * sel) & 7;  // 1, 0, 5, 4, 3, 2, 6, 7
     }
   } else if (f <= s) {
     const uint32_t t = f; f = s; s = t;
-    const int inv8[8] = {1, 0, 7, 6, 5, 4, 3, 2};
-    sel = inv8[sel];
+    sel = 0x23456701 >> (4 * sel) & 7;  // 1, 0, 7, 6, 5, 4, 3, 2
   }
   const uint32_t lo_bits = __reduce_or_sync(FULL_MASK, lane < 10 ? ((uint32_t)sel << (3 * lane)) : 0u);
   const uint32_t hi_bits = __reduce_or_sync(FULL_MASK, (lane >= 10 && lane < 16) ? ((uint32_t)sel << (3 * (lane - 10))) : 0u);
@@ -1892,8 +1916,10 @@ __global__ void __launch_bounds__(128)
                    uint8_t* __restrict__ out, uint32_t out_stride) {
   const uint32_t warp_global = blockIdx.x * 4 + (threadIdx.x >> 5);
   const uint32_t nwarps = gridDim.x * 4;
+  __shared__ AlphaShared shared[4];
   for (uint32_t bi = warp_global; bi < n; bi += nwarps)
-    alpha_block(blocks + (size_t)bi * 64, comp, both, quality, out + (size_t)bi * out_stride);
+    alpha_block(shared[threadIdx.x >> 5], blocks + (size_t)bi * 64, comp, both != 0, quality,
+                out + (size_t)bi * out_stride);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1976,15 +2002,17 @@ __global__ void __launch_bounds__(128)
                           const EncodeSegment* __restrict__ segs) {
   const uint32_t warp_global = blockIdx.x * 4 + (threadIdx.x >> 5);
   const uint32_t nwarps = gridDim.x * 4;
+  __shared__ AlphaShared shared[4];
   for (uint32_t c = warp_global; c < nchunks; c += nwarps) {
     const EncodeChunk ch = chunks[c];
     const EncodeSegment sg = segs[ch.segment];
     const int comp = (int)((sg.options >> kSegCompShift) & 3u);
-    const int both = (sg.options & kSegBothTypes) ? 1 : 0;
+    const bool both = (sg.options & kSegBothTypes) != 0;
     const uint32_t quality = (sg.options >> kSegAlphaQualityShift) & 7u;
     for (uint32_t k = 0; k < ch.count; k++) {
       const uint32_t b = ch.first + k;
-      alpha_block(blocks + (size_t)b * 64, comp, both, quality, sg.out + (size_t)(b - sg.first_block) * sg.stride);
+      alpha_block(shared[threadIdx.x >> 5], blocks + (size_t)b * 64, comp, both, quality,
+                  sg.out + (size_t)(b - sg.first_block) * sg.stride);
     }
   }
 }
