@@ -121,7 +121,7 @@ constexpr int kSeedLanes = 32;
 struct SeedShared {
   // scratch, transposed [i][lane] so lanes never share a bank
   uint32_t t_col[16][kSeedLanes];
-  uint8_t t_w[16][kSeedLanes];
+  float t_w[16][kSeedLanes];
   float t_norm[3][16][kSeedLanes];
   // the warp's 4x4 blocks (RGBA8, 64 bytes each), staged by bulk copies (TMA) that complete on
   // `bar`; the next group's copies are issued once the lanes have read this one
@@ -163,7 +163,7 @@ struct WarpShared {
 static_assert((sizeof(WarpShared) * kWarpsPerCta + 1024) * kCtasPerSm <= 228 * 1024,
               "DXT1 encoder shared memory per CTA");
 constexpr int kSeedCtasPerSm = 4;
-static_assert((sizeof(SeedShared) * kWarpsPerCta + 1024) * kSeedCtasPerSm <= 228 * 1024,
+static_assert((sizeof(SeedShared) * kWarpsPerCta + 2048) * kSeedCtasPerSm <= 228 * 1024,
               "DXT1 phase-1 shared memory per CTA");
 
 // ------------------------------------------------------------------------------------------
@@ -172,10 +172,11 @@ static_assert((sizeof(SeedShared) * kWarpsPerCta + 1024) * kSeedCtasPerSm <= 228
 struct V3f { float x, y, z; };
 
 // intersection::ray_aabb against [0,1]^3 (crn_intersect.h:44-132); true on cSuccess
-__device__ bool ray_unit_box(float o[3], const float d[3], float out[3]) {
+__device__ __forceinline__ bool ray_unit_box(const float* o, const float* d, float* out) {
   int quad[3];
   float cand[3] = {0.f, 0.f, 0.f};
   bool inside = true;
+#pragma unroll
   for (int i = 0; i < 3; i++) {
     if (o[i] < 0.0f) { quad[i] = 1; cand[i] = 0.0f; inside = false; }
     else if (o[i] > 1.0f) { quad[i] = 0; cand[i] = 1.0f; inside = false; }
@@ -183,14 +184,18 @@ __device__ bool ray_unit_box(float o[3], const float d[3], float out[3]) {
   }
   if (inside) return false;
   float mt[3];
+#pragma unroll
   for (int i = 0; i < 3; i++) mt[i] = (quad[i] != 2 && d[i] != 0.0f) ? __fdiv_rn(__fsub_rn(cand[i], o[i]), d[i]) : -1.0f;
   int wp = 0;
-  for (int i = 1; i < 3; i++) if (mt[wp] < mt[i]) wp = i;
-  if (mt[wp] < 0.0f) return false;
+  float far = mt[0];
+#pragma unroll
+  for (int i = 1; i < 3; i++) if (far < mt[i]) { far = mt[i]; wp = i; }
+  if (far < 0.0f) return false;
   float c[3];
+#pragma unroll
   for (int i = 0; i < 3; i++) {
     if (i != wp) {
-      c[i] = __fadd_rn(o[i], __fmul_rn(mt[wp], d[i]));
+      c[i] = __fadd_rn(o[i], __fmul_rn(far, d[i]));
       if (c[i] < 0.0f || c[i] > 1.0f) return false;
     } else {
       c[i] = cand[i];
@@ -200,15 +205,26 @@ __device__ bool ray_unit_box(float o[3], const float d[3], float out[3]) {
   return true;
 }
 
-// fast_random (crnlib/crn_rand.cpp:310-405) with its default seed
+// fast_random (crnlib/crn_rand.cpp:310-405) with its default seed, and its frand(-.00196, .00196):
+// (float)(l + (h - l) (r / 2^32)) in double. The value itself is a whole multiple of 2^-63 (.00196f is one
+// of 2^-32) within 64 bits; the double's roundings move it by less than 4 of them, which only matters
+// where that changes the float it is rounded to (a conversion of a few cycles, against 64 for every
+// double instruction).
 struct FastRandom {
   uint32_t jsr = 0xABCD917Au, jcong = 0x17F3DEADu;
-  __device__ float frand(float l, float h) {
+  __device__ float jitter() {
     jsr ^= (jsr << 17); jsr ^= (jsr >> 13); jsr ^= (jsr << 5);
     jcong = 69069u * jcong + 1234567u;
     const uint32_t r32 = jsr ^ jcong;
+    const float h = .00196f;
+    const long long v = (long long)(int)(r32 - 0x80000000u) * (long long)(h * 4294967296.f);
+    const float lo = __ll2float_rn(v - 4), hi = __ll2float_rn(v + 4);
+    return (lo == hi ? lo * 1.0842022e-19f : in_double(r32));  // 2^-63
+  }
+  static __device__ __noinline__ float in_double(uint32_t r32) {
+    const float l = -.00196f, h = .00196f;
     const double t = __dmul_rn((double)r32, 1.0 / 4294967296.0);
-    float r = (float)__dadd_rn((double)l, __dmul_rn((double)__fsub_rn(h, l), t));
+    const float r = (float)__dadd_rn((double)l, __dmul_rn((double)__fsub_rn(h, l), t));
     return r < l ? l : (r > h ? h : r);
   }
 };
@@ -228,11 +244,65 @@ __device__ __forceinline__ bool is_transparent(uint32_t c, uint32_t opts) {
   return a < ((opts >> kD1ThresholdShift) & 255u);
 }
 
+// The seeds are bound by double precision: an instruction takes a scheduler 64 cycles whatever its
+// active lanes, the SM one every 19 (pow() of a warp 6100 cycles, __ddiv_rn 575, __drcp_rn 365). What
+// only has to come out as the double computation's result rounded to float is therefore computed in
+// pairs of floats (Dekker's double-length arithmetic), and in double when the pair is too close to
+// half way between two floats for its own error, below 2^-44, to leave the rounding certain.
+// With that, the covariance in fused operations, the step of the power iteration in floats and no local
+// array indexed at run time, the seeds of a 64 x 64 image went from 79 to 41 us (half of it still double
+// precision: 6 operations a colour and 24 an iteration), of a 1021 x 683 one from 184 to 87.
+
+// a float as a double; not for denormal numbers
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x);
+  const bool zero = (b << 1) == 0;
+  const uint32_t hi = (b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u);
+  return __hiloint2double((int)(zero ? b : hi), (int)(b << 29));
+}
+// a double of magnitude below 2 as a float, rounded towards zero (below 2^-126 to 0)
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x), mag = hi & 0x7FFFFFFFu;
+  return mag < 0x38100000u ? 0.f
+                           : __uint_as_float((hi & 0x80000000u) | ((mag - 0x38000000u) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ unsigned long long magnitude(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+__device__ __noinline__ float pow_275_double(float s) { return (float)pow((double)s, 2.75); }
+// (float)pow((double)s, 2.75) as s^2 sqrt(s) sqrt(sqrt(s)), s in (0, 1] and not tiny
+__device__ __forceinline__ float pow_275(float s) {
+  const float a1 = __fsqrt_rn(s), a2 = __fdividef(fmaf(-a1, a1, s), 2.f * a1);
+  const float b1 = __fsqrt_rn(a1), b2 = __fdividef(fmaf(-b1, b1, a1) + a2, 2.f * b1);
+  const float t1 = s * s, t2 = fmaf(s, s, -t1);
+  const float p1 = a1 * b1, p2 = fmaf(a1, b1, -p1) + (a1 * b2 + a2 * b1);
+  const float q1 = t1 * p1, q2 = fmaf(t1, p1, -q1) + (t1 * p2 + t2 * p1);
+  const float m = q1 * 9.0949470e-13f;  // 2^-40
+  const float r = q1 + (q2 - m);
+  return r == q1 + (q2 + m) ? r : pow_275_double(s);
+}
+__device__ __noinline__ float inverse_norm_double(float x, float y, float z) {
+  const double n = __dadd_rn(__dadd_rn((double)x, (double)y), (double)z);
+  return n != 0.0 ? (float)__drcp_rn(__dsqrt_rn(n)) : 0.f;
+}
+// (float)(1 / sqrt((double)x + y + z)) by a Newton step from the float's, x, y, z >= 0; 0 for no length
+__device__ __forceinline__ float inverse_norm(float x, float y, float z) {
+  const float s1 = x + y, v1 = s1 - x, e1 = (x - (s1 - v1)) + (y - v1);
+  const float n1 = s1 + z, v2 = n1 - s1, n2 = e1 + ((s1 - (n1 - v2)) + (z - v2));
+  const float f = __frsqrt_rn(n1);
+  const float t1 = f * f, t2 = fmaf(f, f, -t1);
+  const float p = n1 * t1, e = fmaf(n1, t1, -p) + (n1 * t2 + n2 * t1);
+  const float c = f * (((1.f - p) - e) * .5f);
+  const float m = f * 3.6379788e-12f;  // 2^-38
+  const float r = f + (c - m);
+  return r == f + (c + m) && n1 > 1e-20f && n1 < 1e20f ? r : inverse_norm_double(x, y, z);
+}
+
 // Runs handle_multicolor_block up to optimize_endpoints' entry, plus try_median4's seeds, for the
 // block whose 16 texels are pix (lane `slot` of the warp); the hand-off goes to *out.
 template <bool G>
-__device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16], uint32_t opts,
-                             Seed* __restrict__ out) {
+__device__ void phase1_block(SeedShared& S, const float* __restrict__ unit, int slot, const uint32_t (&pix)[16],
+                             uint32_t opts, Seed* __restrict__ out) {
   const int L = slot;
   const bool perceptual = (opts & kD1Perceptual) != 0;
   const uint32_t quality = G ? (opts >> kD1QualityShift) & 7u : kQUber;
@@ -253,17 +323,27 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
     if (has_t || !dark || dark == n) { out->n = -1; return; }
     n = 0;
   }
-  // unique colours of the opaque texels in first-occurrence order (compute_internal :2113-2131)
+  // unique colours of the opaque texels in first-occurrence order (compute_internal :2113-2131); a
+  // transparent texel stands for a colour of its own that is left out. All pairs are compared in
+  // registers: a search through the list so far was a chain of shared-memory loads.
   int opaque = 0;
-  #pragma unroll 1
-  for (int p = 0; p < 16; p++) {
-    if (G && is_transparent(pix[p], opts)) continue;
-    const uint32_t c = pix[p] & 0xFFFFFFu;
-    opaque++;
-    int i = 0;
-    for (; i < n; i++) if (S.t_col[i][L] == c) break;
-    if (i == n) { S.t_col[n][L] = c; S.t_w[n][L] = 1; n++; }
-    else S.t_w[i][L]++;
+  {
+    uint32_t col[16], skip = 0;
+    #pragma unroll
+    for (int p = 0; p < 16; p++) {
+      col[p] = pix[p] & 0xFFFFFFu;
+      if (G && is_transparent(pix[p], opts)) { col[p] = 0xFF000000u | p; skip |= 1u << p; }
+      else opaque++;
+    }
+    #pragma unroll
+    for (int p = 0; p < 16; p++) {
+      int w = 1;
+      #pragma unroll
+      for (int q = p + 1; q < 16; q++) {
+        if (col[q] == col[p]) { w++; skip |= 1u << q; }
+      }
+      if (!(skip & (1u << p))) { S.t_col[n][L] = col[p]; S.t_w[n][L] = (float)w; n++; }
+    }
   }
   out->n = n;
   // no opaque texel, or one colour and no transparency (compute_internal :2205-2227): no search
@@ -280,7 +360,7 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
       const int r = c & 255, g = (c >> 8) & 255, b = c >> 16;
       const int l = (r + g + b + 1) / 3;
       const float lf = (float)l;
-      const float scale = __fdiv_rn((float)S.t_w[i][L], 1.0f > lf ? 1.0f : lf);
+      const float scale = __fdiv_rn(S.t_w[i][L], 1.0f > lf ? 1.0f : lf);
       red = __fadd_rn(red, __fmul_rn(scale, (float)r));
       blue = __fadd_rn(blue, __fmul_rn(scale, (float)b));
       avel = __fadd_rn(avel, lf);
@@ -293,7 +373,7 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
     const float mx = red > blue ? red : blue;
     float s = __fdiv_rn(__fmul_rn(mx, 1.0f), 3.0f);
     s = s < 0.0f ? 0.0f : (s > 1.0f ? 1.0f : s);
-    const float pwr = (float)pow((double)s, 2.75);
+    const float pwr = s > 0.f ? pow_275(s) : 0.f;
     const float p = __fmul_rn(avel, pwr);
     if (!(p >= 1.0f)) {
       passes = 2;
@@ -310,9 +390,8 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
     #pragma unroll 1
     for (int i = 0; i < n; i++) {
       const uint32_t c = S.t_col[i][L];
-      const float wf = (float)S.t_w[i][L];
-      const float v[3] = {__fdiv_rn((float)(c & 255), 255.0f), __fdiv_rn((float)((c >> 8) & 255), 255.0f),
-                          __fdiv_rn((float)(c >> 16), 255.0f)};
+      const float wf = S.t_w[i][L];
+      const float v[3] = {unit[c & 255], unit[(c >> 8) & 255], unit[c >> 16]};
       for (int k = 0; k < 3; k++) {
         mean[k] = __fadd_rn(mean[k], __fmul_rn(v[k], wf));
         meanw[k] = __fadd_rn(meanw[k], __fmul_rn(__fmul_rn(pw[k], v[k]), wf));
@@ -322,12 +401,11 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
     for (int k = 0; k < 3; k++) { mean[k] = __fmul_rn(mean[k], inv); meanw[k] = __fmul_rn(meanw[k], inv); }
     // compute_pca :192-256 (double accumulation in colour order)
     double cov[6] = {0, 0, 0, 0, 0, 0};
-    #pragma unroll 1
+    #pragma unroll 2  // the next colour's products beside this one's sums
     for (int i = 0; i < n; i++) {
       const uint32_t c = S.t_col[i][L];
-      const int w = S.t_w[i][L];
-      const float v[3] = {__fdiv_rn((float)(c & 255), 255.0f), __fdiv_rn((float)((c >> 8) & 255), 255.0f),
-                          __fdiv_rn((float)(c >> 16), 255.0f)};
+      const double w = widen(S.t_w[i][L]);
+      const float v[3] = {unit[c & 255], unit[(c >> 8) & 255], unit[c >> 16]};
       float nv[3];
       for (int k = 0; k < 3; k++) {
         nv[k] = __fsub_rn(v[k], mean[k]);
@@ -337,46 +415,52 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
       const float g = __fsub_rn(__fmul_rn(pw[1], v[1]), meanw[1]);
       const float b = __fsub_rn(__fmul_rn(pw[2], v[2]), meanw[2]);
       const float pr[6] = {__fmul_rn(r, r), __fmul_rn(r, g), __fmul_rn(r, b), __fmul_rn(g, g), __fmul_rn(g, b), __fmul_rn(b, b)};
-      if (w > 1) {
-        for (int k = 0; k < 6; k++) cov[k] = __dadd_rn(cov[k], __dmul_rn((double)pr[k], (double)w));
-      } else {
-        for (int k = 0; k < 6; k++) cov[k] = __dadd_rn(cov[k], (double)pr[k]);
-      }
+      // a product of a float and a weight is exact, so the fused form rounds the sum alone as theirs does
+      for (int k = 0; k < 6; k++) cov[k] = __fma_rn(widen(pr[k]), w, cov[k]);
     }
     double vf[3] = {(double).9f, (double)1.0f, (double).7f};
+    float fv[3] = {.9f, 1.f, .7f};
     #pragma unroll 1
     for (int it = 0; it < 8; it++) {
       double r = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[0]), __dmul_rn(vf[1], cov[1])), __dmul_rn(vf[2], cov[2]));
       double g = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[1]), __dmul_rn(vf[1], cov[3])), __dmul_rn(vf[2], cov[4]));
       double b = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[2]), __dmul_rn(vf[1], cov[4])), __dmul_rn(vf[2], cov[5]));
-      double m = fabs(r);
-      if (fabs(g) > m) m = fabs(g);
-      if (fabs(b) > m) m = fabs(b);
-      if (m > 1e-10) {
-        m = __drcp_rn(m);  // 1.0 / m, correctly rounded
+      // the largest magnitude, compared as integers
+      unsigned long long top = magnitude(r);
+      top = max(top, max(magnitude(g), magnitude(b)));
+      if (top > (unsigned long long)__double_as_longlong(1e-10)) {
+        const double m = __drcp_rn(__longlong_as_double((long long)top));  // 1.0 / m, correctly rounded
         r = __dmul_rn(r, m); g = __dmul_rn(g, m); b = __dmul_rn(b, m);
       }
-      const double d0 = __dsub_rn(vf[0], r), d1 = __dsub_rn(vf[1], g), d2 = __dsub_rn(vf[2], b);
-      const double delta = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
+      // stop once the squared step is below 1e-8: in floats (an error below 1e-10 near that), in double
+      // where those cannot tell
+      const float f[3] = {narrow(r), narrow(g), narrow(b)};
+      bool done = false;
+      if (it > 2) {
+        const float d0 = fv[0] - f[0], d1 = fv[1] - f[1], d2 = fv[2] - f[2];
+        const float step = d0 * d0 + d1 * d1 + d2 * d2;
+        done = step < 1e-8f;
+        if (fabsf(step - 1e-8f) < 2e-10f) {
+          const double e0 = __dsub_rn(vf[0], r), e1 = __dsub_rn(vf[1], g), e2 = __dsub_rn(vf[2], b);
+          done = __dadd_rn(__dadd_rn(__dmul_rn(e0, e0), __dmul_rn(e1, e1)), __dmul_rn(e2, e2)) < 1e-8;
+        }
+      }
       vf[0] = r; vf[1] = g; vf[2] = b;
-      if (it > 2 && delta < 1e-8) break;
+      fv[0] = f[0]; fv[1] = f[1]; fv[2] = f[2];
+      if (done) break;
     }
     const double len = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], vf[0]), __dmul_rn(vf[1], vf[1])), __dmul_rn(vf[2], vf[2]));
     if (len < 1e-10) {
       axis[0] = .2837149f; axis[1] = 0.9540631f; axis[2] = 0.096277453f;
     } else {
-      const double il = __ddiv_rn(1.0, __dsqrt_rn(len));
+      const double il = __drcp_rn(__dsqrt_rn(len));
       axis[0] = (float)__dmul_rn(vf[0], il); axis[1] = (float)__dmul_rn(vf[1], il); axis[2] = (float)__dmul_rn(vf[2], il);
     }
     for (int k = 0; k < 3; k++) axis[k] = __fdiv_rn(axis[k], pw[k]);
     // vec::normalize (crn_vec.h:674-690): float squares accumulated in double
-    double nn = (double)__fmul_rn(axis[0], axis[0]);
-    nn = __dadd_rn(nn, (double)__fmul_rn(axis[1], axis[1]));
-    nn = __dadd_rn(nn, (double)__fmul_rn(axis[2], axis[2]));
-    if (nn != 0.0) {
-      const float sc = (float)__ddiv_rn(1.0, __dsqrt_rn(nn));
+    const float sc = inverse_norm(__fmul_rn(axis[0], axis[0]), __fmul_rn(axis[1], axis[1]), __fmul_rn(axis[2], axis[2]));
+    if (sc != 0.f)
       for (int k = 0; k < 3; k++) axis[k] = __fmul_rn(axis[k], sc);
-    }
     if (passes > 1) {
       if (fabsf(axis[0]) >= .795f) { pw[0] = .424f; pw[1] = .6f; pw[2] = .072f; }
       else if (fabsf(axis[2]) >= .795f) { pw[0] = .212f; pw[1] = .6f; pw[2] = .212f; }
@@ -420,15 +504,19 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
   if (quality < kQBetter) return;
   float means[4][3];
   if (n <= 4) {
+#pragma unroll
     for (int i = 0; i < 4; i++) {
       const int src = i < n - 1 ? i : n - 1;
+#pragma unroll
       for (int k = 0; k < 3; k++) means[i][k] = S.t_norm[k][src][L];
     }
   } else {
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       means[0][k] = __fsub_rn(low[k], mean[k]);
       means[3][k] = __fsub_rn(high[k], mean[k]);
     }
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       means[1][k] = __fadd_rn(means[0][k], __fmul_rn(__fsub_rn(means[3][k], means[0][k]), 1.0f / 3.0f));
       means[2][k] = __fadd_rn(means[0][k], __fmul_rn(__fsub_rn(means[3][k], means[0][k]), 2.0f / 3.0f));
@@ -441,29 +529,43 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
       float nm[4][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
       float nw[4] = {0.f, 0.f, 0.f, 0.f};
       float tot = 0.f;
+      // a colour at a time, the next one's loads ahead of it; the sums are chosen by predicates, as an
+      // index would put them in local memory
+      float v[3] = {S.t_norm[0][0][L], S.t_norm[1][0][L], S.t_norm[2][0][L]}, wf = S.t_w[0][L];
       #pragma unroll 1
       for (int i = 0; i < n; i++) {
-        const float v[3] = {S.t_norm[0][i][L], S.t_norm[1][i][L], S.t_norm[2][i][L]};
+        const int nx = min(i + 1, n - 1);
+        const float u[3] = {S.t_norm[0][nx][L], S.t_norm[1][nx][L], S.t_norm[2][nx][L]}, uw = S.t_w[nx][L];
         float bd = 0.f;
         int bi = 0;
+#pragma unroll
         for (int j = 0; j < 4; j++) {
           float d2 = 0.f;
+#pragma unroll
           for (int k = 0; k < 3; k++) {
             const float d = __fsub_rn(means[j][k], v[k]);
-            d2 = __fadd_rn(d2, __fmul_rn(d, d));
+            d2 = k ? __fadd_rn(d2, __fmul_rn(d, d)) : __fmul_rn(d, d);
           }
           if (j == 0 || d2 < bd) { bd = d2; bi = j; }
         }
         tot = __fadd_rn(tot, bd);
-        const float wf = (float)S.t_w[i][L];
-        for (int k = 0; k < 3; k++) nm[bi][k] = __fadd_rn(nm[bi][k], __fmul_rn(v[k], wf));
-        nw[bi] = __fadd_rn(nw[bi], wf);
+        const float p[3] = {__fmul_rn(v[0], wf), __fmul_rn(v[1], wf), __fmul_rn(v[2], wf)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const bool here = bi == j;
+#pragma unroll
+          for (int k = 0; k < 3; k++) nm[j][k] = here ? __fadd_rn(nm[j][k], p[k]) : nm[j][k];
+          nw[j] = here ? __fadd_rn(nw[j], wf) : nw[j];
+        }
+        v[0] = u[0]; v[1] = u[1]; v[2] = u[2]; wf = uw;
       }
       unsigned hi_idx = 0;
       float hi_w = 0.f;
       bool empty = false;
+#pragma unroll
       for (int j = 0; j < 4; j++) {
         if (nw[j] > 0.0f) {
+#pragma unroll
           for (int k = 0; k < 3; k++) means[j][k] = __fdiv_rn(nm[j][k], nw[j]);
           if (nw[j] > hi_w) { hi_w = nw[j]; hi_idx = j; }
         } else {
@@ -479,35 +581,38 @@ __device__ void phase1_block(SeedShared& S, int slot, const uint32_t (&pix)[16],
       if (empty && it != 7) {
         const unsigned ri = (hi_idx + rover) & 3;
         rover++;
+        float from[3];
+        // (an empty cluster before it in this order has just become its copy, jittered)
+#pragma unroll
         for (int j = 0; j < 4; j++) {
           if (nw[j] == 0.0f) {
-            for (int k = 0; k < 3; k++) means[j][k] = means[ri][k];
-            for (int k = 0; k < 3; k++) means[j][k] = __fadd_rn(means[j][k], rm.frand(-.00196f, .00196f));
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+              from[k] = ri == 0 ? means[0][k] : ri == 1 ? means[1][k] : ri == 2 ? means[2][k] : means[3][k];
+#pragma unroll
+            for (int k = 0; k < 3; k++) means[j][k] = __fadd_rn(from[k], rm.jitter());
           }
         }
       }
     }
   }
-  int slot_i = 0;
-  #pragma unroll 1
-  for (int i = 0; i < 3; i++) {
-    for (int j = i + 1; j < 4; j++) {
-      int q[2][3];
-      for (int k = 0; k < 3; k++) {
-        const float sc = k == 1 ? 63.0f : 31.0f;
-        q[0][k] = (int)floorf(__fadd_rn(.5f, __fmul_rn(__fadd_rn(means[i][k], mean[k]), sc)));
-        q[1][k] = (int)floorf(__fadd_rn(.5f, __fmul_rn(__fadd_rn(means[j][k], mean[k]), sc)));
-      }
-      uint32_t pk[2];
-      for (int e = 0; e < 2; e++) {
-        // color_quad_u8 clamps to 0..255, pack_color(scaled=false) then clamps to 31/63/31
-        const int r = min(clampi(q[e][0], 0, 255), 31), g = min(clampi(q[e][1], 0, 255), 63),
-                  b = min(clampi(q[e][2], 0, 255), 31);
-        pk[e] = pack565(r, g, b);
-      }
-      out->m[slot_i++] = canon_lo(pk[0], pk[1]) | (canon_hi(pk[0], pk[1]) << 16);
+  uint32_t pk[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    int q[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float sc = k == 1 ? 63.0f : 31.0f;
+      q[k] = (int)floorf(__fadd_rn(.5f, __fmul_rn(__fadd_rn(means[j][k], mean[k]), sc)));
     }
+    // color_quad_u8 clamps to 0..255, pack_color(scaled=false) then clamps to 31/63/31
+    pk[j] = pack565(clampi(q[0], 0, 31), clampi(q[1], 0, 63), clampi(q[2], 0, 31));
   }
+  int slot_i = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = i + 1; j < 4; j++) out->m[slot_i++] = canon_lo(pk[i], pk[j]) | (canon_hi(pk[i], pk[j]) << 16);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1634,6 +1739,12 @@ __device__ __forceinline__ void load_pix(const uint8_t* px, uint32_t (&pix)[16])
   }
 }
 
+// v / 255, which phase 1 needs several times for every colour
+__device__ __forceinline__ void fill_unit(float* unit) {
+  for (int v = threadIdx.x; v < 256; v += blockDim.x) unit[v] = __fdiv_rn((float)v, 255.0f);
+  __syncthreads();
+}
+
 // Phase 1 over n blocks: warp w takes the groups of 32 consecutive blocks g = w, w + W, ..., a lane
 // per block, each group staged by one bulk copy. Warps are ranked CTA-first (warp 0 of every CTA,
 // then warp 1, ...), and the grid has a CTA per group up to the resident limit, so a short batch
@@ -1645,6 +1756,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
                  const uint32_t* __restrict__ n_dev) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (n_dev) n = min(n, *n_dev);  // a count the host does not read back: n is then only the grid's bound
+  __shared__ float unit[256];
+  fill_unit(unit);
   SeedShared& S = reinterpret_cast<SeedShared*>(smem_raw)[threadIdx.x >> 5];
   const uint32_t lane = lane_id();
   const uint32_t warp_global = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -1672,7 +1785,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
       run(gn, src, cnt);
       st.next(S, 1, &src, &cnt, &zero);
     }
-    if (b < n) phase1_block<G>(S, (int)lane, pix, opts, seeds + b);
+    if (b < n) phase1_block<G>(S, unit, (int)lane, pix, opts, seeds + b);
   }
   st.finish(S);
 }
@@ -1937,6 +2050,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
     k_dxt1_seeds_chunks(const uint8_t* __restrict__ blocks, const EncodeChunk* __restrict__ chunks, uint32_t nchunks,
                         const EncodeSegment* __restrict__ segs, Seed* __restrict__ seeds) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float unit[256];
+  fill_unit(unit);
   SeedShared& S = reinterpret_cast<SeedShared*>(smem_raw)[threadIdx.x >> 5];
   const uint32_t lane = lane_id();
   const uint32_t warp_global = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
@@ -1971,7 +2086,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
       runs(gn, src, cnt);
       st.next(S, kPer, src, cnt, dst);
     }
-    if (mine) phase1_block<false>(S, (int)lane, pix, segs[ch.segment].options, seeds + ch.first + k);
+    if (mine) phase1_block<false>(S, unit, (int)lane, pix, segs[ch.segment].options, seeds + ch.first + k);
   }
   st.finish(S);
 }
