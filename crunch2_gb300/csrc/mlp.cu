@@ -84,7 +84,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 // and hidden layers go through one 64 KB shared-memory tile (features alias its first 12 KB),
 // accumulators through 256 TMEM columns reused by all three layers. Same arithmetic as the
 // training forward (bf16 operands, fp32 accumulation, bias + tanh-GELU in fp32, bf16 hidden).
-constexpr int kInferThreads = 256;
+// The hidden epilogues (65,536 tanh a tile) are what it spends its time on: a thread per row and
+// quarter of the columns, as with half of them the eight warps left the schedulers idle half the time
+// (87,000 blocks 68 us, now 63 with the texels loaded ahead).
+constexpr int kInferThreads = 512;
+constexpr int kInferCols = kHid / (kInferThreads / BM);  // hidden columns of a thread
 constexpr uint32_t kSmW2 = 0, kSmW1 = kSmW2 + kHid * kHid * 2, kSmW3 = kSmW1 + kHid * kIn * 2,
                    kSmH = kSmW3 + kOutPad * kHid * 2, kSmB1 = kSmH + BM * kHid * 2, kSmB2 = kSmB1 + kHid * 4,
                    kSmB3 = kSmB2 + kHid * 4, kSmBar = kSmB3 + kOutPad * 4, kSmTmem = kSmBar + 8,
@@ -116,12 +120,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// hidden-layer epilogue: TMEM accumulators of this thread's row, columns [c_lo, c_lo + 128),
+// hidden-layer epilogue: TMEM accumulators of this thread's row, columns [c_lo, c_lo + kInferCols),
 // + bias, GELU, bf16 into the K-major hidden tile
 __device__ __forceinline__ void hidden_epilogue(uint32_t tmem, int quarter, int row, int c_lo, const float* bias,
                                                 unsigned char* sH) {
 #pragma unroll 1
-  for (int c0 = c_lo; c0 < c_lo + 128; c0 += 16) {
+  for (int c0 = c_lo; c0 < c_lo + kInferCols; c0 += 16) {
     uint32_t r[16];
     tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
     uint32_t w[8];
@@ -165,19 +169,19 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kSmTmem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  // weights (row-major bf16 [rows x K]) -> K-major core matrices, 16 bytes at a time
-  for (int e = tid; e < kHid * (kHid / 8); e += kInferThreads) {
-    const int r = e >> 5, kg = e & 31;
-    *reinterpret_cast<uint4*>(sW2 + kseg(r, kg, kHid)) = __ldg(reinterpret_cast<const uint4*>(W2 + r * kHid + kg * 8));
-  }
-  for (int e = tid; e < kHid * (kIn / 8); e += kInferThreads) {
-    const int r = e / (kIn / 8), kg = e % (kIn / 8);
-    *reinterpret_cast<uint4*>(sW1 + kseg(r, kg, kIn)) = __ldg(reinterpret_cast<const uint4*>(W1 + r * kIn + kg * 8));
-  }
-  for (int e = tid; e < kOutPad * (kHid / 8); e += kInferThreads) {
-    const int r = e >> 5, kg = e & 31;
-    *reinterpret_cast<uint4*>(sW3 + kseg(r, kg, kHid)) = __ldg(reinterpret_cast<const uint4*>(W3 + r * kHid + kg * 8));
-  }
+  // weights (row-major bf16 [rows x K]) -> K-major core matrices, 16 bytes at a time: the 8 rows of a
+  // core matrix to neighbouring lanes, as a row's segments lie 128 bytes apart (32 lanes on the same
+  // banks took 6.6 us of a launch)
+  auto stage = [&](const __nv_bfloat16* w, unsigned char* dst, int rows, int groups) {
+    for (int e = tid; e < rows * groups; e += kInferThreads) {
+      const int kg = (e >> 3) % groups, r = (e >> 3) / groups * 8 + (e & 7);
+      *reinterpret_cast<uint4*>(dst + kseg(r, kg, groups * 8)) =
+          __ldg(reinterpret_cast<const uint4*>(w + (r * groups + kg) * 8));
+    }
+  };
+  stage(W2, sW2, kHid, kHid / 8);
+  stage(W1, sW1, kHid, kIn / 8);
+  stage(W3, sW3, kOutPad, kHid / 8);
   for (int e = tid; e < kHid; e += kInferThreads) { sB1[e] = b1[e]; sB2[e] = b2[e]; }
   if (tid < kOutPad) sB3[tid] = b3[tid];
   if (warp == 0) {
@@ -194,22 +198,27 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   const uint32_t id256 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kHid >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
   const uint32_t id16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kOutPad >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
   const uint32_t aH = smem_u32(sH), aW1 = smem_u32(sW1), aW2 = smem_u32(sW2), aW3 = smem_u32(sW3);
-  const int quarter = warp & 3, half = warp >> 2;
+  const int quarter = warp & 3, part = warp >> 2;
   const int erow = quarter * 32 + lane;  // the tile row whose accumulators this thread reads
   uint32_t phase = 0;
   bool ok = true;
   const int ntiles = (n + BM - 1) / BM;
+  uint4 v0, v1;  // this thread's texels, loaded a tile ahead
+  auto load = [&](int tile) {
+    const long long row = (long long)tile * BM + (tid & (BM - 1));
+    v0 = v1 = make_uint4(0, 0, 0, 0);
+    if (tid < 2 * BM && row < n) {
+      const uint4* src = reinterpret_cast<const uint4*>(blocks + row * 64 + (tid >> 7) * 32);
+      v0 = __ldg(src);
+      v1 = __ldg(src + 1);
+    }
+  };
+  load(blockIdx.x);
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long row0 = (long long)tile * BM;
-    {  // features: thread (row, half) converts texels 8*half .. 8*half+7 (24 features, 3 K-groups)
+    if (tid < 2 * BM) {  // features: thread (row, half) converts texels 8*half .. 8*half+7 (24 features, 3 K-groups)
       const int r = tid & (BM - 1), hf = tid >> 7;
-      uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-      if (row0 + r < n) {
-        const uint4* src = reinterpret_cast<const uint4*>(blocks + (row0 + r) * 64 + hf * 32);
-        v0 = __ldg(src);
-        v1 = __ldg(src + 1);
-      }
       const uint32_t px[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
       float f[24];
 #pragma unroll
@@ -233,9 +242,10 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                  id256, ks > 0);
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
     }
+    load(min(tile + (int)gridDim.x, ntiles));  // at ntiles every row is past n: nothing is read
     if (!(ok = tile_wait(bar, phase))) break;
     phase ^= 1;
-    hidden_epilogue(tmem, quarter, erow, half * 128, sB1, sH);
+    hidden_epilogue(tmem, quarter, erow, part * kInferCols, sB1, sH);
     asm volatile("fence.proxy.async.shared::cta;");
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -249,7 +259,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     }
     if (!(ok = tile_wait(bar, phase))) break;
     phase ^= 1;
-    hidden_epilogue(tmem, quarter, erow, half * 128, sB2, sH);
+    hidden_epilogue(tmem, quarter, erow, part * kInferCols, sB2, sH);
     asm volatile("fence.proxy.async.shared::cta;");
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -263,7 +273,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     }
     if (!(ok = tile_wait(bar, phase))) break;
     phase ^= 1;
-    if (half == 0) {
+    if (part == 0) {
       uint32_t r[16];
       tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16), r);
       if (row0 + erow < n) {
@@ -748,125 +758,192 @@ __device__ __forceinline__ int q565(float v, int hi) {
   int x = __float2int_rn(v * (float)hi);
   return x < 0 ? 0 : (x > hi ? hi : x);
 }
-__device__ __forceinline__ void expand565(uint32_t c, int* o) {
-  const int r = c >> 11, g = (c >> 5) & 63, b = c & 31;
-  o[0] = (r << 3) | (r >> 2); o[1] = (g << 2) | (g >> 4); o[2] = (b << 3) | (b >> 2);
+// Packed FP32 (sm_100 and later): two colours of a block at a time.
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
 }
-// error of the 4-colour (three = false) or 3-colour palette of (lo, hi); selectors in 2-bit slots
-__device__ uint32_t block_error(const uint32_t* px, uint32_t lo, uint32_t hi, bool perceptual, bool three,
-                                uint32_t* sel_out) {
-  int c[4][3];
-  expand565(lo, c[0]);
-  expand565(hi, c[1]);
-  for (int k = 0; k < 3; k++) {
-    if (three) {
-      c[2][k] = (c[0][k] + c[1][k]) >> 1;
-    } else {
-      c[2][k] = (c[0][k] * 2 + c[1][k]) / 3;
-      c[3][k] = (c[1][k] * 2 + c[0][k]) / 3;
+__device__ __forceinline__ void unpair(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+// A block in registers: the colours in pairs, as floats, and the sum of their weighted squares.
+struct RefitBlock {
+  uint64_t r[8], g[8], b[8];
+  float wr, wg;
+  uint32_t squares;
+};
+// A palette entry p as the distance of a colour x less |x|^2 is evaluated: -2 w p and w p^2 + kOffset,
+// which keeps the whole of it between 2^23 and 2^24 (w p^2 - 2 w p x is between -34 * 255^2 and
+// 34 * 255^2): an integer in the low mantissa bits, every step exact.
+constexpr float kOffset = 13000000.f, kNoEntry = 16000000.f;
+struct RefitEntry {
+  float r, g, b, c;
+  __device__ __forceinline__ void set(const RefitBlock& B, float pr, float pg, float pb) {
+    r = -2.f * B.wr * pr; g = -2.f * B.wg * pg; b = -2.f * pb;
+    c = fmaf(B.wr * pr, pr, fmaf(B.wg * pg, pg, fmaf(pb, pb, kOffset)));
+  }
+};
+__device__ __forceinline__ void refit_palette(const RefitBlock& B, uint32_t lo, uint32_t hi, bool three, RefitEntry (&q)[4]) {
+  auto e5 = [](uint32_t v) { return (int)((v << 3) | (v >> 2)); };
+  auto e6 = [](uint32_t v) { return (int)((v << 2) | (v >> 4)); };
+  const int a[3] = {e5(lo >> 11), e6((lo >> 5) & 63u), e5(lo & 31u)}, c[3] = {e5(hi >> 11), e6((hi >> 5) & 63u), e5(hi & 31u)};
+  q[0].set(B, (float)a[0], (float)a[1], (float)a[2]);
+  q[1].set(B, (float)c[0], (float)c[1], (float)c[2]);
+  if (three) {
+    q[2].set(B, (float)((a[0] + c[0]) >> 1), (float)((a[1] + c[1]) >> 1), (float)((a[2] + c[2]) >> 1));
+    q[3].r = q[3].g = q[3].b = 0.f;
+    q[3].c = kNoEntry;
+  } else {
+    q[2].set(B, (float)((a[0] * 2 + c[0]) / 3), (float)((a[1] * 2 + c[1]) / 3), (float)((a[2] * 2 + c[2]) / 3));
+    q[3].set(B, (float)((c[0] * 2 + a[0]) / 3), (float)((c[1] * 2 + a[1]) / 3), (float)((c[2] * 2 + a[2]) / 3));
+  }
+}
+// Error of the 4-colour (three = false) or 3-colour palette of (lo, hi), and with `selectors` the
+// selectors in 2-bit slots (the first of equally near entries).
+template <bool selectors>
+__device__ __forceinline__ uint32_t block_error(const RefitBlock& B, uint32_t lo, uint32_t hi, bool three, uint32_t* sel_out) {
+  RefitEntry q[4];
+  refit_palette(B, lo, hi, three, q);
+  uint64_t qr[4], qg[4], qb[4], qc[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    qr[k] = pair(q[k].r, q[k].r); qg[k] = pair(q[k].g, q[k].g);
+    qb[k] = pair(q[k].b, q[k].b); qc[k] = pair(q[k].c, q[k].c);
+  }
+  uint32_t sum = 0, sel = 0;
+#pragma unroll
+  for (int p = 0; p < 8; p++) {
+    float d[2][4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      unpair(fma_pair(B.r[p], qr[k], fma_pair(B.g[p], qg[k], fma_pair(B.b[p], qb[k], qc[k]))), d[0][k], d[1][k]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float m = fminf(fminf(d[h][0], d[h][1]), fminf(d[h][2], d[h][3]));
+      sum += __float_as_uint(m);
+      if (selectors) {
+        const uint32_t k = m == d[h][0] ? 0u : m == d[h][1] ? 1u : m == d[h][2] ? 2u : 3u;
+        sel |= k << (4 * p + 2 * h);
+      }
     }
   }
-  const int nk = three ? 3 : 4;
-  const int wr = perceptual ? 8 : 1, wg = perceptual ? 25 : 1;
-  uint32_t err = 0, sel = 0;
-#pragma unroll 4
-  for (int p = 0; p < 16; p++) {
-    const int r = px[p] & 255, g = (px[p] >> 8) & 255, b = (px[p] >> 16) & 255;
-    uint32_t best = 0xFFFFFFFFu;
-    int bi = 0;
-    for (int k = 0; k < nk; k++) {
-      const int dr = r - c[k][0], dg = g - c[k][1], db = b - c[k][2];
-      const uint32_t d = (uint32_t)(wr * dr * dr + wg * dg * dg + db * db);
-      if (d < best) { best = d; bi = k; }
-    }
-    err += best;
-    sel |= (uint32_t)bi << (2 * p);
-  }
-  *sel_out = sel;
-  return err;
+  if (selectors) *sel_out = sel;
+  // a distance's bits are those of 2^23 plus (distance + kOffset - 2^23)
+  return sum - 16u * (0x4B000000u + (uint32_t)(kOffset - 8388608.f)) + B.squares;
 }
 
+// One thread per block: the error of 14 to 38 endpoint pairs over 16 colours and four entries is what
+// it does, in exact packed floats (3 multiply-adds for two colours and an entry, a minimum, an integer
+// add), with selectors only where they are used. In integer arithmetic with selectors for every pair
+// the proposals of 87,000 blocks took 116 us, now 52.
 // y holds the proposals of blocks base .. base + n - 1; indices written to `fallback` are batch-wide
 __global__ void k_learned_refit(const uint8_t* __restrict__ blocks, const float* __restrict__ y, uint32_t base, int n,
                                 int perceptual, uint8_t* __restrict__ out, uint32_t* __restrict__ fallback,
                                 uint32_t* __restrict__ nfall, float threshold) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const long long i = (long long)base + j;
-    uint32_t px[16];
+    RefitBlock B;
+    B.wr = perceptual ? 8.f : 1.f;
+    B.wg = perceptual ? 25.f : 1.f;
+    B.squares = 0;
     const uint4* p4 = reinterpret_cast<const uint4*>(blocks + i * 64);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const uint4 v = __ldg(p4 + q);
-      px[4 * q] = v.x; px[4 * q + 1] = v.y; px[4 * q + 2] = v.z; px[4 * q + 3] = v.w;
+      const uint32_t px[4] = {v.x, v.y, v.z, v.w};
+      float x[4][3];
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) x[t][k] = (float)((px[t] >> (8 * k)) & 255u);
+        B.squares += (uint32_t)fmaf(B.wr * x[t][0], x[t][0], fmaf(B.wg * x[t][1], x[t][1], x[t][2] * x[t][2]));
+      }
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        B.r[2 * q + t] = pair(x[2 * t][0], x[2 * t + 1][0]);
+        B.g[2 * q + t] = pair(x[2 * t][1], x[2 * t + 1][1]);
+        B.b[2 * q + t] = pair(x[2 * t][2], x[2 * t + 1][2]);
+      }
     }
-    const bool perc = perceptual != 0;
     const float* yi = y + (long long)j * kOutPad;
-    int e[6] = {q565(yi[0], 31), q565(yi[1], 63), q565(yi[2], 31), q565(yi[3], 31), q565(yi[4], 63), q565(yi[5], 31)};
-    auto pk = [](const int* v) { return (uint32_t)((v[0] << 11) | (v[1] << 5) | v[2]); };
+    auto pk = [](int r, int g, int b) { return (uint32_t)((r << 11) | (g << 5) | b); };
+    uint32_t lo = pk(q565(yi[0], 31), q565(yi[1], 63), q565(yi[2], 31));
+    uint32_t hi = pk(q565(yi[3], 31), q565(yi[4], 63), q565(yi[5], 31));
     uint32_t sel;
-    uint32_t err = block_error(px, pk(e), pk(e + 3), perc, false, &sel);
+    uint32_t err = block_error<true>(B, lo, hi, false, &sel);
     // least-squares refit from the selectors (points at 1, 0, 2/3, 1/3 of the low endpoint)
     {
       float aa = 0.f, ab = 0.f, bb = 0.f, ax[3] = {0, 0, 0}, bx[3] = {0, 0, 0};
-      const float wlow[4] = {1.f, 0.f, 2.f / 3.f, 1.f / 3.f};
+#pragma unroll
       for (int p = 0; p < 16; p++) {
-        const float a = wlow[(sel >> (2 * p)) & 3], b = 1.f - a;
+        const uint32_t k = (sel >> (2 * p)) & 3u;
+        const float a = k == 0 ? 1.f : k == 1 ? 0.f : k == 2 ? 2.f / 3.f : 1.f / 3.f, b = 1.f - a;
         aa += a * a; ab += a * b; bb += b * b;
-        const float x[3] = {(float)(px[p] & 255), (float)((px[p] >> 8) & 255), (float)((px[p] >> 16) & 255)};
-        for (int k = 0; k < 3; k++) { ax[k] += a * x[k]; bx[k] += b * x[k]; }
+        float x[3], other;
+        if (p & 1) { unpair(B.r[p / 2], other, x[0]); unpair(B.g[p / 2], other, x[1]); unpair(B.b[p / 2], other, x[2]); }
+        else { unpair(B.r[p / 2], x[0], other); unpair(B.g[p / 2], x[1], other); unpair(B.b[p / 2], x[2], other); }
+#pragma unroll
+        for (int k3 = 0; k3 < 3; k3++) { ax[k3] += a * x[k3]; bx[k3] += b * x[k3]; }
       }
       const float det = aa * bb - ab * ab;
       if (fabsf(det) > 1e-6f) {
         const float inv = 1.f / det;
-        const int lim[3] = {31, 63, 31};
         int f[6];
+#pragma unroll
         for (int k = 0; k < 3; k++) {
-          f[k] = q565((ax[k] * bb - bx[k] * ab) * inv / 255.f, lim[k]);
-          f[3 + k] = q565((bx[k] * aa - ax[k] * ab) * inv / 255.f, lim[k]);
+          const int lim = k == 1 ? 63 : 31;
+          f[k] = q565((ax[k] * bb - bx[k] * ab) * inv / 255.f, lim);
+          f[3 + k] = q565((bx[k] * aa - ax[k] * ab) * inv / 255.f, lim);
         }
-        uint32_t nsel;
-        const uint32_t nerr = block_error(px, pk(f), pk(f + 3), perc, false, &nsel);
-        if (nerr < err) { err = nerr; sel = nsel; for (int k = 0; k < 6; k++) e[k] = f[k]; }
+        const uint32_t flo = pk(f[0], f[1], f[2]), fhi = pk(f[3], f[4], f[5]);
+        const uint32_t nerr = block_error<false>(B, flo, fhi, false, nullptr);
+        if (nerr < err) { err = nerr; lo = flo; hi = fhi; }
       }
     }
     // greedy polish: up to three rounds of the best single +-1 move over the six components
 #pragma unroll 1
     for (int round = 0; round < 3; round++) {
-      int best_k = -1, best_d = 0;
-      uint32_t best_err = err, best_sel = sel;
+      uint32_t best_err = err, best_lo = lo, best_hi = hi;
 #pragma unroll 1
-      for (int k = 0; k < 6; k++) {
-        const int lim = (k % 3) == 1 ? 63 : 31;
-        for (int d = -1; d <= 1; d += 2) {
-          const int v = e[k] + d;
-          if (v < 0 || v > lim) continue;
-          int f[6] = {e[0], e[1], e[2], e[3], e[4], e[5]};
-          f[k] = v;
-          uint32_t nsel;
-          const uint32_t nerr = block_error(px, pk(f), pk(f + 3), perc, false, &nsel);
-          if (nerr < best_err) { best_err = nerr; best_sel = nsel; best_k = k; best_d = d; }
-        }
+      for (int t = 0; t < 12; t++) {
+        const int k = t >> 1, c = k % 3, shift = c == 0 ? 11 : c == 1 ? 5 : 0;
+        const uint32_t field = (c == 1 ? 63u : 31u) << shift, from = k < 3 ? lo : hi;
+        if ((from & field) == (t & 1 ? field : 0u)) continue;  // at the component's end
+        const uint32_t to = t & 1 ? from + (1u << shift) : from - (1u << shift);
+        const uint32_t nlo = k < 3 ? to : lo, nhi = k < 3 ? hi : to;
+        const uint32_t nerr = block_error<false>(B, nlo, nhi, false, nullptr);
+        if (nerr < best_err) { best_err = nerr; best_lo = nlo; best_hi = nhi; }
       }
-      if (best_k < 0) break;
-      e[best_k] += best_d;
+      if (best_err == err) break;
       err = best_err;
-      sel = best_sel;
+      lo = best_lo;
+      hi = best_hi;
     }
-    uint32_t lo = pk(e), hi = pk(e + 3);
-    // 4-colour blocks need low > high (swap and remap selectors 0<->1, 2<->3); equal endpoints
-    // are nudged apart as the reference does (crnlib/crn_dxt1.cpp:1563-1583)
+    // 4-colour blocks need low > high; equal endpoints are nudged apart as the reference does
+    // (crnlib/crn_dxt1.cpp:1563-1583). The selectors are those of the order that was searched: with
+    // the endpoints swapped, 0 <-> 1 and 2 <-> 3
+    err = block_error<true>(B, lo, hi, false, &sel);
     if (lo < hi) {
       const uint32_t t = lo; lo = hi; hi = t;
       sel ^= 0x55555555u;
     } else if (lo == hi) {
       if ((lo & 31) != 31) lo++; else hi--;
-      err = block_error(px, lo, hi, perc, false, &sel);
+      err = block_error<true>(B, lo, hi, false, &sel);
     }
     // the 3-colour block on the same endpoints (low <= high, mid-point palette)
     {
-      uint32_t sel3;
-      const uint32_t err3 = block_error(px, hi, lo, perc, true, &sel3);
-      if (err3 < err) { err = err3; sel = sel3; const uint32_t t = lo; lo = hi; hi = t; }
+      const uint32_t err3 = block_error<false>(B, hi, lo, true, nullptr);
+      if (err3 < err) {
+        err = err3;
+        block_error<true>(B, hi, lo, true, &sel);
+        const uint32_t t = lo; lo = hi; hi = t;
+      }
     }
     const float bound = exp2f(yi[6] * 16.f) - 1.f;
     *reinterpret_cast<uint2*>(out + i * 8) = make_uint2(lo | (hi << 16), sel);
