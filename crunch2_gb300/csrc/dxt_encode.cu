@@ -90,21 +90,18 @@ struct State {
 };
 
 // Candidate list kinds consumed by run_list (the reference's candidate loops).
-enum : int { LK_TABLE = 0, LK_PAIRS, LK_LATTICE, LK_REFINE, LK_COMB, LK_COMPS };
+enum : int { LK_TABLE = 0, LK_PAIRS, LK_LATTICE, LK_REFINE, LK_COMB };
 // LK_LATTICE: the 26 adjacent cells, then (Uber) +-2 along each axis, together a warp's 32 candidates:
 // the two lists one after the other took 3.62 ms for a 1024 x 1024 chain, one batch for both 3.38.
 constexpr int kNeighbours = 26;
 
 struct ListDesc {
   int kind, count, dependent, alt, stop_on_accept;
-  int side, nh, row;
-  int base[3];  // LATTICE: centre (packed, base[0]); COMPS: unpacked high endpoint
-  int e[6];     // REFINE: fitted endpoints (At1 triple, At2 triple)
+  int side, nh;  // COMB: nh colours
+  int base;      // LATTICE: centre (packed)
+  int e[6];      // REFINE: fitted endpoints (At1 triple, At2 triple)
   uint32_t pk[2];  // and packed
-  // COMPS: per-component error tables and running bounds
-  int comp, p0;
-  uint32_t packed_lo, e0, best_err;
-  uint32_t W[4], WP2[4], WPP[4], rem[4];
+  uint32_t W[4], WP2[4], WPP[4], rem[4];  // comp_errors' tables
 };
 
 // Phase 1's hand-off for one block, written by k_dxt1_seeds to global memory and read by the
@@ -789,7 +786,7 @@ __device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDes
     }
     case LK_LATTICE: {
       const bool near = i < kNeighbours;
-      const uint32_t base = near ? (uint32_t)d.base[0] : far;
+      const uint32_t base = near ? (uint32_t)d.base : far;
       int r = (int)(base >> 11), g = (int)((base >> 5) & 63), b = (int)(base & 31);
       if (near) {
         // g_adjacency order (crn_dxt1.cpp:489-522): x fastest, then y, then z, centre skipped
@@ -817,35 +814,22 @@ __device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDes
       lo = max(moved, other); hi = min(moved, other);
       return true;
     }
-    case LK_COMB:
-      lo = S.list[d.row];
-      hi = S.list[d.row + 1 + i];
-      return true;
-    default: {  // LK_COMPS: optimize_endpoint_comps inner loop with its table prune (:440-470)
-      const int c1 = i;
-      const uint32_t p1 = (uint32_t)(d.comp == 1 ? exp6(c1) : exp5(c1));
-      const uint32_t p0 = (uint32_t)d.p0;
-      auto E = [&](int s, uint32_t p) { return d.W[s] * p * p - d.WP2[s] * p + d.WPP[s]; };
-      uint32_t e = d.e0 + E(1, p1);
-      if (e + d.rem[2] >= d.best_err) return false;
-      e += E(2, (p0 * 2 + p1) / 3);
-      if (e + d.rem[3] >= d.best_err) return false;
-      e += E(3, (p0 + p1 * 2) / 3);
-      if (e >= d.best_err) return false;
-      int h[3] = {d.base[0], d.base[1], d.base[2]};
-      h[d.comp] = c1;
-      lo = d.packed_lo;
-      hi = pack565(h[0], h[1], h[2]);
+    default: {  // LK_COMB: pair i of the pairs of d.nh endpoints in row order, i (2 nh - 1 - i) / 2 before row i
+      const float half = (float)d.nh - 0.5f;
+      float root;
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(half * half - (float)(2 * i)));
+      const int row = (int)(half - root + 1e-4f);  // the next row's root is at least 1 / nh away
+      lo = S.list[row];
+      hi = S.list[i - row * (2 * d.nh - 1 - row) / 2 + row + 1];
       return true;
     }
   }
 }
 
-// Runs the list described by S.d from position `start` with the reference's sequential
-// semantics; see the file comment. Returns, for stop_on_accept lists, the position of the
+// Runs the list described by S.d with the reference's sequential semantics; see the file comment. Returns, for stop_on_accept lists, the position of the
 // first accepted candidate (or -1); otherwise 1 if anything was accepted, else 0.
 template <bool G>
-__device__ __noinline__ int run_list(WarpShared& S, int start, uint32_t& work) {
+__device__ __noinline__ int run_list(WarpShared& S, uint32_t& work) {
   const ListDesc& d = S.d;
   const uint32_t lane = lane_id();
   const int n = S.st.n;
@@ -853,7 +837,7 @@ __device__ __noinline__ int run_list(WarpShared& S, int start, uint32_t& work) {
   const bool gray = G && S.st.gray != 0;
   const float wr = S.st.wr, wg = S.st.wg;
   bool any = false;
-  int i0 = start;
+  int i0 = 0;
   // Lists whose candidates do not depend on the running best are compacted: the candidates that
   // survive the plane-table prune (against the best when they are generated) queue up in list order
   // in S.pq (a ring of 64), and each batch evaluates 32 of them, so the colour loop runs on full
@@ -1077,7 +1061,7 @@ __device__ __noinline__ bool refine(WarpShared& S, uint32_t& work, int level = 1
     set_list(S, LK_REFINE, 54, 0, 0);
   }
   __syncwarp();
-  return run_list<G>(S, 0, work) != 0;
+  return run_list<G>(S, work) != 0;
 }
 
 template <bool G>
@@ -1131,7 +1115,7 @@ __device__ __noinline__ bool try_solid(WarpShared& S, uint32_t& work) {
   __syncwarp();
   set_list(S, LK_TABLE, S.d.count, 0, 0);
   __syncwarp();
-  return run_list<G>(S, 0, work) != 0;
+  return run_list<G>(S, work) != 0;
 }
 
 // compute_endpoint_component_errors :369-413 as closed-form quadratics; fills S.d.W/WP2/WPP/rem
@@ -1191,8 +1175,8 @@ __device__ __noinline__ void optimize_comps(WarpShared& S, uint32_t& work) {
   for (int comp = 0; comp < 3; comp++) {
     const int p0s = src_lo[comp], p1s = src_hi[comp];
     const uint32_t clo = S.st.best.lo, chi = S.st.best.hi;
-    int lo_u[3] = {(int)(clo >> 11), (int)((clo >> 5) & 63), (int)(clo & 31)};
-    const int hi_u[3] = {(int)(chi >> 11), (int)((chi >> 5) & 63), (int)(chi & 31)};
+    const int shift = comp == 0 ? 11 : comp == 1 ? 5 : 0;
+    const uint32_t field = (comp == 1 ? 63u : 31u) << shift;
     comp_errors<G>(S, comp);
     const int limit = comp == 1 ? 64 : 32;
     auto ex = [&](int c) { return (uint32_t)(comp == 1 ? exp6(c) : exp5(c)); };
@@ -1203,59 +1187,63 @@ __device__ __noinline__ void optimize_comps(WarpShared& S, uint32_t& work) {
     };
     auto E = [&](int k, uint32_t p) { return W[k] * p * p - WP2[k] * p + WPP[k]; };
     load_tables();
-    uint32_t best_err = E(0, ex(lo_u[comp])) + E(1, ex(hi_u[comp])) + E(2, (uint32_t)((p0s * 2 + p1s) / 3)) +
-                        E(3, (uint32_t)((p0s + p1s * 2) / 3));
+    uint32_t best_err = E(0, ex((int)((clo & field) >> shift))) + E(1, ex((int)((chi & field) >> shift))) +
+                        E(2, (uint32_t)((p0s * 2 + p1s) / 3)) + E(3, (uint32_t)((p0s + p1s * 2) / 3));
     if (rem[0] >= best_err) continue;
-    // the low components whose table error leaves room below the best's, from `from` on, 32 at a time
-    // (each visit looks again: an acceptance changes the tables and the best)
+    // Every pair (c0, c1) of components in order, as long as its partial sums stay below the best's:
+    // first the low components with room for a high one, 32 at a time, then theirs. What is left is
+    // gathered into lists for the search; an acceptance changes the tables and the best, and the order
+    // goes on behind it. (A list for each low component was a batch of a few candidates each: half the
+    // time of the slowest blocks.)
+    int from = 0, c1_from = 0;
     #pragma unroll 1
-    for (int from = 0; from < limit;) {
-      const int cl = (from & ~31) + (int)lane;
-      const unsigned room = __ballot_sync(FULL_MASK, cl >= from && E(0, ex(cl)) + rem[1] < best_err);
-      if (!room) { from = (from & ~31) + 32; continue; }
-      const int c0 = (from & ~31) + __ffs(room) - 1;
-      from = c0 + 1;
-      const uint32_t p0 = ex(c0);
-      uint32_t e0 = E(0, p0);
-      {
-        // does any c1 pass the component-table prune for this c0 (:456-466)? lane c1 and c1 + 32;
-        // a pair passes exactly when its component error is below the best's
-        bool pass = false;
-        for (int c1 = (int)lane; c1 < limit; c1 += 32) {
-          const uint32_t p1 = ex(c1);
-          uint32_t e = e0 + E(1, p1);
-          if (e + rem[2] >= best_err) continue;
-          e += E(2, (p0 * 2 + p1) / 3);
-          if (e + rem[3] >= best_err) continue;
-          e += E(3, (p0 + p1 * 2) / 3);
-          pass |= e < best_err;
+    while (from < limit) {
+      int cnt = 0;
+      __syncwarp();  // the last list's reads
+      #pragma unroll 1
+      while (from < limit && cnt <= 32) {
+        const int cl = (from & ~31) + (int)lane;
+        const unsigned room = __ballot_sync(FULL_MASK, cl >= from && E(0, ex(cl)) + rem[1] < best_err);
+        if (!room) { from = (from & ~31) + 32; c1_from = 0; continue; }
+        const int c0 = (from & ~31) + __ffs(room) - 1;
+        if (c0 != from) c1_from = 0;
+        const int c1 = (c1_from & ~31) + (int)lane;
+        // the prune of :456-466
+        const uint32_t p0 = ex(c0), p1 = ex(c1);
+        uint32_t e = E(0, p0) + E(1, p1);
+        bool pass = c1 >= c1_from && e + rem[2] < best_err;
+        e += E(2, (p0 * 2 + p1) / 3);
+        pass &= e + rem[3] < best_err;
+        e += E(3, (p0 + p1 * 2) / 3);
+        pass &= e < best_err;
+        const unsigned m = __ballot_sync(FULL_MASK, pass);
+        if (pass) {
+          const int at = cnt + __popc(m & ((1u << lane) - 1u));
+          S.cand[at] = ((clo & ~field) | ((uint32_t)c0 << shift)) | (((chi & ~field) | ((uint32_t)c1 << shift)) << 16);
+          S.list[at] = (uint16_t)(c0 << 6 | c1);
         }
-        if (!__any_sync(FULL_MASK, pass)) continue;
+        cnt += __popc(m);
+        from = c0;
+        c1_from = (c1_from & ~31) + 32;
+        if (c1_from >= limit) { from++; c1_from = 0; }
       }
-      lo_u[comp] = c0;
+      if (!cnt) break;
       if (lane == 0) {
-        S.d.kind = LK_COMPS; S.d.count = limit; S.d.dependent = 1; S.d.alt = 0; S.d.stop_on_accept = 1;
-        S.d.comp = comp; S.d.p0 = (int)p0; S.d.e0 = e0; S.d.best_err = best_err;
-        S.d.packed_lo = pack565(lo_u[0], lo_u[1], lo_u[2]);
-        S.d.base[0] = hi_u[0]; S.d.base[1] = hi_u[1]; S.d.base[2] = hi_u[2];
+        S.d.kind = LK_TABLE; S.d.count = cnt; S.d.dependent = 1; S.d.alt = 0; S.d.stop_on_accept = 1;
       }
       __syncwarp();
-      int start = 0;
-      while (start < limit) {
-        const int c1 = run_list<G>(S, start, work);
-        if (c1 < 0) break;
-        if (!S.st.best.err) return;
-        compute_selectors(S);
-        comp_errors<G>(S, comp);
-        load_tables();
-        const uint32_t p1 = ex(c1);
-        best_err = E(0, p0) + E(1, p1) + E(2, (p0 * 2 + p1) / 3) + E(3, (p0 + p1 * 2) / 3);
-        e0 = E(0, p0);
-        if (lane == 0) { S.d.e0 = e0; S.d.best_err = best_err; }
-        __syncwarp();
-        if (e0 + rem[1] >= best_err) break;
-        start = c1 + 1;
-      }
+      const int at = run_list<G>(S, work);
+      if (at < 0) continue;
+      if (!S.st.best.err) return;
+      const int c0 = S.list[at] >> 6, c1 = S.list[at] & 63;
+      compute_selectors(S);
+      comp_errors<G>(S, comp);
+      load_tables();
+      const uint32_t p0 = ex(c0), p1 = ex(c1);
+      best_err = E(0, p0) + E(1, p1) + E(2, (p0 * 2 + p1) / 3) + E(3, (p0 + p1 * 2) / 3);
+      from = c0;
+      c1_from = c1 + 1;
+      if (c1_from >= limit) { from++; c1_from = 0; }
     }
   }
 }
@@ -1267,53 +1255,56 @@ __device__ __noinline__ void try_combinatorial(WarpShared& S, uint32_t& work) {
   const int n = S.st.n;
   if (n < 2 || n > 4) return;
   const uint32_t lane = lane_id();
-  if (lane == 0) {
-    // temporary colours (r | g << 8 | b << 16) in S.cand, unique packed endpoints in S.list
-    int cnt = 0;
-    for (int i = 0; i < n; i++) S.cand[cnt++] = S.uci[i];
-    auto push = [&](int a, int b, float f, int rounding) {
-      const float r = rounding ? 1.0f : 0.0f;
-      uint32_t out = 0;
-      for (int ch = 0; ch < 3; ch++) {
-        const float fx = (float)((S.cand[a] >> (8 * ch)) & 255), fy = (float)((S.cand[b] >> (8 * ch)) & 255);
-        const float l = __fadd_rn(fx, __fmul_rn(__fsub_rn(fy, fx), f));
-        out |= (uint32_t)clampi(__float2int_rz(__fadd_rn(r, l)), 0, 255) << (8 * ch);
+  // the block's colours and, for two or three of them, extrapolations from each to each other (a lane
+  // per colour, 42 at most), as 5:6:5 endpoints without repeats in order of first occurrence
+  const int total = n == 2 ? 42 : n == 3 ? 27 : 4;
+  auto endpoint = [&](int t) {
+    uint32_t c = S.uci[min(t, n - 1)];
+    if (t >= n) {
+      int a, b;
+      float f, r;
+      const int u = t - n;
+      if (n == 2) {
+        const int q = u % 10;  // 2, 3, .5, 1.5, -1, 2, -.5, .5, -2, -1 in halves, plus 4
+        f = (float)((int)(0x20538275A8ull >> (4 * q) & 15) - 4) * .5f;
+        r = u >= 20 ? 1.0f : 0.0f;
+        a = u / 10 & 1; b = a ^ 1;
+      } else {
+        const int q = u & 3;
+        f = q == 0 ? 1.5f : q == 1 ? 2.0f / 3.0f : q == 2 ? 1.0f / 3.0f : -.5f;
+        r = 1.0f;
+        a = min(u >> 3, 2); b = u >> 2 & 1;
+        b += b >= a ? 1 : 0;
       }
-      S.cand[cnt++] = out;
-    };
-    if (n == 2) {
-      const float fs[10] = {2.0f, 3.0f, .5f, 1.5f, -1.0f, 2.0f, -.5f, .5f, -2.0f, -1.0f};
-      #pragma unroll 1
-      for (int k = 0; k < 2; k++)
-        for (int q = 0; q < 2; q++)
-          for (int f = 0; f < 10; f++) push(q, q ^ 1, fs[f], k);
-    } else if (n == 3) {
-      #pragma unroll 1
-      for (int i = 0; i <= 2; i++)
-        for (int j = 0; j <= 2; j++) {
-          if (i == j) continue;
-          push(i, j, 1.5f, 1);
-          push(i, j, 2.0f / 3.0f, 1);
-          push(i, j, 1.0f / 3.0f, 1);
-          push(i, j, -.5f, 1);
-        }
+      const uint32_t ca = S.uci[a], cb = S.uci[b];
+      c = 0;
+      for (int ch = 0; ch < 3; ch++) {
+        const float fx = (float)((ca >> (8 * ch)) & 255), fy = (float)((cb >> (8 * ch)) & 255);
+        const float l = __fadd_rn(fx, __fmul_rn(__fsub_rn(fy, fx), f));
+        c |= (uint32_t)clampi(__float2int_rz(__fadd_rn(r, l)), 0, 255) << (8 * ch);
+      }
     }
-    int m = 0;
+    return pack565((int)(((c & 255) * 31u + 127u) / 255u), (int)((((c >> 8) & 255) * 63u + 127u) / 255u),
+                   (int)(((c >> 16) * 31u + 127u) / 255u));
+  };
+  const uint32_t k1 = (int)lane < total ? endpoint((int)lane) : 0x10000u | lane;
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned same = __match_any_sync(FULL_MASK, k1);
+  const bool first = (int)lane < total && !(same & below);
+  const unsigned m1 = __ballot_sync(FULL_MASK, first);
+  if (first) S.list[__popc(m1 & below)] = (uint16_t)k1;
+  int m = __popc(m1);
+  if (n == 2) {
+    const uint32_t k2 = (int)lane < total - 32 ? endpoint((int)lane + 32) : 0x10000u | lane;
     #pragma unroll 1
-    for (int i = 0; i < cnt; i++) {
-      const uint32_t c = S.cand[i];
-      const uint32_t ur = min(((c & 255) * 31u + 127u) / 255u, 31u);
-      const uint32_t ug = min((((c >> 8) & 255) * 63u + 127u) / 255u, 63u);
-      const uint32_t ub = min(((c >> 16) * 31u + 127u) / 255u, 31u);
-      const uint16_t pk = (uint16_t)(ub | (ug << 5) | (ur << 11));
-      bool dup = false;
-      for (int k = 0; k < m; k++) if (S.list[k] == pk) { dup = true; break; }
-      if (!dup) S.list[m++] = pk;
+    for (int j = 0; j < total - 32; j++) {
+      const uint32_t v = __shfl_sync(FULL_MASK, k2, j);
+      if (__any_sync(FULL_MASK, k1 == v || ((int)lane < j && k2 == v))) continue;
+      if (lane == 0) S.list[m] = (uint16_t)v;
+      m++;
     }
-    S.d.nh = m;
   }
   __syncwarp();
-  const int m = S.d.nh;
   #pragma unroll 1
   for (int alt = 0; alt < 2; alt++) {
     uint32_t saved = 0;
@@ -1322,14 +1313,12 @@ __device__ __noinline__ void try_combinatorial(WarpShared& S, uint32_t& work) {
       if (lane == 0 && saved) S.st.best.err = 1;
       __syncwarp();
     }
-    #pragma unroll 1
-    for (int i = 0; S.st.best.err && i + 1 < m; i++) {
-      if (lane == 0) {
-        S.d.kind = LK_COMB; S.d.count = m - 1 - i; S.d.dependent = 0; S.d.alt = alt; S.d.stop_on_accept = 0;
-        S.d.row = i;
-      }
+    if (S.st.best.err) {
+      // all pairs in one list: a list for each first endpoint took most of these blocks' time
+      if (lane == 0) S.d.nh = m;
+      set_list(S, LK_COMB, m * (m - 1) / 2, 0, alt);
       __syncwarp();
-      run_list<G>(S, 0, work);
+      run_list<G>(S, work);
     }
     if (alt) {
       if (lane == 0 && S.st.best.err) S.st.best.err = saved;
@@ -1351,7 +1340,7 @@ __device__ void optimize(WarpShared& S, uint32_t& work) {
     if (lane < 6) S.cand[lane] = S.sd.m[lane];
     set_list(S, LK_TABLE, 6, 0, 0);
     __syncwarp();
-    run_list<G>(S, 0, work);
+    run_list<G>(S, work);
     refine<G>(S, work, quality == kQUber ? 1 : 0);
   }
   const int table = probe_table(quality);
@@ -1406,17 +1395,17 @@ __device__ void optimize(WarpShared& S, uint32_t& work) {
       }
       __syncwarp();
     }
-    run_list<G>(S, 0, work);
+    run_list<G>(S, work);
     // lattice neighbours: low endpoint (26 adjacent cells, then +-2 per axis), then high
     #pragma unroll 1
     for (int side = 0; side < (quality >= kQNormal ? 2 : 0); side++) {
       if (lane == 0) {
-        S.d.base[0] = (int)(side ? S.st.best.hi : S.st.best.lo);
+        S.d.base = (int)(side ? S.st.best.hi : S.st.best.lo);
         S.d.kind = LK_LATTICE; S.d.count = quality == kQUber ? kNeighbours + 6 : kNeighbours; S.d.dependent = 1; S.d.alt = 0;
         S.d.stop_on_accept = 0; S.d.side = side;
       }
       __syncwarp();
-      run_list<G>(S, 0, work);
+      run_list<G>(S, work);
     }
     if (!S.st.best.err || (pass && S.st.best.err == prev)) break;
     if (quality == kQUber) refine<G>(S, work);
@@ -1615,7 +1604,7 @@ __device__ uint32_t phase2_block(WarpShared& S, const uint8_t* __restrict__ px, 
     if (lane == 0) { S.cand[0] = solid_coords(r, g, b, false); S.cand[1] = solid_coords(r, g, b, true); }
     set_list(S, LK_TABLE, use_alpha ? 2 : 1, 0, 0);
     __syncwarp();
-    run_list<G>(S, 0, work);
+    run_list<G>(S, work);
   } else {
     optimize<G>(S, work);
   }
