@@ -1793,65 +1793,124 @@ __device__ __forceinline__ uint32_t tile_pixel(const uint32_t* __restrict__ bloc
 
 __device__ __forceinline__ uint32_t tile_npix(uint32_t kind) { return 16u << (kind >> 2); }
 
-// error of (first, second) over selectors chosen per pixel, plus the least-squares statistics
-struct FitAcc {
-  float aa, ab, bb, ax[3], bx[3];
-  float err;
-};
-
-
 // Unique colours of a cluster in shared memory (open addressing on the packed RGB, count per
 // colour); a cluster with more than kUniqCap / 2 distinct colours skips the probe search.
 constexpr int kUniqCap = 4096;
 constexpr int kMaxCand = 1024;
 __constant__ int16_t c_probe[15] = {0, 1, 2, 3, 5, 7, 9, 10, 13, 15, 19, 27, 43, 59, 91};  // g_uber_probe_table
 
-// The probe search's colour table: per unique colour u, {-2 w_r r, -2 w_g g, -2 w_b b, xx} with
-// xx = w_r r^2 + w_g g^2 + w_b b^2 (w = 8, 25, 1 perceptual, else 1), and its pixel count. For a
-// palette colour p with pp = sum w p^2, the weighted squared distance is xx + pp + a . p, so a
-// pixel's error against the 4-colour palette is xx + min_k (pp_k + a . p_k): three multiply-adds
-// per palette colour, exactly the integer error of cdist.
-__device__ __forceinline__ int4 probe_entry(uint32_t rgb, bool perc) {
-  const int r = (int)(rgb & 255), g = (int)((rgb >> 8) & 255), b = (int)((rgb >> 16) & 255);
-  const int wr = perc ? 8 : 1, wg = perc ? 25 : 1;
-  return make_int4(-2 * wr * r, -2 * wg * g, -2 * b, wr * r * r + wg * g * g + b * b);
-}
-
-// Error of the 4-colour block (lo, hi) over the unique colours, abandoned (returning ~0) as soon as
-// its running sum reaches `bound` (a candidate that cannot win); one thread.
-__device__ __forceinline__ unsigned long long pair_error(uint32_t lo, uint32_t hi, const int4* ut, const uint32_t* uc,
-                                                        int U, bool perc, unsigned long long bound) {
+// A palette colour p for colours x in floats: -2 w . p and w . p^2 (w = 8, 25, 1 perceptual, else 1).
+// With xx = w . x^2 the weighted squared distance is xx + pp - 2 w p . x, and every term an integer
+// below 2^24: exactly the integer error of cdist.
+struct FitEntry {
+  float r, g, b, pp;
+  __device__ __forceinline__ void set(const int* c, float wr, float wg) {
+    r = -2.f * wr * (float)c[0]; g = -2.f * wg * (float)c[1]; b = -2.f * (float)c[2];
+    pp = wr * (float)(c[0] * c[0]) + wg * (float)(c[1] * c[1]) + (float)(c[2] * c[2]);
+  }
+  __device__ __forceinline__ float part(float x, float y, float z) const {
+    return fmaf(x, r, fmaf(y, g, fmaf(z, b, pp)));
+  }
+};
+__device__ __forceinline__ void fit_entries(uint32_t lo, uint32_t hi, float wr, float wg, FitEntry (&q)[4]) {
   int col[4][3];
   colors4(lo, hi, col);
-  const int wr = perc ? 8 : 1, wg = perc ? 25 : 1;
-  int pp[4];
 #pragma unroll
-  for (int k = 0; k < 4; k++) pp[k] = wr * col[k][0] * col[k][0] + wg * col[k][1] * col[k][1] + col[k][2] * col[k][2];
+  for (int k = 0; k < 4; k++) q[k].set(col[k], wr, wg);
+}
+// packed FP32: two colours at a time
+__device__ __forceinline__ uint64_t twice(float v) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(v));
+  return p;
+}
+__device__ __forceinline__ uint64_t fma_two(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(a), "l"(b), "l"(c));
+  return p;
+}
+__device__ __forceinline__ void split_two(uint64_t p, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+
+// The colour table: colours in pairs, {r0, r1, g0, g1, b0, b1, xx0, xx1} with xx + 2^23 in place of xx
+// (a distance added to it is an integer in the low mantissa bits), and their pixel counts after it; an
+// odd last colour is paired with one of count 0.
+struct FitTable {
+  float* col;
+  uint32_t* cnt;
+  int n;
+  float wr, wg;
+  __device__ __forceinline__ void set(int i, uint32_t rgb, uint32_t count) const {
+    float* e = col + (i >> 1) * 8 + (i & 1);
+    const float r = (float)(rgb & 255), g = (float)((rgb >> 8) & 255), b = (float)((rgb >> 16) & 255);
+    e[0] = r; e[2] = g; e[4] = b;
+    e[6] = wr * (r * r) + wg * (g * g) + b * b + 8388608.f;
+    cnt[i] = count;
+  }
+};
+
+// Error of the 4-colour block (lo, hi) over the colour pairs from, from + step, ..., abandoned
+// (returning ~0) as soon as its running sum reaches `bound` (a candidate that cannot win); one thread.
+// Two colours and an entry take three packed multiply-adds; the integer form of the same took three
+// times the instructions.
+__device__ __forceinline__ unsigned long long pair_error(uint32_t lo, uint32_t hi, const FitTable& T, int from, int step,
+                                                        unsigned long long bound) {
+  FitEntry q[4];
+  fit_entries(lo, hi, T.wr, T.wg, q);
+  uint64_t qr[4], qg[4], qb[4], qp[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) { qr[k] = twice(q[k].r); qg[k] = twice(q[k].g); qb[k] = twice(q[k].b); qp[k] = twice(q[k].pp); }
   unsigned long long e = 0;
-  for (int i = 0; i < U; i++) {
-    const int4 t = ut[i];
-    int m = pp[0] + t.x * col[0][0] + t.y * col[0][1] + t.z * col[0][2];
+  const int pairs = (T.n + 1) >> 1;
+  int left = 8;
+  for (int i = from; i < pairs; i += step) {
+    const ulonglong2 rg = reinterpret_cast<const ulonglong2*>(T.col)[2 * i];
+    const ulonglong2 bx = reinterpret_cast<const ulonglong2*>(T.col)[2 * i + 1];
+    const uint2 w = reinterpret_cast<const uint2*>(T.cnt)[i];
+    float d0[4], d1[4], x0, x1;
 #pragma unroll
-    for (int k = 1; k < 4; k++) m = min(m, pp[k] + t.x * col[k][0] + t.y * col[k][1] + t.z * col[k][2]);
-    e += (unsigned long long)(uint32_t)(t.w + m) * uc[i];
-    if ((i & 15) == 15 && e >= bound) return ~0ull;
+    for (int k = 0; k < 4; k++) split_two(fma_two(rg.x, qr[k], fma_two(rg.y, qg[k], fma_two(bx.x, qb[k], qp[k]))), d0[k], d1[k]);
+    split_two(bx.y, x0, x1);
+    const float m0 = fminf(fminf(d0[0], d0[1]), fminf(d0[2], d0[3])), m1 = fminf(fminf(d1[0], d1[1]), fminf(d1[2], d1[3]));
+    e += (unsigned long long)(__float_as_uint(x0 + m0) - 0x4B000000u) * w.x;
+    e += (unsigned long long)(__float_as_uint(x1 + m1) - 0x4B000000u) * w.y;
+    if (--left == 0) {
+      if (e >= bound) return ~0ull;
+      left = 8;
+    }
   }
   return e < bound ? e : ~0ull;
 }
 
-// Evaluates the candidate pairs cand[0..n) (lo | hi << 16), one thread per candidate, and returns
-// to every thread the best (lowest error, then lowest index) among those below `bound`; err = ~0
-// and pair = 0 when none is.
-__device__ void best_candidate(const uint32_t* cand, int n, const int4* ut, const uint32_t* uc, int U, bool perc,
-                               unsigned long long bound, unsigned long long* s_be, uint32_t* s_bi,
-                               unsigned long long& err, uint32_t& pair) {
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Evaluates the candidate pairs cand[0..n) (lo | hi << 16; of the first 32 those in `valid`), kSplit
+// threads per candidate, and returns to every thread the best (lowest error, then lowest index) among
+// those below `bound`; err = ~0 and pair = 0 when none is.
+template <int kSplit>
+__device__ void best_candidate(const uint32_t* cand, int n, uint32_t valid, const FitTable& T, unsigned long long bound,
+                               unsigned long long* s_be, uint32_t* s_bi, unsigned long long& err, uint32_t& pair) {
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, sub = threadIdx.x % kSplit;
   unsigned long long be = ~0ull;
   uint32_t bi = 0xFFFFFFFFu;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    // a later candidate must beat this thread's best strictly (ties go to the lower index)
-    const unsigned long long e = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, ut, uc, U, perc, min(bound, be));
-    if (e < be) { be = e; bi = (uint32_t)i; }
+  if (kSplit > 1) {  // one candidate for each group of threads: n is at most kFitThreads / kSplit
+    const int i = threadIdx.x / kSplit;
+    if (i < n && (valid >> i & 1)) be = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, sub, kSplit, bound);
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < kSplit; o <<= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, be, o);
+      be = be == ~0ull || other == ~0ull ? ~0ull : be + other;
+    }
+    if (be >= bound) be = ~0ull;
+    if (be != ~0ull) bi = (uint32_t)i;
+  } else {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      if (i < 32 && !(valid >> i & 1)) continue;
+      // a later candidate must beat this thread's best strictly (ties go to the lower index)
+      const unsigned long long e = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, 0, 1, min(bound, be));
+      if (e < be) { be = e; bi = (uint32_t)i; }
+    }
+    __syncwarp();
   }
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long oe = __shfl_xor_sync(0xFFFFFFFFu, be, o);
@@ -1869,7 +1928,14 @@ __device__ void best_candidate(const uint32_t* cand, int n, const int4* ut, cons
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __restrict__ blocks,
+// One CTA per cluster. What takes the time is the probe search, up to 840 candidates of 4 palette
+// colours against every unique colour in each of up to four passes (see pair_error); then the latency
+// of the rest, so that a cluster's pixels are fetched through their tiles once and kept in shared
+// memory for the least-squares passes, the principal axis (double precision: 64 cycles an instruction
+// for a warp, whatever the others do) is one warp's work, the probes and moves are listed and scored by
+// a lane each, and the walk's statistics are summed over unique colours by a few threads for each sum.
+// The 2415 clusters of a 1024 x 1024 chain (580 unique colours each) took 4.1 ms, now 1.9.
+__global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* __restrict__ blocks,
                                                              const Chunk* __restrict__ chunks,
                                                              const Tile* __restrict__ tiles,
                                                              const uint32_t* __restrict__ ctile_start,
@@ -1877,6 +1943,12 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
                                                              ClusterOut* __restrict__ out) {
   __shared__ float red[24 * 16];
   __shared__ uint32_t s_tiles[256];
+  // the cluster's pixels, [the thread's pixel][thread]; then the hash of its unique colours, keys in
+  // s_raw[0, kUniqCap), counts in s_raw[kUniqCap, 2 kUniqCap); once compacted (at most kUniqCap / 2
+  // colours): the colour table in s_raw[0, 2 kUniqCap), its counts after it
+  __shared__ __align__(16) uint32_t s_raw[2 * kUniqCap + kUniqCap / 2];
+  constexpr int kPixCap = (2 * kUniqCap + kUniqCap / 2) / kFitThreads;
+  __shared__ float s_axis[4];
   const uint32_t k = blockIdx.x;
   const uint32_t t0 = ctile_start[k], t1 = ctile_start[k + 1];
   const bool perc = perceptual != 0;
@@ -1904,37 +1976,63 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
   // 1. mean and (perceptually weighted) covariance
   float acc[10];
   for (int i = 0; i < 10; i++) acc[i] = 0.f;
+  int np = 0;
   for_pixels([&](uint32_t p) {
+    if (np < kPixCap) s_raw[np * kFitThreads + threadIdx.x] = p;
+    np++;
     const float r = (float)px_r(p), g = (float)px_g(p), b = (float)px_b(p);
     acc[0] += r; acc[1] += g; acc[2] += b; acc[3] += 1.f;
     acc[4] += r * r; acc[5] += r * g; acc[6] += r * b; acc[7] += g * g; acc[8] += g * b; acc[9] += b * b;
   });
+  const bool kept = !__syncthreads_or(np > kPixCap);
+  // the same pixels again, each thread's in the same order
+  auto each_pixel = [&](auto&& fn) {
+    if (kept) {
+      for (int m = 0; m < np; m++) fn(s_raw[m * kFitThreads + threadIdx.x]);
+    } else {
+      for_pixels(fn);
+    }
+  };
   block_sum<10>(acc, red);
   const float cnt = acc[3];
   const float mean[3] = {acc[0] / cnt, acc[1] / cnt, acc[2] / cnt};
   // perceptual weights (crnlib/crn_dxt1.cpp:1074-1108 start from luma-like weights)
   const float pw[3] = {perc ? 0.212f : 1.f, perc ? 0.72f : 1.f, perc ? 0.072f : 1.f};
-  double cov[6] = {acc[4] / cnt - mean[0] * mean[0], acc[5] / cnt - mean[0] * mean[1], acc[6] / cnt - mean[0] * mean[2],
-                   acc[7] / cnt - mean[1] * mean[1], acc[8] / cnt - mean[1] * mean[2], acc[9] / cnt - mean[2] * mean[2]};
-  cov[0] *= pw[0] * pw[0]; cov[1] *= pw[0] * pw[1]; cov[2] *= pw[0] * pw[2];
-  cov[3] *= pw[1] * pw[1]; cov[4] *= pw[1] * pw[2]; cov[5] *= pw[2] * pw[2];
-  double ar = .9, ag = 1.0, ab = .7;
-  for (int it = 0; it < 8; it++) {
-    const double r = ar * cov[0] + ag * cov[1] + ab * cov[2];
-    const double g = ar * cov[1] + ag * cov[3] + ab * cov[4];
-    const double b = ar * cov[2] + ag * cov[4] + ab * cov[5];
-    const double m = fmax(fabs(r), fmax(fabs(g), fabs(b)));
-    if (m > 1e-10) { ar = r / m; ag = g / m; ab = b / m; } else { ar = r; ag = g; ab = b; }
+  float axis[3], sd;
+  if (threadIdx.x < 32) {
+    double cov[6] = {acc[4] / cnt - mean[0] * mean[0], acc[5] / cnt - mean[0] * mean[1], acc[6] / cnt - mean[0] * mean[2],
+                     acc[7] / cnt - mean[1] * mean[1], acc[8] / cnt - mean[1] * mean[2], acc[9] / cnt - mean[2] * mean[2]};
+    cov[0] *= pw[0] * pw[0]; cov[1] *= pw[0] * pw[1]; cov[2] *= pw[0] * pw[2];
+    cov[3] *= pw[1] * pw[1]; cov[4] *= pw[1] * pw[2]; cov[5] *= pw[2] * pw[2];
+    double ar = .9, ag = 1.0, ab = .7;
+    for (int it = 0; it < 8; it++) {
+      const double r = ar * cov[0] + ag * cov[1] + ab * cov[2];
+      const double g = ar * cov[1] + ag * cov[3] + ab * cov[4];
+      const double b = ar * cov[2] + ag * cov[4] + ab * cov[5];
+      const double m = fmax(fabs(r), fmax(fabs(g), fabs(b)));
+      if (m > 1e-10) { ar = r / m; ag = g / m; ab = b / m; } else { ar = r; ag = g; ab = b; }
+    }
+    axis[0] = (float)(ar / pw[0]); axis[1] = (float)(ag / pw[1]); axis[2] = (float)(ab / pw[2]);
+    {
+      const float len = sqrtf(axis[0] * axis[0] + axis[1] * axis[1] + axis[2] * axis[2]);
+      if (len < 1e-10f) { axis[0] = .2837149f; axis[1] = .9540631f; axis[2] = .096277453f; }
+      else for (int i = 0; i < 3; i++) axis[i] /= len;
+    }
+    // spread of the pixels along the axis (unweighted covariance projected on it)
+    const double c_rr = acc[4] / cnt - mean[0] * mean[0], c_rg = acc[5] / cnt - mean[0] * mean[1],
+                 c_rb = acc[6] / cnt - mean[0] * mean[2], c_gg = acc[7] / cnt - mean[1] * mean[1],
+                 c_gb = acc[8] / cnt - mean[1] * mean[2], c_bb = acc[9] / cnt - mean[2] * mean[2];
+    const double var_ax = axis[0] * axis[0] * c_rr + axis[1] * axis[1] * c_gg + axis[2] * axis[2] * c_bb +
+                          2 * (axis[0] * axis[1] * c_rg + axis[0] * axis[2] * c_rb + axis[1] * axis[2] * c_gb);
+    sd = (float)sqrt(fmax(var_ax, 0.0)) * 1.25f;
+    if (threadIdx.x == 0) { s_axis[0] = axis[0]; s_axis[1] = axis[1]; s_axis[2] = axis[2]; s_axis[3] = sd; }
   }
-  float axis[3] = {(float)(ar / pw[0]), (float)(ag / pw[1]), (float)(ab / pw[2])};
-  {
-    const float len = sqrtf(axis[0] * axis[0] + axis[1] * axis[1] + axis[2] * axis[2]);
-    if (len < 1e-10f) { axis[0] = .2837149f; axis[1] = .9540631f; axis[2] = .096277453f; }
-    else for (int i = 0; i < 3; i++) axis[i] /= len;
-  }
+  __syncthreads();
+  axis[0] = s_axis[0]; axis[1] = s_axis[1]; axis[2] = s_axis[2]; sd = s_axis[3];
+  const float wr = perc ? 8.f : 1.f, wg = perc ? 25.f : 1.f;
   // 2. projection bounds
   float pr[2] = {3.4e38f, -3.4e38f};
-  for_pixels([&](uint32_t p) {
+  each_pixel([&](uint32_t p) {
     const float d = ((float)px_r(p) - mean[0]) * axis[0] + ((float)px_g(p) - mean[1]) * axis[1] + ((float)px_b(p) - mean[2]) * axis[2];
     pr[0] = fminf(pr[0], d);
     pr[1] = fmaxf(pr[1], d);
@@ -1954,13 +2052,6 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
               bi = clampi((int)floorf(b * 31.f / 255.f + .5f), 0, 31);
     return (uint32_t)((ri << 11) | (gi << 5) | bi);
   };
-  // spread of the pixels along the axis (unweighted covariance projected on it)
-  const double c_rr = acc[4] / cnt - mean[0] * mean[0], c_rg = acc[5] / cnt - mean[0] * mean[1],
-               c_rb = acc[6] / cnt - mean[0] * mean[2], c_gg = acc[7] / cnt - mean[1] * mean[1],
-               c_gb = acc[8] / cnt - mean[1] * mean[2], c_bb = acc[9] / cnt - mean[2] * mean[2];
-  const double var_ax = axis[0] * axis[0] * c_rr + axis[1] * axis[1] * c_gg + axis[2] * axis[2] * c_bb +
-                        2 * (axis[0] * axis[1] * c_rg + axis[0] * axis[2] * c_rb + axis[1] * axis[2] * c_gb);
-  const float sd = (float)sqrt(fmax(var_ax, 0.0)) * 1.25f;
   // 3. two starts -- the extreme projections and mean +- 1.25 sigma -- each refined by alternating
   // nearest-colour selectors and least-squares endpoints; keep the lowest (perceptual) error
   uint32_t best0 = 0, best1 = 0;
@@ -1970,24 +2061,26 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
     uint32_t e0 = q565(mean[0] + hi_t * axis[0], mean[1] + hi_t * axis[1], mean[2] + hi_t * axis[2]);
     uint32_t e1 = q565(mean[0] + lo_t * axis[0], mean[1] + lo_t * axis[1], mean[2] + lo_t * axis[2]);
     for (int it = 0; it < 8; it++) {
-      int col[4][3];
-      colors4(e0, e1, col);  // DXT order
+      FitEntry q[4];
+      fit_entries(e0, e1, wr, wg, q);  // DXT order
       float a[10];
       for (int i = 0; i < 10; i++) a[i] = 0.f;
-      for_pixels([&](uint32_t p) {
-        const int r = px_r(p), g = px_g(p), b = px_b(p);
-        uint32_t bd = 0xFFFFFFFFu;
+      each_pixel([&](uint32_t p) {
+        const float r = (float)px_r(p), g = (float)px_g(p), b = (float)px_b(p);
+        float bd = q[0].part(r, g, b);
         int bs = 0;
-        for (int q = 0; q < 4; q++) {
-          const uint32_t d = cdist(perc, r, g, b, col[q][0], col[q][1], col[q][2]);
-          if (d < bd) { bd = d; bs = q; }
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+          const float d = q[k].part(r, g, b);
+          if (d < bd) { bd = d; bs = k; }
         }
+        bd += wr * (r * r) + wg * (g * g) + b * b;
         // weight of the first endpoint at DXT selector q: 1, 0, 2/3, 1/3
         const float wa = bs == 0 ? 1.f : bs == 1 ? 0.f : bs == 2 ? (2.f / 3.f) : (1.f / 3.f), wb = 1.f - wa;
         a[0] += wa * wa; a[1] += wa * wb; a[2] += wb * wb;
         a[3] += wa * r; a[4] += wa * g; a[5] += wa * b;
         a[6] += wb * r; a[7] += wb * g; a[8] += wb * b;
-        a[9] += (float)bd;
+        a[9] += bd;
       });
       block_sum<10>(a, red);
       if (a[9] < best_err) { best_err = a[9]; best0 = e0; best1 = e1; }
@@ -2004,22 +2097,19 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
       e0 = n0; e1 = n1;
     }
   }
+  int unique = 0;  // colours in the table, if it holds all
   // 3b. the uber probe search of dxt1_endpoint_optimizer::optimize_endpoints (crnlib/crn_dxt1.cpp:703-1028)
   // over the cluster's unique colours: low and high endpoints probed along the principal axis
   // (g_uber_probe_table steps of 1/64), every low x high pair, then the 26 lattice neighbours and
   // +-2 axis moves of each endpoint of the best pair; up to four passes.
   {
-    // hashing: keys in s_raw[0, kUniqCap), counts in s_raw[kUniqCap, 2 kUniqCap); once compacted (at
-    // most kUniqCap / 2 colours): the int4 probe table in s_raw[0, 2 kUniqCap), counts after it
-    __shared__ __align__(16) uint32_t s_raw[2 * kUniqCap + kUniqCap / 2];
     uint32_t* s_key = s_raw;
     uint32_t* s_cnt = s_raw + kUniqCap;
-    int4* s_ut = reinterpret_cast<int4*>(s_raw);
-    uint32_t* s_uc = s_raw + 2 * kUniqCap;
+    FitTable T{reinterpret_cast<float*>(s_raw), s_raw + 2 * kUniqCap, 0, wr, wg};
     __shared__ uint32_t s_cand[kMaxCand];
     __shared__ unsigned long long s_be[kFitThreads / 32];
     __shared__ uint32_t s_bi[kFitThreads / 32];
-    __shared__ uint32_t s_nu, s_overflow;
+    __shared__ uint32_t s_nu, s_overflow, s_valid;
     __syncthreads();
     for (int i = threadIdx.x; i < kUniqCap; i += blockDim.x) { s_key[i] = 0; s_cnt[i] = 0; }
     if (threadIdx.x == 0) { s_nu = 0; s_overflow = 0; }
@@ -2052,12 +2142,16 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
       const int at = base + incl - nm;
       __syncthreads();
       for (int j = 0; j < nm; j++)
-        if (at + j < kUniqCap / 2) { s_ut[at + j] = probe_entry(mine_key[j], perc); s_uc[at + j] = mine_cnt[j]; }
-      if (threadIdx.x == blockDim.x - 1) s_nu = (uint32_t)(at + nm);
+        if (at + j < kUniqCap / 2) T.set(at + j, mine_key[j], mine_cnt[j]);
+      if (threadIdx.x == blockDim.x - 1) {
+        s_nu = (uint32_t)(at + nm);
+        if (((at + nm) & 1) && at + nm < kUniqCap / 2) T.set(at + nm, 0, 0);
+      }
     }
     __syncthreads();
-    const int U = (int)s_nu;
-    if (!s_overflow && U > 0 && U <= kUniqCap / 2) {
+    T.n = (int)s_nu;
+    if (!s_overflow && T.n > 0 && T.n <= kUniqCap / 2) {
+      unique = cnt < 1e9f ? T.n : 0;
       // best so far: the least-squares fit
       uint32_t bl = best0, bh = best1;
       unsigned long long berr;
@@ -2065,7 +2159,7 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
         uint32_t pair;
         if (threadIdx.x == 0) s_cand[0] = bl | (bh << 16);
         __syncthreads();
-        best_candidate(s_cand, 1, s_ut, s_uc, U, perc, ~0ull, s_be, s_bi, berr, pair);
+        best_candidate<4>(s_cand, 1, 1, T, ~0ull, s_be, s_bi, berr, pair);
       }
       // low / high colours from the axis projection bounds, in 565 units
       float lowc[3], highc[3];
@@ -2084,26 +2178,23 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
           unpack565(bh, ch);
           for (int c = 0; c < 3; c++) { lowc[c] = (float)cl[c] / 255.f * lim[c]; highc[c] = (float)ch[c] / 255.f * lim[c]; }
         }
-        // probe lists (thread 0), then every low x high pair
+        // probe lists (warp 0 the low ones, warp 1 the high ones; lane k: step (k + 1) / 2, backward
+        // for odd k, unless it is where the last step that way already was), then every low x high pair
         __shared__ uint32_t s_pl[32], s_ph[32], s_npl, s_nph;
-        if (threadIdx.x == 0) {
-          for (int which = 0; which < 2; which++) {
-            const float* base = which ? highc : lowc;
-            uint32_t* outp = which ? s_ph : s_pl;
-            int prev[2] = {-1, -1}, n = 0;
-            for (int i = 0; i < 15; i++) {
-              const int x = c_probe[i];
-              for (int sg = i ? 0 : 1; sg < 2; sg++) {
-                const float f = sg ? 1.f : -1.f;
-                const int r = clampi((int)floorf(base[0] + .5f + f * sax[0] * (float)x), 0, 31);
-                const int g = clampi((int)floorf(base[1] + .5f + f * sax[1] * (float)x), 0, 63);
-                const int b = clampi((int)floorf(base[2] + .5f + f * sax[2] * (float)x), 0, 31);
-                const int pc = b | (g << 5) | (r << 11);
-                if (pc != prev[sg]) { outp[n++] = (uint32_t)pc; prev[sg] = pc; }
-              }
-            }
-            if (which) s_nph = (uint32_t)n; else s_npl = (uint32_t)n;
-          }
+        if (threadIdx.x < 64) {
+          const int which = threadIdx.x >> 5, lane = threadIdx.x & 31;
+          const float* base = which ? highc : lowc;
+          const int x = c_probe[min((lane + 1) >> 1, 14)];
+          const float f = (lane + 1) & 1 ? 1.f : -1.f;
+          const int r = clampi((int)floorf(base[0] + .5f + f * sax[0] * (float)x), 0, 31);
+          const int g = clampi((int)floorf(base[1] + .5f + f * sax[1] * (float)x), 0, 63);
+          const int b = clampi((int)floorf(base[2] + .5f + f * sax[2] * (float)x), 0, 31);
+          const uint32_t pc = (uint32_t)(b | (g << 5) | (r << 11));
+          const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, pc, 2);
+          const bool in = lane < 29 && (lane < 2 || pc != prev);
+          const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
+          if (in) (which ? s_ph : s_pl)[__popc(m & ((1u << lane) - 1u))] = pc;
+          if (!lane) (which ? s_nph : s_npl) = (uint32_t)__popc(m);
         }
         __syncthreads();
         const int npl = (int)s_npl, nph = (int)s_nph;
@@ -2112,38 +2203,32 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
         {
           unsigned long long e;
           uint32_t pair;
-          best_candidate(s_cand, npl * nph, s_ut, s_uc, U, perc, berr, s_be, s_bi, e, pair);
+          best_candidate<1>(s_cand, npl * nph, ~0u, T, berr, s_be, s_bi, e, pair);
           if (e < berr) { berr = e; bl = pair & 0xFFFFu; bh = pair >> 16; }
         }
         // lattice neighbours (26) and +-2 axis moves of the low endpoint, then of the high one
         for (int which = 0; which < 2; which++) {
-          if (threadIdx.x == 0) {
-            int n = 0;
+          if (threadIdx.x < 32) {  // lane i: neighbour i of the 26 (centre left out), then a +-2 move
+            const int i = threadIdx.x;
             const uint32_t E = which ? bh : bl, O2 = which ? bl : bh;
-            const int r0 = (E >> 11) & 31, g0 = (E >> 5) & 63, b0 = E & 31;
-            for (int dr = -1; dr <= 1; dr++)
-              for (int dg = -1; dg <= 1; dg++)
-                for (int db = -1; db <= 1; db++) {
-                  if (!dr && !dg && !db) continue;
-                  const int r = r0 + dr, g = g0 + dg, b = b0 + db;
-                  if (r < 0 || r > 31 || g < 0 || g > 63 || b < 0 || b > 31) continue;
-                  const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
-                  s_cand[n++] = which ? (O2 | (X << 16)) : (X | (O2 << 16));
-                }
-            const int d6[6][3] = {{-2, 0, 0}, {2, 0, 0}, {0, -2, 0}, {0, 2, 0}, {0, 0, -2}, {0, 0, 2}};
-            for (int q = 0; q < 6; q++) {
-              const int r = r0 + d6[q][0], g = g0 + d6[q][1], b = b0 + d6[q][2];
-              if (r < 0 || r > 31 || g < 0 || g > 63 || b < 0 || b > 31) continue;
-              const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
-              s_cand[n++] = which ? (O2 | (X << 16)) : (X | (O2 << 16));
+            int r = (E >> 11) & 31, g = (E >> 5) & 63, b = E & 31;
+            if (i < 26) {
+              const int c = i < 13 ? i : i + 1;
+              r += c / 9 - 1; g += c / 3 % 3 - 1; b += c % 3 - 1;
+            } else {
+              const int by = i & 1 ? 2 : -2, axis_i = (i - 26) >> 1;
+              r += axis_i == 0 ? by : 0; g += axis_i == 1 ? by : 0; b += axis_i == 2 ? by : 0;
             }
-            s_npl = (uint32_t)n;
+            const bool in = (unsigned)r <= 31u && (unsigned)g <= 63u && (unsigned)b <= 31u;
+            const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
+            s_cand[i] = which ? (O2 | (X << 16)) : (X | (O2 << 16));
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
+            if (!i) s_valid = m;
           }
           __syncthreads();
-          const int n = (int)s_npl;
           unsigned long long e;
           uint32_t pair;
-          best_candidate(s_cand, n, s_ut, s_uc, U, perc, berr, s_be, s_bi, e, pair);
+          best_candidate<4>(s_cand, 32, s_valid, T, berr, s_be, s_bi, e, pair);
           if (e < berr) { berr = e; bl = pair & 0xFFFFu; bh = pair >> 16; }
         }
         if (pass && berr == prev_err) break;
@@ -2158,7 +2243,6 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
   // selectors re-chosen for the walk's result while the true error keeps falling
   __shared__ unsigned long long s_stat[29];  // hist[4], D2[4][3], DD[4][3] (exact integers), error
   __shared__ uint32_t s_LH[2];
-  __shared__ uint32_t s_sol[54], s_nsol;
   uint32_t L0 = best0 > best1 ? best0 : best1, H0 = best0 > best1 ? best1 : best0;
   if (L0 == H0) { if (L0 < 0xFFFFu) L0++; else H0--; }
   uint32_t keepL = L0, keepH = H0;
@@ -2169,22 +2253,63 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
     __syncthreads();
     if (threadIdx.x < 29) s_stat[threadIdx.x] = 0;
     __syncthreads();
-    for_pixels([&](uint32_t p) {
-      const int r = px_r(p), g = px_g(p), b = px_b(p);
-      uint32_t bd = 0xFFFFFFFFu;
-      int bs = 0;
-      for (int t = 0; t < 4; t++) {
-        const uint32_t d = cdist(perc, r, g, b, col[t][0], col[t][1], col[t][2]);
-        if (d < bd) { bd = d; bs = t; }
+    if (unique) {
+      // selectors into the counts' top bits, then thread 4 i + j adds every fourth colour to sum i
+      float* tc = reinterpret_cast<float*>(s_raw);
+      uint32_t* tn = s_raw + 2 * kUniqCap;
+      constexpr uint32_t kCount = (1u << 30) - 1;
+      FitEntry q[4];
+      fit_entries(L0, H0, wr, wg, q);
+      unsigned long long er = 0;
+      for (int i = threadIdx.x; i < unique; i += blockDim.x) {
+        const float* e = tc + (i >> 1) * 8 + (i & 1);
+        float bd = q[0].part(e[0], e[2], e[4]);
+        uint32_t bs = 0;
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+          const float d = q[k].part(e[0], e[2], e[4]);
+          if (d < bd) { bd = d; bs = (uint32_t)k; }
+        }
+        const uint32_t n = tn[i] & kCount;
+        er += (unsigned long long)(__float_as_uint(e[6] + bd) - 0x4B000000u) * n;
+        tn[i] = n | bs << 30;
       }
-      atomicAdd(&s_stat[bs], 1ull);
-      const int rgb[3] = {r, g, b};
-      for (int c = 0; c < 3; c++) {
-        atomicAdd(&s_stat[4 + bs * 3 + c], (unsigned long long)(2 * rgb[c]));
-        atomicAdd(&s_stat[16 + bs * 3 + c], (unsigned long long)(rgb[c] * rgb[c]));
+      for (int o = 16; o > 0; o >>= 1) er += __shfl_xor_sync(0xFFFFFFFFu, er, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&s_stat[28], er);
+      __syncthreads();
+      {
+        const int id = threadIdx.x >> 2, at = id < 4 ? 0 : (id - 4) % 12;
+        const uint32_t bs = (uint32_t)(id < 4 ? id : at / 3);
+        unsigned long long sum = 0;
+        for (int i = threadIdx.x & 3; i < unique; i += 4) {
+          const uint32_t v = tn[i];
+          const uint32_t x = (uint32_t)tc[(i >> 1) * 8 + (i & 1) + 2 * (at % 3)];
+          const uint32_t term = id < 4 ? 1u : id < 16 ? 2u * x : x * x;
+          if (v >> 30 == bs) sum += (unsigned long long)(v & kCount) * term;
+        }
+        __syncwarp();
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+        if (id < 28 && !(threadIdx.x & 3)) s_stat[id] = sum;
       }
-      atomicAdd(&s_stat[28], (unsigned long long)bd);
-    });
+    } else {
+      for_pixels([&](uint32_t p) {
+        const int r = px_r(p), g = px_g(p), b = px_b(p);
+        uint32_t bd = 0xFFFFFFFFu;
+        int bs = 0;
+        for (int t = 0; t < 4; t++) {
+          const uint32_t d = cdist(perc, r, g, b, col[t][0], col[t][1], col[t][2]);
+          if (d < bd) { bd = d; bs = t; }
+        }
+        atomicAdd(&s_stat[bs], 1ull);
+        const int rgb[3] = {r, g, b};
+        for (int c = 0; c < 3; c++) {
+          atomicAdd(&s_stat[4 + bs * 3 + c], (unsigned long long)(2 * rgb[c]));
+          atomicAdd(&s_stat[16 + bs * 3 + c], (unsigned long long)(rgb[c] * rgb[c]));
+        }
+        atomicAdd(&s_stat[28], (unsigned long long)bd);
+      });
+    }
     __syncthreads();
     const unsigned long long true_err = s_stat[28];
     if (true_err >= keep_err) break;  // uniform: every thread reads the same shared value
@@ -2192,7 +2317,7 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
     keepL = L0;
     keepH = H0;
     if (threadIdx.x < 32) {
-      // the walk runs on warp 0: lane 0 lists the moves, the lanes score them, exactly in 64-bit
+      // the walk runs on warp 0, a lane per move, scored exactly in 64-bit
       // integers (the histogram sums are exact, so the reference's double sums are these values)
       const int lane = threadIdx.x;
       long long hist[4], D2[4][3], DD[4][3];
@@ -2214,62 +2339,45 @@ __global__ void __launch_bounds__(kFitThreads) k_cluster_fit(const uint32_t* __r
       uint32_t wL = L0, wH = H0;
       long long best = err_of(wL, wH);
       const bool preserveL = hist[0] + hist[2] > hist[1] + hist[3];
+      auto apart = [&](uint32_t& L, uint32_t& H) {
+        if (L != H) return;
+        L += !preserveL ? ((~L & 0x1F) ? 0x1 : (~L & 0xF800) ? 0x800 : (~L & 0x7E0) ? 0x20 : 0) : (!L ? 0x1 : 0);
+        H -= preserveL ? ((H & 0x1F) ? 0x1 : (H & 0xF800) ? 0x800 : (H & 0x7E0) ? 0x20 : 0) : (H == 0xFFFF ? 0x1 : 0);
+        L &= 0xFFFFu; H &= 0xFFFFu;
+      };
       bool improved = true;
       for (int iters = 8; improved && iters; iters--) {
         improved = false;
-        if (lane == 0) {
-          int ns = 0;
-          for (int which = 0; which < 2; which++) {
-            const uint32_t E = which ? wH : wL, O2 = which ? wL : wH;
-            const int b0 = E & 31, g0 = (E >> 5) & 63, r0 = (E >> 11) & 31;
-            for (int b = b0 ? b0 - 1 : b0; b <= b0 + 1 && b <= 31; b++)
-              for (int g = g0 ? g0 - 1 : g0; g <= g0 + 1 && g <= 63; g++)
-                for (int r = r0 ? r0 - 1 : r0; r <= r0 + 1 && r <= 31; r++) {
-                  const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
-                  if (X != E) s_sol[ns++] = X > O2 ? (X | (O2 << 16)) : (O2 | (X << 16));
-                }
-          }
-          for (int i = 1; i < ns; i++) {  // sorted, as the reference evaluates them
-            const uint32_t x = s_sol[i];
-            int j = i - 1;
-            while (j >= 0 && s_sol[j] > x) { s_sol[j + 1] = s_sol[j]; j--; }
-            s_sol[j + 1] = x;
-          }
-          s_nsol = (uint32_t)ns;
+        // the neighbours of both endpoints (26 each; lane i the i-th of each), ordered pairs; among equal
+        // errors the lowest pair wins, as the first of the sorted list that the reference walks
+        long long le = LLONG_MAX;
+        uint32_t lp = 0xFFFFFFFFu;
+        for (int which = 0; which < 2; which++) {
+          if (lane >= 26) continue;
+          const uint32_t E = which ? wH : wL, O2 = which ? wL : wH;
+          const int c = lane < 13 ? lane : lane + 1;
+          const int b = (int)(E & 31) + c / 9 - 1, g = (int)((E >> 5) & 63) + c / 3 % 3 - 1, r = (int)(E >> 11 & 31) + c % 3 - 1;
+          if ((unsigned)r > 31u || (unsigned)g > 63u || (unsigned)b > 31u) continue;
+          const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
+          const uint32_t sol = X > O2 ? (X | (O2 << 16)) : (O2 | (X << 16));
+          uint32_t L = sol & 0xFFFFu, H = sol >> 16;
+          apart(L, H);
+          const long long er = err_of(L, H);
+          if (er < le || (er == le && sol < lp)) { le = er; lp = sol; }
         }
         __syncwarp();
-        const int ns = (int)s_nsol;
-        // the first strictly better move in sorted order wins ties: (error, index) minimum
-        long long le = LLONG_MAX;
-        int li = 0x7FFFFFFF;
-        for (int i = lane; i < ns; i += 32) {
-          if (i && s_sol[i] == s_sol[i - 1]) continue;
-          uint32_t L = s_sol[i] & 0xFFFFu, H = s_sol[i] >> 16;
-          if (L == H) {
-            L += !preserveL ? ((~L & 0x1F) ? 0x1 : (~L & 0xF800) ? 0x800 : (~L & 0x7E0) ? 0x20 : 0) : (!L ? 0x1 : 0);
-            H -= preserveL ? ((H & 0x1F) ? 0x1 : (H & 0xF800) ? 0x800 : (H & 0x7E0) ? 0x20 : 0) : (H == 0xFFFF ? 0x1 : 0);
-            L &= 0xFFFFu; H &= 0xFFFFu;
-          }
-          const long long er = err_of(L, H);
-          if (er < le) { le = er; li = i; }
-        }
         for (int o = 16; o > 0; o >>= 1) {
           const long long oe = __shfl_xor_sync(0xFFFFFFFFu, le, o);
-          const int oi = __shfl_xor_sync(0xFFFFFFFFu, li, o);
-          if (oe < le || (oe == le && oi < li)) { le = oe; li = oi; }
+          const uint32_t op = __shfl_xor_sync(0xFFFFFFFFu, lp, o);
+          if (oe < le || (oe == le && op < lp)) { le = oe; lp = op; }
         }
         if (le < best) {
           best = le;
-          uint32_t L = s_sol[li] & 0xFFFFu, H = s_sol[li] >> 16;
-          if (L == H) {
-            L += !preserveL ? ((~L & 0x1F) ? 0x1 : (~L & 0xF800) ? 0x800 : (~L & 0x7E0) ? 0x20 : 0) : (!L ? 0x1 : 0);
-            H -= preserveL ? ((H & 0x1F) ? 0x1 : (H & 0xF800) ? 0x800 : (H & 0x7E0) ? 0x20 : 0) : (H == 0xFFFF ? 0x1 : 0);
-            L &= 0xFFFFu; H &= 0xFFFFu;
-          }
+          uint32_t L = lp & 0xFFFFu, H = lp >> 16;
+          apart(L, H);
           wL = L; wH = H;
           improved = true;
         }
-        __syncwarp();  // s_sol is rewritten by lane 0 in the next step
         if (best == 0) break;
       }
       if (wL <= wH) {  // keep 4-colour order (first > second)
