@@ -1796,7 +1796,7 @@ __device__ __forceinline__ uint32_t tile_npix(uint32_t kind) { return 16u << (ki
 // Unique colours of a cluster in shared memory (open addressing on the packed RGB, count per
 // colour); a cluster with more than kUniqCap / 2 distinct colours skips the probe search.
 constexpr int kUniqCap = 4096;
-constexpr int kMaxCand = 1024;
+constexpr int kMaxCand = 29 * 29;
 __constant__ int16_t c_probe[15] = {0, 1, 2, 3, 5, 7, 9, 10, 13, 15, 19, 27, 43, 59, 91};  // g_uber_probe_table
 
 // A palette colour p for colours x in floats: -2 w . p and w . p^2 (w = 8, 25, 1 perceptual, else 1).
@@ -1850,12 +1850,45 @@ struct FitTable {
   }
 };
 
+// Lower bounds of a pair's error: per component value (5:6:5, the red ones at 0, green 32, blue 96) what
+// the colours below it and above it would cost against it in that component alone. A palette's
+// components lie between its endpoints'. It settles half of the pairs of a probe list; filling it and
+// joining what is left costs about as much as the lists of a cluster of kBoundFrom colours.
+constexpr int kBoundFrom = 128;
+struct FitBound {
+  unsigned long long below[128], above[128];
+  __device__ __forceinline__ unsigned long long of(uint32_t lo, uint32_t hi) const {
+    const uint32_t l[3] = {lo >> 11 & 31, 32 + (lo >> 5 & 63), 96 + (lo & 31)};
+    const uint32_t h[3] = {hi >> 11 & 31, 32 + (hi >> 5 & 63), 96 + (hi & 31)};
+    unsigned long long e = 0;
+#pragma unroll
+    for (int c = 0; c < 3; c++) e += below[min(l[c], h[c])] + above[max(l[c], h[c])];
+    return e;
+  }
+  // thread t of 128 sets entry t
+  __device__ __forceinline__ void fill(const FitTable& T) {
+    const int t = threadIdx.x, c = t < 32 ? 0 : t < 96 ? 1 : 2, v = t - (c == 0 ? 0 : c == 1 ? 32 : 96);
+    const int x = c == 1 ? exp6(v) : exp5(v);
+    unsigned long long b = 0, a = 0;
+    for (int i = 0; i < T.n; i++) {
+      const int d = x - (int)T.col[(i >> 1) * 8 + (i & 1) + 2 * c];
+      const unsigned long long e = (unsigned long long)(uint32_t)(d * d) * T.cnt[i];
+      if (d > 0) b += e; else a += e;
+    }
+    const unsigned w = (unsigned)(c == 0 ? T.wr : c == 1 ? T.wg : 1.f);
+    below[t] = b * w;
+    above[t] = a * w;
+  }
+};
+
 // Error of the 4-colour block (lo, hi) over the colour pairs from, from + step, ..., abandoned
-// (returning ~0) as soon as its running sum reaches `bound` (a candidate that cannot win); one thread.
+// (returning ~0) as soon as its running sum reaches `bound` or is above *best, the lowest error found by
+// any thread so far (a candidate that cannot win); one thread.
 // Two colours and an entry take three packed multiply-adds; the integer form of the same took three
 // times the instructions.
 __device__ __forceinline__ unsigned long long pair_error(uint32_t lo, uint32_t hi, const FitTable& T, int from, int step,
-                                                        unsigned long long bound) {
+                                                        unsigned long long bound,
+                                                        const volatile unsigned long long* best) {
   FitEntry q[4];
   fit_entries(lo, hi, T.wr, T.wg, q);
   uint64_t qr[4], qg[4], qb[4], qp[4];
@@ -1876,7 +1909,7 @@ __device__ __forceinline__ unsigned long long pair_error(uint32_t lo, uint32_t h
     e += (unsigned long long)(__float_as_uint(x0 + m0) - 0x4B000000u) * w.x;
     e += (unsigned long long)(__float_as_uint(x1 + m1) - 0x4B000000u) * w.y;
     if (--left == 0) {
-      if (e >= bound) return ~0ull;
+      if (e >= bound || e > *best) return ~0ull;
       left = 8;
     }
   }
@@ -1885,16 +1918,17 @@ __device__ __forceinline__ unsigned long long pair_error(uint32_t lo, uint32_t h
 
 // Evaluates the candidate pairs cand[0..n) (lo | hi << 16; of the first 32 those in `valid`), kSplit
 // threads per candidate, and returns to every thread the best (lowest error, then lowest index) among
-// those below `bound`; err = ~0 and pair = 0 when none is.
+// those below `bound`; err = ~0 and pair = 0 when none is. *best is at least `bound` on entry.
 template <int kSplit>
 __device__ void best_candidate(const uint32_t* cand, int n, uint32_t valid, const FitTable& T, unsigned long long bound,
-                               unsigned long long* s_be, uint32_t* s_bi, unsigned long long& err, uint32_t& pair) {
+                               unsigned long long* best, unsigned long long* s_be, uint32_t* s_bi,
+                               unsigned long long& err, uint32_t& pair) {
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, sub = threadIdx.x % kSplit;
   unsigned long long be = ~0ull;
   uint32_t bi = 0xFFFFFFFFu;
   if (kSplit > 1) {  // one candidate for each group of threads: n is at most kFitThreads / kSplit
     const int i = threadIdx.x / kSplit;
-    if (i < n && (valid >> i & 1)) be = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, sub, kSplit, bound);
+    if (i < n && (valid >> i & 1)) be = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, sub, kSplit, bound, best);
     __syncwarp();
 #pragma unroll
     for (int o = 1; o < kSplit; o <<= 1) {
@@ -1907,8 +1941,12 @@ __device__ void best_candidate(const uint32_t* cand, int n, uint32_t valid, cons
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       if (i < 32 && !(valid >> i & 1)) continue;
       // a later candidate must beat this thread's best strictly (ties go to the lower index)
-      const unsigned long long e = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, 0, 1, min(bound, be));
-      if (e < be) { be = e; bi = (uint32_t)i; }
+      const unsigned long long e = pair_error(cand[i] & 0xFFFFu, cand[i] >> 16, T, 0, 1, min(bound, be), best);
+      if (e < be) {
+        be = e;
+        bi = (uint32_t)i;
+        atomicMin(best, e);
+      }
     }
     __syncwarp();
   }
@@ -1934,15 +1972,16 @@ __device__ void best_candidate(const uint32_t* cand, int n, uint32_t valid, cons
 // memory for the least-squares passes, the principal axis (double precision: 64 cycles an instruction
 // for a warp, whatever the others do) is one warp's work, the probes and moves are listed and scored by
 // a lane each, and the walk's statistics are summed over unique colours by a few threads for each sum.
-// The 2415 clusters of a 1024 x 1024 chain (580 unique colours each) took 4.1 ms, now 1.9.
+// The 2415 clusters of a 1024 x 1024 chain (580 unique colours each) took 4.1 ms, now 1.6.
 __global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* __restrict__ blocks,
                                                              const Chunk* __restrict__ chunks,
                                                              const Tile* __restrict__ tiles,
                                                              const uint32_t* __restrict__ ctile_start,
                                                              const uint32_t* __restrict__ ctile_list, int perceptual,
                                                              ClusterOut* __restrict__ out) {
-  __shared__ float red[24 * 16];
-  __shared__ uint32_t s_tiles[256];
+  __shared__ float red[10 * 16 + 32];
+  __shared__ uint32_t s_cand[kMaxCand];
+  uint32_t* s_tiles = s_cand;  // 256 of them, while no candidates are listed
   // the cluster's pixels, [the thread's pixel][thread]; then the hash of its unique colours, keys in
   // s_raw[0, kUniqCap), counts in s_raw[kUniqCap, 2 kUniqCap); once compacted (at most kUniqCap / 2
   // colours): the colour table in s_raw[0, 2 kUniqCap), its counts after it
@@ -2106,7 +2145,8 @@ __global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* 
     uint32_t* s_key = s_raw;
     uint32_t* s_cnt = s_raw + kUniqCap;
     FitTable T{reinterpret_cast<float*>(s_raw), s_raw + 2 * kUniqCap, 0, wr, wg};
-    __shared__ uint32_t s_cand[kMaxCand];
+    __shared__ FitBound s_bound;
+    __shared__ unsigned long long s_best;
     __shared__ unsigned long long s_be[kFitThreads / 32];
     __shared__ uint32_t s_bi[kFitThreads / 32];
     __shared__ uint32_t s_nu, s_overflow, s_valid;
@@ -2126,40 +2166,66 @@ __global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* 
     });
     __syncthreads();
     // compact the table in place (slot order); count distinct colours
-    __shared__ uint32_t s_wcnt[kFitThreads / 32 + 1];
     uint32_t mine_key[kUniqCap / kFitThreads], mine_cnt[kUniqCap / kFitThreads];
+    // in four classes by distance from the mean, the farthest first (any order gives the same sums): class
+    // counts as four 16-bit fields, at most kUniqCap in all
+    const float spread = wr * (acc[4] / cnt - mean[0] * mean[0]) + wg * (acc[7] / cnt - mean[1] * mean[1]) +
+                         (acc[9] / cnt - mean[2] * mean[2]);
+    auto level = [&](uint32_t rgb) {
+      const float dr = (float)px_r(rgb) - mean[0], dg = (float)px_g(rgb) - mean[1], db = (float)px_b(rgb) - mean[2];
+      const float d = wr * dr * dr + wg * dg * dg + db * db;
+      return d > 2.5f * spread ? 0 : d > 1.2f * spread ? 16 : d > .5f * spread ? 32 : 48;
+    };
     int nm = 0;
+    unsigned long long mine = 0;
     for (int i = threadIdx.x * (kUniqCap / kFitThreads); i < (int)((threadIdx.x + 1) * (kUniqCap / kFitThreads)); i++)
-      if (s_key[i]) { mine_key[nm] = s_key[i] - 1u; mine_cnt[nm] = s_cnt[i]; nm++; }
+      if (s_key[i]) {
+        mine_key[nm] = s_key[i] - 1u;
+        mine_cnt[nm] = s_cnt[i];
+        mine += 1ull << level(mine_key[nm]);
+        nm++;
+      }
     {
-      // exclusive scan of nm over the CTA
-      int incl = nm;
-      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o); if ((threadIdx.x & 31) >= o) incl += v; }
-      if ((threadIdx.x & 31) == 31) s_wcnt[threadIdx.x >> 5] = incl;
+      // exclusive scan over the CTA
+      unsigned long long incl = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if ((threadIdx.x & 31) >= o) incl += v;
+      }
+      if ((threadIdx.x & 31) == 31) s_be[threadIdx.x >> 5] = incl;
       __syncthreads();
-      int base = 0;
-      for (int w = 0; w < (int)(threadIdx.x >> 5); w++) base += s_wcnt[w];
-      const int at = base + incl - nm;
-      __syncthreads();
-      for (int j = 0; j < nm; j++)
-        if (at + j < kUniqCap / 2) T.set(at + j, mine_key[j], mine_cnt[j]);
-      if (threadIdx.x == blockDim.x - 1) {
-        s_nu = (uint32_t)(at + nm);
-        if (((at + nm) & 1) && at + nm < kUniqCap / 2) T.set(at + nm, 0, 0);
+      unsigned long long before = incl - mine, total = 0;
+      for (int w = 0; w < kFitThreads / 32; w++) {
+        if (w < (int)(threadIdx.x >> 5)) before += s_be[w];
+        total += s_be[w];
+      }
+      // a class begins after the classes before it
+      before += (total << 16) + (total << 32) + (total << 48);
+      const int all = (int)((total & 0xFFFF) + (total >> 16 & 0xFFFF) + (total >> 32 & 0xFFFF) + (total >> 48));
+      for (int j = 0; j < nm; j++) {
+        const int sh = level(mine_key[j]), at = (int)(before >> sh & 0xFFFF);
+        before += 1ull << sh;
+        if (at < kUniqCap / 2) T.set(at, mine_key[j], mine_cnt[j]);
+      }
+      if (threadIdx.x == 0) {
+        s_nu = (uint32_t)all;
+        if ((all & 1) && all < kUniqCap / 2) T.set(all, 0, 0);
       }
     }
     __syncthreads();
     T.n = (int)s_nu;
     if (!s_overflow && T.n > 0 && T.n <= kUniqCap / 2) {
       unique = cnt < 1e9f ? T.n : 0;
+      const bool prune = T.n >= kBoundFrom;
+      if (prune) s_bound.fill(T);  // (read after the barriers below)
       // best so far: the least-squares fit
       uint32_t bl = best0, bh = best1;
       unsigned long long berr;
       {
         uint32_t pair;
-        if (threadIdx.x == 0) s_cand[0] = bl | (bh << 16);
+        if (threadIdx.x == 0) { s_cand[0] = bl | (bh << 16); s_best = ~0ull; }
         __syncthreads();
-        best_candidate<4>(s_cand, 1, 1, T, ~0ull, s_be, s_bi, berr, pair);
+        best_candidate<4>(s_cand, 1, 1, T, ~0ull, &s_best, s_be, s_bi, berr, pair);
       }
       // low / high colours from the axis projection bounds, in 565 units
       float lowc[3], highc[3];
@@ -2198,12 +2264,47 @@ __global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* 
         }
         __syncthreads();
         const int npl = (int)s_npl, nph = (int)s_nph;
-        for (int i = threadIdx.x; i < npl * nph; i += blockDim.x) s_cand[i] = s_pl[i / nph] | (s_ph[i % nph] << 16);
+        // the pairs whose bound leaves them a chance, in order: a warp lists a quarter of them, in place,
+        // and the quarters are then joined
+        int ncand = 0;
+        if (prune) {
+          const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pairs = npl * nph;
+          const int per = (pairs + kFitThreads / 32 - 1) / (kFitThreads / 32), first = warp * per, last = min(pairs, first + per);
+          for (int i0 = first; i0 < last; i0 += 32) {
+            const int i = i0 + lane;
+            const uint32_t lo = s_pl[min(i, pairs - 1) / nph], hi = s_ph[min(i, pairs - 1) % nph];
+            const bool in = i < last && s_bound.of(lo, hi) < berr;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
+            if (in) s_cand[first + ncand + __popc(m & ((1u << lane) - 1u))] = lo | (hi << 16);
+            ncand += __popc(m);
+          }
+          if (!lane) s_bi[warp] = (uint32_t)ncand;
+          if (threadIdx.x == 0) s_best = berr;
+          __syncthreads();
+          const uint32_t* from = s_cand + per;
+          int at = (int)s_bi[0];
+          for (int w = 1; w < kFitThreads / 32; w++, from += per) {  // to lower places: read, then write
+            const int n = (int)s_bi[w];
+            for (int i0 = 0; i0 < n; i0 += kFitThreads) {
+              const int i = i0 + (int)threadIdx.x;
+              const uint32_t v = i < n ? from[i] : 0u;
+              __syncthreads();
+              if (i < n) s_cand[at + i] = v;
+              __syncthreads();
+            }
+            at += n;
+          }
+          ncand = at;
+        } else {
+          ncand = npl * nph;
+          for (int i = threadIdx.x; i < ncand; i += kFitThreads) s_cand[i] = s_pl[i / nph] | (s_ph[i % nph] << 16);
+          if (threadIdx.x == 0) s_best = berr;
+        }
         __syncthreads();
         {
           unsigned long long e;
           uint32_t pair;
-          best_candidate<1>(s_cand, npl * nph, ~0u, T, berr, s_be, s_bi, e, pair);
+          best_candidate<1>(s_cand, ncand, ~0u, T, berr, &s_best, s_be, s_bi, e, pair);
           if (e < berr) { berr = e; bl = pair & 0xFFFFu; bh = pair >> 16; }
         }
         // lattice neighbours (26) and +-2 axis moves of the low endpoint, then of the high one
@@ -2222,13 +2323,13 @@ __global__ void __launch_bounds__(kFitThreads, 4) k_cluster_fit(const uint32_t* 
             const bool in = (unsigned)r <= 31u && (unsigned)g <= 63u && (unsigned)b <= 31u;
             const uint32_t X = (uint32_t)((r << 11) | (g << 5) | b);
             s_cand[i] = which ? (O2 | (X << 16)) : (X | (O2 << 16));
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
-            if (!i) s_valid = m;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, in && (!prune || s_bound.of(X, O2) < berr));
+            if (!i) { s_valid = m; s_best = berr; }
           }
           __syncthreads();
           unsigned long long e;
           uint32_t pair;
-          best_candidate<4>(s_cand, 32, s_valid, T, berr, s_be, s_bi, e, pair);
+          best_candidate<4>(s_cand, 32, s_valid, T, berr, &s_best, s_be, s_bi, e, pair);
           if (e < berr) { berr = e; bl = pair & 0xFFFFu; bh = pair >> 16; }
         }
         if (pass && berr == prev_err) break;
