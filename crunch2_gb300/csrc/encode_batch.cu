@@ -63,7 +63,13 @@ struct EncodeBatch {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   cudaGraphExec_t graph = nullptr;
+  size_t seed_bytes = 0;
 };
+
+// the search's block counter, behind the seeds
+uint32_t* next_block(const EncodeBatch* b) {
+  return reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(b->seeds.ptr) + b->seed_bytes);
+}
 
 int enqueue(EncodeBatch* b, cudaStream_t s, int colour_grid, int alpha_grid) {
   cudaError_t e;
@@ -82,7 +88,7 @@ int enqueue(EncodeBatch* b, cudaStream_t s, int colour_grid, int alpha_grid) {
   if (rc != CRNGPU_OK) return rc;
   if ((e = cudaEventRecord(b->join, b->side)) != cudaSuccess) return cuda_check(e, "record join");
   rc = launch_dxt1_chunks(blk, static_cast<const EncodeChunk*>(b->d_cchunks.ptr), b->ncolour, segs, b->seeds.ptr,
-                          colour_grid, s);
+                          next_block(b), colour_grid, s);
   if (rc != CRNGPU_OK) return rc;
   if ((e = cudaStreamWaitEvent(s, b->join, 0)) != cudaSuccess) return cuda_check(e, "wait join");
   return CRNGPU_OK;
@@ -103,7 +109,7 @@ int autotune(EncodeBatch* b, cudaStream_t s) {
     for (int rep = 0; rep < 2; rep++) {
       cudaEventRecord(ev[0], s);
       const int r = colour ? launch_dxt1_chunks(blk, static_cast<const EncodeChunk*>(b->d_cchunks.ptr), b->ncolour,
-                                                segs, b->seeds.ptr, grid, s)
+                                                segs, b->seeds.ptr, next_block(b), grid, s)
                            : launch_dxt5a_chunks(blk, static_cast<const EncodeChunk*>(b->d_achunks.ptr), b->nalpha,
                                                  segs, grid, s);
       if (r != CRNGPU_OK) return r;
@@ -245,7 +251,8 @@ extern "C" crngpu_encode_batch crngpu_encode_batch_create(const crngpu_encode_it
       rc = cuda_check(e, what);
   };
   if (rc == CRNGPU_OK && (e = b->blocks.ensure(nblocks * 64)) != cudaSuccess) rc = cuda_check(e, "alloc blocks");
-  if (rc == CRNGPU_OK && (e = b->seeds.ensure(nblocks * kDxt1SeedBytes)) != cudaSuccess) rc = cuda_check(e, "alloc seeds");
+  b->seed_bytes = nblocks * kDxt1SeedBytes;
+  if (rc == CRNGPU_OK && (e = b->seeds.ensure(b->seed_bytes + 16)) != cudaSuccess) rc = cuda_check(e, "alloc seeds");
   upload(b->d_tiles, tiles.data(), tiles.size() * sizeof(GatherTile), "upload gather tiles");
   upload(b->d_segs, segs.data(), segs.size() * sizeof(EncodeSegment), "upload segments");
   upload(b->d_cchunks, cchunks.data(), cchunks.size() * sizeof(EncodeChunk), "upload colour chunks");

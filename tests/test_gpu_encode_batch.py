@@ -76,3 +76,21 @@ def test_batch_rejects_bad_items(cg):
         cg.EncodeBatch([(rgba, out, w, h, n, 4)])  # a format this encoder does not write (DXT3)
     with pytest.raises(cg.CrnGpuError):
         cg.EncodeBatch([(rgba, out[:8], w, h, n, f)])  # output too small
+
+
+@pytest.mark.parametrize("blocks_past_two_rounds", [-1, 0, 1, 5])
+@pytest.mark.parametrize("quality", [4, 1])
+def test_block_counts_around_two_per_warp_match_short_calls(cg, blocks_past_two_rounds, quality):
+    # up to two blocks a search warp (32 warps an SM) are dealt out in turn, more through a counter
+    warps = torch.cuda.get_device_properties(0).multi_processor_count * 32
+    n = 2 * warps + blocks_past_two_rounds
+    rng = np.random.default_rng(n)
+    few = rng.integers(0, 256, (n, 4, 4), dtype=np.uint8)  # up to four colours a block
+    px = np.take_along_axis(few, rng.integers(0, 4, (n, 16, 1)), axis=1)
+    px[..., 3] = 255
+    px[::7] = rng.integers(0, 256, px[::7].shape, dtype=np.uint8) | np.uint8([0, 0, 0, 255])
+    blocks = torch.from_numpy(px.reshape(n, 64)).cuda()
+    got = cg.dxt1_optimize(blocks, quality=quality).cpu().numpy()
+    half = n // 2
+    want = [cg.dxt1_optimize(b.contiguous(), quality=quality).cpu().numpy() for b in (blocks[:half - 3], blocks[half - 3:n - 9], blocks[n - 9:])]
+    assert np.array_equal(got, np.concatenate(want))
