@@ -22,7 +22,7 @@
 // expression order without fused multiply-adds (the only FMAs are the explicit fmaf of exact
 // integer terms).
 //
-// DXT5A (dxt5_endpoint_optimizer, crnlib/crn_dxt5a.cpp:40-262) is warp per block, lane per
+// DXT5A (dxt5_endpoint_optimizer, crnlib/crn_dxt5a.cpp:40-262) is half a warp per block, lane per
 // candidate, with the same first-improvement resolution; its probe grid follows the moving
 // centre of the reference.
 #include <cuda_runtime.h>
@@ -1832,12 +1832,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
 }
 
 // ------------------------------------------------------------------------------------------
-// DXT5A: warp per block, lane per (low, high) candidate.
+// DXT5A: half a warp per block, lane per (low, high) candidate.
 
-// A warp's block: its unique values in evaluation order, farthest from the middle of their range first
-// so that the sums pass the best's early, two at a time (one of weight 0 pads them).
+// Half a warp's block: its unique values in evaluation order, farthest from the middle of their range
+// first so that the sums pass the best's early, then values of weight 0.
 struct AlphaShared {
-  float4 val[17];     // v, v + 2^23, weight, distance to 0 or 255
+  float4 val[16];     // v, v + 2^23, weight, distance to 0 or 255
   uint32_t uniq[16];  // first-occurrence order, the order of the pairs
 };
 
@@ -1865,8 +1865,9 @@ struct AlphaRange {
   }
 };
 
-// The errors of the warp's candidates, 8-value preferred on ties; where no lane's can be below `best`
-// any more the rest of the values is left out, and what is returned is at or above `best`.
+// The errors of the lanes' candidates, 8-value preferred on ties, over the first n values (of a half
+// warp that has fewer the rest have weight 0); where no lane's can be below its `best` any more the rest
+// is left out, and what is returned is at or above `best`.
 __device__ __forceinline__ float alpha_errors(const AlphaShared& S, int n, bool both, bool valid, int l, int h,
                                               float best, int& type) {
   const AlphaRange c(l, h);
@@ -1890,106 +1891,100 @@ __device__ __forceinline__ float alpha_errors(const AlphaShared& S, int n, bool 
   return fminf(e8, e6);
 }
 
-// One DXT5A element (dxt5_endpoint_optimizer::compute, crnlib/crn_dxt5a.cpp:40-196) of the 4x4
-// RGBA8 block px on channel comp, written as 8 bytes to o; a whole warp, lane per candidate.
-// quality: crn_dxt_quality; the probe grid is +-16 at Uber, +-8 at Better and absent below (:105-110).
-__device__ __forceinline__ void alpha_block(AlphaShared& S, const uint8_t* __restrict__ px, int comp, bool both,
-                                            uint32_t quality, uint8_t* __restrict__ o) {
-  const uint32_t lane = lane_id();
-  const uint32_t v = lane < 16 ? __ldg(px + lane * 4 + comp) : 0x100u + lane;
-  const unsigned match = __match_any_sync(FULL_MASK, v);
-  const int leader = __ffs(match) - 1;
-  const bool is_leader = lane < 16 && leader == (int)lane;
-  const unsigned lmask = __ballot_sync(FULL_MASK, is_leader);
-  const int n = __popc(lmask);
-  if (n == 1) {
-    if (lane == 0) *reinterpret_cast<uint2*>(o) = make_uint2(v | (v << 8), 0u);
-    return;
-  }
+// Two DXT5A elements (dxt5_endpoint_optimizer::compute, crnlib/crn_dxt5a.cpp:40-196), of the 4x4
+// RGBA8 block px on channel comp for each half of a warp, written as 8 bytes to o if `write`; a lane
+// per candidate. quality: crn_dxt_quality; the probe grid is +-16 at Uber, +-8 at Better and absent
+// below (:105-110). A half warp per block because the blocks of most channels have a handful of values,
+// whose pairs do not fill a warp, and its beginning and end are 16 texels' (a channel of a 2048 x 2048
+// image with a warp per block took 172 us, now 115).
+__device__ __forceinline__ void alpha_blocks(AlphaShared* shared, const uint8_t* __restrict__ px, int comp, bool both,
+                                             uint32_t quality, uint8_t* __restrict__ o, bool write) {
+  const int lane = (int)lane_id() & 15, half = (int)lane_id() >> 4;
+  AlphaShared& S = shared[half];
+  const uint32_t v = __ldg(px + lane * 4 + comp);
+  const unsigned match = __match_any_sync(FULL_MASK, v | (uint32_t)half << 8) >> (16 * half) & 0xFFFFu;
+  const bool is_leader = __ffs(match) - 1 == lane;
+  const unsigned lmask = __ballot_sync(FULL_MASK, is_leader) >> (16 * half) & 0xFFFFu;
+  const int n = __popc(lmask), most = max(n, __shfl_xor_sync(FULL_MASK, n, 16));
   {
     // order of evaluation: by distance from the middle of the range, in half units
-    const int vmin = (int)__reduce_min_sync(FULL_MASK, lane < 16 ? v : 255u);
-    const int vmax = (int)__reduce_max_sync(FULL_MASK, lane < 16 ? v : 0u);
-    const int far = abs(2 * (int)v - vmin - vmax);
+    int vmin = (int)v, vmax = (int)v;
+#pragma unroll
+    for (int k = 8; k; k >>= 1) {
+      vmin = min(vmin, __shfl_xor_sync(FULL_MASK, vmin, k));
+      vmax = max(vmax, __shfl_xor_sync(FULL_MASK, vmax, k));
+    }
+    const int far = is_leader ? abs(2 * (int)v - vmin - vmax) : -1;
     int rank = 0;
-    for (unsigned m = lmask; m; m &= m - 1) {
-      const int j = __ffs(m) - 1, other = __shfl_sync(FULL_MASK, far, j);
-      rank += other > far || (other == far && j < (int)lane);
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int other = __shfl_sync(FULL_MASK, far, j, 16);
+      rank += other > far || (other == far && j < lane);
     }
-    __syncwarp();  // the previous block's reads are done
-    if (is_leader) {
-      const float fv = (float)v;
-      S.val[rank] = make_float4(fv, fv + 8388608.f, (float)__popc(match), fminf(fv, 255.f - fv));
-      S.uniq[__popc(lmask & ((1u << lane) - 1u))] = v;
-    }
-    if (lane == 0) S.val[n] = make_float4(0.f, 8388608.f, 0.f, 0.f);
+    __syncwarp();  // the previous blocks' reads are done
+    const float fv = (float)v;
+    S.val[rank] = make_float4(fv, fv + 8388608.f, is_leader ? (float)__popc(match) : 0.f, fminf(fv, 255.f - fv));
+    if (is_leader) S.uniq[__popc(lmask & ((1u << lane) - 1u))] = v;
     __syncwarp();
   }
-  int first = 0, second = 0, btype = 0;
-  float berr = 1e30f;
-  auto accept_chain = [&](int l, int h, float err, int type, bool dependent) -> int {
-    unsigned ok = __ballot_sync(FULL_MASK, err < berr);
-    int last = -1;
-    while (ok) {
-      const int j = __ffs(ok) - 1;
-      berr = __shfl_sync(FULL_MASK, err, j);
-      last = j;
-      if (dependent) break;
-      const unsigned after = j == 31 ? 0u : (FULL_MASK << (j + 1));
-      ok = __ballot_sync(FULL_MASK, err < berr) & after;
-    }
-    if (last >= 0) {
-      first = __shfl_sync(FULL_MASK, l, last);
-      second = __shfl_sync(FULL_MASK, h, last);
-      btype = __shfl_sync(FULL_MASK, type, last);
-    }
-    return last;
+  int first = (int)v, second = (int)v, btype = 0;
+  float berr = n == 1 ? 0.f : 1e30f;  // a block of one value is done
+  auto take_from = [&](bool any, int j, int l, int h, float err, int type) {
+    const int src = any ? j : lane;
+    const float e = __shfl_sync(FULL_MASK, err, src, 16);
+    const int nl = __shfl_sync(FULL_MASK, l, src, 16), nh = __shfl_sync(FULL_MASK, h, src, 16);
+    const int nt = __shfl_sync(FULL_MASK, type, src, 16);
+    if (any) { berr = e; first = nl; second = nh; btype = nt; }
   };
-  // all unique value pairs i < j (compute :83-96)
-  const int npairs = n * (n - 1) / 2;
-  const float half = (float)n - 0.5f;
+  // all unique value pairs i < j (compute :83-96): the first of the lowest error
+  const int npairs = n * (n - 1) / 2, most_pairs = most * (most - 1) / 2;
+  const float row = (float)n - 0.5f;
 #pragma unroll 1
-  for (int p0 = 0; p0 < npairs; p0 += 32) {
-    const int p = p0 + (int)lane;
+  for (int p0 = 0; p0 < most_pairs; p0 += 16) {
+    const int p = p0 + lane;
     int l = 0, h = 0, type;
     if (p < npairs) {
       // i (2 n - 1 - i) / 2 pairs are before row i; 1e-4 is far below the root's distance to the next row's
-      const int i = (int)(half - sqrtf(half * half - (float)(2 * p)) + 1e-4f);
+      const int i = (int)(row - sqrtf(row * row - (float)(2 * p)) + 1e-4f);
       l = (int)S.uniq[i];
       h = (int)S.uniq[p - i * (2 * n - 1 - i) / 2 + i + 1];
     }
-    const float err = alpha_errors(S, n, both, p < npairs, l, h, berr, type);
-    accept_chain(l, h, err, type, false);
+    const float err = alpha_errors(S, most, both, p < npairs, l, h, berr, type);
+    uint32_t key = err < berr ? (uint32_t)err << 4 | (uint32_t)lane : kInf;  // sums are below 2^24
+#pragma unroll
+    for (int k = 8; k; k >>= 1) key = min(key, __shfl_xor_sync(FULL_MASK, key, k));
+    take_from(key != kInf, (int)(key & 15u), l, h, err, type);
   }
   // +-R probe around the running best (:98-141); the centre moves with each improvement
   const int R = quality == kQUber ? 16 : 8, D = 2 * R + 1;
   const int over_d = R == 16 ? 1986 : 3856;  // p / D is p * over_d >> 16 for the p below
-  if (berr != 0.f && quality >= kQBetter) {
-    int pos = 0, row_l = first - R;
-    const int total = D * D;
+  const int total = berr != 0.f && quality >= kQBetter ? D * D : 0;
+  int pos = 0, row_l = first - R;
 #pragma unroll 1
-    while (pos < total) {
-      const int p = pos + (int)lane;
-      const int row0 = pos * over_d >> 16, r = p * over_d >> 16;
-      int type;
-      const int l = r == row0 ? row_l : first + (r - R);
-      const int h = second + (p - r * D - R);
-      const bool valid = p < total && (unsigned)l <= 255u && (unsigned)h <= 255u;
-      const float err = alpha_errors(S, n, both, valid, l, h, berr, type);
-      const int last = accept_chain(l, h, err, type, true);
-      const int next = last >= 0 ? pos + last + 1 : pos + 32;
-      const int nrow = next * over_d >> 16;
-      // the reference fixes l when a row starts: a row begun inside this batch used the
-      // centre from before the batch, unless it is the accepted candidate's own row
-      const int last_row = last >= 0 ? (pos + last) * over_d >> 16 : -1;
-      if (last >= 0 && nrow == last_row) row_l = __shfl_sync(FULL_MASK, l, last);
-      else if (nrow != row0) row_l = first + (nrow - R);
-      pos = next;
-    }
+  while (__any_sync(FULL_MASK, pos < total)) {
+    const int p = pos + lane;
+    const int row0 = pos * over_d >> 16, r = p * over_d >> 16;
+    int type;
+    const int l = r == row0 ? row_l : first + (r - R);
+    const int h = second + (p - r * D - R);
+    const bool valid = p < total && (unsigned)l <= 255u && (unsigned)h <= 255u;
+    const float err = alpha_errors(S, most, both, valid, l, h, berr, type);
+    const unsigned ok = __ballot_sync(FULL_MASK, err < berr) >> (16 * half) & 0xFFFFu;
+    const int last = ok ? __ffs(ok) - 1 : -1;
+    take_from(ok != 0, last, l, h, err, type);
+    const int at_l = __shfl_sync(FULL_MASK, l, max(last, 0), 16);
+    const int next = last >= 0 ? pos + last + 1 : pos + 16;
+    const int nrow = next * over_d >> 16;
+    // the reference fixes l when a row starts: a row begun inside this batch used the
+    // centre from before the batch, unless it is the accepted candidate's own row
+    const int last_row = last >= 0 ? (pos + last) * over_d >> 16 : -1;
+    if (last >= 0 && nrow == last_row) row_l = at_l;
+    else if (nrow != row0) row_l = first + (nrow - R);
+    if (pos < total) pos = next;
   }
   // selectors of the winner, reorder rules (:143-185), pack (dxt5_block, crn_dxt.h:318-361)
   int sel = 0;
-  if (lane < 16) {
+  {
     const int l = first, h = second;
     int pv[8];
     pv[0] = l; pv[1] = h;
@@ -2020,24 +2015,31 @@ __device__ __forceinline__ void alpha_block(AlphaShared& S, const uint8_t* __res
     const uint32_t t = f; f = s; s = t;
     sel = 0x23456701 >> (4 * sel) & 7;  // 1, 0, 7, 6, 5, 4, 3, 2
   }
-  const uint32_t lo_bits = __reduce_or_sync(FULL_MASK, lane < 10 ? ((uint32_t)sel << (3 * lane)) : 0u);
-  const uint32_t hi_bits = __reduce_or_sync(FULL_MASK, (lane >= 10 && lane < 16) ? ((uint32_t)sel << (3 * (lane - 10))) : 0u);
-  if (lane == 0) {
+  uint32_t lo_bits = lane < 10 ? (uint32_t)sel << (3 * lane) : 0u, hi_bits = lane < 10 ? 0u : (uint32_t)sel << (3 * (lane - 10));
+#pragma unroll
+  for (int k = 8; k; k >>= 1) {
+    lo_bits |= __shfl_xor_sync(FULL_MASK, lo_bits, k);
+    hi_bits |= __shfl_xor_sync(FULL_MASK, hi_bits, k);
+  }
+  if (lane == 0 && write) {
     const uint64_t bits = (uint64_t)lo_bits | ((uint64_t)hi_bits << 30);
     const uint64_t word = (uint64_t)f | ((uint64_t)s << 8) | (bits << 16);
     *reinterpret_cast<uint2*>(o) = make_uint2((uint32_t)word, (uint32_t)(word >> 32));
   }
 }
 
+// A CTA per eight blocks, as many as there are: the hardware's placing of CTAs evens out blocks that
+// differ in cost by a factor of thirty (resident warps that stride over the blocks: 130 us where this
+// takes 115).
 __global__ void __launch_bounds__(128)
     k_dxt5a_encode(const uint8_t* __restrict__ blocks, uint32_t n, int comp, int both, uint32_t quality,
                    uint8_t* __restrict__ out, uint32_t out_stride) {
-  const uint32_t warp_global = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const uint32_t nwarps = gridDim.x * 4;
-  __shared__ AlphaShared shared[4];
-  for (uint32_t bi = warp_global; bi < n; bi += nwarps)
-    alpha_block(shared[threadIdx.x >> 5], blocks + (size_t)bi * 64, comp, both != 0, quality,
-                out + (size_t)bi * out_stride);
+  __shared__ AlphaShared shared[8];
+  const uint32_t pair = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (pair > (n - 1) / 2) return;
+  const uint32_t bi = pair * 2 + (lane_id() >> 4), at = min(bi, n - 1);  // an odd count's last half: the same again
+  alpha_blocks(shared + (threadIdx.x >> 5) * 2, blocks + (size_t)at * 64, comp, both != 0, quality,
+               out + (size_t)at * out_stride, bi < n);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2128,17 +2130,17 @@ __global__ void __launch_bounds__(128)
                           const EncodeSegment* __restrict__ segs) {
   const uint32_t warp_global = blockIdx.x * 4 + (threadIdx.x >> 5);
   const uint32_t nwarps = gridDim.x * 4;
-  __shared__ AlphaShared shared[4];
+  __shared__ AlphaShared shared[8];
   for (uint32_t c = warp_global; c < nchunks; c += nwarps) {
     const EncodeChunk ch = chunks[c];
     const EncodeSegment sg = segs[ch.segment];
     const int comp = (int)((sg.options >> kSegCompShift) & 3u);
     const bool both = (sg.options & kSegBothTypes) != 0;
     const uint32_t quality = (sg.options >> kSegAlphaQualityShift) & 7u;
-    for (uint32_t k = 0; k < ch.count; k++) {
-      const uint32_t b = ch.first + k;
-      alpha_block(shared[threadIdx.x >> 5], blocks + (size_t)b * 64, comp, both, quality,
-                  sg.out + (size_t)(b - sg.first_block) * sg.stride);
+    for (uint32_t k0 = 0; k0 < ch.count; k0 += 2) {
+      const uint32_t k = k0 + (lane_id() >> 4), b = ch.first + min(k, ch.count - 1);
+      alpha_blocks(shared + (threadIdx.x >> 5) * 2, blocks + (size_t)b * 64, comp, both, quality,
+                   sg.out + (size_t)(b - sg.first_block) * sg.stride, k < ch.count);
     }
   }
 }
@@ -2203,20 +2205,6 @@ int ensure_tables() {
 
 // ryg single-colour tables on the host: m5[256][2], m6[256][2] (then the 3-colour variants)
 const void* single_colour_tables_host() { return single_colour_host_tables(); }
-
-namespace {
-
-int grid_for(const void* kernel, int threads, uint32_t work_units) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
-  if (per_sm < 1) per_sm = 1;
-  const uint32_t full = (uint32_t)sms * (uint32_t)per_sm;
-  return (int)(work_units < full ? (work_units ? work_units : 1) : full);
-}
-
-}  // namespace
 
 // Device-pointer launches (no synchronization).
 // Opt-in work counter (profiling hook): candidate x unique-colour evaluations of the DXT1 search.
@@ -2432,8 +2420,7 @@ int launch_dxt5a(const uint8_t* d_blocks, uint32_t n, int comp, bool both, uint3
                  uint32_t out_stride, cudaStream_t s) {
   if (!n) return CRNGPU_OK;
   if (quality > kQUber) { set_error("bad DXT quality"); return CRNGPU_E_PARAM; }
-  const int grid = grid_for((const void*)k_dxt5a_encode, 128, (n + 3) / 4);
-  k_dxt5a_encode<<<grid, 128, 0, s>>>(d_blocks, n, comp, both ? 1 : 0, quality, d_out, out_stride);
+  k_dxt5a_encode<<<n / 8 + (n % 8 != 0), 128, 0, s>>>(d_blocks, n, comp, both ? 1 : 0, quality, d_out, out_stride);
   return cuda_check(cudaGetLastError(), "launch k_dxt5a_encode");
 }
 

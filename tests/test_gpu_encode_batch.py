@@ -94,3 +94,17 @@ def test_block_counts_around_two_per_warp_match_short_calls(cg, blocks_past_two_
     half = n // 2
     want = [cg.dxt1_optimize(b.contiguous(), quality=quality).cpu().numpy() for b in (blocks[:half - 3], blocks[half - 3:n - 9], blocks[n - 9:])]
     assert np.array_equal(got, np.concatenate(want))
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 33])
+def test_alpha_block_counts_match_single_blocks(cg, n):
+    # half a warp a block, eight blocks a CTA: odd counts, short last CTAs, one-value blocks beside full ones
+    rng = np.random.default_rng(n)
+    img = rng.integers(0, 256, (4, 4 * n, 4), dtype=np.uint8)
+    img[..., 3] = np.where(rng.integers(0, 3, (4, 4 * n)) > 0, img[..., 3] // 64 * 60, img[..., 3])
+    img[:, 4 * (n // 2):4 * (n // 2) + 4, 3] = 77
+    flags = cg.FLAG_USE_BOTH_BLOCK_TYPES
+    got = np.asarray(cg.compress_image(img, cg.FMT_DXT5A, flags)).reshape(n, 8)
+    for b in range(n):
+        want = np.asarray(cg.compress_image(np.ascontiguousarray(img[:, 4 * b:4 * b + 4]), cg.FMT_DXT5A, flags))
+        assert np.array_equal(got[b], want.reshape(8)), b
