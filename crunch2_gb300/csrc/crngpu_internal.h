@@ -114,7 +114,8 @@ int dxt5a_chunks_max_grid();
 // dxt1_options() word; d_err (optional) receives each block's error. launch_dxt1_black_trial: the
 // transparent-black trial over blocks already encoded with the same options (d_err_io their
 // errors): a block whose trial is better is rewritten in place, with its new error.
-// launch_dxt5a: quality sets the probe grid (+-16 Uber, +-8 Better, none below).
+// launch_dxt5a: quality sets the probe grid (+-16 Uber, +-8 Better, none below); second >= 0: that
+// channel too, 8 bytes further on in each output block.
 int launch_dxt1(const uint8_t* d_blocks, uint32_t n, uint32_t opts, uint8_t* d_out, uint32_t out_stride,
                 uint64_t* d_err, cudaStream_t s);
 // One image of a host mip chain uploaded as a whole, gathered into 4x4 blocks of cooked texels
@@ -143,7 +144,7 @@ int launch_dxt1_count(const uint8_t* d_blocks, uint32_t n_max, const uint32_t* n
 int launch_dxt1_black_trial(const uint8_t* d_blocks, uint32_t n, uint32_t opts, uint8_t* d_out, uint32_t out_stride,
                             uint64_t* d_err_io, cudaStream_t s);
 int launch_dxt5a(const uint8_t* d_blocks, uint32_t n, int comp, bool both, uint32_t quality, uint8_t* d_out,
-                 uint32_t out_stride, cudaStream_t s);
+                 uint32_t out_stride, cudaStream_t s, int second = -1);
 // the batched colour encode: phase 1 writes one seed record of kDxt1SeedBytes per block to
 // d_seeds (room for every gathered block of the batch), phase 2 reads them; d_next: the number of the
 // next block that phase 2's warps take, set by phase 1

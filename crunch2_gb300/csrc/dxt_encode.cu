@@ -2032,8 +2032,9 @@ __device__ __forceinline__ void alpha_blocks(AlphaShared* shared, const uint8_t*
 // differ in cost by a factor of thirty (resident warps that stride over the blocks: 130 us where this
 // takes 115).
 __global__ void __launch_bounds__(128)
-    k_dxt5a_encode(const uint8_t* __restrict__ blocks, uint32_t n, int comp, int both, uint32_t quality,
+    k_dxt5a_encode(const uint8_t* __restrict__ blocks, uint32_t n, int comp, int second, int both, uint32_t quality,
                    uint8_t* __restrict__ out, uint32_t out_stride) {
+  if (blockIdx.y) { comp = second; out += 8; }
   __shared__ AlphaShared shared[8];
   const uint32_t pair = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (pair > (n - 1) / 2) return;
@@ -2417,10 +2418,11 @@ int stage_wait_counters(uint32_t out[2], bool reset) {
 }
 
 int launch_dxt5a(const uint8_t* d_blocks, uint32_t n, int comp, bool both, uint32_t quality, uint8_t* d_out,
-                 uint32_t out_stride, cudaStream_t s) {
+                 uint32_t out_stride, cudaStream_t s, int second) {
   if (!n) return CRNGPU_OK;
   if (quality > kQUber) { set_error("bad DXT quality"); return CRNGPU_E_PARAM; }
-  k_dxt5a_encode<<<n / 8 + (n % 8 != 0), 128, 0, s>>>(d_blocks, n, comp, both ? 1 : 0, quality, d_out, out_stride);
+  const dim3 grid(n / 8 + (n % 8 != 0), second < 0 ? 1 : 2);
+  k_dxt5a_encode<<<grid, 128, 0, s>>>(d_blocks, n, comp, second, both ? 1 : 0, quality, d_out, out_stride);
   return cuda_check(cudaGetLastError(), "launch k_dxt5a_encode");
 }
 

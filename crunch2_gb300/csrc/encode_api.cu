@@ -29,17 +29,23 @@ bool read_options(const crngpu_block_options* o, uint32_t* quality, uint32_t* th
 }
 
 // Image -> 4x4 blocks with edge clamping (init_task :334-344): texel (x, y) of block (bx, by)
-// is img[min(4by+y, h-1)][min(4bx+x, w-1)]. One thread per output texel.
+// is img[min(4by+y, h-1)][min(4bx+x, w-1)]. A thread per row of a block, its 16 bytes in one load where
+// the image's rows allow it (`wide`: 16-byte aligned); a thread per texel took 17 us for 2048 x 2048.
 __global__ void k_gather_blocks(const uint8_t* __restrict__ img, uint32_t w, uint32_t h, uint32_t pitch,
-                                uint32_t blocks_x, uint64_t total_texels, uint32_t* __restrict__ out) {
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total_texels;
-       t += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t blk = t >> 4;
-    const uint32_t tin = (uint32_t)t & 15;
-    const uint32_t by = (uint32_t)(blk / blocks_x), bx = (uint32_t)(blk - (uint64_t)by * blocks_x);
-    const uint32_t x = min(bx * 4 + (tin & 3), w - 1), y = min(by * 4 + (tin >> 2), h - 1);
-    const uint8_t* p = img + (uint64_t)y * pitch + (uint64_t)x * 4;
-    out[t] = (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
+                                uint32_t blocks_x, uint64_t rows, int wide, uint4* __restrict__ out) {
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t blk = (uint32_t)(t >> 2), by = blk / blocks_x, bx = blk - by * blocks_x;
+    const uint8_t* p = img + (uint64_t)min(by * 4 + ((uint32_t)t & 3), h - 1) * pitch;
+    if (wide && bx * 4 + 4 <= w) {
+      out[t] = __ldg(reinterpret_cast<const uint4*>(p) + bx);
+    } else {
+      uint32_t v[4];
+      for (uint32_t k = 0; k < 4; k++) {
+        const uint8_t* q = p + (uint64_t)min(bx * 4 + k, w - 1) * 4;
+        v[k] = (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16) | ((uint32_t)q[3] << 24);
+      }
+      out[t] = make_uint4(v[0], v[1], v[2], v[3]);
+    }
   }
 }
 
@@ -105,9 +111,7 @@ int encode_device(const uint8_t* d_in, uint32_t n, uint32_t fmt, uint32_t flags,
     case CRNGPU_FMT_DXN_XY:
     case CRNGPU_FMT_DXN_YX: {
       const int c0 = fmt == CRNGPU_FMT_DXN_XY ? 0 : 1;
-      int rc = launch_dxt5a(d_in, n, c0, both, quality, d_out, 16, s);
-      if (rc == CRNGPU_OK) rc = launch_dxt5a(d_in, n, 1 - c0, both, quality, d_out + 8, 16, s);
-      return rc;
+      return launch_dxt5a(d_in, n, c0, both, quality, d_out, 16, s, 1 - c0);
     }
     default: {  // DXT5 family: alpha element, then a colour element that may not use 3-colour blocks
       int rc = launch_dxt5a(d_in, n, 3, both, quality, d_out, 16, s);
@@ -331,9 +335,10 @@ extern "C" int64_t crngpu_compress_image_ex(const uint8_t* rgba, uint32_t width,
       return cuda_check(e, "copy image");
     d_img = static_cast<const uint8_t*>(bi.ptr);
   }
-  const uint64_t texels = n * 16;
-  const uint32_t grid = (uint32_t)((texels + 255) / 256 < 65535 * 8 ? (texels + 255) / 256 : 65535 * 8);
-  k_gather_blocks<<<grid, 256, 0, s>>>(d_img, width, height, pitch_bytes, bx, texels, static_cast<uint32_t*>(blocks.ptr));
+  const uint64_t rows = n * 4;
+  const uint32_t grid = (uint32_t)((rows + 255) / 256 < 65535 * 8 ? (rows + 255) / 256 : 65535 * 8);
+  const int wide = ((uintptr_t)d_img & 15) == 0 && pitch_bytes % 16 == 0;
+  k_gather_blocks<<<grid, 256, 0, s>>>(d_img, width, height, pitch_bytes, bx, rows, wide, static_cast<uint4*>(blocks.ptr));
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_gather_blocks");
   uint8_t* d_out = out;
   DevBuf* so = nullptr;

@@ -108,3 +108,20 @@ def test_alpha_block_counts_match_single_blocks(cg, n):
     for b in range(n):
         want = np.asarray(cg.compress_image(np.ascontiguousarray(img[:, 4 * b:4 * b + 4]), cg.FMT_DXT5A, flags))
         assert np.array_equal(got[b], want.reshape(8)), b
+
+
+@pytest.mark.parametrize("w,h,skip", [(64, 20, 0), (61, 19, 0), (64, 20, 1), (3, 70, 0), (64, 20, 4)])
+def test_images_with_and_without_aligned_rows_match(cg, w, h, skip):
+    # rows of 16-byte pieces are read whole, all others by texel: both, with ragged right and lower edges
+    rng = np.random.default_rng(w)
+    img = rng.integers(0, 256, (h, w, 4), dtype=np.uint8)
+    wide = torch.zeros((h, w + skip, 4), dtype=torch.uint8, device="cuda")
+    wide[:, skip:] = torch.from_numpy(img).cuda()
+    got = cg.compress_image(wide[:, skip:].contiguous(), cg.FMT_DXN_XY, 0)
+    flat = torch.zeros(h * w * 4 + 16, dtype=torch.uint8, device="cuda")
+    shifted = flat[4 * skip:4 * skip + h * w * 4].view(h, w, 4)
+    shifted.copy_(torch.from_numpy(img))
+    again = cg.compress_image(shifted, cg.FMT_DXN_XY, 0)
+    want = np.asarray(cg.compress_image(img, cg.FMT_DXN_XY, 0))
+    to = lambda t: t.cpu().numpy() if hasattr(t, "cpu") else np.asarray(t)
+    assert np.array_equal(to(got).reshape(-1), want.reshape(-1)) and np.array_equal(to(again).reshape(-1), want.reshape(-1))
