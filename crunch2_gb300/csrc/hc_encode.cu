@@ -654,7 +654,7 @@ __host__ __device__ void palettize(const uint32_t* px, int n, bool perc, float* 
 // tiles (k_hc_tile_errors, and k_hc_alpha_errors for the alpha channels' pair search), the chunk's
 // layout from them (k_hc_tile_layout), and the chosen tiles' vectors (k_hc_tile_vectors). A thread
 // has one tile (errors: all of a warp's tiles the same size), not one chunk: with a thread per chunk
-// a 333 x 180 DXT5 chain was 21 CTAs of two warps, 4.8 ms; now TBD. The tile errors are
+// a 333 x 180 DXT5 chain was 21 CTAs of two warps, 4.8 ms; now 0.45. The tile errors are
 // [channel][tile][chunk].
 __global__ void __launch_bounds__(64) k_hc_tile_errors(const uint32_t* __restrict__ blocks, const Chunk* __restrict__ chunks,
                                                        uint32_t nchunks, const SolidTables* __restrict__ st, TileCfg cfg,
@@ -844,7 +844,7 @@ __global__ void k_fast_selector_words(const uint32_t* __restrict__ blocks, uint3
 // nodes get up to 16 CTAs on as many SMs, whose partial sums meet through distributed shared
 // memory.
 
-constexpr int kVqThreads = 512;
+constexpr int kVqThreads = 512, kVqWarps = kVqThreads / 32;
 constexpr uint32_t kDefaultRoundFraction = 4;  // a VQ round splits at most leaves / 4 nodes
 constexpr uint32_t kVqPerCta = 2048;            // vectors per CTA below which a node gets fewer CTAs
 
@@ -883,7 +883,7 @@ __device__ __forceinline__ void block_sum(float* vals, float* red /* smem [N * 1
 
 // block-wide argmax of (value, position): largest value, then smallest position
 __device__ __forceinline__ void block_argmax(float& v, uint32_t& pos, float* rv, uint32_t* rp) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
     const uint32_t op = __shfl_xor_sync(0xFFFFFFFFu, pos, o);
@@ -893,7 +893,8 @@ __device__ __forceinline__ void block_argmax(float& v, uint32_t& pos, float* rv,
   if (lane == 0) { rv[warp] = v; rp[warp] = pos; }
   __syncthreads();
   v = rv[0]; pos = rp[0];
-  for (int w = 1; w < nw; w++)
+#pragma unroll
+  for (int w = 1; w < kVqWarps; w++)
     if (rv[w] > v || (rv[w] == v && rp[w] < pos)) { v = rv[w]; pos = rp[w]; }
 }
 
@@ -954,26 +955,33 @@ struct VqShared {
 // cluster-wide sum of N floats per thread; every CTA adds the partials in rank order, so all of
 // them hold bit-identical totals and take the same branches. Warps reduce by shuffles; the CTA's
 // total of a value is added by one thread per CTA of the cluster, which writes it there (a remote
-// write is not waited for; the barrier that it ends with makes it seen). With N threads adding,
-// partials read from the other CTAs after the barrier, and five shuffles a value, a split round of a
-// 1024 x 1024 DXT1 chain's selector tree took 128 us; now TBD.
+// write is not waited for; the barrier that it ends with makes it seen). Nodes are small enough for
+// this to be most of a pass, so nothing in it waits in turn: the partials of a sum are all on their
+// way before the first is added. (As loops over warps and ranks, with the centroids' divisions one
+// after the other behind it, the splits of a 1024 x 1024 chain's selector tree took 3.8 ms, now 3.0.)
 template <int N>
 __device__ __forceinline__ void cluster_sum(float* vals, VqShared& sh, int& phase, cg::cluster_group& cl) {
   static_assert(N <= kVqSlot, "cluster_sum slot");
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5;
   warp_totals<N>(vals, [&](int k, float t) { sh.red[k * 17 + warp] = t; });
   __syncthreads();
   const unsigned C = cl.num_blocks(), r = cl.block_rank();
-  for (unsigned i = threadIdx.x; i < N * C; i += blockDim.x) {
+  for (unsigned i = threadIdx.x; i < N * C; i += kVqThreads) {
     const unsigned q = i / N, k = i % N;
-    float t = 0.f;
-    for (int wi = 0; wi < nw; wi++) t += sh.red[k * 17 + wi];
+    float p[kVqWarps], t = 0.f;
+#pragma unroll
+    for (int wi = 0; wi < kVqWarps; wi++) p[wi] = sh.red[k * 17 + wi];
+#pragma unroll
+    for (int wi = 0; wi < kVqWarps; wi++) t += p[wi];
     *cl.map_shared_rank(&sh.part[phase][r][k], q) = t;
   }
   cl.sync();
   if (threadIdx.x < N) {
-    float t = 0.f;
-    for (unsigned q = 0; q < C; q++) t += sh.part[phase][q][threadIdx.x];
+    float p[16], t = 0.f;
+#pragma unroll
+    for (unsigned q = 0; q < 16; q++) p[q] = sh.part[phase][q][threadIdx.x];  // those past C are not used
+#pragma unroll
+    for (unsigned q = 0; q < 16; q++) t = q < C ? t + p[q] : t;
     sh.tot[threadIdx.x] = t;
   }
   __syncthreads();
@@ -990,11 +998,13 @@ __device__ __forceinline__ void cluster_argmax(float& v, uint32_t& pos, VqShared
     *cl.map_shared_rank(&sh.pos[phase][r], threadIdx.x) = pos;
   }
   cl.sync();
-  for (unsigned q = 0; q < C; q++) {
-    const float qv = sh.part[phase][q][0];
-    const uint32_t qp = sh.pos[phase][q];
-    if (qv > v || (qv == v && qp < pos)) { v = qv; pos = qp; }
-  }
+  float qv[16];
+  uint32_t qp[16];
+#pragma unroll
+  for (unsigned q = 0; q < 16; q++) { qv[q] = sh.part[phase][q][0]; qp[q] = sh.pos[phase][q]; }
+#pragma unroll
+  for (unsigned q = 0; q < 16; q++)
+    if (q < C && (qv[q] > v || (qv[q] == v && qp[q] < pos))) { v = qv[q]; pos = qp[q]; }
   phase ^= 1;
 }
 
@@ -1024,6 +1034,18 @@ __device__ __forceinline__ float dist2(const float* a, const float* b) {
 #pragma unroll
   for (int k = 0; k < D; k++) { const float d = a[k] - b[k]; s += d * d; }
   return s;
+}
+
+template <int D>
+__device__ __forceinline__ void store_vec(float* __restrict__ p, const float* v) {
+  if constexpr (D % 4 == 0) {
+#pragma unroll
+    for (int k = 0; k < D; k += 4) *reinterpret_cast<float4*>(p + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+  } else {
+    static_assert(D % 2 == 0, "vectors of an even number of floats");
+#pragma unroll
+    for (int k = 0; k < D; k += 2) *reinterpret_cast<float2*>(p + k) = make_float2(v[k], v[k + 1]);
+  }
 }
 
 // Splits each job's parent node into two children (tree_clusterizer::split_node,
@@ -1150,10 +1172,11 @@ __device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float
   }
   // 2-means; the partition is the last assignment (made with the centroids before their update).
   // The updated centroids live in shared memory; the assignment centroids in registers.
-  __shared__ float s_L[D], s_R[D];
+  __shared__ float s_lr[2 * D];  // L, then R
+  const float *s_L = s_lr, *s_R = s_lr + D;
 #pragma unroll
   for (int k = 0; k < D; k++)
-    if (threadIdx.x == k) { s_L[k] = L[k]; s_R[k] = R[k]; }
+    if (threadIdx.x == k) { s_lr[k] = L[k]; s_lr[D + k] = R[k]; }
   float prev = 1e10f, lvar = 0.f, rvar = 0.f, lw = 0.f, rw = 0.f;
   float AL[D], AR[D];  // centroids of the last assignment
   for (int loop = 0; loop < 1024; loop++) {
@@ -1186,9 +1209,7 @@ __device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float
     lvar = acc[2 * D + 2] - ll / lw;
     rvar = acc[2 * D + 3] - rr / rw;
     // every thread read s_L / s_R before cluster_sum's barriers
-#pragma unroll
-    for (int k = 0; k < D; k++)
-      if (threadIdx.x == k) { s_L[k] = acc[k] / lw; s_R[k] = acc[D + k] / rw; }
+    if (threadIdx.x < 2 * D) s_lr[threadIdx.x] = sh.tot[threadIdx.x] / (threadIdx.x < D ? lw : rw);
     const float tv = lvar + rvar;
     if (tv < .00001f) break;
     if ((prev - tv) / tv < .00001f) break;
@@ -1228,7 +1249,7 @@ __device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float
     if (q < r) { left_before += ql; right_before += qn - ql; }
   }
   uint32_t lrun = b0 + left_before, rrun = b0 + left_total + right_before;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int sb = 0;
   for (uint32_t base = s0; base < s1; base += blockDim.x) {
     const uint32_t i = base + threadIdx.x;
@@ -1243,7 +1264,8 @@ __device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float
     if (lane == 0) { sh.scan[sb][warp] = __popc(bl); sh.scan[sb][warp] |= (uint32_t)__popc(br) << 16; }
     __syncthreads();
     uint32_t lpre = 0, rpre = 0, ltot = 0, rtot = 0;
-    for (int wi = 0; wi < nw; wi++) {
+#pragma unroll
+    for (int wi = 0; wi < kVqWarps; wi++) {
       const uint32_t t = sh.scan[sb][wi];
       if (wi < warp) { lpre += t & 0xFFFFu; rpre += t >> 16; }
       ltot += t & 0xFFFFu;
@@ -1251,8 +1273,7 @@ __device__ __forceinline__ void vq_split_cluster(float* __restrict__ vec0, float
     }
     if (live) {
       const uint32_t dst = left ? lrun + lpre + __popc(bl & ((1u << lane) - 1u)) : rrun + rpre + __popc(br & ((1u << lane) - 1u));
-#pragma unroll
-      for (int k = 0; k < D; k++) dvec[(size_t)dst * D + k] = vv[k];
+      store_vec<D>(dvec + (size_t)dst * D, vv);
       dw[dst] = w[i];
     }
     lrun += ltot;
@@ -1471,8 +1492,7 @@ __device__ __forceinline__ void vq_split_warp(float* __restrict__ vec0, float* _
     if (live) {
       const uint32_t below = (1u << lane) - 1u;
       const uint32_t dst = left ? lrun + __popc(bl & below) : rrun + __popc(br & below);
-#pragma unroll
-      for (int k = 0; k < D; k++) dvec[(size_t)dst * D + k] = vv[k];
+      store_vec<D>(dvec + (size_t)dst * D, vv);
       dw[dst] = w[i];
     }
     lrun += __popc(bl);
