@@ -1372,12 +1372,17 @@ __device__ __forceinline__ void vq_split_warp(float* __restrict__ vec0, float* _
       float acc[D];
 #pragma unroll
       for (int k = 0; k < D; k++) acc[k] = 0.f;
+      float ahead[D], wa = 0.f;  // the lane's next vector
+      if (b0 + lane < b1) { load_vec<D>(vec + (size_t)(b0 + lane) * D, ahead); wa = w[b0 + lane]; }
       for (uint32_t i = b0 + lane; i < b1; i += 32) {
         float d[D], dot = 0.f;
-        load_vec<D>(vec + (size_t)i * D, d);
+        const float wi = wa;
+#pragma unroll
+        for (int k = 0; k < D; k++) d[k] = ahead[k];
+        if (i + 32 < b1) { load_vec<D>(vec + (size_t)(i + 32) * D, ahead); wa = w[i + 32]; }
 #pragma unroll
         for (int k = 0; k < D; k++) { d[k] -= c[k]; dot += d[k] * axis[k]; }
-        const float ww = w[i] * dot;
+        const float ww = wi * dot;
 #pragma unroll
         for (int k = 0; k < D; k++) acc[k] += d[k] * ww;
       }
@@ -1453,8 +1458,11 @@ __device__ __forceinline__ void vq_split_warp(float* __restrict__ vec0, float* _
     for (int k = 0; k < D; k++) { ll += acc[k] * acc[k]; rr += acc[D + k] * acc[D + k]; }
     lvar = acc[2 * D + 2] - ll / lw;
     rvar = acc[2 * D + 3] - rr / rw;
+    __syncwarp();  // the totals have been read
+    if (lane < 2 * D) tot[lane] = tot[lane] / (lane < D ? lw : rw);  // a division a lane
+    __syncwarp();
 #pragma unroll
-    for (int k = 0; k < D; k++) { L[k] = acc[k] / lw; R[k] = acc[D + k] / rw; }
+    for (int k = 0; k < D; k++) { L[k] = tot[k]; R[k] = tot[D + k]; }
     const float tv = lvar + rvar;
     if (tv < .00001f) break;
     if ((prev - tv) / tv < .00001f) break;
