@@ -207,10 +207,10 @@ DECODE_SPLIT_DEFAULT, DECODE_LANE_ONLY, DECODE_WIDE_ONLY = 0, 0xFFFFFFFF, 1
 
 
 def set_decode_split(min_blocks: int) -> None:
-    """Which levels run on the wide (CTA-per-level) decoder and which on the lane decoder
-    (crngpu_set_decode_split): DECODE_SPLIT_DEFAULT lets each plan pick the split with the shortest
-    decode; a block count sends levels at least that large to the wide decoder; DECODE_LANE_ONLY /
-    DECODE_WIDE_ONLY force one decoder for every level. Both give the same bytes."""
+    """Which levels run on which decoder (crngpu_set_decode_split): DECODE_SPLIT_DEFAULT lets each plan
+    pick the split over the walk, wide (CTA-per-level) and lane decoders with the shortest decode; a
+    block count sends levels at least that large to the wide decoder; DECODE_LANE_ONLY /
+    DECODE_WIDE_ONLY force one decoder for every level. All give the same bytes."""
     _check(lib().crngpu_set_decode_split(int(min_blocks) & 0xFFFFFFFF), "crngpu_set_decode_split")
 
 

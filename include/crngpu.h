@@ -447,7 +447,8 @@ typedef struct crngpu_unpack_batch_s* crngpu_unpack_batch;
 /* NULL on failure (crngpu_last_error says which item). */
 CRNGPU_API crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_batch_item* items, uint32_t n);
 
-/* Enqueues the batch on `stream` without synchronising: a two-word memset and two kernels.
+/* Enqueues the batch on `stream` without synchronising: memsets, the decoders' launches and the
+ * expansion.
  * flags: CRNGPU_BATCH_GRAPH captures them into a CUDA graph on the first call and replays that
  * graph on later calls (one launch from the host per batch); CRNGPU_BATCH_EXPAND_ONLY re-runs
  * only the expansion kernel from the index records of the last decode (the destinations are
@@ -484,12 +485,14 @@ CRNGPU_API int64_t crngpu_unpack_batch_bytes(crngpu_unpack_batch batch);
  * serial decoder). The wide decoder gives one CTA to a level: per-bit-position step tables built
  * in parallel, a serial walk of chunk and block starts at one shared-memory load per step, then
  * parallel symbol decode and a scan of the endpoint indices. It has the lowest latency per level
- * but does more work per block. The lane decoder runs one level stream per lane, many streams per
- * warp: least work per block, the latency of a serial decode. Both give the same bytes.
- * min_blocks = 0 (the default): each plan sends its largest levels to the wide decoder as long as
- * that shortens the plan's decode (a cost model of both decoders and the device's resident wide
- * CTAs); a single texture's large levels go wide, a batch of many textures mostly stays on the
- * lane decoder. Otherwise levels of at least min_blocks blocks (all faces) go wide: 1 sends every
+ * but does more work per block. The walk decoder spreads the same roles over the device: CTAs that
+ * build tables and decode symbols for segments of a stream beside one walk per level; the shortest
+ * time for the largest levels, several launches. The lane decoder runs one level stream per lane, many
+ * streams per warp: least work per block, the latency of a serial decode. All give the same bytes.
+ * min_blocks = 0 (the default): each plan sends its largest levels to the walk decoder and the next to
+ * the wide one as long as that shortens the plan's decode (a cost model of the three decoders and the
+ * device's resident wide CTAs); a single texture's large levels are walked, a batch of many textures
+ * mostly stays on the lane decoder. Otherwise levels of at least min_blocks blocks (all faces) go wide: 1 sends every
  * level with rows of at most 1024 blocks, 0xFFFFFFFF none. Applies to plans built after the call:
  * contexts' unpack calls and batches created afterwards. */
 CRNGPU_API int crngpu_set_decode_split(uint32_t min_blocks);
