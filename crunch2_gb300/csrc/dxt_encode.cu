@@ -42,7 +42,7 @@ constexpr int kBlocksPerWarp = 8;
 constexpr int kWarpsPerCta = 4;
 // CTAs per SM the encoders are compiled for (registers: 65536 / (128 x 8) = 64 per thread; the
 // phase-1 PCA spills a little, the candidate loops do not). 8 beat 4, 5 and 6 on GB300.
-constexpr int kCtasPerSm = 8;
+constexpr int kCtasPerSm = 8, kFewCtasPerSm = 4;
 constexpr uint32_t kInf = 0xFFFFFFFFu;
 
 // ryg single-colour tables (crnlib/crn_ryg_dxt.cpp:58-99): [value][0]=max, [1]=min endpoint
@@ -1803,8 +1803,12 @@ __device__ __forceinline__ void load_seed(WarpShared& S, const Seed* __restrict_
 // and 528.
 // G = false: Uber quality, perceptual or uniform, no grayscale sampling, transparency or black trial
 // (the default encode, compiled without the general paths); G = true: every option.
-template <bool G>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
+// kCtas: CTAs of an SM that its registers allow. With at most one block for each warp of half of them
+// (a small image, a small level) nothing is gained by more warps, and with twice the registers a block
+// spills nothing on its way: 256 blocks 170 us with 8, 149 with 4; 2400 blocks 230 and 204; 4000 blocks,
+// of which some then wait for others, 262 and 290.
+template <bool G, int kCtas>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, kCtas)
     k_dxt1_encode(const uint8_t* __restrict__ blocks, uint32_t n, uint32_t opts, const Seed* __restrict__ seeds,
                   uint8_t* __restrict__ out, uint32_t out_stride, uint64_t* __restrict__ err_out,
                   uint64_t* __restrict__ err_io, unsigned long long* __restrict__ work_out,
@@ -2266,8 +2270,9 @@ int dxt1_launch_setup(int dev, Dxt1Launch* L) {
   if (!done[dev]) {
     Dxt1Launch c;
     const int smem = (int)(sizeof(WarpShared) * kWarpsPerCta), seed_smem = (int)(sizeof(SeedShared) * kWarpsPerCta);
-    cudaError_t e = cudaFuncSetAttribute(k_dxt1_encode<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_dxt1_encode<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaSuccess;
+    for (auto search : {k_dxt1_encode<false, kCtasPerSm>, k_dxt1_encode<false, kFewCtasPerSm>, k_dxt1_encode<true, kCtasPerSm>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_dxt1_encode_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_dxt1_seeds<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, seed_smem);
@@ -2279,9 +2284,9 @@ int dxt1_launch_setup(int dev, Dxt1Launch* L) {
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.seeds_per_sm, k_dxt1_seeds<true>, kWarpsPerCta * 32, seed_smem);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.search_per_sm[0], k_dxt1_encode<false>, kWarpsPerCta * 32, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.search_per_sm[0], k_dxt1_encode<false, kCtasPerSm>, kWarpsPerCta * 32, smem);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.search_per_sm[1], k_dxt1_encode<true>, kWarpsPerCta * 32, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.search_per_sm[1], k_dxt1_encode<true, kCtasPerSm>, kWarpsPerCta * 32, smem);
     if (e != cudaSuccess) return cuda_check(e, "set up the DXT1 kernels");
     c.seeds_per_sm = c.seeds_per_sm < 1 ? 1 : c.seeds_per_sm;
     for (int k = 0; k < 2; k++) c.search_per_sm[k] = c.search_per_sm[k] < 1 ? 1 : c.search_per_sm[k];
@@ -2324,12 +2329,14 @@ int launch_dxt1_kernel(const uint8_t* d_blocks, uint32_t n, uint32_t opts, uint8
   const uint32_t grid = std::min<uint32_t>((n + kWarpsPerCta - 1) / kWarpsPerCta, full);
   if (general) {
     k_dxt1_seeds<true><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next);
-    k_dxt1_encode<true><<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err,
+    k_dxt1_encode<true, kCtasPerSm><<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err,
                                                              d_err_io, work, n_dev, next);
   } else {
     k_dxt1_seeds<false><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next);
-    k_dxt1_encode<false><<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err,
-                                                              d_err_io, work, n_dev, next);
+    const auto search = n <= (uint32_t)(L.sms * kFewCtasPerSm * kWarpsPerCta) ? k_dxt1_encode<false, kFewCtasPerSm>
+                                                                              : k_dxt1_encode<false, kCtasPerSm>;
+    search<<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err, d_err_io, work, n_dev,
+                                                 next);
   }
   e = cudaGetLastError();
   const cudaError_t fe = cudaFreeAsync(seeds, s);

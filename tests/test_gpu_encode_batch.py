@@ -125,3 +125,17 @@ def test_images_with_and_without_aligned_rows_match(cg, w, h, skip):
     want = np.asarray(cg.compress_image(img, cg.FMT_DXN_XY, 0))
     to = lambda t: t.cpu().numpy() if hasattr(t, "cpu") else np.asarray(t)
     assert np.array_equal(to(got).reshape(-1), want.reshape(-1)) and np.array_equal(to(again).reshape(-1), want.reshape(-1))
+
+
+@pytest.mark.parametrize("past", [-1, 0, 1])
+def test_block_counts_around_the_few_blocks_search_match(cg, past):
+    # up to 16 blocks an SM go to the search with twice the registers: both sides, and one with the other
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 16 + past
+    rng = np.random.default_rng(n)
+    px = rng.integers(0, 256, (n, 16, 4), dtype=np.uint8) // rng.integers(1, 40, (n, 1, 1), dtype=np.uint8)
+    px[..., 3] = 255
+    blocks = torch.from_numpy(px.reshape(n, 64)).cuda()
+    got, err = cg.dxt1_optimize(blocks, with_error=True)
+    twice, terr = cg.dxt1_optimize(torch.cat([blocks, blocks]), with_error=True)
+    for half in (0, 1):
+        assert torch.equal(twice[half * n:(half + 1) * n], got) and torch.equal(terr[half * n:(half + 1) * n], err)
