@@ -160,6 +160,9 @@ struct WarpShared {
 static_assert((sizeof(WarpShared) * kWarpsPerCta + 1024) * kCtasPerSm <= 228 * 1024,
               "DXT1 encoder shared memory per CTA");
 constexpr int kSeedCtasPerSm = 4;
+// blocks of an SM below which four lanes take one: seeds and search of 256 blocks 149 us with a lane
+// each, 140 with four; of 6000 346 and 341, of 8000 416 and 417
+constexpr uint32_t kSharedPerSm = 40;
 static_assert((sizeof(SeedShared) * kWarpsPerCta + 2048) * kSeedCtasPerSm <= 228 * 1024,
               "DXT1 phase-1 shared memory per CTA");
 
@@ -297,10 +300,18 @@ __device__ __forceinline__ float inverse_norm(float x, float y, float z) {
 
 // Runs handle_multicolor_block up to optimize_endpoints' entry, plus try_median4's seeds, for the
 // block whose 16 texels are pix (lane `slot` of the warp); the hand-off goes to *out.
-template <bool G>
+// kShare = 4: four lanes of a warp take the block, alike but for the double precision of the principal
+// axis, of which a lane has two of the six sums and one of the three products, so that a warp of eight
+// blocks has two thirds of the instructions a warp of 32 has.
+template <bool G, int kShare>
 __device__ void phase1_block(SeedShared& S, const float* __restrict__ unit, int slot, const uint32_t (&pix)[16],
                              uint32_t opts, Seed* __restrict__ out) {
-  const int L = slot;
+  const int L = slot, sub = kShare == 4 ? (int)lane_id() & 3 : 0;
+  // a value of the block's lane j (kShare = 4; the four go through everything together)
+  auto from_sharer = [](double x, int j) {
+    const unsigned four = 0xFu << (lane_id() & 28u);
+    return __hiloint2double(__shfl_sync(four, __double2hiint(x), j, 4), __shfl_sync(four, __double2loint(x), j, 4));
+  };
   const bool perceptual = (opts & kD1Perceptual) != 0;
   const uint32_t quality = G ? (opts >> kD1QualityShift) & 7u : kQUber;
   int n = 0;
@@ -413,15 +424,33 @@ __device__ void phase1_block(SeedShared& S, const float* __restrict__ unit, int 
       const float b = __fsub_rn(__fmul_rn(pw[2], v[2]), meanw[2]);
       const float pr[6] = {__fmul_rn(r, r), __fmul_rn(r, g), __fmul_rn(r, b), __fmul_rn(g, g), __fmul_rn(g, b), __fmul_rn(b, b)};
       // a product of a float and a weight is exact, so the fused form rounds the sum alone as theirs does
-      for (int k = 0; k < 6; k++) cov[k] = __fma_rn(widen(pr[k]), w, cov[k]);
+      if constexpr (kShare == 4) {
+        cov[0] = __fma_rn(widen(sub == 0 ? pr[0] : sub == 1 ? pr[1] : sub == 2 ? pr[2] : pr[3]), w, cov[0]);
+        cov[1] = __fma_rn(widen(sub == 0 ? pr[4] : pr[5]), w, cov[1]);
+      } else {
+        for (int k = 0; k < 6; k++) cov[k] = __fma_rn(widen(pr[k]), w, cov[k]);
+      }
     }
+    if constexpr (kShare == 4) {
+      const double mine = cov[0], other = cov[1];
+      for (int k = 0; k < 6; k++) cov[k] = from_sharer(k < 4 ? mine : other, k & 3);
+    }
+    // kShare = 4: the row of the matrix that this lane multiplies (the fourth lane: the third's)
+    const double row[3] = {sub == 0 ? cov[0] : sub == 1 ? cov[1] : cov[2], sub == 0 ? cov[1] : sub == 1 ? cov[3] : cov[4],
+                           sub == 0 ? cov[2] : sub == 1 ? cov[4] : cov[5]};
     double vf[3] = {(double).9f, (double)1.0f, (double).7f};
     float fv[3] = {.9f, 1.f, .7f};
     #pragma unroll 1
     for (int it = 0; it < 8; it++) {
-      double r = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[0]), __dmul_rn(vf[1], cov[1])), __dmul_rn(vf[2], cov[2]));
-      double g = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[1]), __dmul_rn(vf[1], cov[3])), __dmul_rn(vf[2], cov[4]));
-      double b = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[2]), __dmul_rn(vf[1], cov[4])), __dmul_rn(vf[2], cov[5]));
+      double r, g, b;
+      if constexpr (kShare == 4) {
+        const double p = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], row[0]), __dmul_rn(vf[1], row[1])), __dmul_rn(vf[2], row[2]));
+        r = from_sharer(p, 0); g = from_sharer(p, 1); b = from_sharer(p, 2);
+      } else {
+        r = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[0]), __dmul_rn(vf[1], cov[1])), __dmul_rn(vf[2], cov[2]));
+        g = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[1]), __dmul_rn(vf[1], cov[3])), __dmul_rn(vf[2], cov[4]));
+        b = __dadd_rn(__dadd_rn(__dmul_rn(vf[0], cov[2]), __dmul_rn(vf[1], cov[4])), __dmul_rn(vf[2], cov[5]));
+      }
       // the largest magnitude, compared as integers
       unsigned long long top = magnitude(r);
       top = max(top, max(magnitude(g), magnitude(b)));
@@ -1735,14 +1764,14 @@ __device__ __forceinline__ void fill_unit(float* unit) {
 }
 
 // Phase 1 over n blocks: warp w takes the groups of 32 consecutive blocks g = w, w + W, ..., a lane
-// per block, each group staged by one bulk copy. Warps are ranked CTA-first (warp 0 of every CTA,
+// per block (of 8, four lanes per block, below `share_below` blocks), each group staged by one bulk copy. Warps are ranked CTA-first (warp 0 of every CTA,
 // then warp 1, ...), and the grid has a CTA per group up to the resident limit, so a short batch
 // (the learned encoder's fallback blocks, a small mip level) puts one working warp on each SM:
 // the seeds are bound by the SM's FP64 pipe, which the warps of one CTA would share.
 template <bool G>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
     k_dxt1_seeds(const uint8_t* __restrict__ blocks, uint32_t n, uint32_t opts, Seed* __restrict__ seeds,
-                 const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ next) {
+                 const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ next, uint32_t share_below) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (n_dev) n = min(n, *n_dev);  // a count the host does not read back: n is then only the grid's bound
@@ -1752,11 +1781,13 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
   const uint32_t lane = lane_id();
   const uint32_t warp_global = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint32_t nwarps = gridDim.x * kWarpsPerCta;
-  const uint32_t groups = (n + kSeedLanes - 1) / kSeedLanes;
+  const bool share = n < share_below;
+  const uint32_t per = share ? kSeedLanes / 4 : kSeedLanes;  // blocks of a group
+  const uint32_t groups = (n + per - 1) / per;
   const uint32_t zero = 0;
   auto run = [&](uint32_t g, const uint8_t*& src, uint32_t& cnt) {
-    src = blocks + (size_t)g * kSeedLanes * 64;
-    cnt = min((uint32_t)kSeedLanes, n - g * kSeedLanes);
+    src = blocks + (size_t)g * per * 64;
+    cnt = min(per, n - g * per);
   };
   ChunkStager st;
   if (warp_global < groups) {
@@ -1765,17 +1796,20 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
     st.start(S, 1, &src, &cnt, &zero);
   }
   for (uint32_t g = warp_global; g < groups; g += nwarps) {
-    const uint32_t b = g * kSeedLanes + lane;
+    const uint32_t at = share ? lane >> 2 : lane, b = g * per + at;
     const uint8_t* staged = st.acquire(S);
     uint32_t pix[16];
-    if (b < n) load_pix(staged ? staged + (size_t)lane * 64 : blocks + (size_t)b * 64, pix);
+    if (b < n) load_pix(staged ? staged + (size_t)at * 64 : blocks + (size_t)b * 64, pix);
     const uint32_t gn = g + nwarps;
     if (gn < groups) {
       const uint8_t* src; uint32_t cnt;
       run(gn, src, cnt);
       st.next(S, 1, &src, &cnt, &zero);
     }
-    if (b < n) phase1_block<G>(S, unit, (int)lane, pix, opts, seeds + b);
+    if (b < n) {
+      if (share) phase1_block<G, 4>(S, unit, (int)at, pix, opts, seeds + b);
+      else phase1_block<G, 1>(S, unit, (int)at, pix, opts, seeds + b);
+    }
   }
   st.finish(S);
 }
@@ -2099,7 +2133,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
       runs(gn, src, cnt);
       st.next(S, kPer, src, cnt, dst);
     }
-    if (mine) phase1_block<false>(S, unit, (int)lane, pix, segs[ch.segment].options, seeds + ch.first + k);
+    if (mine) phase1_block<false, 1>(S, unit, (int)lane, pix, segs[ch.segment].options, seeds + ch.first + k);
   }
   st.finish(S);
 }
@@ -2321,18 +2355,19 @@ int launch_dxt1_kernel(const uint8_t* d_blocks, uint32_t n, uint32_t opts, uint8
   // the general kernels for anything beyond the default Uber encode
   const bool general = (opts & ~(kD1Perceptual | kD1Three | (7u << kD1QualityShift) | (255u << kD1ThresholdShift))) ||
                        ((opts >> kD1QualityShift) & 7u) != kQUber;
-  const uint32_t seed_warps = (n + kSeedLanes - 1) / kSeedLanes;
+  const uint32_t share_below = (uint32_t)L.sms * kSharedPerSm;
+  const uint32_t seed_warps = n < share_below ? (n + kSeedLanes / 4 - 1) / (kSeedLanes / 4) : (n + kSeedLanes - 1) / kSeedLanes;
   const uint32_t seed_full = (uint32_t)(L.sms * L.seeds_per_sm);
   const uint32_t seed_grid = std::min<uint32_t>(seed_warps, seed_full);
   const size_t seed_smem = sizeof(SeedShared) * kWarpsPerCta, smem = sizeof(WarpShared) * kWarpsPerCta;
   const uint32_t full = (uint32_t)(L.sms * L.search_per_sm[general ? 1 : 0]);
   const uint32_t grid = std::min<uint32_t>((n + kWarpsPerCta - 1) / kWarpsPerCta, full);
   if (general) {
-    k_dxt1_seeds<true><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next);
+    k_dxt1_seeds<true><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next, share_below);
     k_dxt1_encode<true, kCtasPerSm><<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err,
                                                              d_err_io, work, n_dev, next);
   } else {
-    k_dxt1_seeds<false><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next);
+    k_dxt1_seeds<false><<<seed_grid, kWarpsPerCta * 32, seed_smem, s>>>(d_blocks, n, opts, seeds, n_dev, next, share_below);
     const auto search = n <= (uint32_t)(L.sms * kFewCtasPerSm * kWarpsPerCta) ? k_dxt1_encode<false, kFewCtasPerSm>
                                                                               : k_dxt1_encode<false, kCtasPerSm>;
     search<<<grid, kWarpsPerCta * 32, smem, s>>>(d_blocks, n, opts, seeds, d_out, out_stride, d_err, d_err_io, work, n_dev,

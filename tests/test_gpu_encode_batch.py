@@ -139,3 +139,20 @@ def test_block_counts_around_the_few_blocks_search_match(cg, past):
     twice, terr = cg.dxt1_optimize(torch.cat([blocks, blocks]), with_error=True)
     for half in (0, 1):
         assert torch.equal(twice[half * n:(half + 1) * n], got) and torch.equal(terr[half * n:(half + 1) * n], err)
+
+
+@pytest.mark.parametrize("from_line, n", [(0, 1), (0, 7), (0, 9), (0, 33), (1, -1), (1, 0), (1, 1)])
+def test_seeds_of_few_blocks_match_those_of_many(cg, from_line, n):
+    # below 40 blocks an SM four lanes take a block: short groups of eight, and both sides of the line,
+    # against the same blocks among as many again
+    line = torch.cuda.get_device_properties(0).multi_processor_count * 40
+    total = line + n if from_line else n
+    rng = np.random.default_rng(total)
+    px = rng.integers(0, 256, (total, 16, 4), dtype=np.uint8) // rng.integers(1, 60, (total, 1, 4), dtype=np.uint8)
+    px[rng.integers(0, 2, (total, 16)) > 0] &= 0xF0
+    px[..., 3] = 255
+    blocks = torch.from_numpy(px.reshape(total, 64)).cuda()
+    for perceptual in (True, False):
+        got = cg.dxt1_optimize(blocks, perceptual)
+        among = cg.dxt1_optimize(blocks.repeat((line + total) // total + 1, 1), perceptual)
+        assert torch.equal(among[:total], got) and torch.equal(among[-total:], got)
