@@ -751,8 +751,8 @@ def main():
                                     "per_level_calls_parity": per_level_parity,
                                     "dxt5_2048_ms": round(single5_ms, 4),
                                     "dxt5_2048_GB/s": round(single5_bytes / (single5_ms / 1e3) / 1e9, 4),
-                                    "path": "ctx.unpack_levels (crngpu_unpack_levels), device destination: levels of "
-                                            ">= 256 blocks on k_crn_decode_wide (a CTA per level), the rest on the "
+                                    "path": "ctx.unpack_levels (crngpu_unpack_levels), device destination: the largest "
+                                            "levels on k_crn_decode_walk, others on k_crn_decode_wide or the "
                                             "lane decoder; lane_decoder_ms: every level on the lane decoder; per_level_calls_ms: "
                                             "unpack_begin + crngpu_unpack_level per level + unpack_end, wall time "
                                             "per file (the crnd_unpack_level pattern)"},
