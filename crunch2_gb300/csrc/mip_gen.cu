@@ -588,6 +588,12 @@ void add_items(std::vector<Item>& items, Job& job, const std::vector<Span>& sp, 
 // ms, with singles 0.21). Rows: 4 (every row has its own chains; both ways take the same time at 8
 // and 16).
 constexpr int kFewRowSamples = 4, kFewColSamples = 16;
+// Few windows of a small level reach a chunk (5.4 scales wide: 8 pairs of samples at a scale of 16, 4 at
+// 64, for 16 warps), so three levels at a time share their jobs' chunks: 4096 x 4096 1.88 ms with a job
+// for each, 1.51 so (from a scale of 16 on; of 8 1.58, of 4 1.51 and 1000 x 3000 442 us, 471 from 16 on;
+// four levels 1.59). Not for images whose jobs do not fill the SMs (512 x 512 107 us, merged 110).
+constexpr uint32_t kMergeScale = 4, kMergeLevels = 3;
+constexpr uint64_t kMergeTexels = 1u << 21;
 
 bool make_plan(uint32_t width, uint32_t height, uint32_t levels, uint32_t filter, float filter_scale, Plan& plan) {
   std::vector<float> pool;
@@ -610,6 +616,29 @@ bool make_plan(uint32_t width, uint32_t height, uint32_t levels, uint32_t filter
     const std::vector<Span>* sp = axis((int)width, dw);
     if (!sp) return false;
     const bool single = dw <= kFewRowSamples;
+    if (!single && (uint64_t)width * height >= kMergeTexels && (uint32_t)dw * kMergeScale <= width) {
+      // the level and up to two after it in common jobs over the same part of the row
+      uint32_t end = l + 1;
+      while (end < levels && end < l + kMergeLevels && (int)(width >> end) > kFewRowSamples) end++;
+      for (int d = 0; d < dw; d += kPairJob) {
+        Job j = {};
+        j.item = (uint32_t)items.size();
+        for (uint32_t k = l; k < end; k++) {
+          const int kw = (int)(width >> k), from = (int)((int64_t)d * kw / dw),
+                    to = (int)((int64_t)std::min(d + kPairJob, dw) * kw / dw);
+          const std::vector<Span>* ks = axis((int)width, kw);
+          if (!ks) return false;
+          add_items(items, j, *ks, from, to - from, true, tmp_of[k], (uint32_t)kw, 1);
+        }
+        // by their windows' middles, so that the ones that reach a chunk go to different warps
+        std::stable_sort(items.begin() + j.item, items.end(), [](const Item& a, const Item& b) {
+          return a.a0 + std::max(a.b0, a.b1) < b.a0 + std::max(b.b0, b.b1);
+        });
+        rows.push_back(j);
+      }
+      l = end - 1;
+      continue;
+    }
     const int per = single ? kSingles : row_job(*sp);
     for (int d = 0; d < dw; d += per) {
       // the last levels' few samples (4 + 2 + 1, and a side's 1s) share a job: the source is the same

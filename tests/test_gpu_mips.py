@@ -69,3 +69,17 @@ def test_gpu_mips_edges_match_oracle(cg, w, h, filt, scale, wrap, alpha):
     assert len(got) == levels
     for l in range(1, levels):
         assert np.array_equal(got[l].cpu().numpy(), want[l] if len(want) == levels else want[l - 1]), l
+
+
+# images of at least 2^21 texels, whose small levels share their row jobs: sides that are not powers of two,
+# runs of samples cut unevenly between jobs, windows over many chunks, wrap
+@pytest.mark.parametrize("w,h,filt,scale,wrap", [
+    (8209, 257, "kaiser", 0.9, False), (1030, 2053, "lanczos4", 1.3, True), (259, 8101, "box", 0.9, False)])
+def test_gpu_mips_of_large_images_match_oracle(cg, w, h, filt, scale, wrap):
+    from oracle import mip_oracle
+    img = np.random.default_rng(w).integers(0, 256, (h, w, 4), dtype=np.uint8)
+    levels = 7
+    want = mip_oracle.generate_mipmaps(img, filt, scale, True, wrap, alpha=True, levels=levels)
+    got = cg.generate_mipmaps(torch.from_numpy(img).cuda(), filt, scale, True, wrap, alpha=True, levels=levels)
+    for l in range(1, levels):
+        assert np.array_equal(got[l].cpu().numpy(), want[l] if len(want) == levels else want[l - 1]), l
