@@ -365,3 +365,25 @@ def test_compress_crn_bitrate_matches_reference(hc, name):
     assert abs(rate - r["bitrate"]) <= 0.015 * r["bitrate"]
     if r["bitrate"] <= r["target"]:
         assert rate <= r["target"]
+
+
+@pytest.mark.parametrize("cells", [1, 2, 7, 8])
+def test_codebooks_of_few_entries_find_each_cells_own(hc, cells):
+    """Solid 8x8 cells of far apart colours and alphas: with no more entries than lanes that look for the
+    nearest one, every cell must still get its own (5:6:5 rounds a component by at most 4)."""
+    import crunch2_gb300 as cg
+    from dxt_decode import dxt1_colours, dxt5a_values
+    from oracle import port
+    colours = np.array([[0, 0, 0], [255, 255, 255], [255, 0, 0], [0, 255, 0], [0, 0, 255], [255, 255, 0], [0, 255, 255],
+                        [255, 0, 255]], np.uint8)[:cells]
+    img = np.zeros((8, 8 * cells, 4), np.uint8)
+    for i, c in enumerate(colours):
+        img[:, 8 * i:8 * i + 8, :3] = c
+        img[:, 8 * i:8 * i + 8, 3] = 30 * i + 20
+    crn = cg.compress_crn([[img]], cg.FMT_DXT5, quality=255)
+    blocks = port.unpack_level(crn, 0, 16 * 4 * cells).reshape(-1, 16)
+    rgb = dxt1_colours(blocks[:, 8:]).reshape(2, 2 * cells, 16, 3)
+    alpha = dxt5a_values(blocks[:, :8]).reshape(2, 2 * cells, 16)
+    for i in range(cells):
+        assert np.abs(rgb[:, 2 * i:2 * i + 2] - colours[i].astype(int)).max() <= 4, i
+        assert np.abs(alpha[:, 2 * i:2 * i + 2] - (30 * i + 20)).max() <= 1, i
