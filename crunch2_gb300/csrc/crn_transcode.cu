@@ -1,7 +1,8 @@
 // CRN -> DXTn transcoder on the GPU.
 //
 // Restates crnd::crn_unpacker::unpack_level and unpack_dxt1/dxt5/dxn/dxt5a
-// (inc/crn_decomp.h:3537-3619, 3944-4223) as two kernels:
+// (inc/crn_decomp.h:3537-3619, 3944-4223) as a serial and a parallel part, the serial one in one of
+// three decoders (also k_crn_decode_wide and k_crn_decode_walk, below):
 //   k_crn_decode_textures - the serial part. Each level stream is a serial chain of prefix
 //                   codes whose meaning depends on the symbols before it, so one lane owns one
 //                   stream: it Huffman-decodes the reference-group / endpoint-delta / selector
@@ -2265,7 +2266,7 @@ uint64_t level_records(const CrnFile& F, uint32_t l) {
 
 // Which level streams go to k_crn_decode_wide. 0 (the default): the split that minimises the
 // plan's decode time (decide_wide); otherwise levels of at least this many blocks (all faces) go
-// to the wide decoder. Set by crngpu_set_decode_split (tests force either decoder on every level).
+// to the wide decoder. Set by crngpu_set_decode_split (tests force the wide or the lane decoder on every level).
 std::atomic<uint32_t> g_wide_min_blocks{0};
 
 // Decode cost model, in microseconds per block for a one-endpoint format (twice that for DXT5 and
@@ -2935,9 +2936,8 @@ int expand_wait_counters(uint32_t out[2], bool reset) {
 }
 
 
-// A prepared batch: many levels of many contexts, decoded by one persistent launch and expanded
-// by one more. The job tables and record buffer are uploaded/allocated once at creation, so a
-// launch only enqueues a memset and two kernels (and can replay as a CUDA graph).
+// A prepared batch: many levels of many contexts, decoded together and expanded by one launch. The job tables and record buffer are uploaded/allocated once at creation, so a
+// launch only enqueues memsets, the decoders' launches and the expansion (and can replay as a CUDA graph).
 struct UnpackBatch : HostObject {
   uint32_t magic = 0x42415443u;
   int device = -1;

@@ -1,7 +1,7 @@
 // DXT1 / DXT5A block encoders for sm_103a, bit-exact with crnlib's optimizers at every quality.
 //
-// DXT1 (dxt1_endpoint_optimizer, crnlib/crn_dxt1.cpp) runs in two phases inside one kernel:
-//   phase 1, lane per block: unique colours, perceptual weighting (powf), the double-precision
+// DXT1 (dxt1_endpoint_optimizer, crnlib/crn_dxt1.cpp) runs in two phases, a kernel each:
+//   phase 1, lane per block (four lanes for few blocks): unique colours, perceptual weighting (powf), the double-precision
 //     PCA and projection bounds (handle_multicolor_block :1069-1178) and the LBG seeds of
 //     try_median4 (:1181-1308). These are scalar, FP64-heavy and tiny, so lanes work on
 //     different blocks and GB300's narrow FP64 pipe is amortised over the warp.
@@ -19,8 +19,8 @@
 // Distances are exact integers computed in FP32 with the expanded square
 //   w.(x-p)^2 = w.x^2 + (w.p^2 - 2 w.p.x), all terms integers below 2^24.
 // This file must be compiled with --fmad=false: the FP32/FP64 parts restate the reference's
-// expression order without fused multiply-adds (the only FMAs are the explicit fmaf of exact
-// integer terms).
+// expression order without fused multiply-adds (the only FMAs are the explicit ones, of exact terms or
+// where a result's rounding is checked).
 //
 // DXT5A (dxt5_endpoint_optimizer, crnlib/crn_dxt5a.cpp:40-262) is half a warp per block, lane per
 // candidate, with the same first-improvement resolution; its probe grid follows the moving
@@ -38,10 +38,9 @@ namespace crngpu {
 
 #define FULL_MASK 0xFFFFFFFFu
 
-constexpr int kBlocksPerWarp = 8;
 constexpr int kWarpsPerCta = 4;
-// CTAs per SM the encoders are compiled for (registers: 65536 / (128 x 8) = 64 per thread; the
-// phase-1 PCA spills a little, the candidate loops do not). 8 beat 4, 5 and 6 on GB300.
+// CTAs per SM the search is compiled for (registers: 65536 / (128 x 8) = 64 per thread, which spills
+// some 150 bytes): a 1024 x 1024 chain 2.83 ms, with 7 2.85 and with 6 2.88; few blocks, see k_dxt1_encode.
 constexpr int kCtasPerSm = 8, kFewCtasPerSm = 4;
 constexpr uint32_t kInf = 0xFFFFFFFFu;
 

@@ -9,8 +9,8 @@
 //   k_vq_split<D>     tree_clusterizer (crnlib/crn_tree_clusterizer.h:89-570): a node is split by
 //                     furthest/opposite seeds, a 10-step power iteration for its principal axis and
 //                     a 2-means loop. Instead of the reference's one-node-at-a-time priority queue,
-//                     a round splits the top quarter of the leaves by variance at once, one CTA per
-//                     node, until the codebook size is reached.
+//                     a round splits the top quarter of the leaves by variance at once, a cluster of
+//                     CTAs or a warp per node, until the codebook size is reached.
 //   k_nearest_vec6    tile -> nearest endpoint codebook entry (determine_color_endpoint_clusters_task,
 //                     :836-886).
 //   k_cluster_fit     per endpoint cluster, over all pixels of its tiles: principal-axis start, least-
