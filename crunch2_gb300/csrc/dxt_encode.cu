@@ -306,11 +306,17 @@ template <bool G, int kShare>
 __device__ void phase1_block(SeedShared& S, const float* __restrict__ unit, int slot, const uint32_t (&pix)[16],
                              uint32_t opts, Seed* __restrict__ out) {
   const int L = slot, sub = kShare == 4 ? (int)lane_id() & 3 : 0;
-  // a value of the block's lane j (kShare = 4; the four go through everything together)
-  auto from_sharer = [](double x, int j) {
-    const unsigned four = 0xFu << (lane_id() & 28u);
+  // kShare = 4: the four lanes take the same branches and write the same values to their block's scratch,
+  // so they have to meet only where a place is given another value: none may still read the old one
+  const unsigned four = 0xFu << (lane_id() & 28u);
+  auto join_sharers = [&]() {
+    if constexpr (kShare == 4) __syncwarp(four);
+  };
+  // a value of the block's lane j (kShare = 4)
+  auto from_sharer = [&](double x, int j) {
     return __hiloint2double(__shfl_sync(four, __double2hiint(x), j, 4), __shfl_sync(four, __double2loint(x), j, 4));
   };
+  join_sharers();  // the block before
   const bool perceptual = (opts & kD1Perceptual) != 0;
   const uint32_t quality = G ? (opts >> kD1QualityShift) & 7u : kQUber;
   int n = 0;
@@ -329,6 +335,7 @@ __device__ void phase1_block(SeedShared& S, const float* __restrict__ unit, int 
     }
     if (has_t || !dark || dark == n) { out->n = -1; return; }
     n = 0;
+    join_sharers();  // the list above has been searched
   }
   // unique colours of the opaque texels in first-occurrence order (compute_internal :2113-2131); a
   // transparent texel stands for a colour of its own that is left out. All pairs are compared in

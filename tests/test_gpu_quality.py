@@ -153,3 +153,18 @@ def test_rejects_bad_options(cg, gold):
         cg.compress_blocks(gold["edge_in"][:4], cg.FMT_DXT1, quality=5)
     with pytest.raises(cg.CrnGpuError):
         cg.dxt1_optimize(gold["edge_in"][:4], quality=7)
+
+
+@pytest.mark.parametrize("options", [
+    dict(transparent_black=True), dict(transparent_black=True, dxt1a=True), dict(dxt1a=True),
+    dict(grayscale=True), dict(perceptual=False)])
+@pytest.mark.parametrize("quality", [2, 4])
+def test_blocks_seeded_by_four_lanes_equal_those_by_one(cg, gold, options, quality):
+    """Few blocks are seeded by four lanes each, which share their block's scratch: with every option
+    that uses it, what a large batch (a lane each) gives the same blocks."""
+    few = 40 * torch.cuda.get_device_properties(0).multi_processor_count
+    blocks = torch.from_numpy(gold["edge_in"]).cuda()
+    many = blocks.repeat(few // blocks.shape[0] + 1, 1)
+    want = cg.dxt1_optimize(many, quality=quality, **options)
+    for n in (1, 7, 9, blocks.shape[0], few - 1, few):
+        assert torch.equal(cg.dxt1_optimize(many[:n].contiguous(), quality=quality, **options), want[:n]), n
