@@ -79,6 +79,43 @@ void DevBuf::release() {
   device = -1;
 }
 
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+LaunchOrder::~LaunchOrder() {
+  if (last) cudaEventDestroy(last);
+}
+
+OrderedLaunch::OrderedLaunch(LaunchOrder& order, cudaStream_t s)
+    : lock_(order.mu), order_(order), s_(s), captured_(capturing(s)) {
+  if (!captured_ && order_.last) cudaStreamWaitEvent(s_, order_.last, 0);
+}
+
+OrderedLaunch::~OrderedLaunch() {
+  if (captured_) return;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (order_.last && order_.device != dev) {  // an event is recorded on its own device only
+    cudaEventDestroy(order_.last);
+    order_.last = nullptr;
+  }
+  if (!order_.last) {
+    if (cudaEventCreateWithFlags(&order_.last, cudaEventDisableTiming) != cudaSuccess) {
+      order_.last = nullptr;
+      cudaStreamSynchronize(s_);
+      return;
+    }
+    order_.device = dev;
+  }
+  if (cudaEventRecord(order_.last, s_) != cudaSuccess) cudaStreamSynchronize(s_);
+}
+
 // Host allocation hooks of the transcoder's state (host_alloc.h). Each allocation carries a
 // 16-byte header with the hooks that made it, so it is always freed by the same allocator.
 namespace {

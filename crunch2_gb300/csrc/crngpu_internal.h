@@ -77,6 +77,31 @@ DevBuf& staging(int slot);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// True while work enqueued on `s` goes into a graph that the caller is capturing.
+bool capturing(cudaStream_t s);
+
+// Buffers that one launch after another uses: a launch waits on the device for the one before it,
+// which may be on another stream. (A launch that the caller captures runs when their graph does and can
+// neither wait here nor be waited for.)
+struct LaunchOrder {
+  std::mutex mu;  // held while a launch is enqueued
+  cudaEvent_t last = nullptr;  // after the latest launch
+  int device = -1;             // of `last`
+  ~LaunchOrder();
+};
+class OrderedLaunch {
+ public:
+  OrderedLaunch(LaunchOrder& order, cudaStream_t s);
+  ~OrderedLaunch();
+  bool captured() const { return captured_; }
+
+ private:
+  std::lock_guard<std::mutex> lock_;
+  LaunchOrder& order_;
+  cudaStream_t s_;
+  bool captured_;
+};
+
 // Batched block encoding (many textures, mixed formats). A segment is one element of one texture
 // over its gathered blocks [first_block, first_block + count): the colour half of DXT1/DXT5, the
 // alpha of DXT5/DXT5A or one DXN channel; block b's 8 bytes go to out + (b - first_block) * stride.
@@ -147,7 +172,7 @@ int launch_dxt5a(const uint8_t* d_blocks, uint32_t n, int comp, bool both, uint3
                  uint32_t out_stride, cudaStream_t s, int second = -1);
 // the batched colour encode: phase 1 writes one seed record of kDxt1SeedBytes per block to
 // d_seeds (room for every gathered block of the batch), phase 2 reads them; d_next: the number of the
-// next block that phase 2's warps take, set by phase 1
+// next block that phase 2's warps take, set by phase 1; without it each warp takes its share in turn
 constexpr size_t kDxt1SeedBytes = 64;
 int launch_dxt1_chunks(const uint8_t* d_blocks, const EncodeChunk* d_chunks, uint32_t nchunks,
                        const EncodeSegment* d_segs, void* d_seeds, uint32_t* d_next, int grid, cudaStream_t s);

@@ -2105,7 +2105,7 @@ static_assert(kSeedLanes % kColourChunkBlocks == 0 && kSeedLanes / kColourChunkB
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
     k_dxt1_seeds_chunks(const uint8_t* __restrict__ blocks, const EncodeChunk* __restrict__ chunks, uint32_t nchunks,
                         const EncodeSegment* __restrict__ segs, Seed* __restrict__ seeds, uint32_t* __restrict__ next) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
+  if (next && blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float unit[256];
   fill_unit(unit);
@@ -2150,7 +2150,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
 
 // Phase 2 of the batched encode: persistent warps walk the chunk table, a block at a time, taken as in
 // k_dxt1_encode (block k of chunk c is number kColourChunkBlocks c + k; a short chunk's last numbers
-// have none).
+// have none). Without `next` in turn: for launches that may run beside others of the same batch.
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
     k_dxt1_encode_chunks(const uint8_t* __restrict__ blocks, const EncodeChunk* __restrict__ chunks, uint32_t nchunks,
                          const EncodeSegment* __restrict__ segs, const Seed* __restrict__ seeds,
@@ -2161,7 +2161,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
   const uint32_t nwarps = gridDim.x * kWarpsPerCta;
   #pragma unroll 1
   for (uint32_t i = warp_global; i / kColourChunkBlocks < nchunks;) {
-    const uint32_t after = take(next, true);
+    const uint32_t after = take(next, next != nullptr);
     const EncodeChunk ch = chunks[i / kColourChunkBlocks];
     if (i % kColourChunkBlocks < ch.count) {
       const EncodeSegment sg = segs[ch.segment];
@@ -2170,7 +2170,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
       phase2_block<false>(S, blocks + (size_t)b * 64, sg.options, sg.out + (size_t)(b - sg.first_block) * sg.stride,
                           nullptr, nullptr);
     }
-    i = nwarps + __shfl_sync(FULL_MASK, after, 0);
+    i = next ? nwarps + __shfl_sync(FULL_MASK, after, 0) : i + nwarps;
   }
 }
 

@@ -64,14 +64,15 @@ struct EncodeBatch {
   cudaEvent_t fork = nullptr, join = nullptr;
   cudaGraphExec_t graph = nullptr;
   size_t seed_bytes = 0;
+  LaunchOrder order;  // gathered blocks, seeds and counter are the batch's own: one launch at a time
 };
 
-// the search's block counter, behind the seeds
+// the search's block counter, behind the seeds (one for the batch: not for launches that may overlap)
 uint32_t* next_block(const EncodeBatch* b) {
   return reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(b->seeds.ptr) + b->seed_bytes);
 }
 
-int enqueue(EncodeBatch* b, cudaStream_t s, int colour_grid, int alpha_grid) {
+int enqueue(EncodeBatch* b, cudaStream_t s, int colour_grid, int alpha_grid, uint32_t* next) {
   cudaError_t e;
   if (b->ntiles) {
     k_gather_tiles<<<b->ntiles, 256, 0, s>>>(static_cast<const GatherTile*>(b->d_tiles.ptr),
@@ -88,7 +89,7 @@ int enqueue(EncodeBatch* b, cudaStream_t s, int colour_grid, int alpha_grid) {
   if (rc != CRNGPU_OK) return rc;
   if ((e = cudaEventRecord(b->join, b->side)) != cudaSuccess) return cuda_check(e, "record join");
   rc = launch_dxt1_chunks(blk, static_cast<const EncodeChunk*>(b->d_cchunks.ptr), b->ncolour, segs, b->seeds.ptr,
-                          next_block(b), colour_grid, s);
+                          next, colour_grid, s);
   if (rc != CRNGPU_OK) return rc;
   if ((e = cudaStreamWaitEvent(s, b->join, 0)) != cudaSuccess) return cuda_check(e, "wait join");
   return CRNGPU_OK;
@@ -274,9 +275,12 @@ extern "C" int crngpu_encode_batch_launch(crngpu_encode_batch batch, uint32_t fl
   EncodeBatch* b = reinterpret_cast<EncodeBatch*>(batch);
   if (!b || b->magic != 0x454E4342u) { set_error("bad batch"); return CRNGPU_E_PARAM; }
   cudaStream_t s = as_stream(stream);
+  OrderedLaunch ordered(b->order, s);
   int rc;
   if (!b->colour_grid && (rc = autotune(b, s)) != CRNGPU_OK) return rc;
-  if (!(flags & CRNGPU_BATCH_GRAPH)) return enqueue(b, s, b->colour_grid, b->alpha_grid);
+  // a captured launch may later run beside others of the batch, whose counter it then has to leave alone
+  if (!(flags & CRNGPU_BATCH_GRAPH))
+    return enqueue(b, s, b->colour_grid, b->alpha_grid, ordered.captured() ? nullptr : next_block(b));
   cudaError_t e;
   if (!b->graph) {
     // capture on a private stream (the legacy default stream cannot be captured), then replay
@@ -287,7 +291,7 @@ extern "C" int crngpu_encode_batch_launch(crngpu_encode_batch batch, uint32_t fl
       cudaStreamDestroy(cap);
       return cuda_check(e, "begin capture");
     }
-    rc = enqueue(b, cap, b->colour_grid, b->alpha_grid);
+    rc = enqueue(b, cap, b->colour_grid, b->alpha_grid, next_block(b));
     e = cudaStreamEndCapture(cap, &g);
     cudaStreamDestroy(cap);
     if (rc != CRNGPU_OK) { if (g) cudaGraphDestroy(g); return rc; }

@@ -544,7 +544,8 @@ CRNGPU_API crngpu_encode_batch crngpu_encode_batch_create(const crngpu_encode_it
 /* Enqueues the batch on `stream` without synchronising. The first launch runs the autotuner (each
  * encoder timed at several CTAs-per-SM launch shapes on the real blocks; synchronises once).
  * flags: CRNGPU_BATCH_GRAPH captures the launches into a CUDA graph on the first call and replays
- * it on later calls. The items' input and output buffers must stay valid while the batch exists. */
+ * it on later calls. The items' input and output buffers must stay valid while the batch exists.
+ * Launches of one batch on several streams run one after the other. */
 CRNGPU_API int crngpu_encode_batch_launch(crngpu_encode_batch batch, uint32_t flags, void* stream);
 
 /* grids[0], grids[1]: the tuned colour / alpha grid sizes (0 before the first launch); ms: the

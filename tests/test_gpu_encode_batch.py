@@ -156,3 +156,40 @@ def test_seeds_of_few_blocks_match_those_of_many(cg, from_line, n):
         got = cg.dxt1_optimize(blocks, perceptual)
         among = cg.dxt1_optimize(blocks.repeat((line + total) // total + 1, 1), perceptual)
         assert torch.equal(among[:total], got) and torch.equal(among[-total:], got)
+
+
+def test_launches_on_two_streams_and_in_a_callers_graph(cg):
+    """A batch has one set of gathered blocks, seeds and block counter: launches on two streams, directly
+    and from the batch's graph, without a wait between them, and from a graph the caller captured."""
+    items, _ = make_items(cg, [(512, 512, "DXT1", "colour", 8), (256, 256, "DXT5", "colour_alpha", 2)])
+    outs = [it[1] for it in items]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    with cg.EncodeBatch(items) as b:
+        b.launch()
+        torch.cuda.synchronize()
+        want = [o.clone() for o in outs]
+        for use_graph in (False, True):
+            got = []
+            for rep in range(6):
+                with torch.cuda.stream(streams[0]):
+                    for o in outs:
+                        o.zero_()
+                    b.launch(use_graph=use_graph, stream=streams[0])
+                    got.append([o.clone() for o in outs])
+                b.launch(use_graph=use_graph, stream=streams[1])  # beside the copies; writes the same bytes
+            torch.cuda.synchronize()
+            for g in got:
+                assert all(torch.equal(x, y) for x, y in zip(g, want)), use_graph
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            b.launch(stream=streams[0])
+        for rep in range(3):
+            for o in outs:
+                o.zero_()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(streams[0]):
+                graph.replay()
+                got = [o.clone() for o in outs]
+            b.launch(stream=streams[1])
+            torch.cuda.synchronize()
+            assert all(torch.equal(x, y) for x, y in zip(got, want)), rep
