@@ -1111,7 +1111,7 @@ constexpr uint32_t kWalkPosBits = 28;      // anchors: position | combination <<
 
 // A level's progress between launches (zero at the start).
 struct WalkState {
-  uint32_t p, r, e, groups;                // the walk: position, row, chunk or block in the row, groups passed
+  uint32_t p, groups;                      // the walk: position, groups passed
   uint32_t rows, carry, bad, pad;          // the resolver: rows resolved, running indices; 1: bad code, 2: bad index
   uint32_t passed[kWalkMaxSegments + 1];   // groups passed after each segment
   uint32_t bits[kWMaxW / 32];              // the current even row's combinations, a byte per four chunks
@@ -1145,6 +1145,12 @@ __host__ __device__ inline WalkShape walk_shape(uint32_t bx, uint32_t by, uint32
   s.ge = s.W2 / 4 + s.W2 % 4;  // whole groups, then a group per chunk
   s.go = (s.W + 3) / 4;
   return s;
+}
+// Where group g of a level begins: its row, and the chunk (even rows) or block (odd rows) in it.
+__device__ __forceinline__ void walk_group(const WalkShape& sh, uint32_t g, uint32_t& r, uint32_t& e) {
+  const uint32_t pair = g / (sh.ge + sh.go), rem = g - pair * (sh.ge + sh.go), whole = sh.W2 / 4;
+  r = 2 * pair + (rem >= sh.ge ? 1u : 0u);
+  e = rem >= sh.ge ? 4 * (rem - sh.ge) : rem < whole ? 4 * rem : 4 * whole + (rem - whole);
 }
 
 // Shared memory: the walk's ring of table windows (four windows; smaller ones when it holds the row
@@ -1319,7 +1325,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8 * i));
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
-    S.walking = st.r < sh.rows ? 1u : 0u;
+    S.walking = st.groups < sh.rows / 2 * (sh.ge + sh.go) ? 1u : 0u;
   }
   __syncthreads();
   const size_t buf = (size_t)(k & 1u) * job.cap;
@@ -1356,7 +1362,9 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
       if (!walk_wait(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u)) atomicMax(status, (uint32_t)kStWait);
   }
   if (tid) return;
-  uint32_t r = st.r, e = st.e, q = st.p - base, groups = st.groups;
+  // (the row and the place in it from the number of groups, which bounds what is written whatever p says)
+  uint32_t r, e, q = st.p - base, groups = st.groups;
+  walk_group(sh, groups, r, e);
   if (r < sh.rows) {
     const uint8_t* bits = reinterpret_cast<const uint8_t*>(S.bits);
     uint8_t* bits_w = reinterpret_cast<uint8_t*>(S.bits);
@@ -1481,8 +1489,6 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     for (uint32_t i = 0; i < kWMaxW / 32; i++) st.bits[i] = S.bits[i];
   }
   st.p = base + q;
-  st.r = r;
-  st.e = e;
   st.groups = groups;
   st.passed[k] = groups;
 }
@@ -2949,6 +2955,7 @@ struct UnpackBatch : HostObject {
   int variant = -1;          // expansion variant chosen by the autotuner
   float variant_ms[kExpandVariants] = {};
   uint64_t out_bytes = 0;
+  LaunchOrder order;  // records, work counter, status and walk state are the batch's own: one launch at a time
   ~UnpackBatch() {
     if (graph) cudaGraphExecDestroy(graph);
   }
@@ -3106,6 +3113,7 @@ extern "C" int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t fl
   if (!b || b->magic != 0x42415443u) { set_error("bad batch"); return CRNGPU_E_PARAM; }
   if (flags & ~(uint32_t)(CRNGPU_BATCH_GRAPH | CRNGPU_BATCH_EXPAND_ONLY)) { set_error("unknown flags"); return CRNGPU_E_PARAM; }
   cudaStream_t s = as_stream(stream);
+  OrderedLaunch ordered(b->order, s);
   const uint8_t* jobs = static_cast<const uint8_t*>(b->d_jobs.ptr);
   uint32_t* words = static_cast<uint32_t*>(b->d_words.ptr);
   if (b->variant < 0) {
@@ -3192,6 +3200,7 @@ extern "C" int crngpu_unpack_batch_status(crngpu_unpack_batch batch, void* strea
   UnpackBatch* b = reinterpret_cast<UnpackBatch*>(batch);
   if (!b || b->magic != 0x42415443u) { set_error("bad batch"); return CRNGPU_E_PARAM; }
   cudaStream_t s = as_stream(stream);
+  OrderedLaunch ordered(b->order, s);
   cudaError_t e = cudaMemcpyAsync(b->words_host, b->d_words.ptr, 8, cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_check(e, "read status");
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");

@@ -453,7 +453,9 @@ CRNGPU_API crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
  * graph on later calls (one launch from the host per batch); CRNGPU_BATCH_EXPAND_ONLY re-runs
  * only the expansion kernel from the index records of the last decode (the destinations are
  * rewritten; used to time the HBM-bound expansion on its own). The first launch of a batch also
- * runs the expansion autotuner (see crngpu_unpack_batch_tuning) and synchronises once. */
+ * runs the expansion autotuner (see crngpu_unpack_batch_tuning) and synchronises once. Launches of one
+ * batch on several streams run one after the other; one that the caller captures into a graph of their
+ * own must not overlap another of the batch, with which it shares the index records. */
 #define CRNGPU_BATCH_GRAPH 1u
 #define CRNGPU_BATCH_EXPAND_ONLY 2u
 CRNGPU_API int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t flags, void* stream);

@@ -121,3 +121,32 @@ def test_batch_of_walks(cg):
                 assert np.array_equal(o.cpu().numpy(), w)
     for c in ctxs:
         c.close()
+
+
+def test_launches_on_two_streams(cg):
+    """A batch has one set of index records, walk states and counters: launches on two streams, directly and
+    from the batch's graph, without a wait between them."""
+    specs = [("dxt1", 512, 256), ("dxt5", 300, 300), ("dxn", 256, 512), ("dxt1", 64, 64)]
+    crns = [make(cg, f, w, h, 40 + i) for i, (f, w, h) in enumerate(specs)]
+    want = [torch.from_numpy(decode(cg, c, cg.DECODE_LANE_ONLY)[1]).cuda() for c in crns]
+    ctxs = [cg.unpack_begin(c) for c in crns]
+    outs = [torch.zeros_like(w) for w in want]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    with cg.UnpackBatch([(c, 0, c.levels, o) for c, o in zip(ctxs, outs)]) as b:
+        b.launch()
+        torch.cuda.synchronize()
+        for graph in (False, True):
+            got = []
+            for rep in range(6):
+                with torch.cuda.stream(streams[0]):
+                    for o in outs:
+                        o.zero_()
+                    b.launch(use_graph=graph, stream=streams[0])
+                    got.append([o.clone() for o in outs])
+                b.launch(use_graph=graph, stream=streams[1])  # beside the copies; writes the same bytes
+            b.status(streams[0])
+            torch.cuda.synchronize()
+            for g in got:
+                assert all(torch.equal(x, y) for x, y in zip(g, want)), graph
+    for c in ctxs:
+        c.close()
