@@ -92,29 +92,54 @@ LaunchOrder::~LaunchOrder() {
   if (last) cudaEventDestroy(last);
 }
 
-OrderedLaunch::OrderedLaunch(LaunchOrder& order, cudaStream_t s)
-    : lock_(order.mu), order_(order), s_(s), captured_(capturing(s)) {
-  if (!captured_ && order_.last) cudaStreamWaitEvent(s_, order_.last, 0);
+bool LaunchOrder::begin(cudaStream_t s) {
+  if (capturing(s)) return true;
+  if (last) cudaStreamWaitEvent(s, last, 0);
+  return false;
 }
 
-OrderedLaunch::~OrderedLaunch() {
-  if (captured_) return;
+void LaunchOrder::end(cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (order_.last && order_.device != dev) {  // an event is recorded on its own device only
-    cudaEventDestroy(order_.last);
-    order_.last = nullptr;
+  if (last && device != dev) {  // an event is recorded on its own device only
+    cudaEventDestroy(last);
+    last = nullptr;
   }
-  if (!order_.last) {
-    if (cudaEventCreateWithFlags(&order_.last, cudaEventDisableTiming) != cudaSuccess) {
-      order_.last = nullptr;
-      cudaStreamSynchronize(s_);
+  if (!last) {
+    if (cudaEventCreateWithFlags(&last, cudaEventDisableTiming) != cudaSuccess) {
+      last = nullptr;
+      cudaStreamSynchronize(s);
       return;
     }
-    order_.device = dev;
+    device = dev;
   }
-  if (cudaEventRecord(order_.last, s_) != cudaSuccess) cudaStreamSynchronize(s_);
+  if (cudaEventRecord(last, s) != cudaSuccess) cudaStreamSynchronize(s);
 }
+
+// One set per host thread, so callers on different threads never share them.
+namespace {
+struct ThreadStaging {
+  DevBuf bufs[8];
+  LaunchOrder order;
+  int users = 0;  // Staging objects of the calls under way: one call may hold several
+};
+ThreadStaging& thread_staging() {
+  thread_local ThreadStaging t;
+  return t;
+}
+}  // namespace
+
+Staging::Staging(cudaStream_t s) : s_(s) {
+  ThreadStaging& t = thread_staging();
+  if (!t.users++) captured_ = t.order.begin(s);
+}
+
+Staging::~Staging() {
+  ThreadStaging& t = thread_staging();
+  if (!--t.users && !captured_) t.order.end(s_);
+}
+
+DevBuf& Staging::operator[](int slot) const { return thread_staging().bufs[slot & 7]; }
 
 // Host allocation hooks of the transcoder's state (host_alloc.h). Each allocation carries a
 // 16-byte header with the hooks that made it, so it is always freed by the same allocator.
@@ -131,13 +156,6 @@ struct alignas(16) AllocHeader {
   void* user;
 };
 }  // namespace
-
-// Staging buffers for host-memory calls; one set per host thread so concurrent callers on
-// different threads never share them.
-DevBuf& staging(int slot) {
-  thread_local DevBuf bufs[8];
-  return bufs[slot & 7];
-}
 
 void set_host_hooks(HostReallocFn realloc_fn, HostMsizeFn msize_fn, void* user) {
   std::lock_guard<std::mutex> lock(g_host_mu);

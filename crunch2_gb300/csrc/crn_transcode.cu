@@ -2864,9 +2864,10 @@ int unpack_one(UnpackContext* c, const uint8_t* host_src, const uint8_t* dev_src
   }
   LevelTask t = context_task(c, level);
   t.pitch = row_pitch;
+  const Staging staging(s);
   if (dev_src) { t.src = dev_src; t.src_size = src_size; }
   else if (host_src) {
-    DevBuf& sb = staging(2);
+    DevBuf& sb = staging[2];
     if ((e = sb.ensure(src_size + 64)) != cudaSuccess) return cuda_check(e, "alloc segment");
     if ((e = cudaMemcpyAsync(sb.ptr, host_src, src_size, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cuda_check(e, "copy segment");
@@ -2877,7 +2878,7 @@ int unpack_one(UnpackContext* c, const uint8_t* host_src, const uint8_t* dev_src
   if (mem == CRNGPU_MEM_DEVICE) {
     for (uint32_t f = 0; f < F.faces; f++) t.dst[f] = static_cast<uint8_t*>(dst_faces[f]);
   } else {
-    out_stage = &staging(1);
+    out_stage = &staging[1];
     if ((e = out_stage->ensure(face_bytes * F.faces)) != cudaSuccess) return cuda_check(e, "alloc output stage");
     for (uint32_t f = 0; f < F.faces; f++) t.dst[f] = static_cast<uint8_t*>(out_stage->ptr) + face_bytes * f;
     // rows may have pitch padding the transcoder does not write: keep the caller's bytes there
@@ -3032,8 +3033,9 @@ extern "C" int64_t crngpu_unpack_levels(crngpu_unpack_context ctx, uint32_t firs
   cudaError_t e;
   uint8_t* out = static_cast<uint8_t*>(dst);
   DevBuf* stage = nullptr;
+  const Staging staging(s);
   if (mem != CRNGPU_MEM_DEVICE) {
-    stage = &staging(1);
+    stage = &staging[1];
     if ((e = stage->ensure(total)) != cudaSuccess) return cuda_check(e, "alloc output stage");
     out = static_cast<uint8_t*>(stage->ptr);
   }

@@ -71,10 +71,6 @@ struct DevBuf {
   ~DevBuf() { release(); }
 };
 
-// Per-thread scratch for host-memory calls (input/output staging), slots 0..7: 0-3 the encoders,
-// 4-6 mip generation.
-DevBuf& staging(int slot);
-
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // True while work enqueued on `s` goes into a graph that the caller is capturing.
@@ -88,11 +84,16 @@ struct LaunchOrder {
   cudaEvent_t last = nullptr;  // after the latest launch
   int device = -1;             // of `last`
   ~LaunchOrder();
+  bool begin(cudaStream_t s);  // true if the launch is captured
+  void end(cudaStream_t s);    // for launches that are not
 };
 class OrderedLaunch {
  public:
-  OrderedLaunch(LaunchOrder& order, cudaStream_t s);
-  ~OrderedLaunch();
+  OrderedLaunch(LaunchOrder& order, cudaStream_t s) : lock_(order.mu), order_(order), s_(s), captured_(order.begin(s)) {}
+  ~OrderedLaunch() {
+    if (!captured_) order_.end(s_);
+  }
+  OrderedLaunch(const OrderedLaunch&) = delete;
   bool captured() const { return captured_; }
 
  private:
@@ -100,6 +101,22 @@ class OrderedLaunch {
   LaunchOrder& order_;
   cudaStream_t s_;
   bool captured_;
+};
+
+// The calling thread's device buffers for staged inputs and outputs and for what a call needs besides, slots
+// 0..7: 0-3 the encoders and the transcoder, 4-6 mip generation, 4-7 the plain chain encode. A call with
+// device buffers returns while its kernels still use them, so it holds a Staging until it has enqueued
+// everything; the thread's next call, on whatever stream, starts behind it on the device.
+class Staging {
+ public:
+  explicit Staging(cudaStream_t s);
+  ~Staging();
+  Staging(const Staging&) = delete;
+  DevBuf& operator[](int slot) const;
+
+ private:
+  cudaStream_t s_;
+  bool captured_ = false;
 };
 
 // Batched block encoding (many textures, mixed formats). A segment is one element of one texture

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <optional>
 #include <vector>
 
 #include "crngpu_internal.h"
@@ -97,8 +98,9 @@ int encode_device(const uint8_t* d_in, uint32_t n, uint32_t fmt, uint32_t flags,
           dxt1_options(perceptual, both, quality, gray, (flags & CRNGPU_FLAG_DXT1A) != 0, threshold);
       // try_alpha_as_black_optimization runs when 3-colour blocks are allowed (crn_dxt1.cpp:2239)
       const bool black = both && (flags & CRNGPU_FLAG_TRANSPARENT_BLACK);
+      std::optional<Staging> staging;  // until the trial is enqueued
       if (black && !d_err) {
-        DevBuf& be = staging(3);
+        DevBuf& be = staging.emplace(s)[3];
         cudaError_t e = be.ensure((size_t)n * 8);
         if (e != cudaSuccess) return cuda_check(e, "alloc error stage");
         d_err = static_cast<uint64_t*>(be.ptr);
@@ -135,9 +137,10 @@ int with_buffers(const uint8_t* in, size_t in_bytes, uint8_t* out, size_t out_by
     return fn(in, out, err);
   }
   cudaError_t e;
-  DevBuf& bi = staging(0);
-  DevBuf& bo = staging(1);
-  DevBuf& be = staging(3);
+  const Staging staging(s);
+  DevBuf& bi = staging[0];
+  DevBuf& bo = staging[1];
+  DevBuf& be = staging[3];
   if ((e = bi.ensure(in_bytes)) != cudaSuccess) return cuda_check(e, "alloc input stage");
   if ((e = bo.ensure(out_bytes)) != cudaSuccess) return cuda_check(e, "alloc output stage");
   if (err && (e = be.ensure(err_bytes)) != cudaSuccess) return cuda_check(e, "alloc error stage");
@@ -193,10 +196,11 @@ int64_t dds_plain_chain(const uint8_t* rgba_levels, uint32_t width, uint32_t hei
   if (!out || out_capacity < need) return (int64_t)need;
   cudaStream_t s = nullptr;
   cudaError_t e;
-  DevBuf& chain = staging(4);
-  DevBuf& table = staging(5);
-  DevBuf& gathered = staging(6);
-  DevBuf& encoded = staging(7);
+  const Staging staging(s);
+  DevBuf& chain = staging[4];
+  DevBuf& table = staging[5];
+  DevBuf& gathered = staging[6];
+  DevBuf& encoded = staging[7];
   if ((e = chain.ensure(src)) != cudaSuccess || (e = table.ensure(sizeof(GatherImage) * imgs.size())) != cudaSuccess ||
       (e = gathered.ensure((size_t)blocks * 64)) != cudaSuccess || (e = encoded.ensure(need)) != cudaSuccess)
     return cuda_check(e, "alloc chain buffers");
@@ -241,8 +245,9 @@ extern "C" int crngpu_dxt1_optimize_batch(const uint8_t* rgba_blocks, uint32_t n
   return with_buffers(rgba_blocks, (size_t)n * 64, out_blocks, (size_t)n * 8, out_error, (size_t)n * 8, mem, s,
                       [&](const uint8_t* in, uint8_t* out, uint64_t* err) {
                         uint64_t* e = err;
+                        std::optional<Staging> staging;  // until the trial is enqueued
                         if (black && !e) {
-                          DevBuf& be = staging(3);
+                          DevBuf& be = staging.emplace(s)[3];
                           cudaError_t ce = be.ensure((size_t)n * 8);
                           if (ce != cudaSuccess) return cuda_check(ce, "alloc error stage");
                           e = static_cast<uint64_t*>(be.ptr);
@@ -325,11 +330,12 @@ extern "C" int64_t crngpu_compress_image_ex(const uint8_t* rgba, uint32_t width,
   cudaStream_t s = as_stream(stream);
   cudaError_t e;
   const size_t img_bytes = (size_t)pitch_bytes * (height - 1) + (size_t)width * 4;
-  DevBuf& blocks = staging(2);
+  const Staging staging(s);
+  DevBuf& blocks = staging[2];
   if ((e = blocks.ensure(n * 64)) != cudaSuccess) return cuda_check(e, "alloc blocks");
   const uint8_t* d_img = rgba;
   if (mem != CRNGPU_MEM_DEVICE) {
-    DevBuf& bi = staging(0);
+    DevBuf& bi = staging[0];
     if ((e = bi.ensure(img_bytes)) != cudaSuccess) return cuda_check(e, "alloc image stage");
     if ((e = cudaMemcpyAsync(bi.ptr, rgba, img_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cuda_check(e, "copy image");
@@ -343,7 +349,7 @@ extern "C" int64_t crngpu_compress_image_ex(const uint8_t* rgba, uint32_t width,
   uint8_t* d_out = out;
   DevBuf* so = nullptr;
   if (mem != CRNGPU_MEM_DEVICE) {
-    so = &staging(1);
+    so = &staging[1];
     if ((e = so->ensure(need)) != cudaSuccess) return cuda_check(e, "alloc output stage");
     d_out = static_cast<uint8_t*>(so->ptr);
   } else if ((uintptr_t)out & 7) {

@@ -808,8 +808,9 @@ extern "C" int64_t crngpu_generate_mipmaps(const uint8_t* rgba, uint32_t width, 
   const uint64_t texels0 = (uint64_t)width * height;
   cudaError_t e;
   int rc;
-  DevBuf& tables = staging(4);
-  DevBuf& work = staging(5);
+  const Staging staging(s);
+  DevBuf& tables = staging[4];
+  DevBuf& work = staging[5];
   const size_t blob = plan ? plan->blob.size() : 0, o_lin = blob, o_srgb = o_lin + sizeof(gt.to_linear);
   const size_t tmp_bytes = plan ? plan->tmp * sizeof(float4) : 0;
   uint8_t* d_in = nullptr;
@@ -834,7 +835,7 @@ extern "C" int64_t crngpu_generate_mipmaps(const uint8_t* rgba, uint32_t width, 
   if (mem != CRNGPU_MEM_DEVICE) {
     if ((e = cudaMemcpyAsync(d_in, rgba, texels0 * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cuda_check(e, "copy level 0");
-    so = &staging(6);
+    so = &staging[6];
     if ((e = so->ensure(need)) != cudaSuccess) return cuda_check(e, "alloc mip output");
     d_out = static_cast<uint8_t*>(so->ptr);
   } else {

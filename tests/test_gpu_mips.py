@@ -83,3 +83,55 @@ def test_gpu_mips_of_large_images_match_oracle(cg, w, h, filt, scale, wrap):
     got = cg.generate_mipmaps(torch.from_numpy(img).cuda(), filt, scale, True, wrap, alpha=True, levels=levels)
     for l in range(1, levels):
         assert np.array_equal(got[l].cpu().numpy(), want[l] if len(want) == levels else want[l - 1]), l
+
+
+def delayed(stream):
+    """Keeps `stream` busy for some milliseconds, so that what is enqueued next waits there."""
+    with torch.cuda.stream(stream):
+        a = torch.zeros(1 << 28, dtype=torch.uint8, device="cuda")
+        for _ in range(40):
+            a.add_(1)
+
+
+def test_calls_on_two_streams_match_oracle(cg):
+    """Calls with device buffers return before their kernels have run: a second one of another size, from
+    the same thread on another stream, must leave the first one's tables and images alone."""
+    from oracle import mip_oracle
+    from crunch2_gb300 import texgen
+    sizes = [(203, 130), (66, 34), (330, 41)]
+    imgs = [torch.from_numpy(texgen.colour_texture(w, h, w, with_alpha_noise=True)).cuda() for w, h in sizes]
+    want = [mip_oracle.generate_mipmaps(i.cpu().numpy(), "kaiser", 0.9, True, False, alpha=True, levels=4) for i in imgs]
+    for i in imgs:
+        cg.generate_mipmaps(i, levels=4)  # plans made, buffers grown
+    streams = [torch.cuda.Stream() for _ in imgs]
+    torch.cuda.synchronize()
+    for rep in range(3):
+        delayed(streams[rep])
+        got = []
+        for k in range(3):
+            s = streams[(rep + k) % 3]
+            with torch.cuda.stream(s):
+                got.append(cg.generate_mipmaps(imgs[k], levels=4, stream=s))
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            assert all(np.array_equal(a.cpu().numpy(), b) for a, b in zip(g, w)), rep
+
+
+def test_image_encodes_on_two_streams(cg):
+    """The same for compress_image, whose gathered blocks are the thread's."""
+    from crunch2_gb300 import texgen
+    imgs = [torch.from_numpy(texgen.colour_texture(w, h, w, with_alpha_noise=True)).cuda()
+            for w, h in [(256, 128), (64, 44), (200, 180)]]
+    fmts = [cg.FMT_DXT5, cg.FMT_DXT1, cg.FMT_DXT5A]
+    want = [cg.compress_image(i, f) for i, f in zip(imgs, fmts)]
+    streams = [torch.cuda.Stream() for _ in imgs]
+    torch.cuda.synchronize()
+    for rep in range(3):
+        delayed(streams[rep])
+        got = []
+        for k in range(3):
+            s = streams[(rep + k) % 3]
+            with torch.cuda.stream(s):
+                got.append(cg.compress_image(imgs[k], fmts[k], stream=s))
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, w) for g, w in zip(got, want)), rep
