@@ -57,6 +57,7 @@ cudaError_t DevBuf::ensure(size_t bytes) {
   want = (want + want / 4 + 255) & ~(size_t)255;  // grow with headroom, 256-byte multiple
   e = cudaMalloc(&ptr, want);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here: not to the next launch that asks
     ptr = nullptr;
     cap = 0;
     return e;

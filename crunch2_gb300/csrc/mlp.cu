@@ -1035,9 +1035,11 @@ int ensure_batch(Net& net, int tiles) {
   cudaError_t e;
   if ((e = net.errflag.ensure(16)) != cudaSuccess) return cuda_check(e, "alloc flag");
   if (tiles <= net.cap) return CRNGPU_OK;
+  net.cap = 0;  // a buffer that does not get its memory has given up what it had
+  // the largest first, so that a batch that does not fit fails before it holds much
   struct { DevBuf* b; size_t bytes; } need[] = {
-      {&net.h1T, kTileT}, {&net.h2T, kTileT}, {&net.d1T, kTileT}, {&net.d2T, kTileT}, {&net.xT, kTileX},
-      {&net.dyT, kTileDy}, {&net.g1, kHid * BM * 4}, {&net.g2, kHid * BM * 4}, {&net.bias, kBiasSums * 4 * 4}};
+      {&net.g1, kHid * BM * 4}, {&net.g2, kHid * BM * 4}, {&net.h1T, kTileT}, {&net.h2T, kTileT}, {&net.d1T, kTileT},
+      {&net.d2T, kTileT}, {&net.xT, kTileX}, {&net.dyT, kTileDy}, {&net.bias, kBiasSums * 4 * 4}};
   for (auto& n : need)
     if ((e = n.b->ensure(n.bytes * (size_t)tiles)) != cudaSuccess) return cuda_check(e, "alloc training scratch");
   if ((e = net.part.ensure((size_t)std::min(tiles, kMaxSlices) * kGradCols * kHid * 4)) != cudaSuccess)

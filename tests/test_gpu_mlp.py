@@ -190,3 +190,17 @@ def test_training_steps_are_repeatable(L):
         states.append(net.state())
     for name in L.PARAM_NAMES:
         assert np.array_equal(states[0][name], states[1][name]), name
+
+
+def test_a_batch_that_does_not_fit_leaves_the_net_usable(L, batch):
+    """2^28 samples need more scratch than the device has: an error, and the smaller batches that fitted
+    before it fit again."""
+    blocks, targets = (torch.from_numpy(a).cuda() for a in batch)
+    net = L.EndpointNet(seed=5)
+    want = net.gradients(blocks, targets), net.get(2, grad=True)
+    loss = L.ctypes.c_float(0)
+    for call in (lambda n: net.L.crngpu_mlp_gradients(net.h, blocks.data_ptr(), targets.data_ptr(), n, loss, None),
+                 lambda n: net.L.crngpu_mlp_train_step(net.h, blocks.data_ptr(), targets.data_ptr(), n, 0.0, 0.0, loss, None)):
+        assert call(1 << 28) == -3  # CRNGPU_E_DEVICE
+        assert net.gradients(blocks, targets) == want[0]
+        assert np.array_equal(net.get(2, grad=True), want[1])
