@@ -1082,7 +1082,9 @@ struct Adam {
 
 // Loss and gradients of B samples, and with `adam` one AdamW step (betas 0.9/0.999, eps 1e-8); the
 // loss goes to errflag[1].
-int train_pass(Net& net, const uint8_t* blocks, const float* targets, int B, const Adam* adam, cudaStream_t s) {
+int train_pass(Net& net, const uint8_t* blocks, const float* targets, uint32_t n, const Adam* adam, cudaStream_t s) {
+  if (n > (1u << 28)) { set_error("training: at most 2^28 blocks per batch"); return CRNGPU_E_PARAM; }
+  const int B = (int)n;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1098,7 +1100,7 @@ int train_pass(Net& net, const uint8_t* blocks, const float* targets, int B, con
       attr_done[dev] = true;
     }
   }
-  const int tiles = (int)(((long long)B + BM - 1) / BM);
+  const int tiles = (B + BM - 1) / BM;
   int rc = ensure_batch(net, tiles);
   if (rc != CRNGPU_OK) return rc;
   auto f32 = [](DevBuf& b) { return static_cast<float*>(b.ptr); };
@@ -1271,7 +1273,7 @@ extern "C" int crngpu_mlp_gradients(void* h, const uint8_t* d_blocks, const floa
   Net* net = static_cast<Net*>(h);
   if (!net || net->magic != 0x4D4C5030u || !d_blocks || !d_targets || !n) return CRNGPU_E_PARAM;
   cudaStream_t s = as_stream(stream);
-  int rc = train_pass(*net, d_blocks, d_targets, (int)n, nullptr, s);
+  int rc = train_pass(*net, d_blocks, d_targets, n, nullptr, s);
   return rc != CRNGPU_OK ? rc : check_flag(*net, s, loss);
 } catch (...) {
   return crngpu::exception_status();
@@ -1285,7 +1287,7 @@ extern "C" int crngpu_mlp_train_step(void* h, const uint8_t* d_blocks, const flo
   if (!net || net->magic != 0x4D4C5030u || !d_blocks || !d_targets || !n) return CRNGPU_E_PARAM;
   cudaStream_t s = as_stream(stream);
   const Adam adam = {lr, weight_decay};
-  int rc = train_pass(*net, d_blocks, d_targets, (int)n, &adam, s);
+  int rc = train_pass(*net, d_blocks, d_targets, n, &adam, s);
   if (rc != CRNGPU_OK || (rc = check_flag(*net, s, loss)) != CRNGPU_OK) return rc;
   net->step++;
   return CRNGPU_OK;

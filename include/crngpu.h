@@ -370,11 +370,11 @@ CRNGPU_API int crngpu_mlp_make_targets(const uint8_t* d_blocks8, const uint64_t*
  * optimizer's error that holds for a fraction tau of blocks. Endpoint outputs keep squared error. */
 CRNGPU_API int crngpu_mlp_set_bound_loss(void* net, float tau, float weight);
 
-/* Loss gradients for a batch into the gradient buffers; *loss (host) gets the loss. */
+/* Loss gradients for a batch (n <= 2^28) into the gradient buffers; *loss (host) gets the loss. */
 CRNGPU_API int crngpu_mlp_gradients(void* net, const uint8_t* d_blocks, const float* d_targets, uint32_t n,
                                     float* loss, void* stream);
 
-/* One AdamW step (betas 0.9/0.999, eps 1e-8, decoupled weight decay) on a batch. */
+/* One AdamW step (betas 0.9/0.999, eps 1e-8, decoupled weight decay) on a batch (n <= 2^28). */
 CRNGPU_API int crngpu_mlp_train_step(void* net, const uint8_t* d_blocks, const float* d_targets, uint32_t n,
                                      float lr, float weight_decay, float* loss, void* stream);
 

@@ -204,3 +204,13 @@ def test_a_batch_that_does_not_fit_leaves_the_net_usable(L, batch):
         assert call(1 << 28) == -3  # CRNGPU_E_DEVICE
         assert net.gradients(blocks, targets) == want[0]
         assert np.array_equal(net.get(2, grad=True), want[1])
+
+
+@pytest.mark.parametrize("n", [(1 << 28) + 1, 0x80000000, 0xFFFFFF80, 0xFFFFFFFF])
+def test_batches_past_the_limit_are_refused(L, batch, n):
+    blocks, targets = (torch.from_numpy(a).cuda() for a in batch)
+    net = L.EndpointNet(seed=5)
+    loss = L.ctypes.c_float(0)
+    assert net.L.crngpu_mlp_gradients(net.h, blocks.data_ptr(), targets.data_ptr(), n, loss, None) == -1
+    assert net.L.crngpu_mlp_train_step(net.h, blocks.data_ptr(), targets.data_ptr(), n, 0.0, 0.0, loss, None) == -1
+    assert np.isfinite(net.gradients(blocks, targets))
