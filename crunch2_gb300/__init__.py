@@ -169,6 +169,8 @@ def lib():
     L.crngpu_force_wait_timeouts.restype = i32
     L.crngpu_set_decode_split.argtypes = [u32]
     L.crngpu_set_decode_split.restype = i32
+    L.crngpu_decode_counters.argtypes = [ctypes.POINTER(u64), i32]
+    L.crngpu_decode_counters.restype = i32
     _lib = L
     return L
 
@@ -203,15 +205,23 @@ def force_wait_timeouts(on: bool) -> None:
     _check(lib().crngpu_force_wait_timeouts(int(on)), "crngpu_force_wait_timeouts")
 
 
-DECODE_SPLIT_DEFAULT, DECODE_LANE_ONLY, DECODE_WIDE_ONLY = 0, 0xFFFFFFFF, 1
+DECODE_SPLIT_DEFAULT, DECODE_LANE_ONLY, DECODE_WIDE_ONLY, DECODE_WALK_ONLY = 0, 0xFFFFFFFF, 1, 0xFFFFFFFE
 
 
 def set_decode_split(min_blocks: int) -> None:
     """Which levels run on which decoder (crngpu_set_decode_split): DECODE_SPLIT_DEFAULT lets each plan
     pick the split over the walk, wide (CTA-per-level) and lane decoders with the shortest decode; a
     block count sends levels at least that large to the wide decoder; DECODE_LANE_ONLY /
-    DECODE_WIDE_ONLY force one decoder for every level. All give the same bytes."""
+    DECODE_WIDE_ONLY / DECODE_WALK_ONLY force one decoder for every level. All give the same bytes."""
     _check(lib().crngpu_set_decode_split(int(min_blocks) & 0xFFFFFFFF), "crngpu_set_decode_split")
+
+
+def decode_counters(reset: bool = False) -> dict:
+    """Level streams that unpack calls and new batches gave to each decoder, and the segments of the
+    walked ones, since the counts were last cleared (crngpu_decode_counters)."""
+    n = (ctypes.c_uint64 * 4)()
+    _check(lib().crngpu_decode_counters(n, int(reset)), "crngpu_decode_counters")
+    return dict(zip(("lane", "wide", "walk", "walk_segments"), map(int, n)))
 
 
 def _check(rc: int, where: str) -> int:

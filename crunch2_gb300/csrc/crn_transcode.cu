@@ -2252,6 +2252,7 @@ struct Plan {
   uint32_t wide_smem = 0;   // its dynamic shared memory (the largest format's layout)
   size_t wide_ofs = 0;
   uint32_t n_walk = 0;      // level streams for k_crn_decode_walk
+  uint32_t walk_segs = 0;   // their table segments
   uint32_t walk_steps = 0;  // its launches
   struct WalkStep { uint32_t jobs, builds, tiles; };  // jobs with work left, jobs building, their builder CTAs
   HVec<WalkStep> walk_step;
@@ -2270,10 +2271,20 @@ uint64_t level_records(const CrnFile& F, uint32_t l) {
   return (uint64_t)F.level[l].blocks_x * F.level[l].blocks_y * F.faces;
 }
 
-// Which level streams go to k_crn_decode_wide. 0 (the default): the split that minimises the
-// plan's decode time (decide_wide); otherwise levels of at least this many blocks (all faces) go
-// to the wide decoder. Set by crngpu_set_decode_split (tests force the wide or the lane decoder on every level).
+// Which decoder a level stream goes to. 0 (the default): the split that minimises the plan's decode
+// time (decide_decoders); kWalkOnly: the walk decoder for every level it can take; otherwise levels of
+// at least this many blocks (all faces) go to the wide decoder. Set by crngpu_set_decode_split (tests
+// force each decoder on every level).
 std::atomic<uint32_t> g_wide_min_blocks{0};
+constexpr uint32_t kWalkOnly = CRNGPU_DECODE_WALK;
+
+// Level streams that the plans in use gave to each decoder, and the walk's segments
+// (crngpu_decode_counters).
+std::atomic<uint64_t> g_decode_counts[4];
+void count_plan(const Plan& p) {
+  const uint32_t n[4] = {p.n_stream, p.n_wide, p.n_walk, p.walk_segs};
+  for (int i = 0; i < 4; i++) g_decode_counts[i].fetch_add(n[i], std::memory_order_relaxed);
+}
 
 // Decode cost model, in microseconds per block for a one-endpoint format (twice that for DXT5 and
 // DXN), measured on GB300: the lane decoder's serial chain and one wide CTA's phase loop.
@@ -2316,6 +2327,11 @@ enum Decoder : uint8_t { kLane = 0, kWide = 1, kWalk = 2 };
 HVec<uint8_t> decide_decoders(const HVec<LevelTask>& tasks, uint32_t wide_slots, bool walk) {
   HVec<uint8_t> to(tasks.size(), (uint8_t)kLane);
   const uint32_t fixed = g_wide_min_blocks.load(std::memory_order_relaxed);
+  if (fixed == kWalkOnly) {
+    for (size_t i = 0; i < tasks.size(); i++)
+      if (walk && walk_eligible(tasks[i])) to[i] = kWalk;
+    return to;
+  }
   if (fixed) {
     for (size_t i = 0; i < tasks.size(); i++)
       if (wide_eligible(tasks[i]) && task_blocks(tasks[i]) >= fixed) to[i] = kWide;
@@ -2393,6 +2409,7 @@ void plan_walk(HVec<WalkJob>& jobs, Plan& p) {
     w.seg = w.cap - kWalkHalo;
     w.segs = w.bits / w.seg + 1;
     p.walk_steps = std::max(p.walk_steps, w.segs + 3);
+    p.walk_segs += w.segs;
     const bool two = record_bytes(w.j.kind) == 8u;
     w.anchors = reinterpret_cast<uint32_t*>(take((uint64_t)sh.rows / 2 * (sh.ge + sh.go) * 4));
     w.blocks = reinterpret_cast<uint32_t*>(take((uint64_t)sh.rows * sh.W * (two ? 8 : 4)));
@@ -2768,6 +2785,7 @@ int run_levels(UnpackContext* c, HVec<LevelTask>& tasks, cudaStream_t s) {
   if ((e = cudaMemcpyAsync(c->d_jobs.ptr, p.image.data(), p.image.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
     return cuda_check(e, "copy jobs");
   uint32_t* words = static_cast<uint32_t*>(c->d_status.ptr);
+  count_plan(p);
   int rc = enqueue_plan(p, static_cast<const uint8_t*>(c->d_jobs.ptr), words, s);
   if (rc != CRNGPU_OK) return rc;
   // the reference reports a bad stream through its bool result; read the status word back
@@ -3103,6 +3121,7 @@ extern "C" crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
   uint32_t grid = 0;
   size_t smem = 0;
   if (decode_grid(b->plan, &grid, &smem) != CRNGPU_OK) return nullptr;
+  count_plan(b->plan);
   return reinterpret_cast<crngpu_unpack_batch>(b.release());
 } catch (...) {
   crngpu::exception_status();
@@ -3232,6 +3251,17 @@ extern "C" int64_t crngpu_unpack_batch_bytes(crngpu_unpack_batch batch) try {
 extern "C" int crngpu_set_decode_split(uint32_t min_blocks) try {
   clear_error();
   g_wide_min_blocks.store(min_blocks, std::memory_order_relaxed);
+  return CRNGPU_OK;
+} catch (...) {
+  return crngpu::exception_status();
+}
+
+extern "C" int crngpu_decode_counters(uint64_t out[4], int reset) try {
+  clear_error();
+  if (!out) { set_error("NULL output"); return CRNGPU_E_PARAM; }
+  for (int i = 0; i < 4; i++)
+    out[i] = reset ? g_decode_counts[i].exchange(0, std::memory_order_relaxed)
+                   : g_decode_counts[i].load(std::memory_order_relaxed);
   return CRNGPU_OK;
 } catch (...) {
   return crngpu::exception_status();

@@ -494,10 +494,17 @@ CRNGPU_API int64_t crngpu_unpack_batch_bytes(crngpu_unpack_batch batch);
  * min_blocks = 0 (the default): each plan sends its largest levels to the walk decoder and the next to
  * the wide one as long as that shortens the plan's decode (a cost model of the three decoders and the
  * device's resident wide CTAs); a single texture's large levels are walked, a batch of many textures
- * mostly stays on the lane decoder. Otherwise levels of at least min_blocks blocks (all faces) go wide: 1 sends every
+ * mostly stays on the lane decoder. CRNGPU_DECODE_WALK: every level with rows of at most 1024 blocks
+ * is walked. Otherwise levels of at least min_blocks blocks (all faces) go wide: 1 sends every
  * level with rows of at most 1024 blocks, 0xFFFFFFFF none. Applies to plans built after the call:
  * contexts' unpack calls and batches created afterwards. */
+#define CRNGPU_DECODE_WALK 0xFFFFFFFEu
 CRNGPU_API int crngpu_set_decode_split(uint32_t min_blocks);
+
+/* Which decoders the plans really used: out[0..2] = level streams that unpack calls and new batches gave
+ * to the lane, the wide and the walk decoder since the counts were last cleared, out[3] = the segments
+ * that the walked streams were cut into. reset != 0 clears them. Process-wide. */
+CRNGPU_API int crngpu_decode_counters(uint64_t out[4], int reset);
 
 CRNGPU_API int crngpu_unpack_batch_destroy(crngpu_unpack_batch batch);
 

@@ -5,6 +5,8 @@ streams cut short or overwritten (the status and every byte that the two write).
 import numpy as np
 import pytest
 
+import golden_util as G
+
 pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
@@ -150,3 +152,73 @@ def test_launches_on_two_streams(cg):
                 assert all(torch.equal(x, y) for x, y in zip(g, want)), graph
     for c in ctxs:
         c.close()
+
+
+# What follows runs the walk decoder whatever the cost model would choose, and checks that it ran.
+
+@pytest.fixture
+def walk_only(cg):
+    cg.set_decode_split(cg.DECODE_WALK_ONLY)
+    cg.decode_counters(reset=True)
+    yield
+    cg.set_decode_split(cg.DECODE_SPLIT_DEFAULT)
+
+
+@pytest.mark.parametrize("name", sorted(G.manifest().keys()))
+def test_walk_alone_writes_golden_levels(cg, walk_only, name):
+    """Every level of every fixture, 1 x 1 ones and cube faces included, one at a time and all in one plan."""
+    m = G.manifest()[name]
+    with cg.unpack_begin(G.crn_bytes(name)) as ctx:
+        for lvl, info in enumerate(m["levels"]):
+            assert G.sha(ctx.unpack_levels(lvl, 1)) == info["sha256"], (name, lvl)
+        allv = ctx.unpack_levels()
+    pos = 0
+    for lvl, info in enumerate(m["levels"]):
+        assert G.sha(allv[pos:pos + info["bytes"]]) == info["sha256"], (name, lvl, "all levels")
+        pos += info["bytes"]
+    n = cg.decode_counters()
+    assert (n["lane"], n["wide"], n["walk"]) == (0, 0, 2 * len(m["levels"]))
+
+
+# rows of 1, 2, 3, 8, 9, 10, 13 and 1024 blocks: every remainder of the groups of eight, the smallest and
+# the widest; the large ones over many segments
+@pytest.mark.parametrize("fmt,w,h,segments", [
+    ("dxt1", 4, 4, 1), ("dxt5", 8, 12, 1), ("dxn", 12, 100, 1), ("dxt5a", 32, 32, 1), ("dxt5", 36, 60, 1),
+    ("dxn", 40, 64, 1), ("dxt1", 52, 44, 1), ("dxt1", 4096, 64, 2), ("dxt5", 1024, 768, 9), ("dxn", 1000, 600, 5),
+    ("dxt1", 1024, 768, 5)])
+def test_walk_alone_matches_lane(cg, walk_only, fmt, w, h, segments):
+    crn = make(cg, fmt, w, h, w + h, levels=1, quality=255)
+    lane = decode(cg, crn, cg.DECODE_LANE_ONLY)
+    cg.decode_counters(reset=True)
+    walk = decode(cg, crn, cg.DECODE_WALK_ONLY)
+    n = cg.decode_counters()
+    assert (n["lane"], n["wide"], n["walk"]) == (0, 0, 1) and n["walk_segments"] >= segments, n
+    assert lane[0] == walk[0] == 0 and np.array_equal(walk[1], lane[1])
+
+
+@pytest.mark.parametrize("name", ["dxt1_256", "dxt5_256", "dxn_xy_256", "dxt5a_256", "dxt5_cube_64x32"])
+def test_walk_alone_on_corrupt_streams(cg, walk_only, name):
+    """Random bytes over a level's stream: the lane decoder's status, or its bytes where it still decodes."""
+    import struct
+    crn = bytes(G.crn_bytes(name))
+    nlev = len(G.manifest()[name]["levels"])
+    ofs = [struct.unpack(">I", crn[70 + 4 * l:74 + 4 * l])[0] for l in range(nlev)] + [len(crn)]
+    rng = np.random.default_rng(12)
+    for trial in range(16):
+        lvl = trial % 2
+        bad = bytearray(crn)
+        pos = ofs[lvl] + int(rng.integers(0, max(1, ofs[lvl + 1] - ofs[lvl] - 16)))
+        n = int(min(32, ofs[lvl + 1] - pos))
+        bad[pos:pos + n] = rng.integers(0, 256, n, dtype=np.uint8).tobytes()
+        lane = decode(cg, bytes(bad), cg.DECODE_LANE_ONLY, 2)
+        cg.decode_counters(reset=True)
+        walk = decode(cg, bytes(bad), cg.DECODE_WALK_ONLY, 2)
+        assert cg.decode_counters()["walk"] == 2
+        assert walk[0] == lane[0] and (lane[0] or np.array_equal(walk[1], lane[1])), (name, trial)
+
+
+def test_default_split_walks_a_large_level(cg):
+    cg.decode_counters(reset=True)
+    code, _ = decode(cg, make(cg, "dxt1", 1024, 1024, 3, levels=1), cg.DECODE_SPLIT_DEFAULT)
+    n = cg.decode_counters()
+    assert code == 0 and n["walk"] == 1 and n["walk_segments"] > 3, n
