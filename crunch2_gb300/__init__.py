@@ -169,6 +169,8 @@ def lib():
     L.crngpu_force_wait_timeouts.restype = i32
     L.crngpu_set_decode_split.argtypes = [u32]
     L.crngpu_set_decode_split.restype = i32
+    L.crngpu_set_decode_scratch.argtypes = [u64]
+    L.crngpu_set_decode_scratch.restype = i32
     L.crngpu_decode_counters.argtypes = [ctypes.POINTER(u64), i32]
     L.crngpu_decode_counters.restype = i32
     _lib = L
@@ -214,6 +216,12 @@ def set_decode_split(min_blocks: int) -> None:
     block count sends levels at least that large to the wide decoder; DECODE_LANE_ONLY /
     DECODE_WIDE_ONLY / DECODE_WALK_ONLY force one decoder for every level. All give the same bytes."""
     _check(lib().crngpu_set_decode_split(int(min_blocks) & 0xFFFFFFFF), "crngpu_set_decode_split")
+
+
+def set_decode_scratch(most_bytes: int | None = None) -> None:
+    """The most device scratch a plan's walk decoder may take (crngpu_set_decode_scratch); None: no limit."""
+    _check(lib().crngpu_set_decode_scratch((1 << 64) - 1 if most_bytes is None else int(most_bytes)),
+           "crngpu_set_decode_scratch")
 
 
 def decode_counters(reset: bool = False) -> dict:

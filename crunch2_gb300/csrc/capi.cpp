@@ -56,6 +56,10 @@ cudaError_t DevBuf::ensure(size_t bytes) {
   size_t want = bytes < 256 ? 256 : bytes;
   want = (want + want / 4 + 255) & ~(size_t)255;  // grow with headroom, 256-byte multiple
   e = cudaMalloc(&ptr, want);
+  if (e == cudaErrorMemoryAllocation) {
+    trim_decode_pool(dev);
+    e = cudaMalloc(&ptr, want);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();  // reported here: not to the next launch that asks
     ptr = nullptr;

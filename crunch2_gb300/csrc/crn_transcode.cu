@@ -2717,8 +2717,31 @@ int status_to_rc(uint32_t st) {
 }
 
 // The walk decoder's scratch of one call: stream-ordered memory from a per-device pool, given back
-// in stream order. The pool keeps at most kWalkPoolBytes between calls.
+// in stream order. The pool keeps at most kWalkPoolBytes between calls, which go back to the device when
+// another buffer of the library finds no memory (trim_decode_pool) or by crngpu_set_decode_scratch.
 constexpr uint64_t kWalkPoolBytes = 128ull << 20;
+std::atomic<cudaMemPool_t> g_walk_pools[64];
+std::atomic<uint64_t> g_walk_scratch_most{~0ull};  // a plan that would need more does not walk
+
+cudaMemPool_t walk_pool(int dev) {
+  cudaMemPool_t pool = g_walk_pools[dev].load();
+  if (pool) return pool;
+  std::lock_guard<std::mutex> lock(device_setup_mutex());
+  if ((pool = g_walk_pools[dev].load())) return pool;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  uint64_t keep = kWalkPoolBytes;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  g_walk_pools[dev].store(pool);
+  return pool;
+}
+
 struct WalkScratch {
   cudaStream_t s;
   void* ptr = nullptr;
@@ -2727,36 +2750,33 @@ struct WalkScratch {
   ~WalkScratch() {
     if (ptr) cudaFreeAsync(ptr, s);
   }
-  int get(uint64_t bytes) {
-    static cudaMemPool_t pools[64] = {};
+  uint8_t* get(uint64_t bytes) {  // null: there is none
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return cuda_check(e, "cudaGetDevice");
-    if (dev < 0 || dev >= 64) { set_error("device index out of range"); return CRNGPU_E_PARAM; }
-    cudaMemPool_t pool;
-    {
-      std::lock_guard<std::mutex> lock(device_setup_mutex());
-      if (!pools[dev]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t made;
-        if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess) return cuda_check(e, "create decode pool");
-        uint64_t keep = kWalkPoolBytes;
-        if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
-          return cuda_check(e, "decode pool attribute");
-        pools[dev] = made;
-      }
-      pool = pools[dev];
-    }
-    if ((e = cudaMallocFromPoolAsync(&ptr, bytes, pool, s)) != cudaSuccess) {
+    cudaMemPool_t pool = nullptr;
+    if (bytes > g_walk_scratch_most.load() || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 ||
+        !(pool = walk_pool(dev)))
+      return nullptr;
+    if (cudaMallocFromPoolAsync(&ptr, bytes, pool, s) != cudaSuccess) {
+      cudaGetLastError();
       ptr = nullptr;
-      return cuda_check(e, "alloc decode scratch");
     }
-    return CRNGPU_OK;
+    return static_cast<uint8_t*>(ptr);
   }
 };
+
+// make_plan with its walk's scratch from get(bytes), or, if there is none, without the walk decoder: the
+// others need no scratch, so a call never fails for want of it.
+template <class Get>
+bool make_placed_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots, Get get) {
+  if (!make_plan(tasks, p, wide_slots, true)) return false;
+  if (!p.n_walk) return true;
+  if (uint8_t* at = get(p.walk_bytes)) {
+    place_walk(p, at);
+    return true;
+  }
+  p = Plan();
+  return make_plan(tasks, p, wide_slots, false);
+}
 
 // Decodes and expands a list of levels of one context (destinations device memory), then
 // reads the status word back (synchronises `s`).
@@ -2775,11 +2795,10 @@ int run_levels(UnpackContext* c, HVec<LevelTask>& tasks, cudaStream_t s) {
   uint32_t slots = 0;
   int rc0 = wide_slots(&slots);
   if (rc0 != CRNGPU_OK) return rc0;
-  if (!make_plan(tasks, p, slots, true)) { set_error("too many levels in one texture job"); return CRNGPU_E_PARAM; }
   WalkScratch scratch(s);
-  if (p.n_walk) {
-    if ((rc0 = scratch.get(p.walk_bytes)) != CRNGPU_OK) return rc0;
-    place_walk(p, static_cast<uint8_t*>(scratch.ptr));
+  if (!make_placed_plan(tasks, p, slots, [&](uint64_t bytes) { return scratch.get(bytes); })) {
+    set_error("too many levels in one texture job");
+    return CRNGPU_E_PARAM;
   }
   if ((e = c->d_jobs.ensure(p.image.size() + 16)) != cudaSuccess) return cuda_check(e, "alloc jobs");
   if ((e = cudaMemcpyAsync(c->d_jobs.ptr, p.image.data(), p.image.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
@@ -2943,6 +2962,10 @@ void levels_tasks(UnpackContext* c, uint32_t first, uint32_t count, uint8_t* out
 
 }  // namespace
 
+void trim_decode_pool(int dev) {
+  if (cudaMemPool_t pool = g_walk_pools[dev & 63].load()) cudaMemPoolTrimTo(pool, 0);
+}
+
 // Test hook for the expansion's staging waits: polls per wait (drains are not affected).
 int set_expand_wait_polls(uint32_t polls) {
   return cuda_check(cudaMemcpyToSymbol(g_expand_wait_polls, &polls, sizeof(polls)), "set expansion wait polls");
@@ -3105,10 +3128,16 @@ extern "C" crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
   for (LevelTask& t : tasks) t.rec = static_cast<uint8_t*>(b->d_records.ptr) + reinterpret_cast<uintptr_t>(t.rec);
   uint32_t slots = 0;
   if (wide_slots(&slots) != CRNGPU_OK) return nullptr;
-  if (!make_plan(tasks, b->plan, slots, true)) { set_error("too many levels in one batch item"); return nullptr; }
-  if (b->plan.n_walk) {
-    if ((e = b->d_walk.ensure(b->plan.walk_bytes)) != cudaSuccess) { cuda_check(e, "alloc decode scratch"); return nullptr; }
-    place_walk(b->plan, static_cast<uint8_t*>(b->d_walk.ptr));
+  if ((e = b->d_words.ensure(16)) != cudaSuccess) { cuda_check(e, "alloc status"); return nullptr; }
+  if (!make_placed_plan(tasks, b->plan, slots, [&](uint64_t bytes) -> uint8_t* {
+        // the job tables before the scratch, which can be done without
+        if (bytes > g_walk_scratch_most.load() || b->d_jobs.ensure(b->plan.image.size() + 16) != cudaSuccess ||
+            b->d_walk.ensure(bytes) != cudaSuccess)
+          return nullptr;
+        return static_cast<uint8_t*>(b->d_walk.ptr);
+      })) {
+    set_error("too many levels in one batch item");
+    return nullptr;
   }
   if ((e = b->d_jobs.ensure(b->plan.image.size() + 16)) != cudaSuccess) { cuda_check(e, "alloc jobs"); return nullptr; }
   if ((e = cudaMemcpy(b->d_jobs.ptr, b->plan.image.data(), b->plan.image.size(), cudaMemcpyHostToDevice)) !=
@@ -3116,7 +3145,6 @@ extern "C" crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
     cuda_check(e, "copy jobs");
     return nullptr;
   }
-  if ((e = b->d_words.ensure(16)) != cudaSuccess) { cuda_check(e, "alloc status"); return nullptr; }
   // resolve the decoder's launch shape (and its shared-memory attribute) outside any capture
   uint32_t grid = 0;
   size_t smem = 0;
@@ -3251,6 +3279,20 @@ extern "C" int64_t crngpu_unpack_batch_bytes(crngpu_unpack_batch batch) try {
 extern "C" int crngpu_set_decode_split(uint32_t min_blocks) try {
   clear_error();
   g_wide_min_blocks.store(min_blocks, std::memory_order_relaxed);
+  return CRNGPU_OK;
+} catch (...) {
+  return crngpu::exception_status();
+}
+
+extern "C" int crngpu_set_decode_scratch(uint64_t most_bytes) try {
+  clear_error();
+  g_walk_scratch_most.store(most_bytes);
+  for (auto& slot : g_walk_pools)
+    if (cudaMemPool_t pool = slot.load()) {
+      uint64_t keep = std::min<uint64_t>(kWalkPoolBytes, most_bytes);
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaMemPoolTrimTo(pool, keep);
+    }
   return CRNGPU_OK;
 } catch (...) {
   return crngpu::exception_status();

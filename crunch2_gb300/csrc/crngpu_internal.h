@@ -61,6 +61,9 @@ std::mutex& device_setup_mutex();
 // Records `what` + the CUDA error string and returns CRNGPU_E_DEVICE when e != cudaSuccess.
 int cuda_check(cudaError_t e, const char* what);
 
+// Gives the device the memory that the transcoder's pool holds without using it.
+void trim_decode_pool(int dev);
+
 // A device buffer owned by the library; grows on demand, never shrinks.
 struct DevBuf {
   void* ptr = nullptr;

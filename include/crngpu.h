@@ -501,6 +501,13 @@ CRNGPU_API int64_t crngpu_unpack_batch_bytes(crngpu_unpack_batch batch);
 #define CRNGPU_DECODE_WALK 0xFFFFFFFEu
 CRNGPU_API int crngpu_set_decode_split(uint32_t min_blocks);
 
+/* The walk decoder needs device scratch (tables, anchors and decoded blocks: about 5 MB for a large level)
+ * for the time of a call, or of a batch's life. A plan that would need more than most_bytes (the
+ * default is no limit), or whose scratch cannot be allocated, uses the other decoders, which need none;
+ * 0 turns the walk decoder off. Unpack calls keep at most 128 MB of scratch between calls; this call gives
+ * back what is unused of it above most_bytes. */
+CRNGPU_API int crngpu_set_decode_scratch(uint64_t most_bytes);
+
 /* Which decoders the plans really used: out[0..2] = level streams that unpack calls and new batches gave
  * to the lane, the wide and the walk decoder since the counts were last cleared, out[3] = the segments
  * that the walked streams were cut into. reset != 0 clears them. Process-wide. */

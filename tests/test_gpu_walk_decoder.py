@@ -222,3 +222,34 @@ def test_default_split_walks_a_large_level(cg):
     code, _ = decode(cg, make(cg, "dxt1", 1024, 1024, 3, levels=1), cg.DECODE_SPLIT_DEFAULT)
     n = cg.decode_counters()
     assert code == 0 and n["walk"] == 1 and n["walk_segments"] > 3, n
+
+
+@pytest.mark.parametrize("most", [0, 1 << 20])
+def test_plans_without_scratch_use_the_other_decoders(cg, most):
+    """What a failed allocation of the walk's scratch does too: unpack calls, calls by level and batches."""
+    names = ["c1_dxt1_1024", "dxt5_2048", "dxn_xy_2048"]
+    man = G.manifest()
+    cg.set_decode_scratch(most)
+    try:
+        cg.decode_counters(reset=True)
+        ctxs = [cg.unpack_begin(G.crn_bytes(n)) for n in names]
+        outs = [torch.zeros(sum(l["bytes"] for l in man[n]["levels"]), dtype=torch.uint8, device="cuda") for n in names]
+        with cg.UnpackBatch([(c, 0, c.levels, o) for c, o in zip(ctxs, outs)]) as b:
+            b.launch()
+            b.status()
+        for n, c, o in zip(names, ctxs, outs):
+            got = [o.cpu().numpy(), c.unpack_levels()]
+            pos = 0
+            for lvl, info in enumerate(man[n]["levels"]):
+                for g in got:
+                    assert G.sha(g[pos:pos + info["bytes"]]) == info["sha256"], (n, lvl)
+                pos += info["bytes"]
+                assert G.sha(c.unpack_level(lvl).reshape(-1)) == info["sha256"], (n, lvl)
+            c.close()
+        assert cg.decode_counters()["walk"] == 0
+    finally:
+        cg.set_decode_scratch(None)
+    cg.decode_counters(reset=True)
+    with cg.unpack_begin(G.crn_bytes(names[0])) as c:
+        c.unpack_levels()
+    assert cg.decode_counters()["walk"] > 0
