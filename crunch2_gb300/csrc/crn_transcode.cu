@@ -33,7 +33,18 @@
 namespace crngpu {
 
 // Device status word values (written by k_crn_decode_textures, read back by the host).
-enum : uint32_t { kStOk = 0, kStBadCode = 1, kStBadIndex = 2, kStWait = 3 };
+enum : uint32_t { kStOk = 0, kStBadCode = 1, kStBadIndex = 2 };
+
+// Waits for bulk copies into shared memory (the walk's table windows, the expansion's index records) are
+// bounded: one that runs out is counted in g_expand_stage_timeouts, and its kernel goes on without the
+// copies, with the same output. Copies still in flight when a CTA is done are drained with a separate,
+// much longer bound that the test hook does not change; a drain that runs out is counted in
+// g_expand_drain_failures.
+constexpr uint32_t kExpandWaitLimit = 1u << 22;
+constexpr uint32_t kExpandDrainPolls = 1u << 26;
+__device__ uint32_t g_expand_wait_polls = kExpandWaitLimit;
+__device__ unsigned int g_expand_stage_timeouts;
+__device__ unsigned int g_expand_drain_failures;
 
 // Model slots in a context's device model array.
 enum { kMRef = 0, kMEp0 = 1, kMSel0 = 2, kMEp1 = 3, kMSel1 = 4, kNumModels = 5 };
@@ -1061,19 +1072,6 @@ __device__ __forceinline__ void wide_level(const StreamJob& J, WideShared& S, ui
   if (tid == 0 && S.bad) atomicMax(status, (S.bad & 1u) ? (uint32_t)kStBadCode : (uint32_t)kStBadIndex);
 }
 
-// One CTA per large level stream (`jobs`, largest first).
-__global__ void __launch_bounds__(kWThreads, 1) k_crn_decode_wide(const StreamJob* __restrict__ jobs,
-                                                               uint32_t* __restrict__ status) {
-  __shared__ WideShared S;
-  const StreamJob J = jobs[blockIdx.x];
-  switch (J.kind) {
-    case kKDxt1: wide_level<kKDxt1>(J, S, status); break;
-    case kKDxt5: wide_level<kKDxt5>(J, S, status); break;
-    case kKDxn: wide_level<kKDxn>(J, S, status); break;
-    default: wide_level<kKDxt5a>(J, S, status); break;
-  }
-}
-
 // ------------------------------------------------------------------------------------------
 // The largest levels of a plan: k_crn_decode_walk, many CTAs per level stream.
 //
@@ -1112,7 +1110,8 @@ constexpr uint32_t kWalkPosBits = 28;      // anchors: position | combination <<
 // A level's progress between launches (zero at the start).
 struct WalkState {
   uint32_t p, groups;                      // the walk: position, groups passed
-  uint32_t rows, carry, bad, pad;          // the resolver: rows resolved, running indices; 1: bad code, 2: bad index
+  uint32_t rows, carry, bad;               // the resolver: rows resolved, running indices; 1: bad code, 2: bad index
+  uint32_t gave_up;                        // the launch in which a wait of the walk ran out, or 0
   uint32_t passed[kWalkMaxSegments + 1];   // groups passed after each segment
   uint32_t bits[kWMaxW / 32];              // the current even row's combinations, a byte per four chunks
 };
@@ -1281,16 +1280,16 @@ __device__ __forceinline__ void walk_build(const WalkJob& job, WalkShared& S, ui
 }
 
 // ---- the walk over segment k: thread 0 of the CTA, with thread 32 bringing the windows of the
-// tables by bulk copies up to three windows ahead (every wait is bounded; one that runs out ends
-// the walk with an error). A step's chain is a shared-memory load and the addition that gives the
+// tables by bulk copies up to three windows ahead. A wait that runs out ends the level's walk: the
+// launches after it leave the level alone, and k_crn_decode_wide decodes it. A step's chain is a shared-memory load and the addition that gives the
 // next load's address; the loop's own instructions (test, stores) cost as much as the chain unless
 // groups go in fours. Measured on the 1024 x 1024 DXT1 level, cycles per step: 124 with cp.async by
 // the other warps, a barrier per window and a test per group; 103 with bulk copies issued by the
 // walking thread and groups in fours; 72 so.
-constexpr uint32_t kWalkWaitLimit = 1u << 22;
-__device__ __forceinline__ bool walk_wait(uint32_t bar, uint32_t parity, const volatile uint32_t* walking = nullptr) {
+__device__ __forceinline__ bool walk_wait(uint32_t bar, uint32_t parity, uint32_t polls,
+                                          const volatile uint32_t* walking = nullptr) {
   uint32_t done = 0;
-  for (uint32_t i = 0; i < kWalkWaitLimit && !done && !(walking && !*walking); i++)
+  for (uint32_t i = 0; i < polls && !done && !(walking && !*walking); i++)
     asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                  : "=r"(done)
                  : "r"(bar), "r"(parity)
@@ -1309,12 +1308,12 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
 }
 
 template <bool REM>
-__device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t* status) {
+__device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, uint32_t k) {
   using R = WalkRing<REM>;
   const StreamJob& J = job.j;
   const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
   WalkState& st = *job.st;
-  const uint32_t tid = threadIdx.x, base = k * job.seg;
+  const uint32_t tid = threadIdx.x, base = k * job.seg, polls = g_expand_wait_polls;
   if (tid < kWMaxW / 32) S.bits[tid] = st.bits[tid];
   const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(wide_smem);
   const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
@@ -1336,10 +1335,8 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     uint32_t w = 0;
     for (; w < staged && *walking; w++) {
       const uint32_t slot = w & (R::kSlots - 1), bar = full + 8 * slot;
-      if (w >= R::kSlots && !walk_wait(empty + 8 * slot, (w / R::kSlots - 1) & 1u, walking)) {
-        if (*walking) atomicMax(status, (uint32_t)kStWait);
-        break;
-      }
+      // (if the walk does not come on, it is left without windows, and its own wait runs out)
+      if (w >= R::kSlots && !walk_wait(empty + 8 * slot, (w / R::kSlots - 1) & 1u, polls, walking)) break;
       const bool mirror = slot == 0 && w > 0;
       constexpr uint32_t kBytes = R::kWindow * (REM ? 28u : 20u);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(mirror ? 2 * kBytes : kBytes)
@@ -1357,9 +1354,10 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
         if (!mirror) break;
       }
     }
-    // the last copies of each slot
+    // the last copies of each slot land before the CTA exits
     for (uint32_t v = w > R::kSlots ? w - R::kSlots : 0u; v < w; v++)
-      if (!walk_wait(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u)) atomicMax(status, (uint32_t)kStWait);
+      if (!walk_wait(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u, kExpandDrainPolls))
+        atomicAdd(&g_expand_drain_failures, 1u);
   }
   if (tid) return;
   // (the row and the place in it from the number of groups, which bounds what is written whatever p says)
@@ -1372,9 +1370,9 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     const uint2* RM = reinterpret_cast<const uint2*>(wide_smem + R::kRem);
     const uint32_t left = job.bits > base ? job.bits - base : 0u;  // positions before the end of the stream
     uint32_t* out = job.anchors + groups;
-    bool ok = walk_wait(full, 0u);
+    bool ok = walk_wait(full, 0u, polls);
     for (uint32_t w = 0; w < windows && ok && r < sh.rows; w++) {
-      if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u);
+      if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u, polls);
       if (!ok) break;
       const uint32_t lim = min(min((w + 1) * R::kWindow, job.seg), left);
       // four groups of chunks may start while the last of them starts inside window w + 1
@@ -1461,7 +1459,10 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * (w & (R::kSlots - 1))) : "memory");
     }
     *(volatile uint32_t*)&S.walking = 0u;
-    if (!ok) atomicMax(status, (uint32_t)kStWait);
+    if (!ok) {
+      atomicAdd(&g_expand_stage_timeouts, 1u);
+      st.gave_up = k + 1;
+    }
     if (k + 1 == job.segs && ok && r < sh.rows) {
       // the stream has ended (a corrupt or truncated one): every further group starts in its zeros
       const uint32_t zero = (uint32_t)(job.c4[buf + left] >> 16) & 255u;
@@ -1760,10 +1761,16 @@ __device__ __forceinline__ void walk_resolve_rows(const WalkJob& job, WalkShared
   else walk_resolve<TWO, 8>(job, S, k, status);
 }
 
+__device__ __forceinline__ bool walk_gave_up(const WalkJob& job, uint32_t step) {
+  const uint32_t at = job.st->gave_up;
+  return at && at < step;
+}
+
 // Launch `step` of a plan, over the first n jobs (the ones with work left; jobs are ordered by their
 // number of segments): CTAs [0, n) walk segment step - 1 of their level, [n, 2n) resolve rows from
 // segment step - 3, [2n, 2n + n * parts) decode the groups of segment step - 2, the others build
-// tables of segment `step` of the first nb jobs.
+// tables of segment `step` of the first nb jobs. A level that gave up in an earlier launch is left alone
+// (one that does in this launch may be read either way: what its CTAs do is then of no use, but no harm).
 __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJob* __restrict__ jobs, uint32_t n,
                                                                      uint32_t nb, uint32_t parts, uint32_t step,
                                                                      uint32_t* status) {
@@ -1772,15 +1779,15 @@ __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJ
   if (b < n) {
     const WalkJob job = jobs[b];
     const uint32_t k = step - 1;
-    if (step < 1 || k >= job.segs) return;
-    if (job.rem) walk_segment<true>(job, S, k, status); else walk_segment<false>(job, S, k, status);
+    if (step < 1 || k >= job.segs || walk_gave_up(job, step)) return;
+    if (job.rem) walk_segment<true>(job, S, k); else walk_segment<false>(job, S, k);
     return;
   }
   b -= n;
   if (b < n) {
     const WalkJob job = jobs[b];
     const uint32_t k = step - 3;
-    if (step < 3 || k >= job.segs) return;
+    if (step < 3 || k >= job.segs || walk_gave_up(job, step)) return;
     if (record_bytes(job.j.kind) == 8u) walk_resolve_rows<true>(job, S, k, status); else walk_resolve_rows<false>(job, S, k, status);
     return;
   }
@@ -1788,7 +1795,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJ
   if (b < n * parts) {
     const WalkJob job = jobs[b / parts];
     const uint32_t k = step - 2, part = b % parts;
-    if (step < 2 || k >= job.segs) return;
+    if (step < 2 || k >= job.segs || walk_gave_up(job, step)) return;
     switch (job.j.kind) {
       case kKDxt1: walk_decode<kKDxt1>(job, S, k, part, parts); break;
       case kKDxt5: walk_decode<kKDxt5>(job, S, k, part, parts); break;
@@ -1805,6 +1812,22 @@ __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJ
   }
   const WalkJob job = jobs[lo];
   if (step < job.segs) walk_build(job, S, step, b - job.tile0);
+}
+
+// One CTA per large level stream (`jobs`, n of them, largest first), then one per walked level, which has
+// nothing to do unless a wait of that level's walk ran out: then it decodes the level.
+__global__ void __launch_bounds__(kWThreads, 1) k_crn_decode_wide(const StreamJob* __restrict__ jobs, uint32_t n,
+                                                               const WalkJob* __restrict__ walked,
+                                                               uint32_t* __restrict__ status) {
+  __shared__ WideShared S;
+  if (blockIdx.x >= n && !walked[blockIdx.x - n].st->gave_up) return;
+  const StreamJob J = blockIdx.x < n ? jobs[blockIdx.x] : walked[blockIdx.x - n].j;
+  switch (J.kind) {
+    case kKDxt1: wide_level<kKDxt1>(J, S, status); break;
+    case kKDxt5: wide_level<kKDxt5>(J, S, status); break;
+    case kKDxn: wide_level<kKDxn>(J, S, status); break;
+    default: wide_level<kKDxt5a>(J, S, status); break;
+  }
 }
 
 // Palette entry index, clamped so that records left unwritten by a stream the decoder rejected
@@ -1888,14 +1911,7 @@ __device__ __forceinline__ void narrow_emit(const ExpandJob& J, uint32_t first, 
 // before it belong to the previous face of the same buffer) and ends at its last record rounded
 // down to 16 bytes; the up to three records after that are read from global memory. Waits are
 // bounded: a CTA whose wait runs out reads its records from global memory from then on (same
-// output) and counts the event in g_expand_stage_timeouts. Copies still in flight when the CTA is
-// done are drained with a separate, much longer bound (kExpandDrainPolls) that the test hook does
-// not change; a drain that runs out is counted in g_expand_drain_failures.
-constexpr uint32_t kExpandWaitLimit = 1u << 22;
-constexpr uint32_t kExpandDrainPolls = 1u << 26;
-__device__ uint32_t g_expand_wait_polls = kExpandWaitLimit;
-__device__ unsigned int g_expand_stage_timeouts;
-__device__ unsigned int g_expand_drain_failures;
+// output).
 
 __device__ __forceinline__ uint32_t shared_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -2524,6 +2540,7 @@ bool make_plan(const HVec<LevelTask>& tasks, Plan& p, uint32_t wide_slots, bool 
   std::stable_sort(walks.begin(), walks.end(), [](const WalkJob& a, const WalkJob& b) { return a.bits > b.bits; });
   plan_walk(walks, p);
   for (const StreamJob& j : wide) p.wide_smem = std::max(p.wide_smem, wide_layout(models_used(j.kind)).total);
+  for (const WalkJob& w : walks) p.wide_smem = std::max(p.wide_smem, wide_layout(models_used(w.j.kind)).total);
   // largest textures first: the persistent warps then finish at about the same time
   HVec<size_t> order(items.size());
   for (size_t i = 0; i < order.size(); i++) order[i] = i;
@@ -2685,9 +2702,10 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_crn_decode_walk");
   }
-  if (decode && p.n_wide) {
+  if (decode && p.n_wide + p.n_walk) {
     const StreamJob* wj = reinterpret_cast<const StreamJob*>(d_jobs + p.wide_ofs);
-    k_crn_decode_wide<<<p.n_wide, kWThreads, p.wide_smem, s>>>(wj, words + 1);
+    const WalkJob* kj = reinterpret_cast<const WalkJob*>(d_jobs + p.walk_ofs);
+    k_crn_decode_wide<<<p.n_wide + p.n_walk, kWThreads, p.wide_smem, s>>>(wj, p.n_wide, kj, words + 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_crn_decode_wide");
   }
   if (decode && p.n_item) {
@@ -2710,7 +2728,6 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
 
 int status_to_rc(uint32_t st) {
   if (!st) return CRNGPU_OK;
-  if (st == kStWait) { set_error("a wait of the transcoder timed out"); return CRNGPU_E_DEVICE; }
   set_error(st == kStBadCode ? "corrupt block stream (no such prefix code)"
                              : "corrupt block stream (palette index out of range)");
   return CRNGPU_E_CORRUPT;

@@ -253,3 +253,43 @@ def test_plans_without_scratch_use_the_other_decoders(cg, most):
     with cg.unpack_begin(G.crn_bytes(names[0])) as c:
         c.unpack_levels()
     assert cg.decode_counters()["walk"] > 0
+
+
+@pytest.fixture
+def waits_run_out(cg, walk_only):
+    cg.wait_counters(reset=True)
+    cg.force_wait_timeouts(True)
+    yield
+    cg.force_wait_timeouts(False)
+
+
+@pytest.mark.parametrize("name", ["c1_dxt1_1024", "dxt5_256", "dxn_xy_256", "dxt5a_256", "dxt1_100x60", "dxt5_cube_64x32"])
+def test_levels_whose_walk_gives_up_are_decoded_all_the_same(cg, waits_run_out, name):
+    levels = G.manifest()[name]["levels"]
+    with cg.unpack_begin(G.crn_bytes(name)) as ctx:
+        out = torch.zeros(sum(l["bytes"] for l in levels), dtype=torch.uint8, device="cuda")
+        with cg.UnpackBatch([(ctx, 0, len(levels), out)]) as b:
+            b.set_variant(0)  # an expansion without waits of its own
+            for use_graph in (False, True):
+                for forced in (True, False):
+                    out.zero_()
+                    cg.force_wait_timeouts(forced)
+                    cg.wait_counters(reset=True)
+                    b.launch(use_graph=use_graph)
+                    b.status()
+                    n = cg.wait_counters()
+                    assert n["expand_stage_timeouts"] == (len(levels) if forced else 0), n
+                    assert n["expand_drain_failures"] == 0, n
+                    host, pos = out.cpu().numpy(), 0
+                    for lvl, info in enumerate(levels):
+                        assert G.sha(host[pos:pos + info["bytes"]]) == info["sha256"], (lvl, use_graph, forced)
+                        pos += info["bytes"]
+
+
+def test_a_walk_that_gives_up_keeps_the_status_of_a_corrupt_stream(cg, waits_run_out):
+    crn = bytearray(make(cg, "dxt1", 256, 256, 9, levels=1))
+    crn[len(crn) - len(crn) // 3:] = b"\xff" * (len(crn) // 3)
+    lane = decode(cg, bytes(crn), cg.DECODE_LANE_ONLY)
+    walk = decode(cg, bytes(crn), cg.DECODE_WALK_ONLY)
+    assert cg.wait_counters()["expand_stage_timeouts"] > 0
+    assert walk[0] == lane[0] and (lane[0] or np.array_equal(walk[1], lane[1]))
