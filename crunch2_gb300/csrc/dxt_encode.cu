@@ -2150,7 +2150,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kSeedCtasPerSm)
 
 // Phase 2 of the batched encode: persistent warps walk the chunk table, a block at a time, taken as in
 // k_dxt1_encode (block k of chunk c is number kColourChunkBlocks c + k; a short chunk's last numbers
-// have none). Without `next` in turn: for launches that may run beside others of the same batch.
+// have none). kCounter = false: in turn, for launches that may run beside others of the same batch (a kernel
+// of its own: the choice made in one cost the search 0.5 %).
+template <bool kCounter>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
     k_dxt1_encode_chunks(const uint8_t* __restrict__ blocks, const EncodeChunk* __restrict__ chunks, uint32_t nchunks,
                          const EncodeSegment* __restrict__ segs, const Seed* __restrict__ seeds,
@@ -2161,7 +2163,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
   const uint32_t nwarps = gridDim.x * kWarpsPerCta;
   #pragma unroll 1
   for (uint32_t i = warp_global; i / kColourChunkBlocks < nchunks;) {
-    const uint32_t after = take(next, next != nullptr);
+    const uint32_t after = kCounter ? take(next, true) : 0;
     const EncodeChunk ch = chunks[i / kColourChunkBlocks];
     if (i % kColourChunkBlocks < ch.count) {
       const EncodeSegment sg = segs[ch.segment];
@@ -2170,7 +2172,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm)
       phase2_block<false>(S, blocks + (size_t)b * 64, sg.options, sg.out + (size_t)(b - sg.first_block) * sg.stride,
                           nullptr, nullptr);
     }
-    i = next ? nwarps + __shfl_sync(FULL_MASK, after, 0) : i + nwarps;
+    i = kCounter ? nwarps + __shfl_sync(FULL_MASK, after, 0) : i + nwarps;
   }
 }
 
@@ -2317,7 +2319,8 @@ int dxt1_launch_setup(int dev, Dxt1Launch* L) {
     cudaError_t e = cudaSuccess;
     for (auto search : {k_dxt1_encode<false, kCtasPerSm>, k_dxt1_encode<false, kFewCtasPerSm>, k_dxt1_encode<true, kCtasPerSm>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_dxt1_encode_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    for (auto search : {k_dxt1_encode_chunks<true>, k_dxt1_encode_chunks<false>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_dxt1_seeds<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, seed_smem);
     if (e == cudaSuccess)
@@ -2413,7 +2416,7 @@ int dxt1_chunks_max_grid() {
   cudaGetDevice(&dev);
   Dxt1Launch L;
   if (dxt1_launch_setup(dev, &L) != CRNGPU_OK) return -1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dxt1_encode_chunks, kWarpsPerCta * 32, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dxt1_encode_chunks<true>, kWarpsPerCta * 32, smem);
   return L.sms * (per_sm < 1 ? 1 : per_sm);
 }
 
@@ -2440,8 +2443,9 @@ int launch_dxt1_chunks(const uint8_t* d_blocks, const EncodeChunk* d_chunks, uin
   Seed* seeds = static_cast<Seed*>(d_seeds);
   k_dxt1_seeds_chunks<<<seed_grid, kWarpsPerCta * 32, sizeof(SeedShared) * kWarpsPerCta, s>>>(d_blocks, d_chunks, nchunks,
                                                                                            d_segs, seeds, d_next);
-  k_dxt1_encode_chunks<<<grid, kWarpsPerCta * 32, sizeof(WarpShared) * kWarpsPerCta, s>>>(d_blocks, d_chunks, nchunks,
-                                                                                         d_segs, seeds, d_next);
+  const auto search = d_next ? k_dxt1_encode_chunks<true> : k_dxt1_encode_chunks<false>;
+  search<<<grid, kWarpsPerCta * 32, sizeof(WarpShared) * kWarpsPerCta, s>>>(d_blocks, d_chunks, nchunks, d_segs, seeds,
+                                                                           d_next);
   return cuda_check(cudaGetLastError(), "launch k_dxt1_seeds_chunks / k_dxt1_encode_chunks");
 }
 
