@@ -1116,6 +1116,10 @@ struct WalkState {
   uint32_t bits[kWMaxW / 32];              // the current even row's combinations, a byte per four chunks
 };
 
+// A level whose walk gave up in a launch before launch `step` is left alone by walk, decoders and resolver.
+// (Not one that gives up in this very launch, whatever of that is seen: all threads have to agree.)
+__device__ __forceinline__ bool walk_gave_up(uint32_t gave_up, uint32_t step) { return gave_up && gave_up < step; }
+
 struct WalkJob {
   StreamJob j;
   uint4* o4;          // two buffers of `cap` entries
@@ -1281,15 +1285,15 @@ __device__ __forceinline__ void walk_build(const WalkJob& job, WalkShared& S, ui
 
 // ---- the walk over segment k: thread 0 of the CTA, with thread 32 bringing the windows of the
 // tables by bulk copies up to three windows ahead. A wait that runs out ends the level's walk: the
-// launches after it leave the level alone, and k_crn_decode_wide decodes it. A step's chain is a shared-memory load and the addition that gives the
+// launches after it leave the level alone, and another decoder decodes it. A step's chain is a shared-memory load and the addition that gives the
 // next load's address; the loop's own instructions (test, stores) cost as much as the chain unless
 // groups go in fours. Measured on the 1024 x 1024 DXT1 level, cycles per step: 124 with cp.async by
 // the other warps, a barrier per window and a test per group; 103 with bulk copies issued by the
 // walking thread and groups in fours; 72 so.
-__device__ __forceinline__ bool walk_wait(uint32_t bar, uint32_t parity, uint32_t polls,
-                                          const volatile uint32_t* walking = nullptr) {
+template <uint32_t kPolls = kExpandWaitLimit>
+__device__ __forceinline__ bool walk_wait(uint32_t bar, uint32_t parity, const volatile uint32_t* walking = nullptr) {
   uint32_t done = 0;
-  for (uint32_t i = 0; i < polls && !done && !(walking && !*walking); i++)
+  for (uint32_t i = 0; i < kPolls && !done && !(walking && !*walking); i++)
     asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                  : "=r"(done)
                  : "r"(bar), "r"(parity)
@@ -1308,13 +1312,16 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
 }
 
 template <bool REM>
-__device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, uint32_t k) {
+__device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t* given_up) {
   using R = WalkRing<REM>;
   const StreamJob& J = job.j;
   const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
   WalkState& st = *job.st;
-  const uint32_t tid = threadIdx.x, base = k * job.seg, polls = g_expand_wait_polls;
-  if (tid < kWMaxW / 32) S.bits[tid] = st.bits[tid];
+  const uint32_t tid = threadIdx.x, base = k * job.seg;
+  // (the state in one round trip)
+  const uint32_t gave_up = st.gave_up, p0 = st.p, g0 = st.groups, bits0 = tid < kWMaxW / 32 ? st.bits[tid] : 0u;
+  if (walk_gave_up(gave_up, k + 1)) return;
+  if (tid < kWMaxW / 32) S.bits[tid] = bits0;
   const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(wide_smem);
   const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
   const uint32_t windows = (job.seg + R::kWindow - 1) / R::kWindow, staged = job.cap / R::kWindow;
@@ -1324,7 +1331,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8 * i));
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
-    S.walking = st.groups < sh.rows / 2 * (sh.ge + sh.go) ? 1u : 0u;
+    S.walking = g0 < sh.rows / 2 * (sh.ge + sh.go) ? 1u : 0u;
   }
   __syncthreads();
   const size_t buf = (size_t)(k & 1u) * job.cap;
@@ -1336,7 +1343,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     for (; w < staged && *walking; w++) {
       const uint32_t slot = w & (R::kSlots - 1), bar = full + 8 * slot;
       // (if the walk does not come on, it is left without windows, and its own wait runs out)
-      if (w >= R::kSlots && !walk_wait(empty + 8 * slot, (w / R::kSlots - 1) & 1u, polls, walking)) break;
+      if (w >= R::kSlots && !walk_wait(empty + 8 * slot, (w / R::kSlots - 1) & 1u, walking)) break;
       const bool mirror = slot == 0 && w > 0;
       constexpr uint32_t kBytes = R::kWindow * (REM ? 28u : 20u);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(mirror ? 2 * kBytes : kBytes)
@@ -1356,12 +1363,12 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     }
     // the last copies of each slot land before the CTA exits
     for (uint32_t v = w > R::kSlots ? w - R::kSlots : 0u; v < w; v++)
-      if (!walk_wait(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u, kExpandDrainPolls))
+      if (!walk_wait<kExpandDrainPolls>(full + 8 * (v & (R::kSlots - 1)), (v / R::kSlots) & 1u))
         atomicAdd(&g_expand_drain_failures, 1u);
   }
   if (tid) return;
   // (the row and the place in it from the number of groups, which bounds what is written whatever p says)
-  uint32_t r, e, q = st.p - base, groups = st.groups;
+  uint32_t r, e, q = p0 - base, groups = g0;
   walk_group(sh, groups, r, e);
   if (r < sh.rows) {
     const uint8_t* bits = reinterpret_cast<const uint8_t*>(S.bits);
@@ -1370,9 +1377,10 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     const uint2* RM = reinterpret_cast<const uint2*>(wide_smem + R::kRem);
     const uint32_t left = job.bits > base ? job.bits - base : 0u;  // positions before the end of the stream
     uint32_t* out = job.anchors + groups;
-    bool ok = walk_wait(full, 0u, polls);
+    // (the hook's bound is for this first wait: read in the loop it cost 60 cycles a window)
+    bool ok = g_expand_wait_polls && walk_wait(full, 0u);
     for (uint32_t w = 0; w < windows && ok && r < sh.rows; w++) {
-      if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u, polls);
+      if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u);
       if (!ok) break;
       const uint32_t lim = min(min((w + 1) * R::kWindow, job.seg), left);
       // four groups of chunks may start while the last of them starts inside window w + 1
@@ -1461,6 +1469,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     *(volatile uint32_t*)&S.walking = 0u;
     if (!ok) {
       atomicAdd(&g_expand_stage_timeouts, 1u);
+      atomicAdd(given_up, 1u);
       st.gave_up = k + 1;
     }
     if (k + 1 == job.segs && ok && r < sh.rows) {
@@ -1501,8 +1510,8 @@ __device__ __forceinline__ void walk_decode(const WalkJob& job, WalkShared& S, u
   constexpr bool two = KIND == kKDxt5 || KIND == kKDxn, five = KIND == kKDxt5;
   constexpr uint32_t sDB = five ? 3u : 1u, sSB = five ? 4u : 2u;
   const StreamJob& J = job.j;
-  const uint32_t g0 = k ? job.st->passed[k - 1] : 0u, g1 = job.st->passed[k];
-  if (g0 + part * kWalkThreads >= g1) return;
+  const uint32_t gave_up = job.st->gave_up, g0 = k ? job.st->passed[k - 1] : 0u, g1 = job.st->passed[k];
+  if (walk_gave_up(gave_up, k + 2) || g0 + part * kWalkThreads >= g1) return;
   const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
   uint32_t* luts = reinterpret_cast<uint32_t*>(wide_smem);
   walk_stage_models(J, luts, S);
@@ -1586,9 +1595,10 @@ __device__ __forceinline__ void walk_resolve(const WalkJob& job, WalkShared& S, 
   const StreamJob& J = job.j;
   const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
   WalkState& st = *job.st;
-  const uint32_t passed = st.passed[k], pairs = passed / (sh.ge + sh.go);
+  const uint32_t gave_up = st.gave_up, passed = st.passed[k], pairs = passed / (sh.ge + sh.go);
   const uint32_t ready = 2 * pairs + (passed - pairs * (sh.ge + sh.go) >= sh.ge ? 1u : 0u);
   uint32_t r = st.rows;
+  if (walk_gave_up(gave_up, k + 3)) return;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, W = sh.W;
   const uint32_t nA = J.n_a, nB = J.n_b, nSA = J.n_sa, nSB = J.n_sb;
   const uint32_t x0 = tid * kPer;  // rows are even: a pair of blocks is inside or outside
@@ -1761,33 +1771,27 @@ __device__ __forceinline__ void walk_resolve_rows(const WalkJob& job, WalkShared
   else walk_resolve<TWO, 8>(job, S, k, status);
 }
 
-__device__ __forceinline__ bool walk_gave_up(const WalkJob& job, uint32_t step) {
-  const uint32_t at = job.st->gave_up;
-  return at && at < step;
-}
-
 // Launch `step` of a plan, over the first n jobs (the ones with work left; jobs are ordered by their
 // number of segments): CTAs [0, n) walk segment step - 1 of their level, [n, 2n) resolve rows from
 // segment step - 3, [2n, 2n + n * parts) decode the groups of segment step - 2, the others build
-// tables of segment `step` of the first nb jobs. A level that gave up in an earlier launch is left alone
-// (one that does in this launch may be read either way: what its CTAs do is then of no use, but no harm).
+// tables of segment `step` of the first nb jobs.
 __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJob* __restrict__ jobs, uint32_t n,
                                                                      uint32_t nb, uint32_t parts, uint32_t step,
-                                                                     uint32_t* status) {
+                                                                     uint32_t* status /* and levels given up */) {
   __shared__ WalkShared S;
   uint32_t b = blockIdx.x;
   if (b < n) {
     const WalkJob job = jobs[b];
     const uint32_t k = step - 1;
-    if (step < 1 || k >= job.segs || walk_gave_up(job, step)) return;
-    if (job.rem) walk_segment<true>(job, S, k); else walk_segment<false>(job, S, k);
+    if (step < 1 || k >= job.segs) return;
+    if (job.rem) walk_segment<true>(job, S, k, status + 1); else walk_segment<false>(job, S, k, status + 1);
     return;
   }
   b -= n;
   if (b < n) {
     const WalkJob job = jobs[b];
     const uint32_t k = step - 3;
-    if (step < 3 || k >= job.segs || walk_gave_up(job, step)) return;
+    if (step < 3 || k >= job.segs) return;
     if (record_bytes(job.j.kind) == 8u) walk_resolve_rows<true>(job, S, k, status); else walk_resolve_rows<false>(job, S, k, status);
     return;
   }
@@ -1795,7 +1799,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJ
   if (b < n * parts) {
     const WalkJob job = jobs[b / parts];
     const uint32_t k = step - 2, part = b % parts;
-    if (step < 2 || k >= job.segs || walk_gave_up(job, step)) return;
+    if (step < 2 || k >= job.segs) return;
     switch (job.j.kind) {
       case kKDxt1: walk_decode<kKDxt1>(job, S, k, part, parts); break;
       case kKDxt5: walk_decode<kKDxt5>(job, S, k, part, parts); break;
@@ -1814,8 +1818,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) k_crn_decode_walk(const WalkJ
   if (step < job.segs) walk_build(job, S, step, b - job.tile0);
 }
 
-// One CTA per large level stream (`jobs`, n of them, largest first), then one per walked level, which has
-// nothing to do unless a wait of that level's walk ran out: then it decodes the level.
+// One CTA per large level stream (`jobs`, n of them, largest first), then (batches) one per walked level,
+// which has nothing to do unless a wait of that level's walk ran out: then it decodes the level.
 __global__ void __launch_bounds__(kWThreads, 1) k_crn_decode_wide(const StreamJob* __restrict__ jobs, uint32_t n,
                                                                const WalkJob* __restrict__ walked,
                                                                uint32_t* __restrict__ status) {
@@ -2166,7 +2170,7 @@ struct UnpackContext : HostObject {
   CrnFile file;
   DevBuf d_file, d_models, d_pal, d_jobs, d_records, d_status;
   DevPalettes pal{};
-  uint32_t status_host[2] = {0, 0};
+  uint32_t status_host[3] = {0, 0, 0};
   // every level decoded at minimal pitch by the first unpack_level call (0: not tried yet,
   // 1: holds every level, 2: not used for this context)
   DevBuf d_level_cache;
@@ -2673,9 +2677,11 @@ int decode_grid(const Plan& p, uint32_t* grid, size_t* smem) {
 }
 
 // Enqueues the counter/status clear, the decoder and the expansion for a plan whose image is
-// already at d_jobs. `words` = 2 device words: [0] work counter, [1] status. Asynchronous.
-int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStream_t s, bool decode = true,
-                 int variant = -1) {
+// already at d_jobs. `words` = device words: [0] work counter, [1] status, [2] (plans that walk) levels whose
+// walk gave up. Asynchronous. `stand_in`: those levels are decoded behind the walk; without it the caller
+// reads words[2] and sees to them (the launch that nearly never does anything is 5 us).
+int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStream_t s, bool stand_in,
+                 bool decode = true, int variant = -1) {
   if ((size_t)(p.lut_words + p.rb_words) * 4 > kDecodeSmemMax) {
     set_error("texture rows too wide for the decoder");
     return CRNGPU_E_PARAM;
@@ -2689,7 +2695,7 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
   const StreamJob* sj = reinterpret_cast<const StreamJob*>(d_jobs + p.stream_ofs);
   const ExpandJob* ej = reinterpret_cast<const ExpandJob*>(d_jobs + p.expand_ofs);
   if (decode && (p.n_item || p.n_wide || p.n_walk)) {
-    if ((e = cudaMemsetAsync(words, 0, 8, s)) != cudaSuccess) return cuda_check(e, "clear work counter");
+    if ((e = cudaMemsetAsync(words, 0, p.n_walk ? 12 : 8, s)) != cudaSuccess) return cuda_check(e, "clear work counter");
   }
   if (decode && p.n_walk) {
     const WalkJob* kj = reinterpret_cast<const WalkJob*>(d_jobs + p.walk_ofs);
@@ -2702,10 +2708,11 @@ int enqueue_plan(const Plan& p, const uint8_t* d_jobs, uint32_t* words, cudaStre
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_crn_decode_walk");
   }
-  if (decode && p.n_wide + p.n_walk) {
+  const uint32_t walked = stand_in ? p.n_walk : 0;
+  if (decode && p.n_wide + walked) {
     const StreamJob* wj = reinterpret_cast<const StreamJob*>(d_jobs + p.wide_ofs);
     const WalkJob* kj = reinterpret_cast<const WalkJob*>(d_jobs + p.walk_ofs);
-    k_crn_decode_wide<<<p.n_wide + p.n_walk, kWThreads, p.wide_smem, s>>>(wj, p.n_wide, kj, words + 1);
+    k_crn_decode_wide<<<p.n_wide + walked, kWThreads, p.wide_smem, s>>>(wj, p.n_wide, kj, words + 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_check(e, "launch k_crn_decode_wide");
   }
   if (decode && p.n_item) {
@@ -2808,27 +2815,31 @@ int run_levels(UnpackContext* c, HVec<LevelTask>& tasks, cudaStream_t s) {
     t.rec = static_cast<uint8_t*>(c->d_records.ptr) + ofs;
     ofs += (level_records(c->file, t.level) * c->rec_bytes() + 15) & ~(uint64_t)15;
   }
-  Plan p;
   uint32_t slots = 0;
-  int rc0 = wide_slots(&slots);
-  if (rc0 != CRNGPU_OK) return rc0;
-  WalkScratch scratch(s);
-  if (!make_placed_plan(tasks, p, slots, [&](uint64_t bytes) { return scratch.get(bytes); })) {
-    set_error("too many levels in one texture job");
-    return CRNGPU_E_PARAM;
-  }
-  if ((e = c->d_jobs.ensure(p.image.size() + 16)) != cudaSuccess) return cuda_check(e, "alloc jobs");
-  if ((e = cudaMemcpyAsync(c->d_jobs.ptr, p.image.data(), p.image.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-    return cuda_check(e, "copy jobs");
-  uint32_t* words = static_cast<uint32_t*>(c->d_status.ptr);
-  count_plan(p);
-  int rc = enqueue_plan(p, static_cast<const uint8_t*>(c->d_jobs.ptr), words, s);
+  int rc = wide_slots(&slots);
   if (rc != CRNGPU_OK) return rc;
-  // the reference reports a bad stream through its bool result; read the status word back
-  if ((e = cudaMemcpyAsync(c->status_host, words, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-    return cuda_check(e, "read status");
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
-  return status_to_rc(c->status_host[1]);
+  WalkScratch scratch(s);
+  uint32_t* words = static_cast<uint32_t*>(c->d_status.ptr);
+  for (bool walk = true;; walk = false) {
+    Plan p;
+    if (!(walk ? make_placed_plan(tasks, p, slots, [&](uint64_t bytes) { return scratch.get(bytes); })
+               : make_plan(tasks, p, slots, false))) {
+      set_error("too many levels in one texture job");
+      return CRNGPU_E_PARAM;
+    }
+    if ((e = c->d_jobs.ensure(p.image.size() + 16)) != cudaSuccess) return cuda_check(e, "alloc jobs");
+    if ((e = cudaMemcpyAsync(c->d_jobs.ptr, p.image.data(), p.image.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+      return cuda_check(e, "copy jobs");
+    count_plan(p);
+    if ((rc = enqueue_plan(p, static_cast<const uint8_t*>(c->d_jobs.ptr), words, s, false)) != CRNGPU_OK) return rc;
+    // the reference reports a bad stream through its bool result; read the status word back
+    c->status_host[2] = 0;
+    if ((e = cudaMemcpyAsync(c->status_host, words, p.n_walk ? 12 : 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+      return cuda_check(e, "read status");
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
+    if (!c->status_host[2]) return status_to_rc(c->status_host[1]);
+    // a wait of a walk ran out: everything again, by the other decoders
+  }
 }
 
 LevelTask context_task(UnpackContext* c, uint32_t level) {
@@ -3185,7 +3196,7 @@ extern "C" int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t fl
   if (b->variant < 0) {
     // autotuner: decode once, then time every expansion variant on the real records (each writes
     // the same, correct output) and keep the fastest for this batch and as the device default
-    int rc = enqueue_plan(b->plan, jobs, words, s, true, 0);
+    int rc = enqueue_plan(b->plan, jobs, words, s, true, true, 0);
     if (rc != CRNGPU_OK) return rc;
     cudaEvent_t ev[2];
     cudaError_t e;
@@ -3197,7 +3208,7 @@ extern "C" int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t fl
       float tot = 0.f;
       for (int rep = 0; rep < 3; rep++) {
         cudaEventRecord(ev[0], s);
-        if ((rc = enqueue_plan(b->plan, jobs, words, s, false, v)) != CRNGPU_OK) break;
+        if ((rc = enqueue_plan(b->plan, jobs, words, s, true, false, v)) != CRNGPU_OK) break;
         cudaEventRecord(ev[1], s);
         cudaEventSynchronize(ev[1]);
         float ms = 0.f;
@@ -3217,10 +3228,10 @@ extern "C" int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t fl
   }
   if (flags & CRNGPU_BATCH_EXPAND_ONLY) {
     if (!b->decoded) { set_error("no decode has run on this batch"); return CRNGPU_E_PARAM; }
-    return enqueue_plan(b->plan, jobs, words, s, false, b->variant);
+    return enqueue_plan(b->plan, jobs, words, s, true, false, b->variant);
   }
   b->decoded = true;
-  if (!(flags & CRNGPU_BATCH_GRAPH)) return enqueue_plan(b->plan, jobs, words, s, true, b->variant);
+  if (!(flags & CRNGPU_BATCH_GRAPH)) return enqueue_plan(b->plan, jobs, words, s, true, true, b->variant);
   cudaError_t e;
   if (!b->graph) {
     // capture on a private stream (the legacy default stream cannot be captured), then replay
@@ -3231,7 +3242,7 @@ extern "C" int crngpu_unpack_batch_launch(crngpu_unpack_batch batch, uint32_t fl
       cudaStreamDestroy(cap);
       return cuda_check(e, "begin capture");
     }
-    int rc = enqueue_plan(b->plan, jobs, words, cap, true, b->variant);
+    int rc = enqueue_plan(b->plan, jobs, words, cap, true, true, b->variant);
     e = cudaStreamEndCapture(cap, &g);
     cudaStreamDestroy(cap);
     if (rc != CRNGPU_OK) { if (g) cudaGraphDestroy(g); return rc; }
@@ -3493,7 +3504,7 @@ extern "C" int crngpu_unpack_level_noalloc(const void* crn_data, uint32_t crn_si
       return cuda_check(e, "copy into the fixed scratch");
   }
   uint32_t* words = reinterpret_cast<uint32_t*>(base);
-  if ((rc = enqueue_plan(p, base + o_jobs, words, s)) != CRNGPU_OK) return rc;
+  if ((rc = enqueue_plan(p, base + o_jobs, words, s, false)) != CRNGPU_OK) return rc;
   uint32_t st[2] = {0, 0};
   if ((e = cudaMemcpyAsync(st, words, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_check(e, "read status");
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");

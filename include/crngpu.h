@@ -75,7 +75,7 @@ CRNGPU_API int crngpu_profile_counters(int enable, uint64_t* dxt1_evaluations, v
 /* Bounded waits inside the kernels (no counterpart in the reference, whose code runs on the CPU).
  * Every wait on an mbarrier is bounded. A staging wait of the DXT1 encoders or of the TMA
  * expansion variants that runs out falls back to reading global memory, and a level whose walk
- * (see crngpu_set_decode_split) waits too long for its tables is decoded by the wide decoder (the
+ * (see crngpu_set_decode_split) waits too long for its tables is decoded by another decoder (the
  * output does not change either way); a wait on a tcgen05 MMA of the MLP kernels that runs out makes the call return
  * CRNGPU_E_DEVICE. In-flight copies and MMAs are always drained, with a much longer bound, before
  * a CTA exits. crngpu_wait_counters reads how often each happened on the current device (and

@@ -293,3 +293,18 @@ def test_a_walk_that_gives_up_keeps_the_status_of_a_corrupt_stream(cg, waits_run
     walk = decode(cg, bytes(crn), cg.DECODE_WALK_ONLY)
     assert cg.wait_counters()["expand_stage_timeouts"] > 0
     assert walk[0] == lane[0] and (lane[0] or np.array_equal(walk[1], lane[1]))
+
+
+@pytest.mark.parametrize("name", ["c1_dxt1_1024", "dxt5_256", "dxn_xy_256", "dxt1_cube_64"])
+def test_calls_whose_walk_gives_up_decode_again_without_it(cg, waits_run_out, name):
+    levels = G.manifest()[name]["levels"]
+    with cg.unpack_begin(G.crn_bytes(name)) as ctx:
+        out = ctx.unpack_levels()
+        n = cg.decode_counters()
+        assert n["walk"] == len(levels) and n["lane"] + n["wide"] == len(levels)
+        pos = 0
+        for lvl, info in enumerate(levels):
+            assert G.sha(out[pos:pos + info["bytes"]]) == info["sha256"], lvl
+            assert G.sha(ctx.unpack_level(lvl).reshape(-1)) == info["sha256"], lvl
+            pos += info["bytes"]
+    assert cg.wait_counters()["expand_drain_failures"] == 0
