@@ -387,3 +387,40 @@ def test_codebooks_of_few_entries_find_each_cells_own(hc, cells):
     for i in range(cells):
         assert np.abs(rgb[:, 2 * i:2 * i + 2] - colours[i].astype(int)).max() <= 4, i
         assert np.abs(alpha[:, 2 * i:2 * i + 2] - (30 * i + 20)).max() <= 1, i
+
+
+# One cluster over a whole image: its endpoint pairs (first | second << 16) from the implementation that went
+# through every pixel in every pass, hashed nothing away and pruned nothing. Pixels: up to 80 a thread of
+# 128 are kept on chip (10,240), more are fetched again; colours: bounds from 128 on, a table of up to 2,048,
+# above it no probe search, and from 4,096 on a hash that is full.
+FIT_CASES = {
+    "kept_1": (16, 16, 1), "kept_2": (64, 64, 2), "kept_127": (64, 64, 127), "kept_128": (64, 64, 128),
+    "kept_all": (128, 80, 700), "fetched_few": (128, 88, 40), "fetched_700": (128, 88, 700),
+    "fetched_2047": (256, 256, 2047), "fetched_2048": (256, 256, 2048), "no_table_2049": (256, 256, 2049),
+    "hash_full": (256, 256, 20000)}
+
+
+def fit_image(name):
+    """`colours` distinct colours around a line through the colour cube, every one of them used."""
+    w, h, colours = FIT_CASES[name]
+    rng = np.random.default_rng(colours * 1000 + w + h)
+    spread = 24 if colours < 2000 else 60 if colours < 4000 else 255
+    t = rng.integers(0, 256, 64 * colours)
+    rgb = np.stack([t, (t * 3) // 4 + 20, 255 - t], 1) + rng.integers(-spread, spread + 1, (64 * colours, 3))
+    _, first = np.unique(np.clip(rgb, 0, 255) @ np.array([1, 256, 65536]), return_index=True)
+    rgb = np.clip(rgb, 0, 255)[np.sort(first)][:colours]
+    assert len(rgb) == colours
+    pick = np.concatenate([np.arange(colours), rng.integers(0, colours, w * h - colours)])
+    img = np.full((h, w, 4), 255, np.uint8)
+    img[..., :3] = rgb[rng.permutation(pick)].reshape(h, w, 3)
+    return img
+
+
+@pytest.mark.parametrize("perceptual", [True, False])
+@pytest.mark.parametrize("name", sorted(FIT_CASES))
+def test_cluster_fit_of_every_size_class(hc, name, perceptual):
+    with open(os.path.join(G.GOLDEN, "cluster_fit.json")) as fh:
+        want = json.load(fh)
+    _, stats, idx = hc.compress_dxt1([[fit_image(name)]], perceptual=perceptual, codebook=(1, 8), with_indices=True)
+    got = [int(v) & 0xFFFFFFFF for v in idx["endpoints"][:stats["color_endpoints"]]]
+    assert got == want[name]["perceptual" if perceptual else "uniform"]
