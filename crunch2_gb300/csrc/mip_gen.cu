@@ -130,6 +130,47 @@ struct Span {
 
 int floor4(int v) { return v & ~3; }
 
+// Values that depend on their keys alone, the most recently used up to `most` bytes of them.
+template <class Key, class T>
+class Kept {
+ public:
+  explicit Kept(size_t most) : most_(most) {}
+  std::shared_ptr<const T> find(const Key& key) {
+    std::lock_guard<std::mutex> lock(mu_);
+    const auto it = at_.find(key);
+    if (it == at_.end()) return nullptr;
+    items_.splice(items_.begin(), items_, it->second);
+    return it->second->value;
+  }
+  // the value kept under the key: `value`, or one that another thread has added meanwhile
+  std::shared_ptr<const T> add(const Key& key, std::shared_ptr<const T> value, size_t bytes) {
+    std::lock_guard<std::mutex> lock(mu_);
+    const auto it = at_.find(key);
+    if (it != at_.end()) return it->second->value;
+    if (bytes > most_) return value;
+    items_.push_front(Item{key, value, bytes});
+    at_[key] = items_.begin();
+    bytes_ += bytes;
+    while (bytes_ > most_) {
+      bytes_ -= items_.back().bytes;
+      at_.erase(items_.back().key);
+      items_.pop_back();
+    }
+    return value;
+  }
+
+ private:
+  struct Item {
+    Key key;
+    std::shared_ptr<const T> value;
+    size_t bytes;
+  };
+  std::mutex mu_;
+  std::list<Item> items_;  // most recently used first
+  std::map<Key, typename std::list<Item>::iterator> at_;
+  size_t most_, bytes_ = 0;
+};
+
 // Resampler::make_clist (crnlib/crn_resampler.cpp:119-412) with a zero source offset. The spans'
 // weights are appended to `pool`; a sample whose filter arguments equal its predecessor's (every
 // sample of a power-of-two scale) shares them, one copy per alignment of the window.
@@ -193,6 +234,23 @@ bool make_axis(int src, int dst, const Filter& F, float filter_scale, std::vecto
     s.w = (uint32_t)at;
   }
   return true;
+}
+
+struct Axis {
+  std::vector<Span> spans;  // weights in `pool`
+  std::vector<float> pool;
+};
+
+// Textures of many shapes share their sides' axes, which are most of the work of a plan (4096 x 4096:
+// 4.3 ms, 0.3 with the axes at hand), so axes are kept too.
+std::shared_ptr<const Axis> cached_axis(int src, int dst, uint32_t filter, float filter_scale) {
+  static Kept<std::tuple<int, int, uint32_t, float>, Axis> kept(64u << 20);
+  const auto key = std::make_tuple(src, dst, filter, filter_scale);
+  std::shared_ptr<const Axis> axis = kept.find(key);
+  if (axis) return axis;
+  auto made = std::make_shared<Axis>();
+  if (!make_axis(src, dst, kFilters[filter], filter_scale, made->pool, made->spans)) return nullptr;
+  return kept.add(key, made, made->spans.size() * sizeof(Span) + made->pool.size() * sizeof(float));
 }
 
 // One warp's work: one or two neighbouring destination samples (the second window empty, a1 = b1 =
@@ -602,7 +660,13 @@ bool make_plan(uint32_t width, uint32_t height, uint32_t levels, uint32_t filter
   std::map<std::pair<int, int>, std::vector<Span>> axes;
   auto axis = [&](int src, int dst) -> const std::vector<Span>* {
     std::vector<Span>& sp = axes[{src, dst}];
-    if (sp.empty() && !make_axis(src, dst, kFilters[filter], filter_scale, pool, sp)) return nullptr;
+    if (sp.empty()) {
+      const std::shared_ptr<const Axis> a = cached_axis(src, dst, filter, filter_scale);
+      if (!a || pool.size() + a->pool.size() > 0xFFFFFFF0u) return nullptr;
+      sp = a->spans;
+      for (Span& s : sp) s.w += (uint32_t)pool.size();
+      pool.insert(pool.end(), a->pool.begin(), a->pool.end());
+    }
     return &sp;
   };
   uint64_t tmp = 0;
@@ -707,33 +771,18 @@ bool make_plan(uint32_t width, uint32_t height, uint32_t levels, uint32_t filter
   return true;
 }
 
-// Plans depend on sizes and parameters alone. The last few are kept for the process (a program's
-// textures share a few sizes); a caller holds its own reference while it uses one.
+// Plans depend on sizes and parameters alone, and are kept for the process up to 64 MB (about a
+// hundred of 2000 x 1500 images, a thousand of 256 x 256); a caller holds its own reference while it uses
+// one.
 std::shared_ptr<const Plan> cached_plan(uint32_t width, uint32_t height, uint32_t levels, uint32_t filter,
                                         float filter_scale) {
-  using Key = std::tuple<uint32_t, uint32_t, uint32_t, uint32_t, float>;
-  static std::mutex mu;
-  static std::list<std::pair<Key, std::shared_ptr<const Plan>>> kept;  // most recently used first
-  constexpr size_t kPlans = 32, kBytes = 64u << 20;
-  const Key key(width, height, levels, filter, filter_scale);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    for (auto it = kept.begin(); it != kept.end(); ++it)
-      if (it->first == key) {
-        kept.splice(kept.begin(), kept, it);
-        return kept.front().second;
-      }
-  }
-  auto plan = std::make_shared<Plan>();
-  if (!make_plan(width, height, levels, filter, filter_scale, *plan)) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  kept.emplace_front(key, plan);
-  size_t bytes = 0, n = 0;
-  for (auto it = kept.begin(); it != kept.end();) {
-    bytes += it->second->blob.size();
-    if (++n > kPlans || (n > 1 && bytes > kBytes)) it = kept.erase(it); else ++it;
-  }
-  return plan;
+  static Kept<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t, float>, Plan> kept(64u << 20);
+  const auto key = std::make_tuple(width, height, levels, filter, filter_scale);
+  std::shared_ptr<const Plan> plan = kept.find(key);
+  if (plan) return plan;
+  auto made = std::make_shared<Plan>();
+  if (!make_plan(width, height, levels, filter, filter_scale, *made)) return nullptr;
+  return kept.add(key, made, made->blob.size());
 }
 
 struct GammaTables {
