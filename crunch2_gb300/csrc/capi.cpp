@@ -99,13 +99,14 @@ LaunchOrder::~LaunchOrder() {
 
 bool LaunchOrder::begin(cudaStream_t s) {
   if (capturing(s)) return true;
-  if (last) cudaStreamWaitEvent(s, last, 0);
+  if (pending) cudaStreamWaitEvent(s, last, 0);
   return false;
 }
 
 void LaunchOrder::end(cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
+  pending = false;
   if (last && device != dev) {  // an event is recorded on its own device only
     cudaEventDestroy(last);
     last = nullptr;
@@ -118,7 +119,8 @@ void LaunchOrder::end(cudaStream_t s) {
     }
     device = dev;
   }
-  if (cudaEventRecord(last, s) != cudaSuccess) cudaStreamSynchronize(s);
+  if (cudaEventRecord(last, s) == cudaSuccess) pending = true;
+  else cudaStreamSynchronize(s);
 }
 
 // One set per host thread, so callers on different threads never share them.
@@ -141,7 +143,15 @@ Staging::Staging(cudaStream_t s) : s_(s) {
 
 Staging::~Staging() {
   ThreadStaging& t = thread_staging();
-  if (!--t.users && !captured_) t.order.end(s_);
+  if (--t.users || captured_) return;
+  if (idle_) t.order.pending = false;  // what this call waited for is over too
+  else t.order.end(s_);
+}
+
+int Staging::synchronize() {
+  const cudaError_t e = cudaStreamSynchronize(s_);
+  idle_ = e == cudaSuccess;
+  return cuda_check(e, "sync");
 }
 
 DevBuf& Staging::operator[](int slot) const { return thread_staging().bufs[slot & 7]; }

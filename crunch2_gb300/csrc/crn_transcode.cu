@@ -23,6 +23,7 @@
 #include <atomic>
 #include <cstring>
 #include <memory>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -2740,8 +2741,8 @@ int status_to_rc(uint32_t st) {
   return CRNGPU_E_CORRUPT;
 }
 
-// The walk decoder's scratch of one call: stream-ordered memory from a per-device pool, given back
-// in stream order. The pool keeps at most kWalkPoolBytes between calls, which go back to the device when
+// The walk decoder's scratch of one call, or of a batch: stream-ordered memory from a per-device pool, given
+// back in stream order (cudaMalloc and cudaFree for each batch of nine small files took 250 us). The pool keeps at most kWalkPoolBytes between calls, which go back to the device when
 // another buffer of the library finds no memory (trim_decode_pool) or by crngpu_set_decode_scratch.
 constexpr uint64_t kWalkPoolBytes = 128ull << 20;
 std::atomic<cudaMemPool_t> g_walk_pools[64];
@@ -2771,8 +2772,10 @@ struct WalkScratch {
   void* ptr = nullptr;
   explicit WalkScratch(cudaStream_t stream) : s(stream) {}
   WalkScratch(const WalkScratch&) = delete;
-  ~WalkScratch() {
+  ~WalkScratch() { release(); }
+  void release() {
     if (ptr) cudaFreeAsync(ptr, s);
+    ptr = nullptr;
   }
   uint8_t* get(uint64_t bytes) {  // null: there is none
     int dev = 0;
@@ -2929,10 +2932,11 @@ int unpack_one(UnpackContext* c, const uint8_t* host_src, const uint8_t* dev_src
   }
   LevelTask t = context_task(c, level);
   t.pitch = row_pitch;
-  const Staging staging(s);
+  std::optional<Staging> staging;
+  if (host_src || mem != CRNGPU_MEM_DEVICE) staging.emplace(s);
   if (dev_src) { t.src = dev_src; t.src_size = src_size; }
   else if (host_src) {
-    DevBuf& sb = staging[2];
+    DevBuf& sb = (*staging)[2];
     if ((e = sb.ensure(src_size + 64)) != cudaSuccess) return cuda_check(e, "alloc segment");
     if ((e = cudaMemcpyAsync(sb.ptr, host_src, src_size, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cuda_check(e, "copy segment");
@@ -2943,7 +2947,7 @@ int unpack_one(UnpackContext* c, const uint8_t* host_src, const uint8_t* dev_src
   if (mem == CRNGPU_MEM_DEVICE) {
     for (uint32_t f = 0; f < F.faces; f++) t.dst[f] = static_cast<uint8_t*>(dst_faces[f]);
   } else {
-    out_stage = &staging[1];
+    out_stage = &(*staging)[1];
     if ((e = out_stage->ensure(face_bytes * F.faces)) != cudaSuccess) return cuda_check(e, "alloc output stage");
     for (uint32_t f = 0; f < F.faces; f++) t.dst[f] = static_cast<uint8_t*>(out_stage->ptr) + face_bytes * f;
     // rows may have pitch padding the transcoder does not write: keep the caller's bytes there
@@ -2959,9 +2963,8 @@ int unpack_one(UnpackContext* c, const uint8_t* host_src, const uint8_t* dev_src
     for (uint32_t f = 0; f < F.faces; f++)
       if ((e = cudaMemcpyAsync(dst_faces[f], tasks[0].dst[f], face_bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_check(e, "copy output");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
   }
-  return CRNGPU_OK;
+  return staging ? staging->synchronize() : CRNGPU_OK;
 }
 
 // Output bytes of levels [first, first + count) at minimal pitch.
@@ -3018,7 +3021,8 @@ struct UnpackBatch : HostObject {
   uint32_t magic = 0x42415443u;
   int device = -1;
   Plan plan;
-  DevBuf d_jobs, d_records, d_words, d_walk;
+  DevBuf d_jobs, d_records, d_words;
+  WalkScratch walk{nullptr};  // of the legacy default stream, with which creation and end are ordered
   uint32_t words_host[2] = {0, 0};
   cudaGraphExec_t graph = nullptr;
   bool decoded = false;
@@ -3028,6 +3032,14 @@ struct UnpackBatch : HostObject {
   LaunchOrder order;  // records, work counter, status and walk state are the batch's own: one launch at a time
   ~UnpackBatch() {
     if (graph) cudaGraphExecDestroy(graph);
+    if (!walk.ptr) return;
+    // launches on any stream are over before the walk's scratch goes to its next user
+    int cur = -1;
+    cudaGetDevice(&cur);
+    if (device != cur) cudaSetDevice(device);
+    cudaDeviceSynchronize();
+    walk.release();
+    if (device != cur && cur >= 0) cudaSetDevice(cur);
   }
 };
 
@@ -3102,9 +3114,9 @@ extern "C" int64_t crngpu_unpack_levels(crngpu_unpack_context ctx, uint32_t firs
   cudaError_t e;
   uint8_t* out = static_cast<uint8_t*>(dst);
   DevBuf* stage = nullptr;
-  const Staging staging(s);
+  std::optional<Staging> staging;
   if (mem != CRNGPU_MEM_DEVICE) {
-    stage = &staging[1];
+    stage = &staging.emplace(s)[1];
     if ((e = stage->ensure(total)) != cudaSuccess) return cuda_check(e, "alloc output stage");
     out = static_cast<uint8_t*>(stage->ptr);
   }
@@ -3115,7 +3127,7 @@ extern "C" int64_t crngpu_unpack_levels(crngpu_unpack_context ctx, uint32_t firs
   if (stage) {
     if ((e = cudaMemcpyAsync(dst, stage->ptr, total, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return cuda_check(e, "copy output");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
+    if ((rc = staging->synchronize()) != CRNGPU_OK) return rc;
   }
   return (int64_t)total;
 } catch (...) {
@@ -3159,10 +3171,7 @@ extern "C" crngpu_unpack_batch crngpu_unpack_batch_create(const crngpu_unpack_ba
   if ((e = b->d_words.ensure(16)) != cudaSuccess) { cuda_check(e, "alloc status"); return nullptr; }
   if (!make_placed_plan(tasks, b->plan, slots, [&](uint64_t bytes) -> uint8_t* {
         // the job tables before the scratch, which can be done without
-        if (bytes > g_walk_scratch_most.load() || b->d_jobs.ensure(b->plan.image.size() + 16) != cudaSuccess ||
-            b->d_walk.ensure(bytes) != cudaSuccess)
-          return nullptr;
-        return static_cast<uint8_t*>(b->d_walk.ptr);
+        return b->d_jobs.ensure(b->plan.image.size() + 16) == cudaSuccess ? b->walk.get(bytes) : nullptr;
       })) {
     set_error("too many levels in one batch item");
     return nullptr;

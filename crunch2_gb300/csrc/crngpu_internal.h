@@ -86,6 +86,7 @@ struct LaunchOrder {
   std::mutex mu;  // held while a launch is enqueued
   cudaEvent_t last = nullptr;  // after the latest launch
   int device = -1;             // of `last`
+  bool pending = false;        // `last` may still be ahead
   ~LaunchOrder();
   bool begin(cudaStream_t s);  // true if the launch is captured
   void end(cudaStream_t s);    // for launches that are not
@@ -116,10 +117,11 @@ class Staging {
   ~Staging();
   Staging(const Staging&) = delete;
   DevBuf& operator[](int slot) const;
+  int synchronize();  // the stream: the buffers are free again (a call with host buffers ends with this)
 
  private:
   cudaStream_t s_;
-  bool captured_ = false;
+  bool captured_ = false, idle_ = false;
 };
 
 // Batched block encoding (many textures, mixed formats). A segment is one element of one texture

@@ -137,7 +137,7 @@ int with_buffers(const uint8_t* in, size_t in_bytes, uint8_t* out, size_t out_by
     return fn(in, out, err);
   }
   cudaError_t e;
-  const Staging staging(s);
+  Staging staging(s);
   DevBuf& bi = staging[0];
   DevBuf& bo = staging[1];
   DevBuf& be = staging[3];
@@ -153,7 +153,7 @@ int with_buffers(const uint8_t* in, size_t in_bytes, uint8_t* out, size_t out_by
     return cuda_check(e, "copy output");
   if (err && (e = cudaMemcpyAsync(err, be.ptr, err_bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return cuda_check(e, "copy errors");
-  return cuda_check(cudaStreamSynchronize(s), "sync");
+  return staging.synchronize();
 }
 
 }  // namespace
@@ -196,7 +196,7 @@ int64_t dds_plain_chain(const uint8_t* rgba_levels, uint32_t width, uint32_t hei
   if (!out || out_capacity < need) return (int64_t)need;
   cudaStream_t s = nullptr;
   cudaError_t e;
-  const Staging staging(s);
+  Staging staging(s);
   DevBuf& chain = staging[4];
   DevBuf& table = staging[5];
   DevBuf& gathered = staging[6];
@@ -214,9 +214,9 @@ int64_t dds_plain_chain(const uint8_t* rgba_levels, uint32_t width, uint32_t hei
   rc = encode_device(static_cast<const uint8_t*>(gathered.ptr), blocks, format, flags, quality, threshold,
                          static_cast<uint8_t*>(encoded.ptr), nullptr, s);
   if (rc != CRNGPU_OK) return rc;
-  if ((e = cudaMemcpyAsync(out, encoded.ptr, need, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess)
+  if ((e = cudaMemcpyAsync(out, encoded.ptr, need, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return cuda_check(e, "copy result");
+  if ((rc = staging.synchronize()) != CRNGPU_OK) return rc;
   return (int64_t)need;
 }
 
@@ -330,7 +330,7 @@ extern "C" int64_t crngpu_compress_image_ex(const uint8_t* rgba, uint32_t width,
   cudaStream_t s = as_stream(stream);
   cudaError_t e;
   const size_t img_bytes = (size_t)pitch_bytes * (height - 1) + (size_t)width * 4;
-  const Staging staging(s);
+  Staging staging(s);
   DevBuf& blocks = staging[2];
   if ((e = blocks.ensure(n * 64)) != cudaSuccess) return cuda_check(e, "alloc blocks");
   const uint8_t* d_img = rgba;
@@ -362,7 +362,7 @@ extern "C" int64_t crngpu_compress_image_ex(const uint8_t* rgba, uint32_t width,
   if (so) {
     if ((e = cudaMemcpyAsync(out, so->ptr, need, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return cuda_check(e, "copy output");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
+    if ((rc = staging.synchronize()) != CRNGPU_OK) return rc;
   }
   return (int64_t)need;
 } catch (...) {

@@ -857,7 +857,7 @@ extern "C" int64_t crngpu_generate_mipmaps(const uint8_t* rgba, uint32_t width, 
   const uint64_t texels0 = (uint64_t)width * height;
   cudaError_t e;
   int rc;
-  const Staging staging(s);
+  Staging staging(s);
   DevBuf& tables = staging[4];
   DevBuf& work = staging[5];
   const size_t blob = plan ? plan->blob.size() : 0, o_lin = blob, o_srgb = o_lin + sizeof(gt.to_linear);
@@ -913,7 +913,7 @@ extern "C" int64_t crngpu_generate_mipmaps(const uint8_t* rgba, uint32_t width, 
   if (so) {
     if ((e = cudaMemcpyAsync(out, so->ptr, need, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return cuda_check(e, "copy mips");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_check(e, "sync");
+    if ((rc = staging.synchronize()) != CRNGPU_OK) return rc;
   }
   return (int64_t)need;
 } catch (...) {
