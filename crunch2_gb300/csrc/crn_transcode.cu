@@ -1083,9 +1083,9 @@ __device__ __forceinline__ void wide_level(const StreamJob& J, WideShared& S, ui
 // decode and the endpoint indices leave the walking CTA:
 //
 //  * Tables, per bit position p: C4[p] = four times the bits of four chunks starting at p (low half; the
-//    distance to the next entry in bytes) and, for the row below, which of their eight blocks carry endpoint deltas; O4[p][k] = bits - 1 of four
-//    blocks, for each of the 16 combinations k of which carry deltas (a block is at most 64 bits,
-//    so four fit a byte less one). Where a row's blocks are not a multiple of eight, O2 and C1 (two
+//    distance to the next entry in bytes) and, for the row below, which of their eight blocks carry
+//    endpoint deltas; O4[p][k] = bits - 1 of four blocks, for each of the 16 combinations k of which
+//    carry deltas (a block is at most 64 bits, so four fit a byte less one). Where a row's blocks are not a multiple of eight, O2 and C1 (two
 //    blocks, one chunk) for the row's end. A lookup never depends on where the walk is, so every
 //    position's entry is computed by all SMs at once.
 //  * Segments. A level's stream is cut into segments; launch s builds the tables of segment s,
@@ -1286,9 +1286,9 @@ __device__ __forceinline__ void walk_build(const WalkJob& job, WalkShared& S, ui
 
 // ---- the walk over segment k: thread 0 of the CTA, with thread 32 bringing the windows of the
 // tables by bulk copies up to three windows ahead. A wait that runs out ends the level's walk: the
-// launches after it leave the level alone, and another decoder decodes it. A step's chain is a shared-memory load and the addition that gives the
-// next load's address; the loop's own instructions (test, stores) cost as much as the chain unless
-// groups go in fours. Measured on the 1024 x 1024 DXT1 level, cycles per step: 124 with cp.async by
+// launches after it leave the level alone, and another decoder decodes it. A step's chain is a
+// shared-memory load and the addition that gives the next load's address; the loop's own instructions
+// (test, stores) cost as much as the chain unless groups go in fours. Measured on the 1024 x 1024 DXT1 level, cycles per step: 124 with cp.async by
 // the other warps, a barrier per window and a test per group; 103 with bulk copies issued by the
 // walking thread and groups in fours; 72 so.
 template <uint32_t kPolls = kExpandWaitLimit>
@@ -2742,7 +2742,8 @@ int status_to_rc(uint32_t st) {
 }
 
 // The walk decoder's scratch of one call, or of a batch: stream-ordered memory from a per-device pool, given
-// back in stream order (cudaMalloc and cudaFree for each batch of nine small files took 250 us). The pool keeps at most kWalkPoolBytes between calls, which go back to the device when
+// back in stream order (creating and closing a batch of nine small files 230 us, 283 with cudaMalloc, 183
+// without a walk). The pool keeps at most kWalkPoolBytes between calls, which go back to the device when
 // another buffer of the library finds no memory (trim_decode_pool) or by crngpu_set_decode_scratch.
 constexpr uint64_t kWalkPoolBytes = 128ull << 20;
 std::atomic<cudaMemPool_t> g_walk_pools[64];
@@ -3015,8 +3016,9 @@ int expand_wait_counters(uint32_t out[2], bool reset) {
 }
 
 
-// A prepared batch: many levels of many contexts, decoded together and expanded by one launch. The job tables and record buffer are uploaded/allocated once at creation, so a
-// launch only enqueues memsets, the decoders' launches and the expansion (and can replay as a CUDA graph).
+// A prepared batch: many levels of many contexts, decoded together and expanded by one launch. The job
+// tables and record buffer are uploaded/allocated once at creation, so a launch only enqueues memsets, the
+// decoders' launches and the expansion (and can replay as a CUDA graph).
 struct UnpackBatch : HostObject {
   uint32_t magic = 0x42415443u;
   int device = -1;

@@ -1,8 +1,8 @@
 // DXT1 / DXT5A block encoders for sm_103a, bit-exact with crnlib's optimizers at every quality.
 //
 // DXT1 (dxt1_endpoint_optimizer, crnlib/crn_dxt1.cpp) runs in two phases, a kernel each:
-//   phase 1, lane per block (four lanes for few blocks): unique colours, perceptual weighting (powf), the double-precision
-//     PCA and projection bounds (handle_multicolor_block :1069-1178) and the LBG seeds of
+//   phase 1, lane per block (four lanes for few blocks): unique colours, perceptual weighting (powf), the
+//     double-precision PCA and projection bounds (handle_multicolor_block :1069-1178) and the LBG seeds of
 //     try_median4 (:1181-1308). These are scalar, FP64-heavy and tiny, so lanes work on
 //     different blocks and GB300's narrow FP64 pipe is amortised over the warp.
 //   phase 2, warp per block, lane per candidate: every candidate list of optimize_endpoints
@@ -861,8 +861,8 @@ __device__ __forceinline__ bool gen_candidate(const WarpShared& S, const ListDes
   }
 }
 
-// Runs the list described by S.d with the reference's sequential semantics; see the file comment. Returns, for stop_on_accept lists, the position of the
-// first accepted candidate (or -1); otherwise 1 if anything was accepted, else 0.
+// Runs the list described by S.d with the reference's sequential semantics; see the file comment.
+// Returns, for stop_on_accept lists, the position of the first accepted candidate (or -1); otherwise 1 if anything was accepted, else 0.
 template <bool G>
 __device__ __noinline__ int run_list(WarpShared& S, uint32_t& work) {
   const ListDesc& d = S.d;
@@ -1770,8 +1770,8 @@ __device__ __forceinline__ void fill_unit(float* unit) {
 }
 
 // Phase 1 over n blocks: warp w takes the groups of 32 consecutive blocks g = w, w + W, ..., a lane
-// per block (of 8, four lanes per block, below `share_below` blocks), each group staged by one bulk copy. Warps are ranked CTA-first (warp 0 of every CTA,
-// then warp 1, ...), and the grid has a CTA per group up to the resident limit, so a short batch
+// per block (of 8, four lanes per block, below `share_below` blocks), each group staged by one bulk copy.
+// Warps are ranked CTA-first (warp 0 of every CTA, then warp 1, ...), and the grid has a CTA per group up to the resident limit, so a short batch
 // (the learned encoder's fallback blocks, a small mip level) puts one working warp on each SM:
 // the seeds are bound by the SM's FP64 pipe, which the warps of one CTA would share.
 template <bool G>

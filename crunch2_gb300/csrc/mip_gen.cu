@@ -292,11 +292,15 @@ constexpr int kMaxPairJob = 128;
 // two samples' sums, added in the reference's order. Positions are staged chunk by chunk; an item
 // whose window goes on in the next chunk leaves its sums in shared memory.
 //
-// Bound by the FP32 pipe: a row pass multiplies and adds, separately rounded, (support x 2 x filter
-// scale) values per source texel and channel at every level, and no product is shared between
-// levels. Two samples per lane because a texel's 16-byte reads take 4 shared-memory cycles per warp
+// A row pass multiplies and adds, separately rounded, (support x 2 x filter scale) values per source
+// texel and channel at every level, and no product is shared between levels: 0.22 ms of FP32 for 4096 x
+// 4096. Two samples per lane because a texel's 16-byte reads take 4 shared-memory cycles per warp
 // against 8 multiplies and adds per sample, and an SM issues four of those a cycle: with one sample
-// per read the reads would be the bound.
+// per read the reads would be the bound. As it is no pipe is at its limit: the row pass (1.15 ms) issues
+// on 47 % of its cycles, the FMA pipe is busy for 25 % and the shared-memory data path for 55 %, 8 % of its
+// loads' cycles for bank conflicts; warps wait for the chunks' barriers (5.4 of 16 cycles between two
+// issues) and for weights and texels (4.2). Every job stages and converts its
+// texels anew, each texel about ten times.
 
 __device__ __forceinline__ int source_index(int j, int n, int wrap) {
   if (j >= 0 && j < n) return j;

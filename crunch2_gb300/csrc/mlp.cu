@@ -973,7 +973,7 @@ __global__ void k_scatter_idx(const uint8_t* __restrict__ enc, const uint32_t* _
 // Host side
 
 struct Param {
-  int rows, cols, rows_live;
+  int rows, cols;
   DevBuf w, g, m, v, wb;  // fp32 master, grad, Adam moments, bf16 copy (weights only)
   DevBuf wbT;             // bf16 transposed copy (W2, W3: the backward products)
   size_t n() const { return (size_t)rows * cols; }
@@ -984,7 +984,7 @@ struct Net {
   int device = -1;
   Param W1, b1, W2, b2, W3, b3;
   int step = 0;
-  float bound_tau = 0.f, bound_weight = 1.f;  // loss of the error-bound output (see k_loss_grad)
+  float bound_tau = 0.f, bound_weight = 1.f;  // loss of the error-bound output (see k_train_tile)
   // training scratch sized for the largest batch seen (tiles of 128 samples, see TrainArgs)
   int cap = 0;
   DevBuf h1T, h2T, d1T, d2T, xT, dyT, g1, g2, bias, part;
@@ -994,8 +994,8 @@ struct Net {
   std::vector<Param*> params() { return {&W1, &b1, &W2, &b2, &W3, &b3}; }
 };
 
-int alloc_param(Param& p, int rows, int cols, int rows_live, bool bf16, bool transposed) {
-  p.rows = rows; p.cols = cols; p.rows_live = rows_live;
+int alloc_param(Param& p, int rows, int cols, bool bf16, bool transposed) {
+  p.rows = rows; p.cols = cols;
   cudaError_t e;
   if ((e = p.w.ensure(p.n() * 4)) != cudaSuccess) return cuda_check(e, "alloc weights");
   if ((e = p.g.ensure(p.n() * 4)) != cudaSuccess) return cuda_check(e, "alloc grads");
@@ -1185,7 +1185,7 @@ extern "C" void* crngpu_mlp_create(uint64_t seed) try {
   cudaGetDevice(&net->device);
   std::mt19937_64 rng(seed);
   auto init = [&](Param& p, int rows, int cols, int rows_live, bool is_bias, int fan_in) {
-    if (alloc_param(p, rows, cols, rows_live, !is_bias, &p == &net->W2 || &p == &net->W3) != CRNGPU_OK) return false;
+    if (alloc_param(p, rows, cols, !is_bias, &p == &net->W2 || &p == &net->W3) != CRNGPU_OK) return false;
     std::vector<float> h(p.n(), 0.f);
     if (!is_bias) {
       const float bound = std::sqrt(6.0f / (float)fan_in) * 0.5f;

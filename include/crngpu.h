@@ -429,8 +429,8 @@ CRNGPU_API int64_t crngpu_unpack_levels(crngpu_unpack_context ctx, uint32_t firs
 
 /* Batched transcode (no single counterpart in the reference, which transcodes one level per
  * crnd_unpack_level call, inc/crn_decomp.h:3537-3619): many levels of many open contexts, of any
- * mix of sizes and formats, decoded by ONE persistent launch (one lane per level stream, streams
- * taken largest-first from a work counter) and expanded by one more. Each item writes levels
+ * mix of sizes and formats, decoded together (each level by one of three decoders, see
+ * crngpu_set_decode_split) and expanded by one launch. Each item writes levels
  * [first_level, first_level + level_count) of its context back to back into `dst` (device
  * memory), exactly as crngpu_unpack_levels does. Creation validates every item, uploads the job
  * tables and allocates the index-record buffer once; the contexts must stay open while the batch
