@@ -1113,6 +1113,7 @@ struct WalkState {
   uint32_t p, groups;                      // the walk: position, groups passed
   uint32_t rows, carry, bad;               // the resolver: rows resolved, running indices; 1: bad code, 2: bad index
   uint32_t gave_up;                        // the launch in which a wait of the walk ran out, or 0
+  uint32_t polls;                          // g_expand_wait_polls, as launch 0 found it
   uint32_t passed[kWalkMaxSegments + 1];   // groups passed after each segment
   uint32_t bits[kWMaxW / 32];              // the current even row's combinations, a byte per four chunks
 };
@@ -1204,6 +1205,7 @@ __device__ __forceinline__ uint32_t walk_stage_models(const StreamJob& J, uint32
 __device__ __forceinline__ void walk_build(const WalkJob& job, WalkShared& S, uint32_t k, uint32_t tile) {
   const StreamJob& J = job.j;
   const uint32_t P0 = k * job.seg + tile * kWalkTile, tid = threadIdx.x;
+  if (P0 == 0 && tid == 0) job.st->polls = g_expand_wait_polls;
   if (P0 > job.bits + kWalkHalo) return;
   const bool two = J.kind == kKDxt5 || J.kind == kKDxn, five = J.kind == kKDxt5;
   uint32_t* luts = reinterpret_cast<uint32_t*>(wide_smem);
@@ -1320,12 +1322,15 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
   WalkState& st = *job.st;
   const uint32_t tid = threadIdx.x, base = k * job.seg;
   // (the state in one round trip)
-  const uint32_t gave_up = st.gave_up, p0 = st.p, g0 = st.groups, bits0 = tid < kWMaxW / 32 ? st.bits[tid] : 0u;
+  const uint32_t gave_up = st.gave_up, polls = st.polls, p0 = st.p, g0 = st.groups;
+  const uint32_t bits0 = tid < kWMaxW / 32 ? st.bits[tid] : 0u;
   if (walk_gave_up(gave_up, k + 1)) return;
   if (tid < kWMaxW / 32) S.bits[tid] = bits0;
   const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(wide_smem);
   const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
-  const uint32_t windows = (job.seg + R::kWindow - 1) / R::kWindow, staged = job.cap / R::kWindow;
+  // (the test hook's bound of no polls: after the first wait, as if that had run out. A bound that the waits
+  // themselves look at cost 60 cycles a window)
+  const uint32_t windows = polls ? (job.seg + R::kWindow - 1) / R::kWindow : 0u, staged = job.cap / R::kWindow;
   if (tid == 0) {
     for (uint32_t i = 0; i < R::kSlots; i++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * i));
@@ -1378,8 +1383,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
     const uint2* RM = reinterpret_cast<const uint2*>(wide_smem + R::kRem);
     const uint32_t left = job.bits > base ? job.bits - base : 0u;  // positions before the end of the stream
     uint32_t* out = job.anchors + groups;
-    // (the hook's bound is for this first wait: read in the loop it cost 60 cycles a window)
-    bool ok = g_expand_wait_polls && walk_wait(full, 0u);
+    bool ok = walk_wait(full, 0u);
     for (uint32_t w = 0; w < windows && ok && r < sh.rows; w++) {
       if (w + 1 < staged) ok = walk_wait(full + 8 * ((w + 1) & (R::kSlots - 1)), ((w + 1) / R::kSlots) & 1u);
       if (!ok) break;
@@ -1468,6 +1472,7 @@ __device__ __forceinline__ void walk_segment(const WalkJob& job, WalkShared& S, 
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * (w & (R::kSlots - 1))) : "memory");
     }
     *(volatile uint32_t*)&S.walking = 0u;
+    if (!windows) ok = false;
     if (!ok) {
       atomicAdd(&g_expand_stage_timeouts, 1u);
       atomicAdd(given_up, 1u);
@@ -1596,10 +1601,10 @@ __device__ __forceinline__ void walk_resolve(const WalkJob& job, WalkShared& S, 
   const StreamJob& J = job.j;
   const WalkShape sh = walk_shape(J.bx, J.by, J.faces);
   WalkState& st = *job.st;
-  const uint32_t gave_up = st.gave_up, passed = st.passed[k], pairs = passed / (sh.ge + sh.go);
-  const uint32_t ready = 2 * pairs + (passed - pairs * (sh.ge + sh.go) >= sh.ge ? 1u : 0u);
+  const bool over = walk_gave_up(st.gave_up, k + 3);  // then no rows (a return here would hold up the loads below)
+  const uint32_t passed = st.passed[k], pairs = passed / (sh.ge + sh.go);
   uint32_t r = st.rows;
-  if (walk_gave_up(gave_up, k + 3)) return;
+  const uint32_t ready = over ? r : 2 * pairs + (passed - pairs * (sh.ge + sh.go) >= sh.ge ? 1u : 0u);
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, W = sh.W;
   const uint32_t nA = J.n_a, nB = J.n_b, nSA = J.n_sa, nSB = J.n_sb;
   const uint32_t x0 = tid * kPer;  // rows are even: a pair of blocks is inside or outside
@@ -1758,7 +1763,7 @@ __device__ __forceinline__ void walk_resolve(const WalkJob& job, WalkShared& S, 
   if (tid == 0) {
     st.rows = ready;
     st.carry = S.carry[ready & 1u];
-    const uint32_t bad = k + 1 == job.segs ? atomicOr(&st.bad, 0u) : 0u;
+    const uint32_t bad = k + 1 == job.segs && !over ? atomicOr(&st.bad, 0u) : 0u;
     if (bad) atomicMax(status, (bad & 1u) ? (uint32_t)kStBadCode : (uint32_t)kStBadIndex);
   }
 }
